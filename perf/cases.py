@@ -325,3 +325,119 @@ TOLERANCE = {
 
 def tolerance(case):
     return TOLERANCE[case["kind"]]
+
+
+# ------------------------------------------------------------------------------ the same passes in 64 bits
+def _swiglu64(x, w1, w2, w3):
+    gate = x @ w1.t()
+    return (gate * torch.sigmoid(gate) * (x @ w3.t())) @ w2.t()
+
+
+def _attention64(state, causal, rotate):
+    """Output and gradients of attention, one (sequence, KV head) at a time."""
+    q, k, v, dy = (state[n].detach().double() for n in ("q", "k", "v", "dy"))
+    B, S, H, Hkv = *q.shape[:3], k.shape[2]
+
+    def turn(x, sign):
+        """Rotates adjacent pairs of ``[S, ..., 128]`` by their position's angle."""
+        if not rotate:
+            return x
+        cos, sin = (state[n][:S].double().view(S, *[1] * (x.dim() - 2), -1) for n in ("cos", "sin"))
+        a, b = x[..., 0::2], x[..., 1::2]
+        return torch.stack((a * cos - sign * b * sin, sign * a * sin + b * cos), -1).flatten(-2)
+
+    out, dq, dk, dv = torch.empty_like(q), torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+    hidden = torch.ones(S, S, dtype=torch.bool, device=q.device).triu(1) if causal else None
+    for b in range(B):
+        for j in range(Hkv):
+            keys, values = turn(k[b, :, j], 1), v[b, :, j]
+            dkeys, dvalues = torch.zeros_like(keys), torch.zeros_like(values)
+            for h in range(j * (H // Hkv), (j + 1) * (H // Hkv)):
+                queries, g = turn(q[b, :, h], 1), dy[b, :, h]
+                p = queries @ keys.t() * HEAD_DIM ** -0.5
+                if hidden is not None:
+                    p.masked_fill_(hidden, -math.inf)
+                p = p.softmax(-1)
+                out[b, :, h] = p @ values
+                dvalues += p.t() @ g
+                ds = (g @ values.t() - (g * out[b, :, h]).sum(-1, keepdim=True)) * p * HEAD_DIM ** -0.5
+                dq[b, :, h] = turn(ds @ keys, -1)
+                dkeys += ds.t() @ queries
+            dk[b, :, j], dv[b, :, j] = turn(dkeys, -1), dvalues
+    return [out, dq, dk, dv]
+
+
+def _moe64(x, router, w1, w2, w3):
+    """Top-2 routed experts with renormalised weights; differentiable."""
+    top, idx = (x @ router.t()).softmax(-1).topk(2, dim=-1)
+    weights = top / top.sum(-1, keepdim=True)
+    out = torch.zeros_like(x)
+    for e in range(w1.shape[0]):
+        token, j = (idx == e).nonzero(as_tuple=True)
+        out = out.index_add(0, token, _swiglu64(x[token], w1[e], w2[e], w3[e]) * weights[token, j, None])
+    return out
+
+
+def _norm64(x, weight):
+    return x * torch.rsqrt(x.square().mean(-1, keepdim=True) + 1e-5) * weight.double()
+
+
+def _logits64(case, wrapped, ids):
+    model, S, H = wrapped.module, case["seq"], case["heads"]
+
+    def bf16(weight):      # the wrapped model computes with bf16 copies of its fp32 weights
+        return weight.detach().to(BF16).double()
+
+    angles = torch.arange(S, device="cuda").double()[:, None] * 10000.0 ** (
+        -torch.arange(0, HEAD_DIM, 2, device="cuda").double() / HEAD_DIM)[None]
+    x = bf16(model.token_embeddings.weight)[ids]
+    B = x.shape[0]
+    for layer in model.layers:
+        n, a = _norm64(x, layer.ln1.weight), layer.attn
+        heads = {name: (n @ bf16(getattr(a, name + "_proj").weight).t()).view(B, S, -1, HEAD_DIM) for name in "qkv"}
+        state = {**heads, "dy": torch.zeros_like(heads["q"]), "cos": angles.cos(), "sin": angles.sin()}
+        x = x + _attention64(state, True, True)[0].view(B, S, H * HEAD_DIM) @ bf16(a.output_proj.weight).t()
+        n, f = _norm64(x, layer.ln2.weight).view(B * S, -1), layer.ffn
+        experts = [p.detach().double() for p in (f.experts.w1, f.experts.w2, f.experts.w3)]
+        x = x + _moe64(n, bf16(f.router.weight), *experts).view(x.shape)
+    return _norm64(x, model.ln_final.weight) @ bf16(model.lm_head.weight).t()
+
+
+def exact(case, seed):
+    kind = case["kind"]
+    if kind == "step":
+        return None      # thousands of roundings in a row, then updates that follow the gradients' signs
+    state = prepare(case, seed)
+    if kind == "logits":
+        with torch.no_grad():
+            return _logits64(case, state["model"], state["x"])
+    if kind == "moe":
+        module = state["model"].module
+        leaves = [state["x"], module.router.weight.to(BF16), module.experts.w1, module.experts.w2, module.experts.w3]
+        leaves = [t.detach().double().requires_grad_(True) for t in leaves]
+        out = _moe64(*leaves)
+        dx, drouter, dw1, dw2, dw3 = torch.autograd.grad(out, leaves, state["dy"].double())
+        return [out.detach(), dx, drouter, dw1, dw2, dw3]
+    if kind == "ffn":
+        params = list(state["model"].parameters())
+        leaves = [t.detach().double().requires_grad_(True) for t in (state["x"], *params)]
+        out = leaves[0]
+        for w1, w2, w3 in zip(leaves[1::3], leaves[2::3], leaves[3::3]):
+            out = _swiglu64(out, w1, w2, w3)
+        return [out.detach(), *torch.autograd.grad(out, leaves, state["dy"].double())]
+    if kind in ("rope_attn", "attn"):
+        return _attention64(state, kind == "rope_attn" or case["causal"], kind == "rope_attn")
+    if kind == "flash":
+        q, k, v = (state[n].double() for n in "qkv")
+        return torch.stack([(q[b] @ k[b].mT * HEAD_DIM ** -0.5).softmax(-1) @ v[b] for b in range(q.shape[0])])
+    if kind == "head":
+        hidden, weight = (state[n].detach().double().requires_grad_(True) for n in ("hidden", "weight"))
+        loss = torch.nn.functional.cross_entropy(hidden @ weight.t(), state["targets"])
+        return [loss.detach(), *torch.autograd.grad(loss, (hidden, weight))]
+    results = []
+    for p in state["params"]:      # first update of lr 1e-3, betas 0.9 and 0.999, eps 1e-8, decay 0.01
+        g = p.grad.double()
+        m, v = 0.1 * g, 0.001 * g * g
+        step = 1e-3 * math.sqrt(1 - 0.999) / (1 - 0.9)
+        results.append([p.detach().double() * (1 - 1e-3 * 0.01) - step * m / (v.sqrt() + 1e-8), m, v])
+    return results
