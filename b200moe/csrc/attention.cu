@@ -8,17 +8,14 @@
 // it into bf16 P in place, and P feeds the next MMA straight from TMEM (A operand in
 // tensor memory), so P never touches shared memory.
 //
-// Forward, one CTA per (128 queries, head, batch), 320 threads:
-//   warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 softmax / correction / epilogue
-//   (two threads per query row, 64 key columns each).  Two S buffers let QK^T of tile j+1 run under the
-//   softmax of tile j; O is rescaled only when a row maximum grew by more than 2^8.
-// Backward kernels run 320 threads: two softmax groups split the 128 columns of a tile.
+// Forward, one CTA per (256 queries, head, batch): see attn_fwd_kernel.
 // Backward dK/dV, one CTA per (128 keys, kv head, batch): loops over the 4 query heads
 //   of the group and their causal query tiles with S^T = K Q^T, dP^T = V dO^T, so P^T
 //   and dS^T are A operands in TMEM; dV and dK accumulate in TMEM over the whole loop
 //   (the GQA reduction needs no atomics).
 // Backward dQ, one CTA per (128 queries, head, batch): recomputes S and dP per key tile
 //   and accumulates dQ += dS K in TMEM.
+// A sequence may have any length: its last tile reads zeros behind it and is masked.
 // Every barrier wait is bounded; a wait that runs out sets the status word.
 #include "ptx.cuh"
 #include "tensormap.cuh"
@@ -30,8 +27,7 @@ constexpr int TQ = 128;
 constexpr int TK = 128;
 constexpr int TILE_BYTES = 128 * HD * 2;      // 32 KiB: two swizzle atoms of [128 rows x 64 cols]
 constexpr int ATOM_BYTES = 16384;
-constexpr int ATTN_THREADS = 192;
-constexpr int ATTN_BWD_THREADS = 320;   // TMA warp, MMA warp, two softmax groups of four warps
+constexpr int ATTN_THREADS = 320;       // two softmax warpgroups, TMA warp, MMA warp
 
 struct AttnParams {
   CUtensorMap map_q, map_k, map_v, map_do;
@@ -39,9 +35,11 @@ struct AttnParams {
   int causal;             // 1: keys after the query are masked; 0: every query sees every key
   float scale;            // 1/sqrt(head_dim)
   float scale_log2;       // scale * log2(e)
-  __nv_bfloat16* out;     // forward: [B,S,Hq,128] contiguous
-  float* lse;             // [B,Hq,S] natural-log row sums (forward writes, backward reads)
-  const float* delta;     // [B,Hq,S] rowsum(dO * O) (backward)
+  int set_heads;          // heads that share a launch-order set (attn_work)
+  void* out;              // forward: [B,S,Hq,128] contiguous, in the type of q, k, v
+  float* lse;             // [B,Hq,S] natural-log row sums (forward writes)
+  const float* stats;     // backward: [B*Hq][2][Sp] with Sp = S rounded up to 128: -lse * log2(e), then -rowsum(dO * O);
+                          // -inf and 0 behind the sequence (such queries get zero probabilities)
   __nv_bfloat16* dq;      // [B,S,Hq,128]
   __nv_bfloat16* dk;      // [B,S,Hkv,128]
   __nv_bfloat16* dv;      // [B,S,Hkv,128]
@@ -86,9 +84,45 @@ __device__ __forceinline__ uint64_t desc_mnmajor(uint32_t tile, int ks) {
   return umma_smem_desc(tile + ks * 2048, ATOM_BYTES, 1024);
 }
 
-__device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int col0, int row0) {
-  tma_load_2d(dst, map, bar, col0, row0);
-  tma_load_2d(dst + ATOM_BYTES, map, bar, col0 + 64, row0);
+// 128 tokens x 128 columns of one batch entry; tokens behind the sequence read as zeros.
+__device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int col0, int token0,
+                                          int batch) {
+  tma_load_3d(dst, map, bar, col0, token0, batch);
+  tma_load_3d(dst + ATOM_BYTES, map, bar, col0 + 64, token0, batch);
+}
+
+template <int F16>
+constexpr uint32_t attn_idesc(int b_mn_major) {
+  return F16 ? umma_idesc_f16(128, 128, 0, b_mn_major) : umma_idesc_bf16(128, 128, 0, b_mn_major);
+}
+
+// Two fp32 values in a 64-bit register: one instruction of the FMA pipe works on both (same rounding as two).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 make_f32x2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 bits_f32x2(const uint32_t* two) {
+  return make_f32x2(__uint_as_float(two[0]), __uint_as_float(two[1]));
+}
+__device__ __forceinline__ void split_f32x2(f32x2 v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma_f32x2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 add_f32x2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul_f32x2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
 }
 
 #define ATTN_FAIL(code)            \
@@ -99,27 +133,53 @@ __device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* map, 
 
 // ================================================================= forward
 struct FwdBars {
-  uint64_t q_full, k_full[2], v_full[2], k_empty[2], v_empty[2], s_full[2], p_full[2], o_done, mx_ready;
+  uint64_t q_full, k_full[2], v_full[2], k_empty[2], v_empty[2], s_full[2], p_lo[2], p_hi[2], o_done[2];
 };
 
-__global__ void __launch_bounds__(ATTN_BWD_THREADS, 1) attn_fwd_kernel(const __grid_constant__ AttnParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sQ = smem;
-  uint8_t* sK = sQ + TILE_BYTES;            // 2 stages
+// Which tile a CTA works on.  CTAs are numbered so that the longest causal rows of a set of heads start first, and a
+// set holds as many heads as keep the tensors they re-read inside the L2 (p.set_heads, host side).
+struct AttnWork {
+  int tile, head;          // 0 = longest; flattened batch * heads + head
+};
+__device__ __forceinline__ AttnWork attn_work(const AttnParams& p, int tiles, int heads) {
+  const int per_set = p.set_heads * tiles;
+  const int set = static_cast<int>(blockIdx.x) / per_set;
+  const int rest = static_cast<int>(blockIdx.x) - set * per_set;
+  const int count = min(p.set_heads, heads - set * p.set_heads);
+  return {rest / count, set * p.set_heads + rest % count};
+}
+
+// One CTA per (two adjacent 128-query tiles, head, batch): the tiles ping-pong, so the tensor core works on one while
+// the softmax warpgroup of the other turns scores into probabilities.  A thread owns a whole query row (128 score
+// columns in registers): no exchange of row maxima, one barrier per half of a probability tile.  S and O of both tiles
+// fill tensor memory; P overwrites S.  MMA order O0(j) S0(j+1) O1(j) S1(j+1): a tile's next scores are issued behind
+// the product that still reads its probabilities, so "scores ready" also means "output of the previous key tile
+// accumulated", and the rare rescale of O (row maximum grew by more than 2^8) needs no further wait.
+// Bound by the chain scores -> exponentials -> product of each tile.  32/8 heads of 8192 tokens, causal: 447 us, 1230
+// TFLOP/s (one query tile per CTA with two threads per row: 622 us); 32 heads of 2048 tokens, every key, fp16: 77 us
+// (bf16 kernel 95 us plus 96 us of casts).
+template <int F16>
+__global__ void __launch_bounds__(ATTN_THREADS, 1) attn_fwd_kernel(const __grid_constant__ AttnParams p) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = smem_raw;
+  uint8_t* sQ = smem;                       // 2 tiles
+  uint8_t* sK = sQ + 2 * TILE_BYTES;        // 2 stages
   uint8_t* sV = sK + 2 * TILE_BYTES;        // 2 stages
-  float* s_rowmax = reinterpret_cast<float*>(sV + 2 * TILE_BYTES);   // [2 buffers][2 halves][128] + [2][128] sums
-  FwdBars* bars = reinterpret_cast<FwdBars*>(s_rowmax + 6 * TQ);
+  FwdBars* bars = reinterpret_cast<FwdBars*>(sV + 2 * TILE_BYTES);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int q_tiles = p.S / TQ;
-  const int qt = q_tiles - 1 - blockIdx.x;      // long tiles first
-  const int h = blockIdx.y, b = blockIdx.z;
+  const int kv_tiles = (p.S + TK - 1) / TK;
+  const int pairs = (kv_tiles + 1) / 2;
+  const AttnWork work = attn_work(p, pairs, p.B * p.Hq);
+  const int qt0 = 2 * (pairs - 1 - work.tile);
+  const int b = work.head / p.Hq, h = work.head - b * p.Hq;
   const int hk = h / (p.Hq / p.Hkv);
-  const int n_kv = p.causal ? qt + 1 : q_tiles;
-  const int row_q = b * p.S + qt * TQ;
+  // key tiles that each of the two query tiles sees (the second one may lie behind the sequence)
+  const int n0 = p.causal ? qt0 + 1 : kv_tiles;
+  const int n1 = qt0 + 1 >= kv_tiles ? 0 : (p.causal ? qt0 + 2 : kv_tiles);
+  const int n_kv = max(n0, n1);
 
   if (threadIdx.x == 0) {
     mbar_init(&bars->q_full, 1);
@@ -129,666 +189,752 @@ __global__ void __launch_bounds__(ATTN_BWD_THREADS, 1) attn_fwd_kernel(const __g
       mbar_init(&bars->k_empty[s], 1);
       mbar_init(&bars->v_empty[s], 1);
       mbar_init(&bars->s_full[s], 1);
-      mbar_init(&bars->p_full[s], 8);
+      mbar_init(&bars->p_lo[s], 4);
+      mbar_init(&bars->p_hi[s], 4);
+      mbar_init(&bars->o_done[s], 1);
     }
-    mbar_init(&bars->o_done, 1);
-    mbar_init(&bars->mx_ready, 8);
     *abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == 1) {
+  if (warp == 9) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
-  const uint32_t tmem_o = tmem + 256;
+  const uint32_t tmem = *tmem_slot;         // S0 | S1 | O0 | O1, 128 columns each
 
-  if (warp == 0) {
+  if (warp == 8) {
     if (elect_one()) {
-      mbar_expect_tx(&bars->q_full, TILE_BYTES);
-      load_tile(sQ, &p.map_q, &bars->q_full, h * HD, row_q);
+      mbar_expect_tx(&bars->q_full, (n1 ? 2 : 1) * TILE_BYTES);
+      load_tile(sQ, &p.map_q, &bars->q_full, h * HD, qt0 * TQ, b);
+      if (n1) load_tile(sQ + TILE_BYTES, &p.map_q, &bars->q_full, h * HD, (qt0 + 1) * TQ, b);
       for (int j = 0; j < n_kv && !*abort_flag; ++j) {
         const int s = j & 1;
         const uint32_t ph = ((j >> 1) & 1) ^ 1;
-        const int row_k = b * p.S + j * TK;
         if (!mbar_wait(&bars->k_empty[s], ph)) { ATTN_FAIL(201); break; }
         mbar_expect_tx(&bars->k_full[s], TILE_BYTES);
-        load_tile(sK + s * TILE_BYTES, &p.map_k, &bars->k_full[s], hk * HD, row_k);
+        load_tile(sK + s * TILE_BYTES, &p.map_k, &bars->k_full[s], hk * HD, j * TK, b);
         if (!mbar_wait(&bars->v_empty[s], ph)) { ATTN_FAIL(202); break; }
         mbar_expect_tx(&bars->v_full[s], TILE_BYTES);
-        load_tile(sV + s * TILE_BYTES, &p.map_v, &bars->v_full[s], hk * HD, row_k);
+        load_tile(sV + s * TILE_BYTES, &p.map_v, &bars->v_full[s], hk * HD, j * TK, b);
       }
     }
-  } else if (warp == 1) {
+  } else if (warp == 9) {
     if (elect_one()) {
-      constexpr uint32_t idesc_qk = umma_idesc_bf16(128, 128, 0, 0);
-      constexpr uint32_t idesc_pv = umma_idesc_bf16(128, 128, 0, 1);
-      const uint32_t q_addr = smem_u32(sQ);
-      bool ok = mbar_wait(&bars->q_full, 0);
-      if (!ok) ATTN_FAIL(203);
-      auto issue_s = [&](int j) -> bool {
-        const int s = j & 1;
-        if (!mbar_wait(&bars->k_full[s], (j >> 1) & 1)) return false;
-        tc_fence_after();
-        const uint32_t k_addr = smem_u32(sK + s * TILE_BYTES);
+      constexpr uint32_t idesc_qk = attn_idesc<F16>(0);
+      constexpr uint32_t idesc_pv = attn_idesc<F16>(1);
+      auto issue_s = [&](int t, int j) {
+        const uint32_t q_addr = smem_u32(sQ + t * TILE_BYTES), k_addr = smem_u32(sK + (j & 1) * TILE_BYTES);
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
-          umma_bf16_ss(tmem + s * 128, desc_kmajor(q_addr, ks), desc_kmajor(k_addr, ks), idesc_qk, ks != 0);
-        umma_commit(&bars->k_empty[s]);
-        umma_commit(&bars->s_full[s]);
-        return true;
+          umma_bf16_ss(tmem + t * 128, desc_kmajor(q_addr, ks), desc_kmajor(k_addr, ks), idesc_qk, ks != 0);
+        umma_commit(&bars->s_full[t]);
       };
-      if (ok && !issue_s(0)) { ATTN_FAIL(204); ok = false; }
-      if (ok && n_kv > 1 && !issue_s(1)) { ATTN_FAIL(204); ok = false; }
+      bool ok = mbar_wait(&bars->q_full, 0) && mbar_wait(&bars->k_full[0], 0);
+      if (!ok) ATTN_FAIL(203);
+      if (ok) {
+        tc_fence_after();
+        issue_s(0, 0);
+        if (n1) issue_s(1, 0);
+        umma_commit(&bars->k_empty[0]);
+      }
       for (int j = 0; j < n_kv && ok && !*abort_flag; ++j) {
-        const int s = j & 1;
-        if (!mbar_wait(&bars->p_full[s], (j >> 1) & 1) || !mbar_wait(&bars->v_full[s], (j >> 1) & 1)) {
-          ATTN_FAIL(205);
+        const uint32_t ph = j & 1;
+        if (!mbar_wait(&bars->v_full[j & 1], (j >> 1) & 1) ||
+            (j + 1 < n_kv && !mbar_wait(&bars->k_full[(j + 1) & 1], ((j + 1) >> 1) & 1))) {
+          ATTN_FAIL(204);
           break;
         }
-        tc_fence_after();
-        const uint32_t v_addr = smem_u32(sV + s * TILE_BYTES);
+        const uint32_t v_addr = smem_u32(sV + (j & 1) * TILE_BYTES);
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks)
-          umma_bf16_ts(tmem_o, tmem + s * 128 + (ks >> 2) * 64 + (ks & 3) * 8, desc_mnmajor(v_addr, ks), idesc_pv,
-                       (j | ks) != 0);
-        umma_commit(&bars->v_empty[s]);
-        umma_commit(&bars->o_done);
-        if (j + 2 < n_kv && !issue_s(j + 2)) { ATTN_FAIL(204); break; }
+        for (int t = 0; t < 2; ++t) {
+          const int n = t ? n1 : n0;
+          if (j >= n || !ok) continue;
+          if (!mbar_wait(&bars->p_lo[t], ph)) { ok = false; continue; }
+          tc_fence_after();
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks)
+            umma_bf16_ts(tmem + 256 + t * 128, tmem + t * 128 + ks * 8, desc_mnmajor(v_addr, ks), idesc_pv, (j | ks) != 0);
+          if (!mbar_wait(&bars->p_hi[t], ph)) { ok = false; continue; }
+          tc_fence_after();
+#pragma unroll
+          for (int ks = 4; ks < 8; ++ks)
+            umma_bf16_ts(tmem + 256 + t * 128, tmem + t * 128 + ks * 8, desc_mnmajor(v_addr, ks), idesc_pv, 1);
+          if (j + 1 == n) umma_commit(&bars->o_done[t]);
+          else issue_s(t, j + 1);
+        }
+        if (!ok) { ATTN_FAIL(205); break; }
+        umma_commit(&bars->v_empty[j & 1]);
+        if (j + 1 < n_kv) umma_commit(&bars->k_empty[(j + 1) & 1]);
       }
     }
   } else {
-    // Two softmax groups of four warps; group ``half`` owns key columns [64 half, 64 half + 64) of every
-    // score tile.  The two threads that share a query row exchange their partial row maxima through shared
-    // memory (one bounded mbarrier phase per tile) and keep separate partial row sums until the end.
+    const int t = warp >> 2;                              // query tile of this warpgroup
     const int quad = warp & 3;
-    const int half = (warp - 2) >> 2;
     const int r = quad * 32 + lane;                       // query row inside the tile
-    const int col0 = half * 64;
+    const int qt = qt0 + t;
+    const int n = t ? n1 : n0;
     const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
+    const uint32_t ts = tmem + t * 128 + lane_base, to = tmem + 256 + t * 128 + lane_base;
     float m_ref = -INFINITY, l = 0.f;
-    for (int j = 0; j < n_kv && !*abort_flag; ++j) {
-      const int s = j & 1;
-      if (!mbar_wait(&bars->s_full[s], (j >> 1) & 1)) { ATTN_FAIL(206); break; }
+    for (int j = 0; j < n && !*abort_flag; ++j) {
+      if (!mbar_wait(&bars->s_full[t], j & 1)) { ATTN_FAIL(206); break; }
       tc_fence_after();
-      const uint32_t ts = tmem + s * 128 + lane_base + col0;
-      uint32_t raw[2][32];
-      tmem_ld_32x32(ts, raw[0]);
-      tmem_ld_32x32(ts + 32, raw[1]);
+      uint32_t raw[4][32];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tmem_ld_32x32(ts + c * 32, raw[c]);
       tmem_ld_wait();
-      if (p.causal && j == qt) {                       // diagonal tile: keys after the query are masked
+      auto score = [&](int i) { return __uint_as_float(raw[i >> 5][i & 31]); };
+      // keys that the row does not see: after the query (causal, diagonal tile) or behind the sequence
+      const bool diagonal = p.causal && j == qt;
+      if (diagonal || (j + 1) * TK > p.S) {
+        const int limit = diagonal ? r + 1 : p.S - j * TK;
 #pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (col0 + c * 32 + i > r) raw[c][i] = 0xff800000u;   // -inf
+        for (int i = 0; i < 128; ++i)
+          if (i >= limit) raw[i >> 5][i & 31] = 0xff800000u;   // -inf
       }
-      float mpart[8];
+      float mpart[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-      for (int i = 0; i < 8; ++i) mpart[i] = -INFINITY;
-#pragma unroll
-      for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int i = 0; i < 32; ++i) mpart[i & 7] = fmaxf(mpart[i & 7], __uint_as_float(raw[c][i]));
-      float mx = fmaxf(fmaxf(fmaxf(mpart[0], mpart[1]), fmaxf(mpart[2], mpart[3])),
-                       fmaxf(fmaxf(mpart[4], mpart[5]), fmaxf(mpart[6], mpart[7])));
-      // exchange with the thread that owns the other 64 columns of this row
-      s_rowmax[(s * 2 + half) * TQ + r] = mx;
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->mx_ready);
-      if (!mbar_wait(&bars->mx_ready, j & 1)) { ATTN_FAIL(209); break; }
-      mx = fmaxf(fmaxf(mx, s_rowmax[(s * 2 + (half ^ 1)) * TQ + r]), m_ref);
+      for (int i = 0; i < 128; i += 2) mpart[(i >> 1) & 3] = fmaxf(fmaxf(mpart[(i >> 1) & 3], score(i)), score(i + 1));
+      const float mx = fmaxf(fmaxf(fmaxf(mpart[0], mpart[1]), fmaxf(mpart[2], mpart[3])), m_ref);
       const bool need = (mx - m_ref) * p.scale_log2 > 8.f;      // also true on the first tile (m_ref = -inf)
-      const bool any = __any_sync(0xffffffffu, need);
-      float alpha = 1.f;
-      if (any) {
-        alpha = ex2((m_ref - mx) * p.scale_log2);               // 0 on the first tile
+      if (__any_sync(0xffffffffu, need)) {
+        const float alpha = ex2((m_ref - mx) * p.scale_log2);   // 0 on the first tile
         m_ref = mx;
-      }
-      const float neg = -m_ref * p.scale_log2;
-      float part[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};   // independent partial sums: no long add chain
-      uint32_t packed[32];
-#pragma unroll
-      for (int c = 0; c < 2; ++c)
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          const float x0 = fmaf(__uint_as_float(raw[c][i]), p.scale_log2, neg);
-          const float x1 = fmaf(__uint_as_float(raw[c][i + 1]), p.scale_log2, neg);
-          const float p0 = ex2(x0), p1 = ex2(x1);
-          part[(i >> 1) & 7] += p0 + p1;
-          packed[c * 16 + (i >> 1)] = pack_bf16(p0, p1);
-        }
-      const float sum = ((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]));
-      l = l * alpha + sum;
-      // P (bf16 pairs) overwrites the first 32 of the 64 columns this thread has just read
-      tmem_st_32x32(ts, packed);
-      if (j > 0) {
-        if (!mbar_wait(&bars->o_done, (j - 1) & 1)) { ATTN_FAIL(207); break; }
-        tc_fence_after();
-        if (any) {
+        l *= alpha;
+        if (j > 0) {
 #pragma unroll 1
-          for (int c = 0; c < 2; ++c) {
-            uint32_t o[32];
-            tmem_ld_32x32(tmem_o + lane_base + col0 + c * 32, o);
+          for (int c = 0; c < 8; ++c) {
+            uint32_t o[16];
+            tmem_ld_32x16(to + c * 16, o);
             tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-            tmem_st_32x32(tmem_o + lane_base + col0 + c * 32, o);
+            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+            tmem_st_32x16(to + c * 16, o);
           }
         }
       }
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->p_full[s]);
+      const float neg = -m_ref * p.scale_log2;
+      const f32x2 scale2 = make_f32x2(p.scale_log2, p.scale_log2), neg2 = make_f32x2(neg, neg);
+      f32x2 sum2[4] = {0, 0, 0, 0};          // independent partial sums: no long add chain
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t packed[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const int k = hf * 64 + c * 32 + 2 * i;
+            float x0, x1;
+            split_f32x2(fma_f32x2(make_f32x2(score(k), score(k + 1)), scale2, neg2), x0, x1);
+            const float p0 = ex2(x0), p1 = ex2(x1);
+            sum2[i & 3] = add_f32x2(sum2[i & 3], make_f32x2(p0, p1));
+            packed[i] = F16 ? pack_f16(p0, p1) : pack_bf16(p0, p1);
+          }
+          tmem_st_32x16(ts + hf * 32 + c * 16, packed);      // pairs over the score columns read above
+        }
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(hf ? &bars->p_hi[t] : &bars->p_lo[t]);
+      }
+      float s0, s1;
+      split_f32x2(add_f32x2(add_f32x2(sum2[0], sum2[1]), add_f32x2(sum2[2], sum2[3])), s0, s1);
+      l += s0 + s1;
     }
-    // epilogue: combine the two partial row sums, normalise, store this thread's 64 output columns
-    if (!*abort_flag) {
-      s_rowmax[(4 + half) * TQ + r] = l;
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->mx_ready);
-      if (!mbar_wait(&bars->mx_ready, n_kv & 1)) ATTN_FAIL(210);
-      l += s_rowmax[(4 + (half ^ 1)) * TQ + r];
-      if (!mbar_wait(&bars->o_done, (n_kv - 1) & 1)) ATTN_FAIL(208);
+    // epilogue: normalise and store this thread's query row
+    if (n > 0 && !*abort_flag) {
+      if (!mbar_wait(&bars->o_done[t], 0)) ATTN_FAIL(208);
       tc_fence_after();
       const float inv = 1.f / l;
-      const size_t token = static_cast<size_t>(row_q + r);
-      __nv_bfloat16* dst = p.out + (token * p.Hq + h) * HD + col0;
+      const int pos = qt * TQ + r;
+      uint8_t* dst = static_cast<uint8_t*>(p.out) + ((static_cast<size_t>(b) * p.S + pos) * p.Hq + h) * HD * 2;
 #pragma unroll 1
-      for (int c = 0; c < 2; ++c) {
+      for (int c = 0; c < 4; ++c) {
         uint32_t o[32];
-        tmem_ld_32x32(tmem_o + lane_base + col0 + c * 32, o);
+        tmem_ld_32x32(to + c * 32, o);
         tmem_ld_wait();
-        uint4* d4 = reinterpret_cast<uint4*>(dst + c * 32);
+        if (pos < p.S) {
+          uint4* d4 = reinterpret_cast<uint4*>(dst + c * 64);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          d4[i] = make_uint4(pack_bf16(__uint_as_float(o[8 * i]) * inv, __uint_as_float(o[8 * i + 1]) * inv),
-                             pack_bf16(__uint_as_float(o[8 * i + 2]) * inv, __uint_as_float(o[8 * i + 3]) * inv),
-                             pack_bf16(__uint_as_float(o[8 * i + 4]) * inv, __uint_as_float(o[8 * i + 5]) * inv),
-                             pack_bf16(__uint_as_float(o[8 * i + 6]) * inv, __uint_as_float(o[8 * i + 7]) * inv));
+          for (int i = 0; i < 4; ++i) {
+            uint32_t w[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const float a = __uint_as_float(o[8 * i + 2 * k]) * inv, e = __uint_as_float(o[8 * i + 2 * k + 1]) * inv;
+              w[k] = F16 ? pack_f16(a, e) : pack_bf16(a, e);
+            }
+            d4[i] = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+        }
+        __syncwarp();
       }
-      if (half == 0) p.lse[(static_cast<size_t>(b) * p.Hq + h) * p.S + qt * TQ + r] = m_ref * p.scale + logf(l);
+      if (pos < p.S) p.lse[static_cast<size_t>(work.head) * p.S + pos] = m_ref * p.scale + logf(l);
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) {
+  if (warp == 9) {
     tc_fence_after();
     tmem_dealloc(tmem, 512);
   }
 }
 
-// ================================================================= backward: delta = rowsum(dO * O)
-__global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ out,
-                                  float* __restrict__ delta, int B, int S, int Hq) {
-  // one warp per (token, head); delta layout [B, Hq, S]
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  const int total = B * S * Hq;
-  if (warp >= total) return;
-  const int h = warp % Hq;
-  const int token = warp / Hq;
-  const size_t base = static_cast<size_t>(warp) * HD + lane * 4;
-  const uint2 a = *reinterpret_cast<const uint2*>(dout + base);
-  const uint2 o = *reinterpret_cast<const uint2*>(out + base);
-  const float2 a0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a.x));
-  const float2 a1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&a.y));
-  const float2 o0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&o.x));
-  const float2 o1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&o.y));
-  float s = a0.x * o0.x + a0.y * o0.y + a1.x * o1.x + a1.y * o1.y;
+// ================================================================= backward: row statistics
+// stats[head][0][pos] = -lse * log2(e), stats[head][1][pos] = -rowsum(dO * O); -inf and 0 behind the sequence.  Half a
+// warp per row (16 bytes a lane), sixteen consecutive positions of one head per block: 64-byte stores.  Memory bound:
+// 134 MB in 32 us at 32 heads of 8192 tokens (a warp per row with 8-byte loads: 48 us).
+__global__ void __launch_bounds__(256) attn_stats_kernel(const __nv_bfloat16* __restrict__ dout,
+                                                         const __nv_bfloat16* __restrict__ out,
+                                                         const float* __restrict__ lse, float* __restrict__ stats, int S,
+                                                         int Sp, int Hq) {
+  const int sub = threadIdx.x & 15;
+  const int blocks_per_head = Sp / 16;
+  const int head = blockIdx.x / blocks_per_head;           // batch * Hq + h
+  const int pos = (blockIdx.x - head * blocks_per_head) * 16 + (threadIdx.x >> 4);
+  const int b = head / Hq, h = head - b * Hq;
+  float sum = 0.f;
+  if (pos < S) {
+    const size_t base = ((static_cast<size_t>(b) * S + pos) * Hq + h) * HD + sub * 8;
+    const uint4 a = *reinterpret_cast<const uint4*>(dout + base);
+    const uint4 o = *reinterpret_cast<const uint4*>(out + base);
+    const uint32_t av[4] = {a.x, a.y, a.z, a.w}, ov[4] = {o.x, o.y, o.z, o.w};
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  if (lane == 0) {
-    const int b = token / S, pos = token - b * S;
-    delta[(static_cast<size_t>(b) * Hq + h) * S + pos] = s;
+    for (int i = 0; i < 4; ++i) {
+      const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&av[i]));
+      const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ov[i]));
+      sum += x.x * y.x + x.y * y.y;
+    }
+  }
+#pragma unroll
+  for (int off = 8; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+  if (sub == 0) {
+    float* row = stats + static_cast<size_t>(head) * 2 * Sp + pos;
+    row[0] = pos < S ? -lse[static_cast<size_t>(head) * S + pos] * 1.4426950408889634f : -INFINITY;
+    row[Sp] = -sum;
+  }
+}
+
+// A finished accumulator row of 128 fp32 columns: scaled, rotated back if tables are given, stored as bf16.  The whole
+// warp calls it (tcgen05.ld is a warp instruction); rows behind the sequence are not stored.  CHUNKS of 32 columns from
+// chunk ``first`` on.
+template <int CHUNKS = 4>
+__device__ __forceinline__ void store_grad_row(uint32_t taddr, __nv_bfloat16* dst, int pos, int S, float scale,
+                                               const float* rope_cos, const float* rope_sin, int first = 0) {
+#pragma unroll 1
+  for (int c = first; c < first + CHUNKS; ++c) {
+    uint32_t a[32];
+    tmem_ld_32x32(taddr + c * 32, a);
+    tmem_ld_wait();
+    if (pos < S) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) a[i] = __float_as_uint(__uint_as_float(a[i]) * scale);
+      if (rope_cos) unrotate32(a, rope_cos, rope_sin, pos, c * 16);
+      uint4* d4 = reinterpret_cast<uint4*>(dst + c * 32);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        d4[i] = make_uint4(pack_bf16(__uint_as_float(a[8 * i]), __uint_as_float(a[8 * i + 1])),
+                           pack_bf16(__uint_as_float(a[8 * i + 2]), __uint_as_float(a[8 * i + 3])),
+                           pack_bf16(__uint_as_float(a[8 * i + 4]), __uint_as_float(a[8 * i + 5])),
+                           pack_bf16(__uint_as_float(a[8 * i + 6]), __uint_as_float(a[8 * i + 7])));
+    }
+    __syncwarp();
   }
 }
 
 // ================================================================= backward: dK, dV
-struct KvBars {
-  uint64_t kv_full, qd_full[2], qd_empty[2], st_full, dpt_full, p_ready, ds_ready, acc_done;
+// Both backward kernels are bound by the chain MMA -> softmax warps -> MMA of a 128 x 128 tile (of 3500 cycles 1050 on
+// the special-function unit and 2050 on the tensor core when the two warpgroups ran in step), so the tile is cut into
+// two 64-column halves with their own barriers: half a period apart, one half's exponentials run under the other half's
+// products and hand-overs.  32/8 heads of 8192 tokens, causal: dK/dV 1058 -> 932 us, dQ 848 -> 714 us.
+struct BwdBars {
+  uint64_t fixed_full, a_full[3], a_empty[3], b_full[2], b_empty[2], st_full[2], dpt_full[2], p_ready[2], ds_ready[2],
+      acc_done;
+};
+constexpr int HALF = 64;
+template <bool V> struct Constant { static constexpr bool value = V; };
+
+// Shared memory of both kernels: two tiles that stay, a ring of three (read last by the products of the previous
+// step), a ring of two, and per ring slot 128 row statistics (dK/dV kernel only).
+struct BwdSmem {
+  uint8_t fixed[2][TILE_BYTES];
+  uint8_t a[3][TILE_BYTES];
+  uint8_t b[2][TILE_BYTES];
+  float a_stat[3][TQ], b_stat[2][TQ];
+  BwdBars bars;
+  uint32_t tmem_slot;
+  int abort_flag;
 };
 
-// TMEM: S^T / P^T [0,128), dP^T / dS^T [128,256), dV [256,384), dK [384,512).
-// 320 threads: warp 0 TMA, warp 1 MMA, warps 2-9 two softmax groups; group g handles query columns
-// [64 g, 64 g + 64) of the 128 x 128 tile (two warps per scheduler hide each other's latency).
-// MMA order per query tile: dV(it), S^T(it+1), dK(it), dP^T(it+1) - S^T of the next tile runs on the
-// tensor core while the softmax warps turn dP^T into dS^T.
-__global__ void __launch_bounds__(ATTN_BWD_THREADS, 1) attn_bwd_dkv_kernel(const __grid_constant__ AttnParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sK = smem;
-  uint8_t* sV = sK + TILE_BYTES;
-  uint8_t* sQ = sV + TILE_BYTES;             // 2 stages
-  uint8_t* sDO = sQ + 2 * TILE_BYTES;        // 2 stages
-  KvBars* bars = reinterpret_cast<KvBars*>(sDO + 2 * TILE_BYTES);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+__device__ __forceinline__ void bwd_init(BwdSmem& sm, int warp) {
+  if (threadIdx.x == 0) {
+    mbar_init(&sm.bars.fixed_full, 1);
+    for (int s = 0; s < 3; ++s) {
+      mbar_init(&sm.bars.a_full[s], 1);
+      mbar_init(&sm.bars.a_empty[s], 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&sm.bars.b_full[s], 1);
+      mbar_init(&sm.bars.b_empty[s], 1);
+      mbar_init(&sm.bars.st_full[s], 1);
+      mbar_init(&sm.bars.dpt_full[s], 1);
+      mbar_init(&sm.bars.p_ready[s], 4);
+      mbar_init(&sm.bars.ds_ready[s], 4);
+    }
+    mbar_init(&sm.bars.acc_done, 1);
+    sm.abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 9) {
+    tmem_alloc(&sm.tmem_slot, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+}
+
+__device__ __forceinline__ void bwd_exit(BwdSmem& sm, int warp, uint32_t tmem) {
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 9) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 512);
+  }
+}
+
+// Slot and phase of step i in a ring of three.
+__device__ __forceinline__ int slot3(int i) { return i % 3; }
+__device__ __forceinline__ uint32_t phase3(int i) { return (i / 3) & 1; }
+
+__device__ __forceinline__ void arrive_half(uint64_t* bar, int lane) {
+  tc_fence_before();
+  __syncwarp();
+  if (lane == 0) mbar_arrive(bar);
+}
+
+// TMEM: S^T / P^T [0,128), dP^T / dS^T [128,256) (64 columns per half), dV [256,384), dK [384,512).  320 threads: warps
+// 0-7 two softmax warpgroups, group g handles query columns [64 g, 64 g + 64) of every tile; warp 8 TMA, warp 9 MMA.
+// The ring of three holds Q tiles (with -rowsum(dO O)), the ring of two dO tiles (with -lse).  MMA order per query tile:
+//   dV0(i) S0(i+1) | dK1(i-1) dP1(i) | dV1(i) S1(i+1) | dK0(i) dP0(i+1)
+// each group of products waits for one half's P or dS, which the other half's turn has given time to appear.
+__global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dkv_kernel(const __grid_constant__ AttnParams p) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  BwdSmem& sm = *reinterpret_cast<BwdSmem*>(smem_raw);
+  BwdBars* bars = &sm.bars;
+  volatile int* abort_flag = &sm.abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int q_tiles = p.S / TQ;
-  const int kt = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
+  const int q_tiles = (p.S + TQ - 1) / TQ;
+  const AttnWork work = attn_work(p, q_tiles, p.B * p.Hkv);
+  const int kt = work.tile, b = work.head / p.Hkv, hk = work.head - b * p.Hkv;
   const int group = p.Hq / p.Hkv;
   const int q_first = p.causal ? kt : 0;           // causal: query tiles kt .. q_tiles-1
   const int per_head = q_tiles - q_first;
   const int iters = group * per_head;
-  const int row_k = b * p.S + kt * TK;
 
-  if (threadIdx.x == 0) {
-    mbar_init(&bars->kv_full, 1);
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&bars->qd_full[s], 1);
-      mbar_init(&bars->qd_empty[s], 1);
-    }
-    mbar_init(&bars->st_full, 1);
-    mbar_init(&bars->dpt_full, 1);
-    mbar_init(&bars->p_ready, 8);
-    mbar_init(&bars->ds_ready, 8);
-    mbar_init(&bars->acc_done, 1);
-    *abort_flag = 0;
-    mbar_fence_init();
-  }
-  if (warp == 1) {
-    tmem_alloc(tmem_slot, 512);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  bwd_init(sm, warp);
+  const uint32_t tmem = sm.tmem_slot;
   const uint32_t t_st = tmem, t_dpt = tmem + 128, t_dv = tmem + 256, t_dk = tmem + 384;
 
-  if (warp == 0) {
+  if (warp == 8) {
     if (elect_one()) {
-      mbar_expect_tx(&bars->kv_full, 2 * TILE_BYTES);
-      load_tile(sK, &p.map_k, &bars->kv_full, hk * HD, row_k);
-      load_tile(sV, &p.map_v, &bars->kv_full, hk * HD, row_k);
+      mbar_expect_tx(&bars->fixed_full, 2 * TILE_BYTES);
+      load_tile(sm.fixed[0], &p.map_k, &bars->fixed_full, hk * HD, kt * TK, b);
+      load_tile(sm.fixed[1], &p.map_v, &bars->fixed_full, hk * HD, kt * TK, b);
       for (int it = 0; it < iters && !*abort_flag; ++it) {
-        const int s = it & 1;
+        const int s3 = slot3(it), s2 = it & 1;
         const int hq = hk * group + it / per_head;
         const int qi = q_first + it % per_head;
-        const int row_q = b * p.S + qi * TQ;
-        if (!mbar_wait(&bars->qd_empty[s], ((it >> 1) & 1) ^ 1)) { ATTN_FAIL(211); break; }
-        mbar_expect_tx(&bars->qd_full[s], 2 * TILE_BYTES);
-        load_tile(sQ + s * TILE_BYTES, &p.map_q, &bars->qd_full[s], hq * HD, row_q);
-        load_tile(sDO + s * TILE_BYTES, &p.map_do, &bars->qd_full[s], hq * HD, row_q);
+        const float* stat = p.stats + (static_cast<size_t>(b) * p.Hq + hq) * 2 * q_tiles * TQ + qi * TQ;
+        if (!mbar_wait(&bars->a_empty[s3], phase3(it) ^ 1)) { ATTN_FAIL(211); break; }
+        mbar_expect_tx(&bars->a_full[s3], TILE_BYTES + TQ * 4);
+        load_tile(sm.a[s3], &p.map_q, &bars->a_full[s3], hq * HD, qi * TQ, b);
+        bulk_load(sm.a_stat[s3], stat + q_tiles * TQ, &bars->a_full[s3], TQ * 4);
+        if (!mbar_wait(&bars->b_empty[s2], ((it >> 1) & 1) ^ 1)) { ATTN_FAIL(212); break; }
+        mbar_expect_tx(&bars->b_full[s2], TILE_BYTES + TQ * 4);
+        load_tile(sm.b[s2], &p.map_do, &bars->b_full[s2], hq * HD, qi * TQ, b);
+        bulk_load(sm.b_stat[s2], stat, &bars->b_full[s2], TQ * 4);
       }
     }
-  } else if (warp == 1) {
+  } else if (warp == 9) {
     if (elect_one()) {
-      constexpr uint32_t idesc_kk = umma_idesc_bf16(128, 128, 0, 0);   // both operands K-major
+      constexpr uint32_t idesc_kk = umma_idesc_bf16(128, HALF, 0, 0);  // both operands K-major
       constexpr uint32_t idesc_tn = umma_idesc_bf16(128, 128, 0, 1);   // A from TMEM, B MN-major
-      const uint32_t k_addr = smem_u32(sK), v_addr = smem_u32(sV);
-      auto issue_st = [&](int it) {          // S^T[key, q] = K Q^T
-        const uint32_t q_addr = smem_u32(sQ + (it & 1) * TILE_BYTES);
+      const uint32_t k_addr = smem_u32(sm.fixed[0]), v_addr = smem_u32(sm.fixed[1]);
+      auto issue_st = [&](int it, int g) {          // S^T[key, q half] = K Q^T
+        const uint32_t q_addr = smem_u32(sm.a[slot3(it)]) + g * HALF * 128;
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
-          umma_bf16_ss(t_st, desc_kmajor(k_addr, ks), desc_kmajor(q_addr, ks), idesc_kk, ks != 0);
-        umma_commit(&bars->st_full);
+          umma_bf16_ss(t_st + g * HALF, desc_kmajor(k_addr, ks), desc_kmajor(q_addr, ks), idesc_kk, ks != 0);
+        umma_commit(&bars->st_full[g]);
       };
-      auto issue_dpt = [&](int it) {         // dP^T[key, q] = V dO^T
-        const uint32_t do_addr = smem_u32(sDO + (it & 1) * TILE_BYTES);
+      auto issue_dpt = [&](int it, int g) {         // dP^T[key, q half] = V dO^T
+        const uint32_t do_addr = smem_u32(sm.b[it & 1]) + g * HALF * 128;
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
-          umma_bf16_ss(t_dpt, desc_kmajor(v_addr, ks), desc_kmajor(do_addr, ks), idesc_kk, ks != 0);
-        umma_commit(&bars->dpt_full);
+          umma_bf16_ss(t_dpt + g * HALF, desc_kmajor(v_addr, ks), desc_kmajor(do_addr, ks), idesc_kk, ks != 0);
+        umma_commit(&bars->dpt_full[g]);
       };
-      bool ok = mbar_wait(&bars->kv_full, 0) && mbar_wait(&bars->qd_full[0], 0);
-      if (!ok) ATTN_FAIL(212);
+      auto issue_dv = [&](int it, int g) {          // dV[key, d] += P^T[key, q half] dO[q half, d]
+        const uint32_t do_addr = smem_u32(sm.b[it & 1]);
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks)
+          umma_bf16_ts(t_dv, t_st + g * HALF + ks * 8, desc_mnmajor(do_addr, g * 4 + ks), idesc_tn, (it | g | ks) != 0);
+      };
+      auto issue_dk = [&](int it, int g) {          // dK[key, d] += dS^T[key, q half] Q[q half, d]
+        const uint32_t q_addr = smem_u32(sm.a[slot3(it)]);
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks)
+          umma_bf16_ts(t_dk, t_dpt + g * HALF + ks * 8, desc_mnmajor(q_addr, g * 4 + ks), idesc_tn, (it | g | ks) != 0);
+      };
+      bool ok = mbar_wait(&bars->fixed_full, 0) && mbar_wait(&bars->a_full[0], 0) && mbar_wait(&bars->b_full[0], 0);
       if (ok) {
         tc_fence_after();
-        issue_st(0);
-        issue_dpt(0);
+        issue_st(0, 0);
+        issue_st(0, 1);
+        issue_dpt(0, 0);
       }
       for (int it = 0; it < iters && ok && !*abort_flag; ++it) {
-        const int s = it & 1;
         const uint32_t ph = it & 1;
-        const uint32_t q_addr = smem_u32(sQ + s * TILE_BYTES), do_addr = smem_u32(sDO + s * TILE_BYTES);
-        if (!mbar_wait(&bars->p_ready, ph)) { ATTN_FAIL(214); break; }
-        tc_fence_after();
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks)      // dV[key, d] += P^T[key, q] dO[q, d]
-          umma_bf16_ts(t_dv, t_st + (ks >> 2) * 64 + (ks & 3) * 8, desc_mnmajor(do_addr, ks), idesc_tn, (it | ks) != 0);
         const bool more = it + 1 < iters;
-        if (more) {
-          if (!mbar_wait(&bars->qd_full[(it + 1) & 1], ((it + 1) >> 1) & 1)) { ATTN_FAIL(213); break; }
-          tc_fence_after();
-          issue_st(it + 1);                 // overwrites P^T only after dV above (same-thread issue order)
-        }
-        if (!mbar_wait(&bars->ds_ready, ph)) { ATTN_FAIL(215); break; }
+        if (!(ok = mbar_wait(&bars->p_ready[0], ph))) break;
         tc_fence_after();
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks)      // dK[key, d] += dS^T[key, q] Q[q, d]
-          umma_bf16_ts(t_dk, t_dpt + (ks >> 2) * 64 + (ks & 3) * 8, desc_mnmajor(q_addr, ks), idesc_tn, (it | ks) != 0);
-        umma_commit(&bars->qd_empty[s]);
-        umma_commit(&bars->acc_done);
-        if (more) issue_dpt(it + 1);        // overwrites dS^T only after dK above
+        issue_dv(it, 0);
+        if (more) {
+          if (!(ok = mbar_wait(&bars->a_full[slot3(it + 1)], phase3(it + 1)))) break;
+          tc_fence_after();
+          issue_st(it + 1, 0);              // overwrites P^T only after dV above (same-thread issue order)
+        }
+        if (it > 0) {
+          if (!(ok = mbar_wait(&bars->ds_ready[1], ph ^ 1))) break;
+          tc_fence_after();
+          issue_dk(it - 1, 1);
+          umma_commit(&bars->a_empty[slot3(it - 1)]);
+        }
+        issue_dpt(it, 1);                   // overwrites dS^T only after dK above
+        if (!(ok = mbar_wait(&bars->p_ready[1], ph))) break;
+        tc_fence_after();
+        issue_dv(it, 1);
+        umma_commit(&bars->b_empty[it & 1]);
+        if (more) issue_st(it + 1, 1);
+        if (!(ok = mbar_wait(&bars->ds_ready[0], ph))) break;
+        tc_fence_after();
+        issue_dk(it, 0);
+        if (more) {
+          if (!(ok = mbar_wait(&bars->b_full[(it + 1) & 1], ((it + 1) >> 1) & 1))) break;
+          tc_fence_after();
+          issue_dpt(it + 1, 0);
+        }
       }
+      if (ok && !*abort_flag && (ok = mbar_wait(&bars->ds_ready[1], (iters - 1) & 1))) {
+        tc_fence_after();
+        issue_dk(iters - 1, 1);
+        umma_commit(&bars->acc_done);
+      }
+      if (!ok) ATTN_FAIL(213);
     }
   } else {
+    const int half = warp >> 2;                            // which 64 query columns this thread handles
     const int quad = warp & 3;
-    const int half = (warp - 2) >> 2;                      // which 64 query columns this thread handles
     const int r = quad * 32 + lane;                        // key row inside the tile
     const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
-    const int col0 = half * 64;
+    const int col0 = half * HALF;
+    const uint32_t ts = t_st + lane_base + col0, tp = t_dpt + lane_base + col0;
+    const f32x2 scale2 = make_f32x2(p.scale_log2, p.scale_log2);
     for (int it = 0; it < iters && !*abort_flag; ++it) {
-      const int hq = hk * group + it / per_head;
       const int qi = q_first + it % per_head;
       const uint32_t ph = it & 1;
-      const size_t stat = (static_cast<size_t>(b) * p.Hq + hq) * p.S + qi * TQ + col0;
-      // statistics of my 64 query columns: lane i keeps those of columns 32c + i and the warp shuffles them
-      float lse_reg[2], dl_reg[2];
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        lse_reg[c] = p.lse[stat + c * 32 + lane] * 1.4426950408889634f;
-        dl_reg[c] = p.delta[stat + c * 32 + lane];
+      // statistics of my 64 query columns: four columns per 16-byte broadcast read
+      const float4* nlse = reinterpret_cast<const float4*>(sm.b_stat[it & 1] + col0);
+      const float4* ndelta = reinterpret_cast<const float4*>(sm.a_stat[slot3(it)] + col0);
+      if (!mbar_wait(&bars->b_full[it & 1], (it >> 1) & 1) || !mbar_wait(&bars->a_full[slot3(it)], phase3(it)) ||
+          !mbar_wait(&bars->st_full[half], ph)) {
+        ATTN_FAIL(216);
+        break;
       }
-      if (!mbar_wait(&bars->st_full, ph)) { ATTN_FAIL(216); break; }
       tc_fence_after();
-      const bool diag = p.causal && qi == kt;
-      uint32_t pk[32];
-      float pf[64];
+      uint32_t raw[2][32], pk[16];
+      f32x2 pf[32];
+      tmem_ld_32x32(ts, raw[0]);
+      tmem_ld_32x32(ts + 32, raw[1]);
+      tmem_ld_wait();
+      // P^T as bf16 pairs, written over the first 32 of the 64 columns this thread has just read
+      auto probabilities = [&](auto diagonal) {
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t raw[32];
-        tmem_ld_32x32(t_st + lane_base + col0 + c * 32, raw);
-        tmem_ld_wait();
+        for (int g = 0; g < 16; ++g) {
+          const float4 n = nlse[g];
+          const uint32_t* x = &raw[g >> 3][(g & 7) * 4];
+          float e[4];
+          split_f32x2(fma_f32x2(bits_f32x2(x), scale2, make_f32x2(n.x, n.y)), e[0], e[1]);
+          split_f32x2(fma_f32x2(bits_f32x2(x + 2), scale2, make_f32x2(n.z, n.w)), e[2], e[3]);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const float lq = __shfl_sync(0xffffffffu, lse_reg[c], i);
-          pf[c * 32 + i] = ex2(fmaf(__uint_as_float(raw[i]), p.scale_log2, -lq));
+          for (int i = 0; i < 4; ++i) {
+            e[i] = ex2(e[i]);
+            if (decltype(diagonal)::value && r > col0 + g * 4 + i) e[i] = 0.f;   // key after query
+          }
+          pf[2 * g] = make_f32x2(e[0], e[1]);
+          pf[2 * g + 1] = make_f32x2(e[2], e[3]);
+          pk[(2 * g) & 15] = pack_bf16(e[0], e[1]);
+          pk[(2 * g + 1) & 15] = pack_bf16(e[2], e[3]);
+          if ((g & 7) == 7) tmem_st_32x16(ts + (g >> 3) * 16, pk);
         }
-      }
-      if (diag) {                                           // key after query
-#pragma unroll
-        for (int q = 0; q < 64; ++q)
-          if (r > col0 + q) pf[q] = 0.f;
-      }
-#pragma unroll
-      for (int i = 0; i < 64; i += 2) pk[i >> 1] = pack_bf16(pf[i], pf[i + 1]);
-      // P^T as bf16 pairs, written over the columns this thread has just read: queries 0-63 land in columns
-      // [0,32), queries 64-127 in [64,96)
-      tmem_st_32x32(t_st + lane_base + col0, pk);
+      };
+      if (p.causal && qi == kt) probabilities(Constant<true>());
+      else probabilities(Constant<false>());
       tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->p_ready);
-      if (!mbar_wait(&bars->dpt_full, ph)) { ATTN_FAIL(217); break; }
+      arrive_half(&bars->p_ready[half], lane);
+      if (!mbar_wait(&bars->dpt_full[half], ph)) { ATTN_FAIL(217); break; }
       tc_fence_after();
+      tmem_ld_32x32(tp, raw[0]);
+      tmem_ld_32x32(tp + 32, raw[1]);
+      tmem_ld_wait();
+      // dS without the factor 1/sqrt(head_dim), which the epilogue applies to the fp32 sum
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t raw[32];
-        tmem_ld_32x32(t_dpt + lane_base + col0 + c * 32, raw);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          const int q = c * 32 + i;
-          const float dq0 = __shfl_sync(0xffffffffu, dl_reg[c], i), dq1 = __shfl_sync(0xffffffffu, dl_reg[c], i + 1);
-          const float d0 = pf[q] * (__uint_as_float(raw[i]) - dq0) * p.scale;
-          const float d1 = pf[q + 1] * (__uint_as_float(raw[i + 1]) - dq1) * p.scale;
-          pk[q >> 1] = pack_bf16(d0, d1);
-        }
+      for (int g = 0; g < 16; ++g) {
+        const float4 n = ndelta[g];
+        const uint32_t* x = &raw[g >> 3][(g & 7) * 4];
+        float e[4];
+        split_f32x2(mul_f32x2(pf[2 * g], add_f32x2(bits_f32x2(x), make_f32x2(n.x, n.y))), e[0], e[1]);
+        split_f32x2(mul_f32x2(pf[2 * g + 1], add_f32x2(bits_f32x2(x + 2), make_f32x2(n.z, n.w))), e[2], e[3]);
+        pk[(2 * g) & 15] = pack_bf16(e[0], e[1]);
+        pk[(2 * g + 1) & 15] = pack_bf16(e[2], e[3]);
+        if ((g & 7) == 7) tmem_st_32x16(tp + (g >> 3) * 16, pk);
       }
-      tmem_st_32x32(t_dpt + lane_base + col0, pk);
       tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->ds_ready);
+      arrive_half(&bars->ds_ready[half], lane);
     }
-    if (!*abort_flag && half == 0) {
-      if (!mbar_wait(&bars->acc_done, (iters - 1) & 1)) ATTN_FAIL(218);
+    // epilogue: group 0 stores dV, group 1 dK
+    if (!*abort_flag) {
+      if (!mbar_wait(&bars->acc_done, 0)) ATTN_FAIL(218);
       tc_fence_after();
-      const size_t token = static_cast<size_t>(row_k + r);
-      __nv_bfloat16* dvp = p.dv + token * p.dv_pitch + hk * HD;
-      __nv_bfloat16* dkp = p.dk + token * p.dk_pitch + hk * HD;
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t a[32], k2[32];
-        tmem_ld_32x32(t_dv + lane_base + c * 32, a);
-        tmem_ld_32x32(t_dk + lane_base + c * 32, k2);
-        tmem_ld_wait();
-        if (p.rope_cos) unrotate32(k2, p.rope_cos, p.rope_sin, token % static_cast<size_t>(p.S), c * 16);
-        uint4* d4 = reinterpret_cast<uint4*>(dvp + c * 32);
-        uint4* k4 = reinterpret_cast<uint4*>(dkp + c * 32);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          d4[i] = make_uint4(pack_bf16(__uint_as_float(a[8 * i]), __uint_as_float(a[8 * i + 1])),
-                             pack_bf16(__uint_as_float(a[8 * i + 2]), __uint_as_float(a[8 * i + 3])),
-                             pack_bf16(__uint_as_float(a[8 * i + 4]), __uint_as_float(a[8 * i + 5])),
-                             pack_bf16(__uint_as_float(a[8 * i + 6]), __uint_as_float(a[8 * i + 7])));
-          k4[i] = make_uint4(pack_bf16(__uint_as_float(k2[8 * i]), __uint_as_float(k2[8 * i + 1])),
-                             pack_bf16(__uint_as_float(k2[8 * i + 2]), __uint_as_float(k2[8 * i + 3])),
-                             pack_bf16(__uint_as_float(k2[8 * i + 4]), __uint_as_float(k2[8 * i + 5])),
-                             pack_bf16(__uint_as_float(k2[8 * i + 6]), __uint_as_float(k2[8 * i + 7])));
-        }
-      }
+      const int pos = kt * TK + r;
+      const size_t token = static_cast<size_t>(b) * p.S + pos;
+      __nv_bfloat16* dst = half ? p.dk + token * p.dk_pitch + hk * HD : p.dv + token * p.dv_pitch + hk * HD;
+      store_grad_row(half ? t_dk + lane_base : t_dv + lane_base, dst, pos, p.S, half ? p.scale : 1.f,
+                     half ? p.rope_cos : nullptr, p.rope_sin);
     }
   }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 1) {
-    tc_fence_after();
-    tmem_dealloc(tmem, 512);
-  }
+  bwd_exit(sm, warp, tmem);
 }
 
 // ================================================================= backward: dQ
-struct DqBars {
-  uint64_t qd_full, kv_full[2], kv_empty[2], s_full, s_taken, dp_full, ds_ready, acc_done;
-};
-
-// TMEM: S [0,128), dP / dS [128,256), dQ [256,384).  320 threads like the dK/dV kernel: softmax group g
-// handles key columns [64 g, 64 g + 64).  P stays in registers, so S of the next key tile is issued as soon
-// as both groups have read S (s_taken) and runs under the dS computation.
-__global__ void __launch_bounds__(ATTN_BWD_THREADS, 1) attn_bwd_dq_kernel(const __grid_constant__ AttnParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sQ = smem;
-  uint8_t* sDO = sQ + TILE_BYTES;
-  uint8_t* sK = sDO + TILE_BYTES;            // 2 stages
-  uint8_t* sV = sK + 2 * TILE_BYTES;         // 2 stages
-  DqBars* bars = reinterpret_cast<DqBars*>(sV + 2 * TILE_BYTES);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+// TMEM: S [0,128), dP / dS [128,256), dQ [256,384).  Thread layout as above with query rows: group g handles key columns
+// [64 g, 64 g + 64).  The ring of three holds K tiles, the ring of two V tiles.  P stays in registers, so the next
+// scores of a half are issued as soon as its warps have read the present ones (p_ready counts that).  MMA order:
+//   S0(j+1) | dQ1(j-1) dP1(j) | S1(j+1) | dQ0(j) dP0(j+1)
+__global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dq_kernel(const __grid_constant__ AttnParams p) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  BwdSmem& sm = *reinterpret_cast<BwdSmem*>(smem_raw);
+  BwdBars* bars = &sm.bars;
+  volatile int* abort_flag = &sm.abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int q_tiles = p.S / TQ;
-  const int qt = q_tiles - 1 - blockIdx.x;
-  const int h = blockIdx.y, b = blockIdx.z;
+  const int q_tiles = (p.S + TQ - 1) / TQ;
+  const AttnWork work = attn_work(p, q_tiles, p.B * p.Hq);
+  const int qt = q_tiles - 1 - work.tile;
+  const int b = work.head / p.Hq, h = work.head - b * p.Hq;
   const int hk = h / (p.Hq / p.Hkv);
   const int n_kv = p.causal ? qt + 1 : q_tiles;
-  const int row_q = b * p.S + qt * TQ;
 
-  if (threadIdx.x == 0) {
-    mbar_init(&bars->qd_full, 1);
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&bars->kv_full[s], 1);
-      mbar_init(&bars->kv_empty[s], 1);
-    }
-    mbar_init(&bars->s_full, 1);
-    mbar_init(&bars->s_taken, 8);
-    mbar_init(&bars->dp_full, 1);
-    mbar_init(&bars->ds_ready, 8);
-    mbar_init(&bars->acc_done, 1);
-    *abort_flag = 0;
-    mbar_fence_init();
-  }
-  if (warp == 1) {
-    tmem_alloc(tmem_slot, 512);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  bwd_init(sm, warp);
+  const uint32_t tmem = sm.tmem_slot;
   const uint32_t t_s = tmem, t_dp = tmem + 128, t_dq = tmem + 256;
 
-  if (warp == 0) {
+  if (warp == 8) {
     if (elect_one()) {
-      mbar_expect_tx(&bars->qd_full, 2 * TILE_BYTES);
-      load_tile(sQ, &p.map_q, &bars->qd_full, h * HD, row_q);
-      load_tile(sDO, &p.map_do, &bars->qd_full, h * HD, row_q);
+      mbar_expect_tx(&bars->fixed_full, 2 * TILE_BYTES);
+      load_tile(sm.fixed[0], &p.map_q, &bars->fixed_full, h * HD, qt * TQ, b);
+      load_tile(sm.fixed[1], &p.map_do, &bars->fixed_full, h * HD, qt * TQ, b);
       for (int j = 0; j < n_kv && !*abort_flag; ++j) {
-        const int s = j & 1;
-        const int row_k = b * p.S + j * TK;
-        if (!mbar_wait(&bars->kv_empty[s], ((j >> 1) & 1) ^ 1)) { ATTN_FAIL(221); break; }
-        mbar_expect_tx(&bars->kv_full[s], 2 * TILE_BYTES);
-        load_tile(sK + s * TILE_BYTES, &p.map_k, &bars->kv_full[s], hk * HD, row_k);
-        load_tile(sV + s * TILE_BYTES, &p.map_v, &bars->kv_full[s], hk * HD, row_k);
+        const int s3 = slot3(j), s2 = j & 1;
+        if (!mbar_wait(&bars->a_empty[s3], phase3(j) ^ 1)) { ATTN_FAIL(221); break; }
+        mbar_expect_tx(&bars->a_full[s3], TILE_BYTES);
+        load_tile(sm.a[s3], &p.map_k, &bars->a_full[s3], hk * HD, j * TK, b);
+        if (!mbar_wait(&bars->b_empty[s2], ((j >> 1) & 1) ^ 1)) { ATTN_FAIL(222); break; }
+        mbar_expect_tx(&bars->b_full[s2], TILE_BYTES);
+        load_tile(sm.b[s2], &p.map_v, &bars->b_full[s2], hk * HD, j * TK, b);
       }
     }
-  } else if (warp == 1) {
+  } else if (warp == 9) {
     if (elect_one()) {
-      constexpr uint32_t idesc_kk = umma_idesc_bf16(128, 128, 0, 0);
+      constexpr uint32_t idesc_kk = umma_idesc_bf16(128, HALF, 0, 0);
       constexpr uint32_t idesc_tn = umma_idesc_bf16(128, 128, 0, 1);
-      const uint32_t q_addr = smem_u32(sQ), do_addr = smem_u32(sDO);
-      auto issue_s = [&](int j) {           // S[q, key] = Q K^T
-        const uint32_t k_addr = smem_u32(sK + (j & 1) * TILE_BYTES);
+      const uint32_t q_addr = smem_u32(sm.fixed[0]), do_addr = smem_u32(sm.fixed[1]);
+      auto issue_s = [&](int j, int g) {           // S[q, key half] = Q K^T
+        const uint32_t k_addr = smem_u32(sm.a[slot3(j)]) + g * HALF * 128;
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
-          umma_bf16_ss(t_s, desc_kmajor(q_addr, ks), desc_kmajor(k_addr, ks), idesc_kk, ks != 0);
-        umma_commit(&bars->s_full);
+          umma_bf16_ss(t_s + g * HALF, desc_kmajor(q_addr, ks), desc_kmajor(k_addr, ks), idesc_kk, ks != 0);
+        umma_commit(&bars->st_full[g]);
       };
-      auto issue_dp = [&](int j) {          // dP[q, key] = dO V^T
-        const uint32_t v_addr = smem_u32(sV + (j & 1) * TILE_BYTES);
+      auto issue_dp = [&](int j, int g) {          // dP[q, key half] = dO V^T
+        const uint32_t v_addr = smem_u32(sm.b[j & 1]) + g * HALF * 128;
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
-          umma_bf16_ss(t_dp, desc_kmajor(do_addr, ks), desc_kmajor(v_addr, ks), idesc_kk, ks != 0);
-        umma_commit(&bars->dp_full);
+          umma_bf16_ss(t_dp + g * HALF, desc_kmajor(do_addr, ks), desc_kmajor(v_addr, ks), idesc_kk, ks != 0);
+        umma_commit(&bars->dpt_full[g]);
       };
-      bool ok = mbar_wait(&bars->qd_full, 0) && mbar_wait(&bars->kv_full[0], 0);
-      if (!ok) ATTN_FAIL(222);
+      auto issue_dq = [&](int j, int g) {          // dQ[q, d] += dS[q, key half] K[key half, d]
+        const uint32_t k_addr = smem_u32(sm.a[slot3(j)]);
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks)
+          umma_bf16_ts(t_dq, t_dp + g * HALF + ks * 8, desc_mnmajor(k_addr, g * 4 + ks), idesc_tn, (j | g | ks) != 0);
+      };
+      bool ok = mbar_wait(&bars->fixed_full, 0) && mbar_wait(&bars->a_full[0], 0) && mbar_wait(&bars->b_full[0], 0);
       if (ok) {
         tc_fence_after();
-        issue_s(0);
-        issue_dp(0);
+        issue_s(0, 0);
+        issue_s(0, 1);
+        issue_dp(0, 0);
       }
       for (int j = 0; j < n_kv && ok && !*abort_flag; ++j) {
-        const int s = j & 1;
         const uint32_t ph = j & 1;
         const bool more = j + 1 < n_kv;
         if (more) {
-          if (!mbar_wait(&bars->kv_full[(j + 1) & 1], ((j + 1) >> 1) & 1) || !mbar_wait(&bars->s_taken, ph)) {
-            ATTN_FAIL(223);
-            break;
-          }
+          if (!(ok = mbar_wait(&bars->a_full[slot3(j + 1)], phase3(j + 1)) && mbar_wait(&bars->p_ready[0], ph))) break;
           tc_fence_after();
-          issue_s(j + 1);
+          issue_s(j + 1, 0);
         }
-        if (!mbar_wait(&bars->ds_ready, ph)) { ATTN_FAIL(224); break; }
+        if (j > 0) {
+          if (!(ok = mbar_wait(&bars->ds_ready[1], ph ^ 1))) break;
+          tc_fence_after();
+          issue_dq(j - 1, 1);
+          umma_commit(&bars->a_empty[slot3(j - 1)]);
+        }
+        issue_dp(j, 1);                     // overwrites dS only after dQ above
+        umma_commit(&bars->b_empty[j & 1]);
+        if (more) {
+          if (!(ok = mbar_wait(&bars->p_ready[1], ph))) break;
+          tc_fence_after();
+          issue_s(j + 1, 1);
+        }
+        if (!(ok = mbar_wait(&bars->ds_ready[0], ph))) break;
         tc_fence_after();
-        const uint32_t k_addr = smem_u32(sK + s * TILE_BYTES);
-#pragma unroll
-        for (int ks = 0; ks < 8; ++ks)      // dQ[q, d] += dS[q, key] K[key, d]
-          umma_bf16_ts(t_dq, t_dp + (ks >> 2) * 64 + (ks & 3) * 8, desc_mnmajor(k_addr, ks), idesc_tn, (j | ks) != 0);
-        umma_commit(&bars->kv_empty[s]);
-        umma_commit(&bars->acc_done);
-        if (more) issue_dp(j + 1);          // overwrites dS only after dQ above
+        issue_dq(j, 0);
+        if (more) {
+          if (!(ok = mbar_wait(&bars->b_full[(j + 1) & 1], ((j + 1) >> 1) & 1))) break;
+          tc_fence_after();
+          issue_dp(j + 1, 0);
+        }
       }
+      if (ok && !*abort_flag && (ok = mbar_wait(&bars->ds_ready[1], (n_kv - 1) & 1))) {
+        tc_fence_after();
+        issue_dq(n_kv - 1, 1);
+        umma_commit(&bars->acc_done);
+      }
+      if (!ok) ATTN_FAIL(223);
     }
   } else {
+    const int half = warp >> 2;
     const int quad = warp & 3;
-    const int half = (warp - 2) >> 2;
     const int r = quad * 32 + lane;                        // query row inside the tile
     const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
-    const int col0 = half * 64;
-    const size_t stat = (static_cast<size_t>(b) * p.Hq + h) * p.S + qt * TQ + r;
-    const float lse2 = p.lse[stat] * 1.4426950408889634f;
-    const float dl = p.delta[stat];
+    const int col0 = half * HALF;
+    const uint32_t ts = t_s + lane_base + col0, tp = t_dp + lane_base + col0;
+    const float* stat = p.stats + static_cast<size_t>(work.head) * 2 * q_tiles * TQ + qt * TQ + r;
+    const f32x2 scale2 = make_f32x2(p.scale_log2, p.scale_log2);
+    const f32x2 nlse2 = make_f32x2(stat[0], stat[0]);
+    const f32x2 ndelta2 = make_f32x2(stat[q_tiles * TQ], stat[q_tiles * TQ]);
     for (int j = 0; j < n_kv && !*abort_flag; ++j) {
       const uint32_t ph = j & 1;
-      if (!mbar_wait(&bars->s_full, ph)) { ATTN_FAIL(225); break; }
+      if (!mbar_wait(&bars->st_full[half], ph)) { ATTN_FAIL(225); break; }
       tc_fence_after();
-      float pf[64];
+      uint32_t raw[2][32];
+      f32x2 pf[32];
+      tmem_ld_32x32(ts, raw[0]);
+      tmem_ld_32x32(ts + 32, raw[1]);
+      tmem_ld_wait();
+      arrive_half(&bars->p_ready[half], lane);
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t raw[32];
-        tmem_ld_32x32(t_s + lane_base + col0 + c * 32, raw);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) pf[c * 32 + i] = ex2(fmaf(__uint_as_float(raw[i]), p.scale_log2, -lse2));
+      for (int i = 0; i < 32; ++i) {
+        float e0, e1;
+        split_f32x2(fma_f32x2(bits_f32x2(&raw[i >> 4][(i & 15) * 2]), scale2, nlse2), e0, e1);
+        pf[i] = make_f32x2(ex2(e0), ex2(e1));
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->s_taken);
-      if (p.causal && j == qt) {                                        // diagonal tile: keys after the query
+      // keys that the row does not see: after the query (causal, diagonal tile) or behind the sequence
+      const bool diagonal = p.causal && j == qt;
+      if (diagonal || (j + 1) * TK > p.S) {
+        const int limit = (diagonal ? r + 1 : p.S - j * TK) - col0;
 #pragma unroll
-        for (int k = 0; k < 64; ++k)
-          if (col0 + k > r) pf[k] = 0.f;
-      }
-      if (!mbar_wait(&bars->dp_full, ph)) { ATTN_FAIL(226); break; }
-      tc_fence_after();
-      uint32_t pk[32];
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        uint32_t raw[32];
-        tmem_ld_32x32(t_dp + lane_base + col0 + c * 32, raw);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          const int k = c * 32 + i;
-          const float d0 = pf[k] * (__uint_as_float(raw[i]) - dl) * p.scale;
-          const float d1 = pf[k + 1] * (__uint_as_float(raw[i + 1]) - dl) * p.scale;
-          pk[k >> 1] = pack_bf16(d0, d1);
+        for (int i = 0; i < 32; ++i) {
+          float e0, e1;
+          split_f32x2(pf[i], e0, e1);
+          pf[i] = make_f32x2(2 * i < limit ? e0 : 0.f, 2 * i + 1 < limit ? e1 : 0.f);
         }
       }
-      tmem_st_32x32(t_dp + lane_base + col0, pk);          // dS pairs over the columns just read
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->ds_ready);
-    }
-    if (!*abort_flag && half == 0) {
-      if (!mbar_wait(&bars->acc_done, (n_kv - 1) & 1)) ATTN_FAIL(227);
+      if (!mbar_wait(&bars->dpt_full[half], ph)) { ATTN_FAIL(226); break; }
       tc_fence_after();
-      const size_t token = static_cast<size_t>(row_q + r);
-      __nv_bfloat16* dst = p.dq + token * p.dq_pitch + h * HD;
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        uint32_t a[32];
-        tmem_ld_32x32(t_dq + lane_base + c * 32, a);
-        tmem_ld_wait();
-        if (p.rope_cos) unrotate32(a, p.rope_cos, p.rope_sin, token % static_cast<size_t>(p.S), c * 16);
-        uint4* d4 = reinterpret_cast<uint4*>(dst + c * 32);
+      uint32_t pk[32];
+      tmem_ld_32x32(tp, raw[0]);
+      tmem_ld_32x32(tp + 32, raw[1]);
+      tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          d4[i] = make_uint4(pack_bf16(__uint_as_float(a[8 * i]), __uint_as_float(a[8 * i + 1])),
-                             pack_bf16(__uint_as_float(a[8 * i + 2]), __uint_as_float(a[8 * i + 3])),
-                             pack_bf16(__uint_as_float(a[8 * i + 4]), __uint_as_float(a[8 * i + 5])),
-                             pack_bf16(__uint_as_float(a[8 * i + 6]), __uint_as_float(a[8 * i + 7])));
+      for (int i = 0; i < 32; ++i) {      // dS without the factor 1/sqrt(head_dim): the epilogue applies it
+        float e0, e1;
+        split_f32x2(mul_f32x2(pf[i], add_f32x2(bits_f32x2(&raw[i >> 4][(i & 15) * 2]), ndelta2)), e0, e1);
+        pk[i] = pack_bf16(e0, e1);
       }
+      tmem_st_32x32(tp, pk);              // dS pairs over the columns just read
+      tmem_st_wait();
+      arrive_half(&bars->ds_ready[half], lane);
+    }
+    if (!*abort_flag) {                   // each group stores 64 of the 128 columns
+      if (!mbar_wait(&bars->acc_done, 0)) ATTN_FAIL(227);
+      tc_fence_after();
+      const int pos = qt * TQ + r;
+      store_grad_row<2>(t_dq + lane_base, p.dq + (static_cast<size_t>(b) * p.S + pos) * p.dq_pitch + h * HD, pos, p.S,
+                        p.scale, p.rope_cos, p.rope_sin, 2 * half);
     }
   }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 1) {
-    tc_fence_after();
-    tmem_dealloc(tmem, 512);
-  }
+  bwd_exit(sm, warp, tmem);
 }
 
 // ================================================================= host
-// [tokens, heads*128] bf16 with token pitch ``pitch`` elements; box = [128 tokens, 64 columns].
+// [B, S, heads*128] 16-bit elements with token pitch ``pitch`` elements; box = 128 tokens x 64 columns of one batch
+// entry (tokens behind the sequence are out of bounds, so they read as zeros instead of the next entry's rows).
 static int g_last_encode_result = 0;     // CUresult of the last tensor-map encode that failed (diagnostics)
 
-static int attn_map(CUtensorMap* map, const void* base, long long tokens, int heads, long long pitch) {
+static int attn_map(CUtensorMap* map, const void* base, int B, int S, int heads, long long pitch, bool f16 = false) {
   EncodeTiledFn fn = encode_fn();      // binds this thread's context first (tensormap.cuh)
   if (!fn) return -1;
-  cuuint64_t dims[2] = {static_cast<cuuint64_t>(heads) * HD, static_cast<cuuint64_t>(tokens)};
-  cuuint64_t strides[1] = {static_cast<cuuint64_t>(pitch) * 2};
-  cuuint32_t box[2] = {64, 128};
-  cuuint32_t estr[2] = {1, 1};
-  const CUresult rc = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  cuuint64_t dims[3] = {static_cast<cuuint64_t>(heads) * HD, static_cast<cuuint64_t>(S), static_cast<cuuint64_t>(B)};
+  cuuint64_t strides[2] = {static_cast<cuuint64_t>(pitch) * 2, static_cast<cuuint64_t>(pitch) * 2 * S};
+  cuuint32_t box[3] = {64, 128, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult rc = fn(map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3,
+                         const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (rc != CUDA_SUCCESS) g_last_encode_result = static_cast<int>(rc);
   return rc == CUDA_SUCCESS ? 0 : -2;
 }
 
-constexpr int FWD_SMEM = 5 * TILE_BYTES + 1024 + 6 * TQ * 4 + 512;
-constexpr int BWD_SMEM = 6 * TILE_BYTES + 1024 + 512;
+// Heads per launch-order set: as many as keep the tensors that their CTAs read again and again (``bytes_per_head``)
+// inside 48 MB of the 126 MB L2; the longest tiles of the whole set start first.
+static int heads_per_set(int heads, long long bytes_per_head) {
+  const long long fit = (48LL << 20) / (bytes_per_head > 0 ? bytes_per_head : 1);
+  return static_cast<int>(fit < 1 ? 1 : (fit > heads ? heads : fit));
+}
+
+// The dynamic windows start 1024-byte aligned (the kernels have no static shared memory).
+constexpr int FWD_SMEM = 6 * TILE_BYTES + 512;
+constexpr int BWD_SMEM = sizeof(BwdSmem);
+static_assert(BWD_SMEM <= 227 * 1024, "shared memory of a backward CTA");
+
+template <int F16>
+static int launch_fwd(const AttnParams& p, long long ctas, cudaStream_t stream) {
+  static bool set = false;
+  if (!set) {
+    if (cudaFuncSetAttribute(attn_fwd_kernel<F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM) != cudaSuccess)
+      return -3;
+    set = true;
+  }
+  attn_fwd_kernel<F16><<<static_cast<unsigned>(ctas), ATTN_THREADS, FWD_SMEM, stream>>>(p);
+  return cudaGetLastError() == cudaSuccess ? 0 : -4;
+}
 
 }  // namespace b2
 
@@ -799,72 +945,54 @@ extern "C" {
 // After an entry point returned -11 (a tensor map could not be encoded): the driver's result code of that encode.
 int b2_attention_last_encode_result() { return g_last_encode_result; }
 
-// q: [B,S,Hq,128], k, v: [B,S,Hkv,128] bf16 with token pitches (elements); out [B,S,Hq,128] contiguous; lse [B,Hq,S].
+// q: [B,S,Hq,128], k, v: [B,S,Hkv,128] with token pitches (elements), bf16 or (f16 != 0) fp16; out [B,S,Hq,128]
+// contiguous in the same type; lse [B,Hq,S].
 int b2_attention_fwd_ex(const void* q, const void* k, const void* v, long long q_pitch, long long k_pitch,
                         long long v_pitch, void* out, float* lse, int B, int S, int Hq, int Hkv, float scale,
-                        int causal, int* status, cudaStream_t stream) {
-  if (S % 128 || Hq % Hkv || q_pitch % 8 || k_pitch % 8 || v_pitch % 8) return -10;
+                        int causal, int f16, int* status, cudaStream_t stream) {
+  if (S < 1 || B < 1 || Hkv < 1 || Hq % Hkv || q_pitch % 8 || k_pitch % 8 || v_pitch % 8) return -10;
   AttnParams p{};
-  const long long tokens = static_cast<long long>(B) * S;
-  if (attn_map(&p.map_q, q, tokens, Hq, q_pitch) || attn_map(&p.map_k, k, tokens, Hkv, k_pitch) ||
-      attn_map(&p.map_v, v, tokens, Hkv, v_pitch))
-    return -11;
+  if (attn_map(&p.map_q, q, B, S, Hq, q_pitch, f16 != 0)) return -11;
+  if (attn_map(&p.map_k, k, B, S, Hkv, k_pitch, f16 != 0)) return -12;
+  if (attn_map(&p.map_v, v, B, S, Hkv, v_pitch, f16 != 0)) return -13;
   p.B = B; p.S = S; p.Hq = Hq; p.Hkv = Hkv; p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
   p.causal = causal != 0;
-  p.out = static_cast<__nv_bfloat16*>(out); p.lse = lse; p.status = status;
-  static bool set = false;
-  if (!set) {
-    if (cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM) != cudaSuccess)
-      return -3;
-    set = true;
-  }
-  attn_fwd_kernel<<<dim3(S / TQ, Hq, B), ATTN_BWD_THREADS, FWD_SMEM, stream>>>(p);
-  return cudaGetLastError() == cudaSuccess ? 0 : -4;
+  p.set_heads = heads_per_set(B * Hq, 4LL * S * HD * Hkv / Hq);
+  p.out = out; p.lse = lse; p.status = status;
+  const long long tiles = (S + TQ - 1) / TQ;
+  const long long ctas = (tiles + 1) / 2 * B * Hq;
+  if (ctas > 0x7fffffffLL) return -10;
+  return f16 ? launch_fwd<1>(p, ctas, stream) : launch_fwd<0>(p, ctas, stream);
 }
 
 // Causal form (the one the model uses).
 int b2_attention_fwd(const void* q, const void* k, const void* v, long long q_pitch, long long k_pitch,
                      long long v_pitch, void* out, float* lse, int B, int S, int Hq, int Hkv, float scale, int* status,
                      cudaStream_t stream) {
-  return b2_attention_fwd_ex(q, k, v, q_pitch, k_pitch, v_pitch, out, lse, B, S, Hq, Hkv, scale, 1, status, stream);
+  return b2_attention_fwd_ex(q, k, v, q_pitch, k_pitch, v_pitch, out, lse, B, S, Hq, Hkv, scale, 1, 0, status, stream);
 }
 
+// Gradients.  dout, out: [B,S,Hq,128] contiguous; stats: fp32 scratch [B*Hq, 2, Sp] with Sp = S rounded up to 128; dq
+// [B,S,Hq,128], dk, dv [B,S,Hkv,128] with token pitches dq_pitch, dk_pitch, dv_pitch (they may be views into one fused
+// gradient buffer).  With rotary tables (fp32 [S, 64]) q and k are the ROTATED tensors the forward pass saw, and dq, dk
+// are stored rotated back, i.e. as gradients of the unrotated projections.
 int b2_attention_bwd_rope(const void* dout, const void* q, const void* k, const void* v, const void* out,
-                          const float* lse, long long q_pitch, long long k_pitch, long long v_pitch, float* delta,
-                          void* dq, void* dk, void* dv, long long dq_pitch, long long dk_pitch, long long dv_pitch,
-                          int B, int S, int Hq, int Hkv, float scale, int causal, const float* rope_cos,
-                          const float* rope_sin, int* status, cudaStream_t stream);
-
-// dout, out: [B,S,Hq,128] contiguous; delta: fp32 [B,Hq,S] scratch; dq [B,S,Hq,128], dk, dv [B,S,Hkv,128] with
-// token pitches dq_pitch, dk_pitch, dv_pitch (they may be views into one fused gradient buffer).
-int b2_attention_bwd_ex(const void* dout, const void* q, const void* k, const void* v, const void* out,
-                        const float* lse, long long q_pitch, long long k_pitch, long long v_pitch, float* delta,
-                        void* dq, void* dk, void* dv, long long dq_pitch, long long dk_pitch, long long dv_pitch,
-                        int B, int S, int Hq, int Hkv, float scale, int causal, int* status, cudaStream_t stream) {
-  return b2_attention_bwd_rope(dout, q, k, v, out, lse, q_pitch, k_pitch, v_pitch, delta, dq, dk, dv, dq_pitch,
-                               dk_pitch, dv_pitch, B, S, Hq, Hkv, scale, causal, nullptr, nullptr, status, stream);
-}
-
-// The same with optional rotary tables (fp32 [S, 64]): q and k are the ROTATED tensors the forward pass saw, and dq,
-// dk are stored rotated back, i.e. as gradients of the unrotated projections.
-int b2_attention_bwd_rope(const void* dout, const void* q, const void* k, const void* v, const void* out,
-                          const float* lse, long long q_pitch, long long k_pitch, long long v_pitch, float* delta,
+                          const float* lse, long long q_pitch, long long k_pitch, long long v_pitch, float* stats,
                           void* dq, void* dk, void* dv, long long dq_pitch, long long dk_pitch, long long dv_pitch,
                           int B, int S, int Hq, int Hkv, float scale, int causal, const float* rope_cos,
                           const float* rope_sin, int* status, cudaStream_t stream) {
-  if (S % 128 || Hq % Hkv) return -10;
+  if (S < 1 || B < 1 || Hkv < 1 || Hq % Hkv) return -10;
   AttnParams p{};
-  const long long tokens = static_cast<long long>(B) * S;
   // -11 / -12 / -13 / -14: the tensor map of q / k / v / dout could not be encoded (base not 16-byte aligned, pitch
   // not a multiple of 8 elements, ...); b2_attention_last_encode_result() has the driver's code
   if (q_pitch % 8 || k_pitch % 8 || v_pitch % 8) return -10;
-  if (attn_map(&p.map_q, q, tokens, Hq, q_pitch)) return -11;
-  if (attn_map(&p.map_k, k, tokens, Hkv, k_pitch)) return -12;
-  if (attn_map(&p.map_v, v, tokens, Hkv, v_pitch)) return -13;
-  if (attn_map(&p.map_do, dout, tokens, Hq, static_cast<long long>(Hq) * HD)) return -14;
+  if (attn_map(&p.map_q, q, B, S, Hq, q_pitch)) return -11;
+  if (attn_map(&p.map_k, k, B, S, Hkv, k_pitch)) return -12;
+  if (attn_map(&p.map_v, v, B, S, Hkv, v_pitch)) return -13;
+  if (attn_map(&p.map_do, dout, B, S, Hq, static_cast<long long>(Hq) * HD)) return -14;
   p.B = B; p.S = S; p.Hq = Hq; p.Hkv = Hkv; p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
   p.causal = causal != 0;
-  p.lse = const_cast<float*>(lse); p.delta = delta; p.dq = static_cast<__nv_bfloat16*>(dq);
+  p.stats = stats; p.dq = static_cast<__nv_bfloat16*>(dq);
   p.dk = static_cast<__nv_bfloat16*>(dk); p.dv = static_cast<__nv_bfloat16*>(dv); p.status = status;
   p.dq_pitch = dq_pitch; p.dk_pitch = dk_pitch; p.dv_pitch = dv_pitch;
   p.rope_cos = rope_cos; p.rope_sin = rope_sin;
@@ -875,20 +1003,16 @@ int b2_attention_bwd_rope(const void* dout, const void* q, const void* k, const 
       return -3;
     set = true;
   }
-  const long long warps = tokens * Hq;
-  attn_delta_kernel<<<static_cast<unsigned>((warps * 32 + 255) / 256), 256, 0, stream>>>(
-      static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(out), delta, B, S, Hq);
-  attn_bwd_dkv_kernel<<<dim3(S / TK, Hkv, B), ATTN_BWD_THREADS, BWD_SMEM, stream>>>(p);
-  attn_bwd_dq_kernel<<<dim3(S / TQ, Hq, B), ATTN_BWD_THREADS, BWD_SMEM, stream>>>(p);
+  const long long tiles = (S + TQ - 1) / TQ, Sp = tiles * TQ;
+  if (Sp / 16 * B * Hq > 0x7fffffffLL) return -10;
+  attn_stats_kernel<<<static_cast<unsigned>(Sp / 16 * B * Hq), 256, 0, stream>>>(
+      static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(out), lse, stats, S,
+      static_cast<int>(Sp), Hq);
+  p.set_heads = heads_per_set(B * Hkv, 4LL * S * HD * (Hq / Hkv));
+  attn_bwd_dkv_kernel<<<static_cast<unsigned>(tiles * B * Hkv), ATTN_THREADS, BWD_SMEM, stream>>>(p);
+  p.set_heads = heads_per_set(B * Hq, 4LL * S * HD * Hkv / Hq);
+  attn_bwd_dq_kernel<<<static_cast<unsigned>(tiles * B * Hq), ATTN_THREADS, BWD_SMEM, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
-}
-
-int b2_attention_bwd(const void* dout, const void* q, const void* k, const void* v, const void* out, const float* lse,
-                     long long q_pitch, long long k_pitch, long long v_pitch, float* delta, void* dq, void* dk,
-                     void* dv, long long dq_pitch, long long dk_pitch, long long dv_pitch, int B, int S, int Hq,
-                     int Hkv, float scale, int* status, cudaStream_t stream) {
-  return b2_attention_bwd_ex(dout, q, k, v, out, lse, q_pitch, k_pitch, v_pitch, delta, dq, dk, dv, dq_pitch, dk_pitch,
-                             dv_pitch, B, S, Hq, Hkv, scale, 1, status, stream);
 }
 
 }  // extern "C"

@@ -158,7 +158,7 @@ class MultiHeadLayerLL(nn.Module):
             from ..ops.attention import attention_backend, fused_qkv_attention
             x2d = x.reshape(batch * seq, -1)
             if (token_positions is None and mask is None and ops.use_native(x2d, "attention")
-                    and attention_backend() == "native" and hd == 128 and seq % 128 == 0):
+                    and attention_backend() == "native" and hd == 128):
                 # RoPE rides in the projection GEMM's epilogue (forward) and in the attention backward kernels'
                 # epilogues (its transpose), so q and k are never re-read just to be rotated
                 cos, sin = (self.RoPE.cos, self.RoPE.sin) if self.use_rope else (None, None)

@@ -18,16 +18,54 @@ def _native():
     return native
 
 
+def _eager(*tensors) -> bool:
+    """Plain tensors outside every transformation that looks through PyTorch operations (vmap and the other function
+    transforms, forward-mode differentiation, tracing) or changes their types (autocast to another one)."""
+    from torch.autograd import forward_ad
+    return (all(type(t) in (torch.Tensor, torch.nn.Parameter) for t in tensors)
+            and not torch._C._are_functorch_transforms_active() and forward_ad._current_level < 0
+            and not torch.compiler.is_compiling() and not torch.jit.is_tracing()
+            and not (torch.is_autocast_enabled("cuda") and torch.get_autocast_dtype("cuda") != torch.bfloat16))
+
+
+def _ragged_ok(q, k, v, cos=None, sin=None) -> bool:
+    """Whether the kernels take a sequence that is no multiple of 128 (their last tile is masked).  Everything that the
+    PyTorch formula accepts beyond that stays with it: other types, head sizes, layouts, key lengths, and tables of
+    other shapes."""
+    if not (_eager(q, k, v) and q.dtype == k.dtype == v.dtype == torch.bfloat16 and q.dim() == k.dim() == 4
+            and k.shape == v.shape and q.shape[:2] == k.shape[:2] and q.shape[3] == k.shape[3] == 128
+            and k.device == v.device == q.device and min(q.numel(), k.numel()) > 0
+            and q.shape[2] % k.shape[2] == 0):
+        return False
+    tables = (cos is None) == (sin is None) and all(
+        t is None or (_eager(t) and t.dim() == 2 and t.dtype == torch.float32 and t.shape[1] == 64
+                      and t.shape[0] >= q.shape[1] and t.is_contiguous() and t.data_ptr() % 16 == 0
+                      and t.device == q.device and not t.requires_grad) for t in (cos, sin))
+    return tables and all(_native()._pitched(t) for t in (q, k, v))
+
+
+def _second_order(q, k, v, dout, cos, sin, causal):
+    """Gradients as differentiable functions of the inputs (``create_graph=True``), through the PyTorch formula; for
+    the sequences that only came to the kernels when these learnt to mask their last tile."""
+    out = Fn.attention_ref(q, k, v, cos, sin, causal=causal)
+    wanted = [t for t in (q, k, v) if t.requires_grad]
+    grads = iter(torch.autograd.grad(out, wanted, dout, create_graph=True))
+    return tuple(next(grads) if t.requires_grad else None for t in (q, k, v))
+
+
 class _RopeAttention(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, cos, sin):
         out, lse, q_rot, k_rot = _native().attention_fwd(q, k, v, cos, sin)
-        ctx.save_for_backward(q_rot, k_rot, v, out, lse, cos, sin)
+        ctx.ragged = q.shape[1] % 128 != 0
+        ctx.save_for_backward(q_rot, k_rot, v, out, lse, cos, sin, *((q, k) if ctx.ragged else ()))
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        q_rot, k_rot, v, out, lse, cos, sin = ctx.saved_tensors
+        q_rot, k_rot, v, out, lse, cos, sin, *inputs = ctx.saved_tensors
+        if ctx.ragged and torch.is_grad_enabled():
+            return (*_second_order(*inputs, v, dout, cos, sin, True), None, None)
         dq, dk, dv = _native().attention_bwd(dout.contiguous(), q_rot, k_rot, v, out, lse, cos, sin)
         return dq, dk, dv, None, None
 
@@ -113,7 +151,8 @@ def rope_attention(q, k, v, cos, sin):
     """Returns ``[B, S, Hq, head_dim]``.  ``cos``/``sin`` are ``[S_max, hd/2]``
     fp32 tables or ``None`` for no rotation."""
     from . import use_native
-    if use_native(q, "attention") and attention_backend() == "native" and q.shape[-1] == 128 and q.shape[1] % 128 == 0:
+    if use_native(q, "attention") and attention_backend() == "native" and q.shape[-1] == 128 and (
+            q.shape[1] % 128 == 0 or _ragged_ok(q, k, v, cos, sin)):
         return _RopeAttention.apply(q, k, v, cos, sin)
     if q.is_cuda:
         # library attention on the GPU (A/B baseline only)
@@ -140,8 +179,15 @@ class _PlainAttention(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout):
         q, k, v, out, lse = ctx.saved_tensors
+        if q.shape[1] % 128 and torch.is_grad_enabled():
+            return (*_second_order(q, k, v, dout, None, None, ctx.causal), None)
         dq, dk, dv = _native().attention_bwd(dout, q, k, v, out, lse, causal=ctx.causal)
         return dq, dk, dv, None
+
+
+def _native_attention(q) -> bool:
+    from . import use_native
+    return use_native(q, "attention") and q.dim() == 4
 
 
 def _native_shape_ok(q, k) -> bool:
@@ -152,8 +198,9 @@ def _native_shape_ok(q, k) -> bool:
 
 def attention(q, k, v, causal: bool = True):
     """Differentiable attention on ``[B, S, H, hd]`` tensors (``Hq`` a multiple of ``Hkv``); no rotation.  Runs the
-    tcgen05 kernels for bf16, head_dim 128, ``S % 128 == 0`` on a GPU and the PyTorch formula otherwise."""
-    if _native_shape_ok(q, k):
+    tcgen05 kernels for bf16 and head_dim 128 on a GPU (any ``S``, see ``_ragged_ok``) and the PyTorch formula
+    otherwise."""
+    if _native_shape_ok(q, k) or (_native_attention(q) and q.shape[1] % 128 and _ragged_ok(q, k, v)):
         return _PlainAttention.apply(q, k, v, bool(causal))
     return Fn.attention_ref(q, k, v, causal=causal)
 
@@ -163,11 +210,17 @@ def flash_attention_forward(q, k, v, causal: bool = False):
     entry point of the reference's hand-written kernel (implementation/kernels/flash_attention.cu:390-448, fp16,
     ``mma.sync``/``wmma``, 32 queries per CTA).  Here every (batch, head) pair is a batch entry of the tcgen05
     forward kernel with one head — ``[B, H, S, 128]`` is read in place as ``[B·H, S, 1, 128]`` — so no transposed
-    copy is made.  fp16 inputs are computed in bf16 and returned as fp16; shapes the kernel does not cover
-    (head_dim ≠ 128, ``S % 128 ≠ 0``, CPU) take the PyTorch formula, like the reference's scalar fallback kernel."""
+    copy is made.  The kernel exists for both types (fp16 inputs went through bf16 before: three casts in, one out, 8
+    bits of mantissa instead of 11); shapes it does not cover (head_dim ≠ 128, ``S % 128 ≠ 0``, CPU) take the PyTorch formula, like the reference's scalar fallback kernel."""
     B, H, S, hd = q.shape
     want = q.dtype
     if q.is_cuda and want in (torch.float16, torch.bfloat16):
+        if (want == k.dtype == v.dtype == torch.float16 and _native_attention(q) and _eager(q, k, v) and hd == 128
+                and S % 128 == 0):
+            heads = [t.contiguous().view(B * H, S, 1, hd) for t in (q, k, v)]
+            if all(t.data_ptr() % 16 == 0 for t in heads):
+                with torch.no_grad():
+                    return _native().attention_fwd(*heads, None, None, causal=causal)[0].view(B, H, S, hd)
         q, k, v = (t.to(torch.bfloat16).contiguous().view(B * H, S, 1, hd) for t in (q, k, v))
         if _native_shape_ok(q, k):
             with torch.no_grad():

@@ -504,21 +504,34 @@ def _token_pitch(t):
     return t.stride(1)
 
 
+def _pitched(t) -> bool:
+    """``[B, S, H, 128]`` with contiguous heads, one token pitch throughout, and the alignment that 16-byte vectors and
+    tensor maps need."""
+    S, H, hd = t.shape[1:]
+    return (hd == 128 and t.stride(3) == 1 and t.stride(2) == hd and t.stride(0) == S * t.stride(1)
+            and t.stride(1) >= H * hd and t.stride(1) % 8 == 0 and t.data_ptr() % 16 == 0)
+
+
 def attention_fwd(q, k, v, cos=None, sin=None, causal=True):
     """GQA attention, causal by default.  ``q [B,S,Hq,128]``, ``k, v [B,S,Hkv,128]`` bf16 (views of a fused projection are
-    fine).  With ``cos``/``sin`` the rotation is applied to copies of q and k first.  Returns
-    ``(out [B,S,Hq,128], lse fp32 [B,Hq,S], q_used, k_used)``."""
+    fine), or all three fp16 without a rotation; any ``S``.  With ``cos``/``sin`` (fp32 ``[>= S, 64]``) rotated copies of
+    q and k are made first.  Returns ``(out [B,S,Hq,128], lse fp32 [B,Hq,S], q_used, k_used)``."""
     B, S, Hq, hd = q.shape
     Hkv = k.shape[2]
+    f16 = q.dtype == k.dtype == v.dtype == torch.float16 and cos is None
     if cos is not None:
-        q, k = q.contiguous().clone(), k.contiguous().clone()
-        rope_inplace(q, 0, B * S, S, Hq, hd, Hq * hd, cos, sin, 1.0)
-        rope_inplace(k, 0, B * S, S, Hkv, hd, Hkv * hd, cos, sin, 1.0)
-    out = torch.empty(B, S, Hq, hd, dtype=torch.bfloat16, device=q.device)
+        q, k = (t if _pitched(_bf16(t)) else t.clone(memory_format=torch.contiguous_format) for t in (q, k))
+        qr, kr = (torch.empty(t.shape, dtype=torch.bfloat16, device=t.device) for t in (q, k))
+        _call("b2_rope_copy", _p(q), _p(k), _p(qr), _p(kr), _p(cos), _p(sin), _I(B * S), _I(S), _I(Hq), _I(Hkv),
+              _L(_token_pitch(q)), _L(_token_pitch(k)), _stream())
+        q, k = qr, kr
+    if not f16:
+        _bf16(q), _bf16(k), _bf16(v)
+    out = torch.empty(B, S, Hq, hd, dtype=q.dtype, device=q.device)
     lse = torch.empty(B, Hq, S, dtype=torch.float32, device=q.device)
-    _call("b2_attention_fwd_ex", _p(_bf16(q)), _p(_bf16(k)), _p(_bf16(v)), _L(_token_pitch(q)), _L(_token_pitch(k)),
+    _call("b2_attention_fwd_ex", _p(q), _p(k), _p(v), _L(_token_pitch(q)), _L(_token_pitch(k)),
           _L(_token_pitch(v)), _p(out), _p(lse), _I(B), _I(S), _I(Hq), _I(Hkv), _F(hd ** -0.5), _I(int(causal)),
-          _p(status_word(q.device)), _stream())
+          _I(int(f16)), _p(status_word(q.device)), _stream())
     return out, lse, q, k
 
 
@@ -534,12 +547,13 @@ def attention_bwd(dout, q, k, v, out, lse, cos=None, sin=None, grads=None, causa
                  torch.empty(B, S, Hkv, hd, dtype=torch.bfloat16, device=q.device),
                  torch.empty(B, S, Hkv, hd, dtype=torch.bfloat16, device=q.device))
     dq, dk, dv = grads
-    delta = torch.empty(B, Hq, S, dtype=torch.float32, device=q.device)
+    # per query row -lse*log2(e) and -rowsum(dO*O), rows padded to whole tiles
+    stats = torch.empty(B * Hq, 2, (S + 127) // 128 * 128, dtype=torch.float32, device=q.device)
     dout = _bf16(dout).contiguous()
     if cos is not None and (cos.shape[-1] != 64 or not cos.is_contiguous() or cos.shape[0] < S):
         raise ValueError("rotary tables must be contiguous fp32 [>= S, 64]")
     _call("b2_attention_bwd_rope", _p(dout), _p(q), _p(k), _p(v), _p(_bf16(out)), _p(lse), _L(_token_pitch(q)),
-          _L(_token_pitch(k)), _L(_token_pitch(v)), _p(delta), _p(dq), _p(dk), _p(dv), _L(_token_pitch(dq)),
+          _L(_token_pitch(k)), _L(_token_pitch(v)), _p(stats), _p(dq), _p(dk), _p(dv), _L(_token_pitch(dq)),
           _L(_token_pitch(dk)), _L(_token_pitch(dv)), _I(B), _I(S), _I(Hq), _I(Hkv), _F(hd ** -0.5),
           _I(int(causal)), _p(cos), _p(sin), _p(status_word(q.device)), _stream(), n=3)
     return dq, dk, dv

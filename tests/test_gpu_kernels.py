@@ -449,6 +449,65 @@ def test_attention_non_causal(native, B, S, Hq, Hkv):
     native.check_status()
 
 
+@pytest.mark.parametrize("S", [1, 100, 127, 129, 257, 387])
+@pytest.mark.parametrize("causal", [True, False])
+def test_attention_of_ragged_sequences(native, S, causal):
+    """Sequences around the 128-row tile edges (one and two query tiles per CTA, a masked last key tile), with rotation
+    where causal.  The second batch entry starts with non-finite rows: the first one's last tile must not read them.
+    Bounds as for whole tiles: bf16 inputs, probabilities and outputs."""
+    from b200moe.ops import functional as Fn, rope_attention
+    from b200moe.ops.attention import attention
+    torch.manual_seed(S)
+    B, Hq, Hkv, hd = 2, 4, 2, 128
+    cos, sin = Fn.rope_tables(10000.0, hd, 512, device="cuda")
+    q, k, v = (_rand(B, S, h, hd) for h in (Hq, Hkv, Hkv))
+    dout = _rand(B, S, Hq, hd)
+    for t in (q, k, v, dout):
+        t[1, 0] = float("inf")
+    leaves = [t.requires_grad_(True) for t in (q, k, v)]
+    before = native.launch_count()
+    out = rope_attention(*leaves, cos, sin) if causal else attention(*leaves, causal=False)
+    out.backward(dout)
+    assert native.launch_count() >= before + 4
+    exact = [t.detach()[:1].double().requires_grad_(True) for t in leaves]
+    heads = [t.transpose(1, 2) for t in exact]
+    if causal:
+        def turn(x):
+            a, b, c, s_ = x[..., 0::2], x[..., 1::2], cos[:S].double(), sin[:S].double()
+            return torch.stack((a * c - b * s_, a * s_ + b * c), -1).flatten(-2)
+        heads[0], heads[1] = turn(heads[0]), turn(heads[1])
+    kh, vh = (t.repeat_interleave(Hq // Hkv, 1) for t in heads[1:])
+    scores = heads[0] @ kh.mT / math.sqrt(hd)
+    if causal:
+        scores = scores.masked_fill(torch.triu(torch.ones(S, S, dtype=torch.bool, device="cuda"), 1), float("-inf"))
+    ref = (scores.softmax(-1) @ vh).transpose(1, 2)
+    ref.backward(dout[:1].double())
+    assert _rel(out[:1], ref) < 1e-2
+    for got, want in zip(leaves, exact):
+        # dq and dk vanish where a row sees one key only: what is left is the rounding of dP - rowsum(dO O)
+        floor = 2e-2 * float(want.grad.norm()) + (1e-2 * math.sqrt(want.numel()) if S == 1 else 0.0)
+        assert float((got.grad[:1].double() - want.grad).norm()) <= floor
+    native.check_status()
+
+
+@pytest.mark.parametrize("S", [128, 384])
+@pytest.mark.parametrize("causal", [True, False])
+def test_flash_attention_in_fp16_keeps_fp16_precision(native, S, causal):
+    """fp16 inputs are multiplied as fp16: against 64 bits the error is that of fp16 probabilities and outputs (2^-11
+    each), which a pass through bf16 (2^-9 per input) cannot reach."""
+    from b200moe.ops.attention import flash_attention_forward
+    torch.manual_seed(S)
+    q, k, v = (torch.randn(2, 3, S, 128, device="cuda").half() for _ in range(3))
+    scores = q.double() @ k.double().mT / math.sqrt(128)
+    if causal:
+        scores = scores.masked_fill(torch.triu(torch.ones(S, S, dtype=torch.bool, device="cuda"), 1), float("-inf"))
+    got = flash_attention_forward(q, k, v, causal=causal)
+    assert got.dtype == torch.float16
+    want = scores.softmax(-1) @ v.double()
+    assert float((got.double() - want).norm() / want.norm()) < 1e-3
+    native.check_status()
+
+
 def test_flash_attention_forward_entry(native):
     """``[B, H, S, 128]`` forward-only entry point, fp16 in and out, against an fp32 softmax(QK^T)V."""
     from b200moe.ops.attention import flash_attention_forward
