@@ -9,10 +9,10 @@
 // SwiGLU epilogue for the gate/up projection and a K-concatenated form for
 // dx = dgate W1 + dup W3.
 //
-// Layout of one CTA (192 threads, one CTA per SM):
+// Layout of one CTA (320 threads, one CTA per SM):
 //   warp 0       TMA producer (one elected lane)
 //   warp 1       tensor-memory allocation, MMA issue (one elected lane)
-//   warps 2..5   epilogue: tcgen05.ld the 128 x BN fp32 tile, convert, store
+//   warps 2..9   epilogue: tcgen05.ld the 128 x BN fp32 tile, convert, store
 // The accumulator is double-buffered in TMEM (2 x 256 columns), so the epilogue
 // of tile i overlaps the main loop of tile i+1.  Shared memory holds a 4-stage
 // ring of {A 128x64, B 256x64} bf16 tiles in the 128-byte-swizzled layout that
@@ -28,7 +28,6 @@ constexpr int BN = 256;
 constexpr int BK = 64;
 constexpr int A_SUB_BYTES = BM * BK * 2;   // 16 KiB per 128-row sub-tile of A
 constexpr int B_BYTES = BN * BK * 2;       // 32 KiB
-constexpr int GEMM_THREADS = 192;
 // MT = 128-row sub-tiles of A per CTA tile.  MT=1: 128x256 tile, 4 stages, accumulator double-buffered in
 // TMEM (epilogue overlaps the next main loop).  MT=2: 256x256 tile (two MMAs per k-step share the B tile in
 // shared memory, a third fewer operand bytes per FLOP), 3 stages, both accumulators fill TMEM.
@@ -44,11 +43,13 @@ template <int MT, int PAIR = 0> struct Cfg {
   static constexpr int NACC = MT == 2 ? 1 : 2;
   static constexpr int TM = PAIR ? 2 : MT;     // 128-row units per output tile
   static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
-  static constexpr int PUSH_STAGING = 4 * 32 * 256;   // EPI_PUSH: 32 rows x 128 bf16 columns per epilogue warp
 };
-template <int EPI, int MT, int PAIR = 0> constexpr int smem_bytes() {
-  return Cfg<MT, PAIR>::SMEM + (EPI == 5 /*EPI_PUSH*/ ? Cfg<MT, PAIR>::PUSH_STAGING : 0);
-}
+// Epilogue: eight warps, each 32 rows of one half of the tile's columns, through 4 KiB of shared memory per warp (see
+// ``staged`` below).  EPI_PUSH: four warps with 8 KiB each, so that a row leaves in pieces of 256 bytes.
+constexpr int EPI_STAGING = 32 * 1024;
+template <int EPI> constexpr int epi_warps() { return EPI == 5 /*EPI_PUSH*/ ? 4 : 8; }
+template <int EPI> constexpr int gemm_threads() { return 64 + 32 * epi_warps<EPI>(); }
+template <int EPI, int MT, int PAIR = 0> constexpr int smem_bytes() { return Cfg<MT, PAIR>::SMEM + EPI_STAGING; }
 constexpr int GROUP_M = 8;
 
 enum Epilogue : int {
@@ -59,6 +60,9 @@ enum Epilogue : int {
   EPI_STORE_F32 = 4,    // D[M,N] fp32 = acc
   EPI_ROPE = 6,         // D[M,N] bf16 = acc with the rotary embedding applied to the leading rope_cols columns
                         // (adjacent pairs, heads of 128 columns, position = row mod rope_seq): the fused q/k/v projection
+  EPI_SWIGLU_BWD = 7,   // acc = dh; with the saved pre-activations g, u of the same element: D[M,2N] = [dg | du], H[M,N] =
+                        // silu(g) u.  Memory traffic of the epilogue: 2 reads and 3 writes of 2 bytes per element, under
+                        // the next tile's main loop; a kernel of its own moved 6 and the GEMM's store of dh a seventh
   EPI_PUSH = 5,         // expert-parallel return: row r, scaled by push_w[r], is stored as bf16 into row push_tag[r]
                         // of rank push_src[r]'s buffer through its peer pointer; the last CTA raises a flag
 };
@@ -83,6 +87,7 @@ struct GemmParams {
   void* d;                     // output
   void* d_gate;                // optional gate pre-activation (SwiGLU)
   void* d_up;                  // optional up pre-activation (SwiGLU)
+  void* h;                     // EPI_SWIGLU_BWD: [M, N]; d_gate and d_up are inputs there
   long long ldd;               // leading dimension of d (elements)
   long long d_expert_stride;   // elements between experts in d (SCHED_WGRAD)
   float beta;                  // 1 accumulate, 0 overwrite (EPI_ACC_*)
@@ -139,7 +144,7 @@ __device__ __forceinline__ TileCoord decode_tile(const GemmParams& p, long long 
 }
 
 template <int A_MN, int B_MN, int EPI, int SCHED, int MT, int PAIR>
-__global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __grid_constant__ GemmParams p) {
+__global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(const __grid_constant__ GemmParams p) {
   static_assert(!PAIR || MT == 1, "a CTA of a pair holds one 128-row sub-tile");
   constexpr int STAGES = Cfg<MT, PAIR>::STAGES;
   constexpr int A_BYTES = Cfg<MT, PAIR>::A_BYTES;
@@ -174,7 +179,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tmem_full[a], 1);
-      mbar_init(&tmem_empty[a], PAIR ? 8 : 4);   // epilogue warps (of both CTAs of a pair)
+      mbar_init(&tmem_empty[a], (PAIR ? 2 : 1) * epi_warps<EPI>());   // epilogue warps (of both CTAs of a pair)
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -329,9 +334,18 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       }
     }
   } else {
-    // ------------------------------------------------------------ epilogue (warps 2..5)
+    // ------------------------------------------------------------ epilogue (warps 2..9; EPI_PUSH: 2..5)
     const int quad = warp & 3;                 // TMEM lane group this warp may read
     const int row_in_tile = quad * 32 + lane;
+    const int half = (warp - 2) >> 2;          // which half of the tile's columns (EPI_PUSH: all of them)
+    // A thread reads one row of the accumulator.  Loads and stores of global memory straight from that layout put 16
+    // bytes per lane at 32 rows into one instruction: half sectors, 32 lines.  Instead each warp passes 32 rows x 32
+    // fp32 columns through shared memory (16-byte units, XOR-swizzled by row: conflict-free both ways), after which
+    // four lanes hold 32 consecutive columns of a row.  Products with a short reduction are bound by this part; before
+    // (four warps, straight stores) and after, us: bf16 store 8192 x 3584 K 1024 60 -> 53, SwiGLU 4096 x 14336 K 4096
+    // 756 -> 711 and 4096 x 1536 K 1024 45 -> 34, fp32 accumulate 4096 x 14336 K 4096 412 -> 375 and K 512 183 -> 130.
+    uint4* const staged = reinterpret_cast<uint4*>(smem + STAGES * STAGE_BYTES + 256) + (warp - 2) * 256;
+    auto swz = [](int r) { return (r & 1) | ((r & 2) << 1) | ((r & 4) >> 1); };
     int acc = 0;
     uint32_t acc_phase = 0;
     for (long long tile = worker; tile < total_tiles && !*abort_flag; tile += num_workers) {
@@ -348,42 +362,51 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       const uint32_t taddr = tmem_base + (MT == 2 ? sub * BN : acc * BN) + (static_cast<uint32_t>(quad * 32) << 16);
       const long long row = static_cast<long long>(t.m_tile) * TILE_M + (PAIR ? static_cast<int>(cta) : sub) * BM + row_in_tile;
       const bool row_ok = row < p.M;
+      const long long row0 = row - lane;
       if (EPI == EPI_SWIGLU) {
+        // 16 gate and 16 up columns at a time; afterwards two lanes per row, eight features each
         __nv_bfloat16* h = reinterpret_cast<__nv_bfloat16*>(p.d);
         const long long half_n = p.N / 2;
         const long long col0 = static_cast<long long>(t.n_tile) * 128;
+        const int q = lane & 1;
 #pragma unroll 1
-        for (int c = 0; c < 128; c += 32) {
-          uint32_t g[32], u[32];
-          tmem_ld_32x32(taddr + c, g);
-          tmem_ld_32x32(taddr + 128 + c, u);
+        for (int c = half * 64; c < half * 64 + 64; c += 16) {
+          uint32_t g[16], u[16];
+          tmem_ld_32x16(taddr + c, g);
+          tmem_ld_32x16(taddr + 128 + c, u);
           tmem_ld_wait();
-          if (row_ok && col0 + c < half_n) {
-            uint32_t out[16], og[16], ou[16];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const float g0 = __uint_as_float(g[2 * i]), g1 = __uint_as_float(g[2 * i + 1]);
-              const float u0 = __uint_as_float(u[2 * i]), u1 = __uint_as_float(u[2 * i + 1]);
-              const float h0 = g0 / (1.f + __expf(-g0)) * u0;
-              const float h1 = g1 / (1.f + __expf(-g1)) * u1;
-              out[i] = pack_bf16(h0, h1);
-              og[i] = pack_bf16(g0, g1);
-              ou[i] = pack_bf16(u0, u1);
-            }
-            const long long off = row * half_n + col0 + c;
-            uint4* dst = reinterpret_cast<uint4*>(h + off);
+          for (int i = 0; i < 4; ++i) {
+            staged[lane * 8 + (i ^ swz(lane))] = make_uint4(g[4 * i], g[4 * i + 1], g[4 * i + 2], g[4 * i + 3]);
+            staged[lane * 8 + ((4 + i) ^ swz(lane))] = make_uint4(u[4 * i], u[4 * i + 1], u[4 * i + 2], u[4 * i + 3]);
+          }
+          __syncwarp();
 #pragma unroll
-            for (int i = 0; i < 4; ++i) dst[i] = make_uint4(out[4 * i], out[4 * i + 1], out[4 * i + 2], out[4 * i + 3]);
-            if (p.d_gate) {
-              uint4* dg = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.d_gate) + off);
-              uint4* du = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.d_up) + off);
+          for (int it = 0; it < 2; ++it) {
+            const int r = it * 16 + (lane >> 1);
+            const uint4 ga = staged[r * 8 + ((2 * q) ^ swz(r))], gb = staged[r * 8 + ((2 * q + 1) ^ swz(r))];
+            const uint4 ua = staged[r * 8 + ((4 + 2 * q) ^ swz(r))], ub = staged[r * 8 + ((5 + 2 * q) ^ swz(r))];
+            const uint32_t gw[8] = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, gb.w};
+            const uint32_t uw[8] = {ua.x, ua.y, ua.z, ua.w, ub.x, ub.y, ub.z, ub.w};
+            if (row0 + r < p.M && col0 + c < half_n) {
+              uint32_t out[4], og[4], ou[4];
 #pragma unroll
               for (int i = 0; i < 4; ++i) {
-                dg[i] = make_uint4(og[4 * i], og[4 * i + 1], og[4 * i + 2], og[4 * i + 3]);
-                du[i] = make_uint4(ou[4 * i], ou[4 * i + 1], ou[4 * i + 2], ou[4 * i + 3]);
+                const float g0 = __uint_as_float(gw[2 * i]), g1 = __uint_as_float(gw[2 * i + 1]);
+                const float u0 = __uint_as_float(uw[2 * i]), u1 = __uint_as_float(uw[2 * i + 1]);
+                out[i] = pack_bf16(g0 / (1.f + __expf(-g0)) * u0, g1 / (1.f + __expf(-g1)) * u1);
+                og[i] = pack_bf16(g0, g1);
+                ou[i] = pack_bf16(u0, u1);
+              }
+              const long long off = (row0 + r) * half_n + col0 + c + q * 8;
+              *reinterpret_cast<uint4*>(h + off) = make_uint4(out[0], out[1], out[2], out[3]);
+              if (p.d_gate) {
+                *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.d_gate) + off) = make_uint4(og[0], og[1], og[2], og[3]);
+                *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.d_up) + off) = make_uint4(ou[0], ou[1], ou[2], ou[3]);
               }
             }
           }
+          __syncwarp();
         }
       } else if (EPI == EPI_PUSH) {
         // Rows leave for other GPUs.  A thread owns one row of the accumulator, so storing straight from registers
@@ -434,8 +457,37 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
       } else {
         const long long col_base = static_cast<long long>(t.n_tile) * BN;
         const long long expert_off = SCHED == SCHED_WGRAD ? t.expert * p.d_expert_stride : 0;
+        const int q = lane & 3;
+        const bool add = (EPI == EPI_ACC_F32 || EPI == EPI_ACC_BF16) && p.beta != 0.f;
 #pragma unroll 1
-        for (int c = 0; c < BN; c += 32) {
+        for (int c = half * 128; c < half * 128 + 128; c += 32) {
+          const long long col = col_base + c + q * 8;     // N is a multiple of 32 (checked on the host)
+          if (col_base + c >= p.N) break;
+          // what the epilogue reads from global memory, all of the chunk in flight before the accumulator arrives
+          constexpr int OLD = EPI == EPI_ACC_BF16 ? 1 : (EPI == EPI_ACC_F32 || EPI == EPI_ROPE || EPI == EPI_SWIGLU_BWD) ? 2 : 0;
+          uint4 old[4][OLD ? OLD : 1];
+          if (OLD) {
+#pragma unroll
+            for (int it = 0; it < 4; ++it) {
+              const long long rr = row0 + it * 8 + (lane >> 2);
+              if (rr >= p.M) continue;
+              const long long off = expert_off + rr * p.ldd + col;
+              if (EPI == EPI_ACC_F32 && add) {
+                old[it][0] = reinterpret_cast<const uint4*>(reinterpret_cast<const float*>(p.d) + off)[0];
+                old[it][OLD - 1] = reinterpret_cast<const uint4*>(reinterpret_cast<const float*>(p.d) + off)[1];
+              } else if (EPI == EPI_ACC_BF16 && add) {
+                old[it][0] = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.d) + off);
+              } else if (EPI == EPI_ROPE && col < p.rope_cols) {
+                // four adjacent pairs (2j, 2j+1) of a head: table entries [position][(col mod 128)/2 + j]
+                const size_t tab = static_cast<size_t>(static_cast<int>(rr) % p.rope_seq) * 64 + ((col & 127) >> 1);
+                old[it][0] = *reinterpret_cast<const uint4*>(p.rope_cos + tab);
+                old[it][OLD - 1] = *reinterpret_cast<const uint4*>(p.rope_sin + tab);
+              } else if (EPI == EPI_SWIGLU_BWD) {
+                old[it][0] = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.d_gate) + rr * p.N + col);
+                old[it][OLD - 1] = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.d_up) + rr * p.N + col);
+              }
+            }
+          }
           uint32_t v[32];
           if (!empty_k) {
             tmem_ld_32x32(taddr + c, v);
@@ -444,84 +496,72 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tcgen05_kernel(const __g
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = 0;
           }
-          const long long col = col_base + c;
-          if (!row_ok || col >= p.N) continue;   // N is a multiple of 32 (checked on the host)
-          const long long off = expert_off + row * p.ldd + col;
-          if (EPI == EPI_ROPE) {
-            if (col < p.rope_cols) {
-              // 32 consecutive columns of one head: pairs (2j, 2j+1), table entries [pos][(col mod 128)/2 + j]
-              const size_t tab = static_cast<size_t>(row % p.rope_seq) * 64 + ((col & 127) >> 1);
-              const float4* c4 = reinterpret_cast<const float4*>(p.rope_cos + tab);
-              const float4* s4 = reinterpret_cast<const float4*>(p.rope_sin + tab);
 #pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                const float4 cc = c4[q], ss = s4[q];
-                const float cv[4] = {cc.x, cc.y, cc.z, cc.w}, sv[4] = {ss.x, ss.y, ss.z, ss.w};
+          for (int i = 0; i < 8; ++i)
+            staged[lane * 8 + (i ^ swz(lane))] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+          __syncwarp();
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  const float x0 = __uint_as_float(v[8 * q + 2 * j]), x1 = __uint_as_float(v[8 * q + 2 * j + 1]);
-                  v[8 * q + 2 * j] = __float_as_uint(x0 * cv[j] - x1 * sv[j]);
-                  v[8 * q + 2 * j + 1] = __float_as_uint(x0 * sv[j] + x1 * cv[j]);
+          for (int it = 0; it < 4; ++it) {
+            const int r = it * 8 + (lane >> 2);
+            const uint4 a = staged[r * 8 + ((2 * q) ^ swz(r))], b = staged[r * 8 + ((2 * q + 1) ^ swz(r))];
+            float x[8] = {__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z), __uint_as_float(a.w),
+                          __uint_as_float(b.x), __uint_as_float(b.y), __uint_as_float(b.z), __uint_as_float(b.w)};
+            const uint4 o0 = old[it][0], o1 = old[it][OLD ? OLD - 1 : 0];
+            const uint32_t w0[4] = {o0.x, o0.y, o0.z, o0.w}, w1[4] = {o1.x, o1.y, o1.z, o1.w};
+            if (row0 + r >= p.M) continue;
+            const long long off = expert_off + (row0 + r) * p.ldd + col;
+            if (EPI == EPI_ACC_F32 || EPI == EPI_STORE_F32) {
+              if (add) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                  x[i] += __uint_as_float(w0[i]);
+                  x[4 + i] += __uint_as_float(w1[i]);
                 }
               }
-            }
-            uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.d) + off);
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              dst[i] = make_uint4(pack_bf16(__uint_as_float(v[8 * i]), __uint_as_float(v[8 * i + 1])),
-                                  pack_bf16(__uint_as_float(v[8 * i + 2]), __uint_as_float(v[8 * i + 3])),
-                                  pack_bf16(__uint_as_float(v[8 * i + 4]), __uint_as_float(v[8 * i + 5])),
-                                  pack_bf16(__uint_as_float(v[8 * i + 6]), __uint_as_float(v[8 * i + 7])));
-          } else if (EPI == EPI_STORE_BF16) {
-            uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.d) + off);
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              dst[i] = make_uint4(pack_bf16(__uint_as_float(v[8 * i]), __uint_as_float(v[8 * i + 1])),
-                                  pack_bf16(__uint_as_float(v[8 * i + 2]), __uint_as_float(v[8 * i + 3])),
-                                  pack_bf16(__uint_as_float(v[8 * i + 4]), __uint_as_float(v[8 * i + 5])),
-                                  pack_bf16(__uint_as_float(v[8 * i + 6]), __uint_as_float(v[8 * i + 7])));
-          } else if (EPI == EPI_ACC_F32 || EPI == EPI_STORE_F32) {
-            float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.d) + off);
-            const bool add = EPI == EPI_ACC_F32 && p.beta != 0.f;
-            float4 old[8];
-            if (add) {
-#pragma unroll
-              for (int i = 0; i < 8; ++i) old[i] = dst[i];
-            }
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              float4 r = make_float4(__uint_as_float(v[4 * i]), __uint_as_float(v[4 * i + 1]),
-                                     __uint_as_float(v[4 * i + 2]), __uint_as_float(v[4 * i + 3]));
-              if (add) {
-                r.x += old[i].x; r.y += old[i].y; r.z += old[i].z; r.w += old[i].w;
-              }
-              dst[i] = r;
-            }
-          } else if (EPI == EPI_ACC_BF16) {
-            uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.d) + off);
-            const bool add = p.beta != 0.f;
-            uint4 old[4];
-            if (add) {
-#pragma unroll
-              for (int i = 0; i < 4; ++i) old[i] = dst[i];
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              uint32_t o[4] = {old[i].x, old[i].y, old[i].z, old[i].w};
-              uint32_t r[4];
+              float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.d) + off);
+              dst[0] = make_float4(x[0], x[1], x[2], x[3]);
+              dst[1] = make_float4(x[4], x[5], x[6], x[7]);
+            } else if (EPI == EPI_SWIGLU_BWD) {
+              uint32_t og[4], ou[4], oh[4];
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
-                float a = __uint_as_float(v[8 * i + 2 * j]), b = __uint_as_float(v[8 * i + 2 * j + 1]);
-                if (add) {
-                  const __nv_bfloat162 prev = *reinterpret_cast<__nv_bfloat162*>(&o[j]);
-                  a += __low2float(prev);
-                  b += __high2float(prev);
-                }
-                r[j] = pack_bf16(a, b);
+                const float2 g = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w0[j]));
+                const float2 u = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w1[j]));
+                const float s0 = 1.f / (1.f + __expf(-g.x)), s1 = 1.f / (1.f + __expf(-g.y));
+                const float l0 = g.x * s0, l1 = g.y * s1;
+                og[j] = pack_bf16(x[2 * j] * u.x * s0 * (1.f + g.x * (1.f - s0)),
+                                  x[2 * j + 1] * u.y * s1 * (1.f + g.y * (1.f - s1)));
+                ou[j] = pack_bf16(x[2 * j] * l0, x[2 * j + 1] * l1);
+                oh[j] = pack_bf16(l0 * u.x, l1 * u.y);
               }
-              dst[i] = make_uint4(r[0], r[1], r[2], r[3]);
+              __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.d) + off;
+              *reinterpret_cast<uint4*>(dst) = make_uint4(og[0], og[1], og[2], og[3]);
+              *reinterpret_cast<uint4*>(dst + p.N) = make_uint4(ou[0], ou[1], ou[2], ou[3]);
+              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.h) + (row0 + r) * p.N + col) =
+                  make_uint4(oh[0], oh[1], oh[2], oh[3]);
+            } else {
+              if (EPI == EPI_ACC_BF16 && add) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  const float2 prev = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w0[j]));
+                  x[2 * j] += prev.x;
+                  x[2 * j + 1] += prev.y;
+                }
+              }
+              if (EPI == EPI_ROPE && col < p.rope_cols) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  const float cv = __uint_as_float(w0[j]), sv = __uint_as_float(w1[j]);
+                  const float x0 = x[2 * j], x1 = x[2 * j + 1];
+                  x[2 * j] = x0 * cv - x1 * sv;
+                  x[2 * j + 1] = x0 * sv + x1 * cv;
+                }
+              }
+              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.d) + off) =
+                  make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
             }
           }
+          __syncwarp();
         }
       }
       }  // sub
@@ -567,7 +607,7 @@ static int launch_mt(const GemmParams& p, int sms, cudaStream_t stream) {
       return -3;
     configured = true;
   }
-  kernel<<<sms, GEMM_THREADS, smem_bytes<EPI, MT>(), stream>>>(p);
+  kernel<<<sms, gemm_threads<EPI>(), smem_bytes<EPI, MT>(), stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
@@ -580,7 +620,7 @@ static int pairs_resident(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, in
   attr->val.clusterDim.x = 2;
   attr->val.clusterDim.y = 1;
   attr->val.clusterDim.z = 1;
-  cfg->blockDim = dim3(GEMM_THREADS);
+  cfg->blockDim = dim3(gemm_threads<EPI>());
   cfg->dynamicSmemBytes = smem_bytes<EPI, 1, 1>();
   cfg->attrs = attr;
   cfg->numAttrs = 1;
@@ -739,6 +779,22 @@ int b2_gemm_nn(const void* a, const void* w, const void* w2, void* d, int M, int
   p.tile_expert = tile_expert; p.num_m_tiles = num_m_tiles; p.d = d; p.ldd = ldd; p.status = status;
   p.group_align256 = group_align256;
   return launch<0, 1, EPI_STORE_BF16, SCHED_FLAT>(p, sm_count(), stream);
+}
+
+// SwiGLU backward of the hidden layer in one launch: dh[M,F] = a[M,K] * w[e][K,F] stays in tensor memory; with the saved
+// pre-activations gate, up [M,F] the epilogue stores dgu[M,2F] = [dh u silu'(g) | dh silu(g)] and h[M,F] = silu(g) u.
+int b2_gemm_nn_swiglu_bwd(const void* a, const void* w, const void* gate, const void* up, void* dgu, void* h, int M,
+                          int F, int K, long long lda, int num_experts, const int* tile_expert, const int* num_m_tiles,
+                          int group_align256, int* status, cudaStream_t stream) {
+  if (F % 32 || K % 64) return -10;
+  GemmParams p{};
+  if (make_map(&p.map_a, a, K, M, lda, BM)) return -11;
+  if (make_map(&p.map_b, w, F, static_cast<long long>(num_experts) * K, F, 64)) return -12;
+  p.M = M; p.N = F; p.K = K; p.num_experts = num_experts; p.b_expert_rows = K;
+  p.tile_expert = tile_expert; p.num_m_tiles = num_m_tiles; p.group_align256 = group_align256;
+  p.d = dgu; p.ldd = 2LL * F; p.h = h; p.d_gate = const_cast<void*>(gate); p.d_up = const_cast<void*>(up);
+  p.status = status;
+  return launch<0, 1, EPI_SWIGLU_BWD, SCHED_FLAT>(p, sm_count(), stream);
 }
 
 // y[M,N] = a[M,K] * w[N,K]^T with the rotary embedding applied to columns [0, rope_cols) in the epilogue: column c

@@ -74,7 +74,7 @@ class _MoEFused(torch.autograd.Function):
         tokens, dim, experts, cap, recompute = ctx.meta_py
         saved = list(ctx.saved_tensors)
         x_perm, y_perm, weights, offs, tile_expert, meta, slot_row, row_slot = saved[:8]
-        tiles, live_rows = meta[0:1], meta[1:2]
+        tiles = meta[0:1]
         dout = dout.contiguous()
         ffn = w1.shape[1]
         if recompute:
@@ -84,9 +84,9 @@ class _MoEFused(torch.autograd.Function):
         dweights = torch.zeros(tokens, 2, dtype=torch.float32, device=dout.device)
         dy_perm = native.moe_gather(dout, row_slot, meta, cap, scale=weights.view(-1), y_perm=y_perm,
                                     dweights=dweights.view(-1))
-        dh = native.gemm_nn(dy_perm, w2, tile_expert=tile_expert, num_m_tiles=tiles, num_experts=experts, align256=True)
-        dgu, h = native.swiglu_bwd(dh, gate, up, live_rows=live_rows)
-        del dh, gate, up
+        dgu, h = native.gemm_nn_swiglu_bwd(dy_perm, w2, gate, up, tile_expert=tile_expert, num_m_tiles=tiles,
+                                           num_experts=experts, align256=True, live_rows=meta[1:2])
+        del gate, up
         dx_perm = native.gemm_nn(dgu, w1, w2=w3, tile_expert=tile_expert, num_m_tiles=tiles, num_experts=experts,
                                  align256=True)
         dw2 = _wgrad(dy_perm, h, w2, offs, experts)
