@@ -69,6 +69,14 @@ def _trunc_normal(shape, std, device=None, dtype=None):
     return tensor.to(dtype) if dtype is not None else tensor
 
 
+def _hooked(module) -> bool:
+    """Whether somebody watches calls of ``module`` (its own or global hooks), so that it has to be called."""
+    from torch.nn.modules import module as m
+    own = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks")
+    return "forward" in module.__dict__ or any(getattr(module, name, None) for name in own) or any(
+        getattr(m, "_global" + name, None) for name in own)
+
+
 class LinearLayer(nn.Module):
     """``y = x Wᵀ`` with ``W [d_out, d_in]``, fp32 master, truncated-normal init
     ``σ = sqrt(2/(d_in+d_out))`` cut at ±3σ, no bias (reference layers.py:55-69)."""
@@ -230,6 +238,12 @@ class PositionWiseFFLayer(nn.Module):
         self.w3 = LinearLayer(d_model, d_ff, device=device)
 
     def forward(self, x):
+        projections = (self.w1, self.w3, self.w2)
+        if all(type(p) is LinearLayer and not _hooked(p) for p in projections):
+            out = ops.swiglu_ffn(x, *(p.compute_weight if p.compute_weight is not None else p.weight
+                                      for p in projections))
+            if out is not None:
+                return out
         gate, up = self.w1(x), self.w3(x)
         return self.w2(Fn.swiglu_ref(gate, up))
 

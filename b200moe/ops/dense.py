@@ -98,6 +98,59 @@ def linear_rope(x: torch.Tensor, weight: torch.Tensor, cos, sin, rope_cols: int,
     return _Linear.apply(x, weight, (cos[:seq].contiguous(), sin[:seq].contiguous(), rope_cols, seq))
 
 
+class _SwiGLUFFN(torch.autograd.Function):
+    """``(silu(x W1ᵀ) · (x W3ᵀ)) W2ᵀ``: gate/up product with the SwiGLU in its epilogue and the down projection; backward:
+    ``dh`` product with the SwiGLU backward in its epilogue, ``dx`` over the concatenated reduction, three weight
+    gradients."""
+
+    @staticmethod
+    def forward(ctx, x, w1, w3, w2):
+        native = _native()
+        x2d = x.reshape(-1, x.shape[-1])
+        keep = any(ctx.needs_input_grad)
+        h, gate, up = native.gemm_swiglu(x2d, w1.unsqueeze(0), w3.unsqueeze(0), save_gate_up=keep)
+        y = native.gemm_nt(h, w2)
+        ctx.weights = (w1, w3, w2)
+        if keep:
+            ctx.save_for_backward(x, gate, up)
+        return y.view(*x.shape[:-1], w2.shape[0])
+
+    @staticmethod
+    def backward(ctx, dy):
+        native = _native()
+        x, gate, up = ctx.saved_tensors
+        w1, w3, w2 = ctx.weights
+        x2d, ffn = x.reshape(-1, x.shape[-1]), w1.shape[0]
+        dy2d = dy.reshape(-1, dy.shape[-1]).contiguous()
+        dgu, h = native.gemm_nn_swiglu_bwd(dy2d, w2, gate, up)
+        dx = native.gemm_nn(dgu, w1, w2=w3).view_as(x) if ctx.needs_input_grad[0] else None
+        grads = []
+        for i, (weight, left, right) in enumerate(((w1, dgu[:, :ffn], x2d), (w3, dgu[:, ffn:], x2d), (w2, dy2d, h))):
+            main_grad = getattr(weight, "main_grad", None)
+            if main_grad is not None:
+                native.gemm_tn(left, right, out=main_grad, accumulate=True)
+            grads.append(native.gemm_tn(left, right, out_dtype=weight.dtype)
+                         if main_grad is None and ctx.needs_input_grad[i + 1] else None)
+        return dx, *grads
+
+
+def swiglu_ffn(x, w1, w3, w2):
+    """The dense SwiGLU layer on the fused kernels, or ``None`` where its three products have to run one by one: CPU,
+    other types, a weight that is still to be gathered, layouts and widths that the fused epilogues do not tile (they
+    take 128 gate columns beside 128 up columns, and reduce in steps of 64).  4096 x 4096 -> 14336, forward and
+    backward: 3.8 ms of products instead of 3.45 ms plus 1.6 ms of elementwise passes over the hidden layer."""
+    weights = (w1, w3, w2)
+    if not (_use_native(x, "gemm") and x.dtype == torch.bfloat16 and x.numel() > 0 and x.data_ptr() % 16 == 0
+            and x.is_contiguous() and all(
+                w.dtype == torch.bfloat16 and w.dim() == 2 and w.is_contiguous() and w.data_ptr() % 16 == 0
+                and w.device == x.device and getattr(w, "pending_gather", None) is None for w in weights)):
+        return None
+    ffn, dim = w1.shape
+    if w3.shape != w1.shape or w2.shape != (dim, ffn) or ffn % 128 or dim % 64 or x.shape[-1] != dim:
+        return None
+    return _SwiGLUFFN.apply(x, *weights)
+
+
 class _Embedding(torch.autograd.Function):
     @staticmethod
     def forward(ctx, ids, table):

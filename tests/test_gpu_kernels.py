@@ -129,6 +129,38 @@ def test_grouped_expert_gemms(native, tile_mode, counts, pad):
     native.check_status()
 
 
+@pytest.mark.parametrize("tokens,dim,ffn,launches", [(1, 64, 128, 7), (129, 192, 384, 7), (300, 512, 640, 7),
+                                                     (5500, 64, 384, 8)])
+def test_dense_swiglu_layer_on_the_fused_kernels(native, tile_mode, tokens, dim, ffn, launches):
+    """Rows and widths around the tile edges, in every tile kind, forward and all gradients against 64 bits; a hook on
+    one projection sends the same layer through the three separate products."""
+    from b200moe.models.layers import PositionWiseFFLayer
+    torch.manual_seed(tokens)
+    layer = PositionWiseFFLayer(dim, ffn, device="cuda").to(torch.bfloat16)
+    x = _rand(tokens, dim).requires_grad_(True)
+    dy = _rand(tokens, dim)
+    leaves = [t.detach().double().requires_grad_(True) for t in (x, layer.w1.weight, layer.w3.weight, layer.w2.weight)]
+    gate = leaves[0] @ leaves[1].t()
+    ref = (gate * torch.sigmoid(gate) * (leaves[0] @ leaves[2].t())) @ leaves[3].t()
+    wanted = torch.autograd.grad(ref, leaves, dy.double())
+    calls = []
+    for hook in (False, True):
+        if hook:
+            layer.w3.register_forward_hook(lambda *_: calls.append(1))
+        for p in (x, *layer.parameters()):
+            p.grad = None
+        before = native.launch_count()
+        out = layer(x)
+        out.backward(dy)
+        assert native.launch_count() - before == (9 if hook else launches)
+        # bf16 hidden layer and gradients of it: 2^-9 each, three roundings deep
+        assert _rel(out, ref) < 1e-2
+        for got, want in zip((x.grad, layer.w1.weight.grad, layer.w3.weight.grad, layer.w2.weight.grad), wanted):
+            assert _rel(got, want) < 1.2e-2
+    assert calls
+    native.check_status()
+
+
 def test_rmsnorm_forward_backward(native):
     from b200moe import ops
     from b200moe.ops import functional as Fn
