@@ -652,20 +652,20 @@ static int launch_pair(const GemmParams& p, int sms, cudaStream_t stream) {
   return 0;
 }
 
-static int g_tile_mode = 0;   // 0 auto (single-CTA kinds), 1 force 128x256, 2 force 256x256 on one CTA,
-                              // 3 force CTA pairs where legal, 4 auto with CTA pairs for large problems
+static int g_tile_mode = 0;   // 0 auto, 1 force 128x256, 2 force 256x256 on one CTA, 3 force CTA pairs where legal, 4 auto
+                              // (EPI_PUSH included), 5 auto among the single-CTA kinds
 
 enum TileKind : int { TILE_128 = 0, TILE_256 = 1, TILE_PAIR = 2 };
 
 // 256-row tiles (one CTA with two sub-tiles, or a CTA pair) need whole 256-row tiles of one expert: the caller says
 // whether its segments are padded to 256 rows.
-// Measured in isolation (burst clocks) CTA pairs are the fastest kind everywhere: 16384 x 6144 x 4096 runs at
-// 1351 TFLOP/s with 128x256 tiles and 1494 on pairs, grouped weight gradients gain 13-28 %.  Inside a training
-// step, which runs against the 1000 W power cap for seconds, the same kernels pull the SM clock down further
-// (median 1175 MHz against 1385 MHz with the single-CTA kinds, same power) and the step gets 7 % slower (3141 ms
-// against 2940 ms, measured twice, alternating).  So the automatic choice uses the single-CTA kinds — 256x256 for
-// long K, where the exposed epilogue is amortised, 128x256 otherwise — and pairs are opt-in (mode 3 or 4).
-template <int SCHED>
+// CTA pairs wherever their tiles reach half of the machine's pairs or more.  Whole passes, us, single-CTA kinds -> pairs:
+// three-layer dense SwiGLU stack 11374 -> 10544, 5003-token expert layer 11142 -> 10905, one-block step of 2 x 16384
+// tokens 109651 -> 104820, head and loss of 6001 tokens 3519 -> 3307; the eight-block step that runs against the 1000 W
+// power cap for ten seconds 10649 -> 10669 ms, which is the same.  (With the four-warp epilogue pairs lost 7 % there.)
+// Below that the single-CTA kinds: 256x256 for long K, where the exposed epilogue is amortised, else 128x256.  The
+// expert-parallel return (EPI_PUSH) stays with those: its time depends on the links, which one GPU does not show.
+template <int SCHED, int EPI>
 static TileKind choose_tile(const GemmParams& p, int sms, bool pair_available) {
   const long long k_eff = SCHED == SCHED_WGRAD ? p.K / (p.num_experts > 0 ? p.num_experts : 1) : p.K;
   const bool legal = SCHED == SCHED_WGRAD ||
@@ -674,8 +674,10 @@ static TileKind choose_tile(const GemmParams& p, int sms, bool pair_available) {
                              (SCHED == SCHED_WGRAD ? p.num_experts : 1);
   if (!legal || g_tile_mode == 1) return TILE_128;
   if (g_tile_mode == 2) return TILE_256;
-  if (pair_available && (g_tile_mode == 3 || (g_tile_mode == 4 && tiles256 >= sms / 2))) return TILE_PAIR;
+  if (pair_available && g_tile_mode == 3) return TILE_PAIR;
   if (g_tile_mode == 3) return TILE_128;
+  const bool pairs = g_tile_mode == 4 || (g_tile_mode == 0 && EPI != EPI_PUSH);
+  if (pair_available && pairs && tiles256 >= sms / 2) return TILE_PAIR;
   return tiles256 >= 2LL * sms && k_eff >= 6144 ? TILE_256 : TILE_128;
 }
 
@@ -696,7 +698,7 @@ static int launch(const GemmParams& p, TileKind kind, int sms, cudaStream_t stre
 // Convenience for entry points whose tensor maps do not depend on the tile kind.
 template <int A_MN, int B_MN, int EPI, int SCHED>
 static int launch(const GemmParams& p, int sms, cudaStream_t stream) {
-  return launch<A_MN, B_MN, EPI, SCHED>(p, choose_tile<SCHED>(p, sms, pair_available<A_MN, B_MN, EPI, SCHED>(sms)),
+  return launch<A_MN, B_MN, EPI, SCHED>(p, choose_tile<SCHED, EPI>(p, sms, pair_available<A_MN, B_MN, EPI, SCHED>(sms)),
                                         sms, stream);
 }
 
@@ -722,8 +724,8 @@ using namespace b2;
 //   status         device int32 word, set non-zero if an in-kernel wait ran out
 extern "C" {
 
-// 0 automatic among the single-CTA kinds, 1 always 128x256 tiles, 2 single-CTA 256x256 tiles wherever they are legal,
-// 3 CTA pairs wherever legal, 4 automatic with CTA pairs for problems that fill the machine.
+// 0 automatic, 1 always 128x256 tiles, 2 single-CTA 256x256 tiles wherever they are legal, 3 CTA pairs wherever legal,
+// 4 automatic for the expert-parallel return too, 5 automatic among the single-CTA kinds.
 void b2_gemm_set_tile_mode(int mode) { g_tile_mode = mode; }
 
 // y[M,N] = a[M,K] * w[e][N,K]^T      (a K-major, w K-major)
@@ -740,7 +742,7 @@ int b2_gemm_nt(const void* a, const void* w, void* d, int M, int N, int K, long 
   const int sms = sm_count();
   const bool pairs = epi == EPI_STORE_BF16 ? pair_available<0, 0, EPI_STORE_BF16, SCHED_FLAT>(sms)
                                            : pair_available<0, 0, EPI_STORE_F32, SCHED_FLAT>(sms);
-  const TileKind kind = choose_tile<SCHED_FLAT>(p, sms, pairs);
+  const TileKind kind = choose_tile<SCHED_FLAT, EPI_STORE_BF16>(p, sms, pairs);
   if (make_map(&p.map_a, a, K, M, lda, BM)) return -11;
   // a CTA of a pair stages 128 of the tile's 256 weight rows
   if (make_map(&p.map_b, w, K, static_cast<long long>(num_experts) * N, ldw, kind == TILE_PAIR ? BN / 2 : BN))
@@ -809,7 +811,7 @@ int b2_gemm_nt_rope(const void* a, const void* w, void* d, int M, int N, int K, 
   p.d = d; p.ldd = ldd; p.status = status; p.beta = 0.f;
   p.rope_cos = cos_t; p.rope_sin = sin_t; p.rope_cols = rope_cols; p.rope_seq = seq;
   const int sms = sm_count();
-  const TileKind kind = choose_tile<SCHED_FLAT>(p, sms, pair_available<0, 0, EPI_ROPE, SCHED_FLAT>(sms));
+  const TileKind kind = choose_tile<SCHED_FLAT, EPI_ROPE>(p, sms, pair_available<0, 0, EPI_ROPE, SCHED_FLAT>(sms));
   if (make_map(&p.map_a, a, K, M, lda, BM)) return -11;
   if (make_map(&p.map_b, w, K, N, K, kind == TILE_PAIR ? BN / 2 : BN)) return -12;
   return launch<0, 0, EPI_ROPE, SCHED_FLAT>(p, kind, sms, stream);
@@ -842,7 +844,7 @@ int b2_gemm_nt_push(const void* a, const void* w, int M, int N, int K, long long
   p.group_align256 = group_align256;
   fill_push(p, push_dst, push_tag, push_src, push_w, sig, sig_slot, seq, rank, n, ticket);
   const int sms = sm_count();
-  const TileKind kind = choose_tile<SCHED_FLAT>(p, sms, pair_available<0, 0, EPI_PUSH, SCHED_FLAT>(sms));
+  const TileKind kind = choose_tile<SCHED_FLAT, EPI_PUSH>(p, sms, pair_available<0, 0, EPI_PUSH, SCHED_FLAT>(sms));
   if (make_map(&p.map_a, a, K, M, lda, BM)) return -11;
   if (make_map(&p.map_b, w, K, static_cast<long long>(num_experts) * N, K, kind == TILE_PAIR ? BN / 2 : BN))
     return -12;

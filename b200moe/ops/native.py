@@ -219,10 +219,9 @@ def _bf16(t):
 
 # ------------------------------------------------------------------------------ GEMM
 def set_gemm_tile_mode(mode: int) -> None:
-    """0: automatic among the single-CTA kinds (the default: fastest under the sustained power cap of a training
-    step); 1: always 128x256 CTA tiles; 2: single-CTA 256x256 tiles wherever legal; 3: 256x256 tiles on CTA pairs
-    (``cta_group::2``) wherever legal; 4: automatic with CTA pairs for problems that fill the machine (fastest for
-    a kernel run in isolation).  The environment variable ``B200MOE_GEMM_TILE_MODE`` sets it at load time."""
+    """0: automatic (the default): 256x256 tiles on CTA pairs (``cta_group::2``) for problems that fill the machine,
+    else the single-CTA kinds; 1: always 128x256 CTA tiles; 2: single-CTA 256x256 tiles wherever legal; 3: CTA pairs
+    wherever legal; 4: like 0, the expert-parallel return included; 5: automatic among the single-CTA kinds.  The environment variable ``B200MOE_GEMM_TILE_MODE`` sets it at load time."""
     require().b2_gemm_set_tile_mode(_I(mode))
 
 
