@@ -10,12 +10,7 @@ from __future__ import annotations
 import torch
 import torch.nn.functional as F
 
-from . import functional as Fn
-
-
-def _native():
-    from . import native
-    return native
+from . import functional as Fn, native, use_native
 
 
 def _eager(*tensors) -> bool:
@@ -41,7 +36,7 @@ def _ragged_ok(q, k, v, cos=None, sin=None) -> bool:
         t is None or (_eager(t) and t.dim() == 2 and t.dtype == torch.float32 and t.shape[1] == 64
                       and t.shape[0] >= q.shape[1] and t.is_contiguous() and t.data_ptr() % 16 == 0
                       and t.device == q.device and not t.requires_grad) for t in (cos, sin))
-    return tables and all(_native()._pitched(t) for t in (q, k, v))
+    return tables and all(native._pitched(t) for t in (q, k, v))
 
 
 def _second_order(q, k, v, dout, cos, sin, causal):
@@ -56,7 +51,7 @@ def _second_order(q, k, v, dout, cos, sin, causal):
 class _RopeAttention(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, cos, sin):
-        out, lse, q_rot, k_rot = _native().attention_fwd(q, k, v, cos, sin)
+        out, lse, q_rot, k_rot = native.attention_fwd(q, k, v, cos, sin)
         ctx.ragged = q.shape[1] % 128 != 0
         ctx.save_for_backward(q_rot, k_rot, v, out, lse, cos, sin, *((q, k) if ctx.ragged else ()))
         return out
@@ -66,7 +61,7 @@ class _RopeAttention(torch.autograd.Function):
         q_rot, k_rot, v, out, lse, cos, sin, *inputs = ctx.saved_tensors
         if ctx.ragged and torch.is_grad_enabled():
             return (*_second_order(*inputs, v, dout, cos, sin, True), None, None)
-        dq, dk, dv = _native().attention_bwd(dout.contiguous(), q_rot, k_rot, v, out, lse, cos, sin)
+        dq, dk, dv = native.attention_bwd(dout.contiguous(), q_rot, k_rot, v, out, lse, cos, sin)
         return dq, dk, dv, None, None
 
 
@@ -77,7 +72,7 @@ class _RopeQK(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, qkv, seq, total, heads, hd, cos, sin):
-        _native().rope_inplace(qkv, 0, qkv.shape[0], seq, heads, hd, total * hd, cos, sin, 1.0)
+        native.rope_inplace(qkv, 0, qkv.shape[0], seq, heads, hd, total * hd, cos, sin, 1.0)
         ctx.mark_dirty(qkv)
         ctx.meta = (seq, total, heads, hd, cos, sin)
         return qkv
@@ -86,7 +81,7 @@ class _RopeQK(torch.autograd.Function):
     def backward(ctx, dqkv):
         seq, total, heads, hd, cos, sin = ctx.meta
         dqkv = dqkv.contiguous().clone()
-        _native().rope_inplace(dqkv, 0, dqkv.shape[0], seq, heads, hd, total * hd, cos, sin, -1.0)
+        native.rope_inplace(dqkv, 0, dqkv.shape[0], seq, heads, hd, total * hd, cos, sin, -1.0)
         return dqkv, None, None, None, None, None, None
 
 
@@ -104,7 +99,6 @@ class _FusedQKVAttention(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, qkv, batch, seq, hq, hkv, hd, cos, sin, pre_rotated):
-        native = _native()
         total = hq + 2 * hkv
         if cos is not None and not pre_rotated:      # the projection GEMM did not rotate q and k in its epilogue
             native.rope_inplace(qkv, 0, qkv.shape[0], seq, hq + hkv, hd, total * hd, cos, sin, 1.0)
@@ -117,7 +111,6 @@ class _FusedQKVAttention(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, _dqkv_unused, dout):
-        native = _native()
         qkv, out, lse = ctx.saved_tensors
         batch, seq, hq, hkv, hd, cos, sin = ctx.meta
         total = hq + 2 * hkv
@@ -150,7 +143,6 @@ def attention_backend() -> str:
 def rope_attention(q, k, v, cos, sin):
     """Returns ``[B, S, Hq, head_dim]``.  ``cos``/``sin`` are ``[S_max, hd/2]``
     fp32 tables or ``None`` for no rotation."""
-    from . import use_native
     if use_native(q, "attention") and attention_backend() == "native" and q.shape[-1] == 128 and (
             q.shape[1] % 128 == 0 or _ragged_ok(q, k, v, cos, sin)):
         return _RopeAttention.apply(q, k, v, cos, sin)
@@ -171,7 +163,7 @@ class _PlainAttention(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, v, causal):
-        out, lse, _, _ = _native().attention_fwd(q, k, v, None, None, causal=causal)
+        out, lse, _, _ = native.attention_fwd(q, k, v, None, None, causal=causal)
         ctx.save_for_backward(q, k, v, out, lse)
         ctx.causal = causal
         return out
@@ -181,17 +173,15 @@ class _PlainAttention(torch.autograd.Function):
         q, k, v, out, lse = ctx.saved_tensors
         if q.shape[1] % 128 and torch.is_grad_enabled():
             return (*_second_order(q, k, v, dout, None, None, ctx.causal), None)
-        dq, dk, dv = _native().attention_bwd(dout, q, k, v, out, lse, causal=ctx.causal)
+        dq, dk, dv = native.attention_bwd(dout, q, k, v, out, lse, causal=ctx.causal)
         return dq, dk, dv, None
 
 
 def _native_attention(q) -> bool:
-    from . import use_native
     return use_native(q, "attention") and q.dim() == 4
 
 
 def _native_shape_ok(q, k) -> bool:
-    from . import use_native
     return (use_native(q, "attention") and q.dtype == torch.bfloat16 and q.shape[-1] == 128
             and q.shape[1] % 128 == 0 and k.shape[1] == q.shape[1])
 
@@ -220,11 +210,11 @@ def flash_attention_forward(q, k, v, causal: bool = False):
             heads = [t.contiguous().view(B * H, S, 1, hd) for t in (q, k, v)]
             if all(t.data_ptr() % 16 == 0 for t in heads):
                 with torch.no_grad():
-                    return _native().attention_fwd(*heads, None, None, causal=causal)[0].view(B, H, S, hd)
+                    return native.attention_fwd(*heads, None, None, causal=causal)[0].view(B, H, S, hd)
         q, k, v = (t.to(torch.bfloat16).contiguous().view(B * H, S, 1, hd) for t in (q, k, v))
         if _native_shape_ok(q, k):
             with torch.no_grad():
-                out, _, _, _ = _native().attention_fwd(q, k, v, None, None, causal=causal)
+                out, _, _, _ = native.attention_fwd(q, k, v, None, None, causal=causal)
             return out.view(B, H, S, hd).to(want)
         q, k, v = (t.view(B, H, S, hd) for t in (q, k, v))
     with torch.no_grad():

@@ -13,17 +13,7 @@ from __future__ import annotations
 
 import torch
 
-from . import functional as Fn
-
-
-def _native():
-    from . import native
-    return native
-
-
-def _use_native(t, op):
-    from . import use_native
-    return use_native(t, op)
+from . import functional as Fn, native, use_native
 
 
 class _Linear(torch.autograd.Function):
@@ -43,12 +33,12 @@ class _Linear(torch.autograd.Function):
             y = gather(x2d if x2d.is_contiguous() else x2d.contiguous())
             if rope is not None:
                 cos, sin, cols, seq = rope
-                _native().rope_inplace(y, 0, y.shape[0], seq, cols // 128, 128, y.shape[1], cos, sin, 1.0)
+                native.rope_inplace(y, 0, y.shape[0], seq, cols // 128, 128, y.shape[1], cos, sin, 1.0)
         elif rope is not None:
             cos, sin, cols, seq = rope
-            y = _native().gemm_nt_rope(x2d, weight, cos, sin, cols, seq)
-        elif _use_native(x, "gemm"):
-            y = _native().gemm_nt(x2d, weight)
+            y = native.gemm_nt_rope(x2d, weight, cos, sin, cols, seq)
+        elif use_native(x, "gemm"):
+            y = native.gemm_nt(x2d, weight)
         else:
             w = weight if weight.dtype == x.dtype else weight.to(x.dtype)
             y = x2d @ w.t()
@@ -62,11 +52,11 @@ class _Linear(torch.autograd.Function):
         dy2d = dy.reshape(-1, dy.shape[-1])
         if not dy2d.is_contiguous():
             dy2d = dy2d.contiguous()
-        native = _use_native(x, "gemm")
+        on_gpu = use_native(x, "gemm")
         dx = None
         if ctx.needs_input_grad[0]:
-            if native:
-                dx = _native().gemm_nn(dy2d, weight)
+            if on_gpu:
+                dx = native.gemm_nn(dy2d, weight)
             else:
                 w = weight if weight.dtype == dy2d.dtype else weight.to(dy2d.dtype)
                 dx = dy2d @ w
@@ -74,13 +64,13 @@ class _Linear(torch.autograd.Function):
         dw = None
         main_grad = getattr(weight, "main_grad", None)
         if main_grad is not None:
-            if native:
-                _native().gemm_tn(dy2d, x2d, out=main_grad, accumulate=True)
+            if on_gpu:
+                native.gemm_tn(dy2d, x2d, out=main_grad, accumulate=True)
             else:
                 main_grad.addmm_(dy2d.t().to(main_grad.dtype), x2d.to(main_grad.dtype))
         elif ctx.needs_input_grad[1]:
-            if native:
-                dw = _native().gemm_tn(dy2d, x2d, out_dtype=weight.dtype)
+            if on_gpu:
+                dw = native.gemm_tn(dy2d, x2d, out_dtype=weight.dtype)
             else:
                 dw = (dy2d.t() @ x2d).to(weight.dtype)
         return dx, dw, None
@@ -105,7 +95,6 @@ class _SwiGLUFFN(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, w1, w3, w2):
-        native = _native()
         x2d = x.reshape(-1, x.shape[-1])
         keep = any(ctx.needs_input_grad)
         h, gate, up = native.gemm_swiglu(x2d, w1.unsqueeze(0), w3.unsqueeze(0), save_gate_up=keep)
@@ -117,7 +106,6 @@ class _SwiGLUFFN(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dy):
-        native = _native()
         x, gate, up = ctx.saved_tensors
         w1, w3, w2 = ctx.weights
         x2d, ffn = x.reshape(-1, x.shape[-1]), w1.shape[0]
@@ -140,7 +128,7 @@ def swiglu_ffn(x, w1, w3, w2):
     take 128 gate columns beside 128 up columns, and reduce in steps of 64).  4096 x 4096 -> 14336, forward and
     backward: 3.8 ms of products instead of 3.45 ms plus 1.6 ms of elementwise passes over the hidden layer."""
     weights = (w1, w3, w2)
-    if not (_use_native(x, "gemm") and x.dtype == torch.bfloat16 and x.numel() > 0 and x.data_ptr() % 16 == 0
+    if not (use_native(x, "gemm") and x.dtype == torch.bfloat16 and x.numel() > 0 and x.data_ptr() % 16 == 0
             and x.is_contiguous() and all(
                 w.dtype == torch.bfloat16 and w.dim() == 2 and w.is_contiguous() and w.data_ptr() % 16 == 0
                 and w.device == x.device and getattr(w, "pending_gather", None) is None for w in weights)):
@@ -156,8 +144,8 @@ class _Embedding(torch.autograd.Function):
     def forward(ctx, ids, table):
         ctx.table = table
         ctx.save_for_backward(ids)
-        if _use_native(table, "embedding"):
-            return _native().embedding_fwd(ids, table)
+        if use_native(table, "embedding"):
+            return native.embedding_fwd(ids, table)
         return table[ids]
 
     @staticmethod
@@ -168,8 +156,8 @@ class _Embedding(torch.autograd.Function):
         dy2d = dy.reshape(-1, dy.shape[-1])
         main_grad = getattr(table, "main_grad", None)
         if main_grad is not None:
-            if _use_native(dy, "embedding"):
-                _native().embedding_bwd(flat_ids, dy2d, main_grad)
+            if use_native(dy, "embedding"):
+                native.embedding_bwd(flat_ids, dy2d, main_grad)
             else:
                 main_grad.index_add_(0, flat_ids, dy2d.to(main_grad.dtype))
             return None, None
@@ -186,20 +174,20 @@ def embedding(ids: torch.Tensor, table: torch.Tensor) -> torch.Tensor:
 class _RMSNorm(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, eps):
-        y, rstd = _native().rmsnorm_fwd(x, weight, eps)
+        y, rstd = native.rmsnorm_fwd(x, weight, eps)
         ctx.save_for_backward(x, weight, rstd)
         return y
 
     @staticmethod
     def backward(ctx, dy):
         x, weight, rstd = ctx.saved_tensors
-        dx, dw = _native().rmsnorm_bwd(dy.contiguous(), x, weight, rstd)
+        dx, dw = native.rmsnorm_bwd(dy.contiguous(), x, weight, rstd)
         return dx, dw.to(weight.dtype), None
 
 
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5) -> torch.Tensor:
     """``x · rsqrt(mean(x²) + eps) · weight`` evaluated in fp32, cast back."""
-    if _use_native(x, "rmsnorm"):
+    if use_native(x, "rmsnorm"):
         return _RMSNorm.apply(x, weight, eps)
     return Fn.rmsnorm_ref(x, weight, eps)
 
@@ -207,21 +195,21 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5) -> torch.T
 class _AddRMSNorm(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, delta, weight, eps):
-        summed, y, rstd = _native().add_rmsnorm_fwd(x, delta, weight, eps)
+        summed, y, rstd = native.add_rmsnorm_fwd(x, delta, weight, eps)
         ctx.save_for_backward(summed, weight, rstd)
         return summed, y
 
     @staticmethod
     def backward(ctx, dsum, dy):
         summed, weight, rstd = ctx.saved_tensors
-        dx, dw = _native().rmsnorm_bwd(dy.contiguous(), summed, weight, rstd, residual_grad=dsum)
+        dx, dw = native.rmsnorm_bwd(dy.contiguous(), summed, weight, rstd, residual_grad=dsum)
         return dx, dx, dw.to(weight.dtype), None
 
 
 def add_rmsnorm(x: torch.Tensor, delta: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5):
     """Residual add fused with the following norm: returns ``(x + delta,
     rmsnorm(x + delta))``."""
-    if _use_native(x, "rmsnorm"):
+    if use_native(x, "rmsnorm"):
         return _AddRMSNorm.apply(x, delta, weight, eps)
     summed = x + delta
     return summed, Fn.rmsnorm_ref(summed, weight, eps)

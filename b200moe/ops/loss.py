@@ -22,14 +22,9 @@ from __future__ import annotations
 
 import torch
 
-from . import functional as Fn
+from . import functional as Fn, native, use_native
 
 CHUNK_TOKENS = 4096
-
-
-def _native():
-    from . import native
-    return native
 
 
 def _chunks(total: int, size: int):
@@ -40,7 +35,6 @@ def _chunks(total: int, size: int):
 class _LMHeadCE(torch.autograd.Function):
     @staticmethod
     def forward(ctx, hidden, weight, targets, grad_scale):
-        native = _native()
         h2d = hidden.reshape(-1, hidden.shape[-1])
         flat_targets = targets.reshape(-1).contiguous()
         tokens = h2d.shape[0]
@@ -64,7 +58,6 @@ class _LMHeadCE(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dloss):
-        native = _native()
         weight = ctx.weight
         if ctx.eager:
             (dh,) = ctx.saved_tensors
@@ -91,7 +84,6 @@ def lm_head_cross_entropy(hidden: torch.Tensor, weight: torch.Tensor, targets: t
                           grad_scale: float | None = None) -> torch.Tensor:
     """Mean next-token loss of ``hidden @ weightᵀ`` against ``targets``.  ``grad_scale``: the factor the caller will
     back-propagate into the returned loss, when it is known in advance (see the module text)."""
-    from . import use_native
     from .dense import linear
     if use_native(hidden, "lmhead_ce"):
         return _LMHeadCE.apply(hidden, weight, targets, grad_scale)

@@ -24,26 +24,16 @@ import torch
 import torch.distributed as dist
 import torch.nn.functional as F
 
-from . import functional as Fn
+from . import functional as Fn, native, use_native
 
 ALIGN = 128
-
-
-def _native():
-    from . import native
-    return native
-
-
-def _use_native(t, op):
-    from . import use_native
-    return use_native(t, op)
 
 
 # ----------------------------------------------------------------------------- router
 class _RouterTop2(torch.autograd.Function):
     @staticmethod
     def forward(ctx, logits):
-        weights, idx, probs = _native().router_top2_fwd(logits)
+        weights, idx, probs = native.router_top2_fwd(logits)
         ctx.save_for_backward(probs, idx, weights)
         ctx.mark_non_differentiable(idx)
         return weights, idx
@@ -51,13 +41,13 @@ class _RouterTop2(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dweights, _didx):
         probs, idx, weights = ctx.saved_tensors
-        return _native().router_top2_bwd(dweights.contiguous(), probs, idx, weights)
+        return native.router_top2_bwd(dweights.contiguous(), probs, idx, weights)
 
 
 def router_top2(logits: torch.Tensor):
     """``(weights fp32 [T,2], idx int64 [T,2])``: softmax over experts, top-2,
     weights renormalised to sum to one."""
-    if _use_native(logits, "router"):
+    if use_native(logits, "router"):
         return _RouterTop2.apply(logits)
     return Fn.router_top2_ref(logits, 2)
 
@@ -252,7 +242,7 @@ def moe_ffn(x: torch.Tensor, weights: torch.Tensor, idx: torch.Tensor, w1, w2, w
     renormalised weights.  ``w1, w3: [E_local, d_ff, D]``, ``w2: [E_local, D, d_ff]``."""
     tokens, k = idx.shape
     ep = 1 if group is None else dist.get_world_size(group)
-    if _use_native(x, "moe") and ep == 1:
+    if use_native(x, "moe") and ep == 1:
         from .moe_fused import moe_ffn_fused
         return moe_ffn_fused(x, weights, idx, w1, w2, w3, recompute=recompute, budget=budget)
     plan = build_plan(idx, w1.shape[0] * ep, group)

@@ -81,7 +81,7 @@ class _MoEFused(torch.autograd.Function):
             _, gate, up = native.gemm_swiglu(x_perm, w1, w3, tile_expert, tiles, save_gate_up=True, align256=True)
         else:
             gate, up = saved[8:10]
-        dweights = torch.zeros(tokens, 2, dtype=torch.float32, device=dout.device)
+        dweights = torch.empty(tokens, 2, dtype=torch.float32, device=dout.device)   # every slot has its row
         dy_perm = native.moe_gather(dout, row_slot, meta, cap, scale=weights.view(-1), y_perm=y_perm,
                                     dweights=dweights.view(-1))
         dgu, h = native.gemm_nn_swiglu_bwd(dy_perm, w2, gate, up, tile_expert=tile_expert, num_m_tiles=tiles,

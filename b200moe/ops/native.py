@@ -23,6 +23,8 @@ _lib = None
 _load_error = None
 _launches = 0
 _status = {}
+_entries = {}        # entry point name -> ctypes function
+_has = {}            # op family -> whether the library has it
 
 _FAMILIES = {
     "gemm": "b2_gemm_nt", "rmsnorm": "b2_rmsnorm_fwd", "router": "b2_router_top2_fwd",
@@ -58,11 +60,14 @@ def require():
 
 
 def has(op: str) -> bool:
-    lib = _load()
-    if lib is None:
-        return False
-    symbol = _FAMILIES.get(op)
-    return symbol is not None and hasattr(lib, symbol)
+    known = _has.get(op)
+    if known is None:
+        lib = _load()
+        symbol = _FAMILIES.get(op)
+        known = lib is not None and symbol is not None and hasattr(lib, symbol)
+        if lib is not None:
+            _has[op] = known
+    return known
 
 
 def available_ops() -> list:
@@ -83,12 +88,21 @@ def _p(t):
     return ctypes.c_void_p(0 if t is None else t.data_ptr())
 
 
+# Stream and device as plain integers: ``torch.cuda.current_stream()`` builds two objects and looks the device up three
+# times, which was a quarter of the host time of a small training step.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_raw_device = getattr(torch._C, "_cuda_getDevice", None)
+
+
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(_raw_stream(_raw_device()))
 
 
 def status_word(device=None) -> torch.Tensor:
     """Device int32 word that kernels set non-zero when a bounded wait ran out."""
+    word = _status.get(device) if type(device) is torch.device else None
+    if word is not None:
+        return word
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     word = _status.get(device)
     if word is None:
@@ -175,24 +189,30 @@ def launch_times() -> dict:
 
 def _call(name, *args, n: int = 1, tag: str = ""):
     global _launches
+    entry = _entries.get(name)
+    if entry is None:
+        entry = _entries[name] = getattr(require(), name)
+    if _timed is None and not _nvtx:
+        rc = entry(*args)
+        if rc != 0:
+            raise RuntimeError(f"{name} failed with code {rc}{_failure_detail(name, rc)}")
+        _launches += n
+        return
     if _timed is not None:
         begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         begin.record()
-        rc = getattr(require(), name)(*args)
+        rc = entry(*args)
         end.record()
         _timed.append((f"{name} {tag}".strip(), begin, end))
         if rc != 0:
             raise RuntimeError(f"{name} failed with code {rc}")
         _launches += n
         return
-    if _nvtx:
-        torch.cuda.nvtx.range_push(name)
-        try:
-            rc = getattr(require(), name)(*args)
-        finally:
-            torch.cuda.nvtx.range_pop()
-    else:
-        rc = getattr(require(), name)(*args)
+    torch.cuda.nvtx.range_push(name)
+    try:
+        rc = entry(*args)
+    finally:
+        torch.cuda.nvtx.range_pop()
     if rc != 0:
         raise RuntimeError(f"{name} failed with code {rc}{_failure_detail(name, rc)}")
     _launches += n
@@ -587,13 +607,10 @@ def attention_bwd(dout, q, k, v, out, lse, cos=None, sin=None, grads=None, causa
 def moe_plan(idx, num_experts, capacity_rows):
     slots = idx.numel()
     dev = idx.device
-    i32 = dict(dtype=torch.int32, device=dev)
-    slot_row = torch.empty(slots, **i32)
-    row_slot = torch.empty(capacity_rows, **i32)
-    offs = torch.empty(num_experts, **i32)
-    tile_expert = torch.empty(capacity_rows // 128, **i32)
-    meta = torch.zeros(4, **i32)
-    counts = torch.empty(num_experts, **i32)
+    # one allocation, cut into the six tables (the kernel writes what it promises of each)
+    sizes = (slots, capacity_rows, num_experts, capacity_rows // 128, 4, num_experts)
+    slot_row, row_slot, offs, tile_expert, meta, counts = torch.empty(sum(sizes), dtype=torch.int32,
+                                                                      device=dev).split(sizes)
     _call("b2_moe_plan", _p(idx.contiguous()), _I(slots), _I(num_experts), _p(slot_row), _p(row_slot), _p(offs),
           _p(tile_expert), _p(meta), _p(counts), _I(capacity_rows), _stream())
     return slot_row, row_slot, offs, tile_expert, meta, counts
