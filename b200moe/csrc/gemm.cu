@@ -91,6 +91,7 @@ struct GemmParams {
   long long ldd;               // leading dimension of d (elements)
   long long d_expert_stride;   // elements between experts in d (SCHED_WGRAD)
   float beta;                  // 1 accumulate, 0 overwrite (EPI_ACC_*)
+  const float* alpha;          // optional device scalar that multiplies the product (EPI_STORE_*, EPI_ACC_*)
   int* status;                 // device word; non-zero = a wait ran out
   // EPI_ROPE only
   const float* rope_cos;       // [rope_seq, 64] fp32
@@ -459,6 +460,8 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
         const long long expert_off = SCHED == SCHED_WGRAD ? t.expert * p.d_expert_stride : 0;
         const int q = lane & 3;
         const bool add = (EPI == EPI_ACC_F32 || EPI == EPI_ACC_BF16) && p.beta != 0.f;
+        constexpr bool SCALED = EPI == EPI_ACC_F32 || EPI == EPI_ACC_BF16 || EPI == EPI_STORE_BF16 || EPI == EPI_STORE_F32;
+        const float alpha = SCALED && p.alpha ? *p.alpha : 1.f;
 #pragma unroll 1
         for (int c = half * 128; c < half * 128 + 128; c += 32) {
           const long long col = col_base + c + q * 8;     // N is a multiple of 32 (checked on the host)
@@ -509,6 +512,10 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
             const uint4 o0 = old[it][0], o1 = old[it][OLD ? OLD - 1 : 0];
             const uint32_t w0[4] = {o0.x, o0.y, o0.z, o0.w}, w1[4] = {o1.x, o1.y, o1.z, o1.w};
             if (row0 + r >= p.M) continue;
+            if (SCALED) {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) x[i] *= alpha;
+            }
             const long long off = expert_off + (row0 + r) * p.ldd + col;
             if (EPI == EPI_ACC_F32 || EPI == EPI_STORE_F32) {
               if (add) {
@@ -767,12 +774,14 @@ int b2_gemm_swiglu(const void* a, const void* w1, const void* w3, void* h, void*
 }
 
 // dx[M,N] = a[M,K] * w[e][K,N]     (w MN-major: its rows are the reduction index).
+// ``alpha`` (optional device scalar) multiplies the result.
 // If w2 is given, K = k_split + K2 and rows k >= k_split come from w2 (dx = dg W1 + du W3 in one pass).
 int b2_gemm_nn(const void* a, const void* w, const void* w2, void* d, int M, int N, int K, int k_split, long long lda,
                long long ldw, long long ldd, int num_experts, const int* tile_expert, const int* num_m_tiles,
-               int group_align256, int* status, cudaStream_t stream) {
+               int group_align256, const float* alpha, int* status, cudaStream_t stream) {
   if (N % 32 || K % 64 || (w2 && k_split % 64)) return -10;
   GemmParams p{};
+  p.alpha = alpha;
   const int rows = w2 ? k_split : K;
   if (make_map(&p.map_a, a, K, M, lda, BM)) return -11;
   if (make_map(&p.map_b, w, N, static_cast<long long>(num_experts) * rows, ldw, 64)) return -12;
@@ -871,12 +880,14 @@ int b2_gemm_nn_push(const void* a, const void* w, const void* w2, int M, int N, 
 }
 
 // dw[e][M,N] (+)= a[rows_e, M]^T * b[rows_e, N]   (both MN-major; rows_e from cumulative offsets, or all R rows
-// when expert_offsets is null).  out_kind: 1 fp32 (+= if beta), 2 bf16 (+= if beta).
+// when expert_offsets is null).  out_kind: 1 fp32 (+= if beta), 2 bf16 (+= if beta).  ``alpha`` (optional device scalar)
+// multiplies the product before it is added.
 int b2_gemm_tn(const void* a, const void* b, void* d, int M, int N, int R, long long lda, long long ldb,
-               long long ldd, int num_experts, const int* expert_offsets, int out_kind, float beta, int* status,
-               cudaStream_t stream) {
+               long long ldd, int num_experts, const int* expert_offsets, int out_kind, float beta,
+               const float* alpha, int* status, cudaStream_t stream) {
   if (N % 32 || M % 8) return -10;
   GemmParams p{};
+  p.alpha = alpha;
   if (make_map(&p.map_a, a, M, R, lda, 64)) return -11;
   if (make_map(&p.map_b, b, N, R, ldb, 64)) return -12;
   p.M = M; p.N = N; p.K = R; p.num_experts = num_experts; p.b_expert_rows = 0; p.k_split = 0;

@@ -279,12 +279,13 @@ def gemm_nt_rope(x, w, cos, sin, rope_cols: int, seq: int):
 
 
 def gemm_nn(dy, w, w2=None, tile_expert=None, num_m_tiles=None, num_experts: int = 1, align256: bool = False,
-            out=None):
+            out=None, alpha=None):
     """``dy [M,K] @ w[e] [K,N]`` (``w`` rows are the reduction index).  With ``w2``
-    the reduction continues over ``w2``'s rows: ``dy = [a | b]``, result ``a w + b w2``."""
+    the reduction continues over ``w2``'s rows: ``dy = [a | b]``, result ``a w + b w2``.  ``alpha``: fp32 device scalar
+    that multiplies the result in the epilogue."""
     M, K = dy.shape
     N = w.shape[-1]
-    if K <= 16 and num_experts == 1 and w2 is None:
+    if K <= 16 and num_experts == 1 and w2 is None and alpha is None:
         out = torch.empty(M, N, dtype=torch.bfloat16, device=dy.device)
         _call("b2_skinny_nn", _p(dy.float().contiguous()), _p(_bf16(w)), _p(out), _I(M), _I(K), _I(N), _stream())
         return out
@@ -294,7 +295,7 @@ def gemm_nn(dy, w, w2=None, tile_expert=None, num_m_tiles=None, num_experts: int
     assert dy.stride(-1) == 1 and w.is_contiguous() and out.stride(-1) == 1 and out.shape == (M, N)
     _call("b2_gemm_nn", _p(_bf16(dy)), _p(_bf16(w)), _p(w2), _p(_bf16(out)), _I(M), _I(N), _I(K), _I(k_split),
           _L(dy.stride(0)), _L(N), _L(out.stride(0)), _I(num_experts), _p(tile_expert), _p(num_m_tiles), _I(int(align256)),
-          _p(status_word(dy.device)), _stream(), tag=f"{'grouped ' if tile_expert is not None else ''}N={N} K={K}")
+          _p(alpha), _p(status_word(dy.device)), _stream(), tag=f"{'grouped ' if tile_expert is not None else ''}N={N} K={K}")
     return out
 
 
@@ -323,11 +324,13 @@ def gemm_nn_swiglu_bwd(dy, w, gate, up, tile_expert=None, num_m_tiles=None, num_
     return dgu, h
 
 
-def gemm_tn(dy, x, out=None, accumulate: bool = False, out_dtype=None, expert_offsets=None, num_experts: int = 1):
-    """``out[e] (+)= dy[rows_e]ᵀ @ x[rows_e]`` -> ``[E?, N_out, K_in]``; fp32 or bf16 output."""
+def gemm_tn(dy, x, out=None, accumulate: bool = False, out_dtype=None, expert_offsets=None, num_experts: int = 1,
+            alpha=None):
+    """``out[e] (+)= dy[rows_e]ᵀ @ x[rows_e]`` -> ``[E?, N_out, K_in]``; fp32 or bf16 output.  ``alpha``: fp32 device
+    scalar that multiplies the product."""
     R, M = dy.shape
     N = x.shape[1]
-    if M <= 16 and expert_offsets is None:
+    if M <= 16 and expert_offsets is None and alpha is None:
         if out is None:
             out = torch.zeros(M, N, dtype=torch.float32, device=dy.device)
             accumulate = True
@@ -348,7 +351,7 @@ def gemm_tn(dy, x, out=None, accumulate: bool = False, out_dtype=None, expert_of
     assert dy.stride(-1) == 1 and x.stride(-1) == 1 and out.is_contiguous()
     _call("b2_gemm_tn", _p(_bf16(dy)), _p(_bf16(x)), _p(out), _I(M), _I(N), _I(R), _L(dy.stride(0)), _L(x.stride(0)),
           _L(N), _I(num_experts), _p(expert_offsets), _I(kind), _F(1.0 if accumulate else 0.0),
-          _p(status_word(dy.device)), _stream(),
+          _p(alpha), _p(status_word(dy.device)), _stream(),
           tag=f"{'grouped ' if expert_offsets is not None else ''}{M}x{N} {'fp32' if kind == 1 else 'bf16'}")
     return out if want is None or want == out.dtype else out.to(want)
 

@@ -206,6 +206,49 @@ def test_router_linear_and_top2(native):
     assert _rel(x.grad, xr.grad) < 1e-2 and _rel(w.grad, wr.grad) < 1e-2
 
 
+@pytest.mark.parametrize("T,N,K", [(1, 2, 8), (31, 5, 264), (33, 8, 520), (300, 9, 512), (2051, 16, 1032)])
+def test_skinny_products(native, T, N, K):
+    """Router-shaped products: token counts around the four-token and 32-token groups, outputs on both sides of eight,
+    widths that leave lanes and column blocks partly empty.  fp32 sums of bf16 products: 1e-5; bf16 output: 2^-8."""
+    torch.manual_seed(T)
+    x, w = _rand(T, K), _rand(N, K)
+    dy = torch.randn(T, N, device="cuda")
+    assert _rel(native.gemm_nt(x, w).double(), x.double() @ w.double().t()) < 1e-5
+    assert _rel(native.gemm_nn(dy, w).double(), dy.double() @ w.double()) < 4e-3
+    base = torch.randn(N, K, device="cuda")
+    got = native.gemm_tn(dy, x, out=base.clone(), accumulate=True)
+    assert _rel(got.double() - base.double(), dy.double().t() @ x.double()) < 1e-5
+    native.check_status()
+
+
+@pytest.mark.parametrize("keep", [True, False])
+def test_lm_head_without_a_known_factor_keeps_or_rebuilds_its_logits(native, keep, monkeypatch):
+    """Both forms of the head against 64 bits, with a factor on the loss, twice through the same graph (nothing that
+    the first backward pass read is changed by it), for a weight gradient and for an accumulator."""
+    from b200moe import ops
+    from b200moe.ops import loss as L
+    if not keep:
+        monkeypatch.setattr(L, "KEEP_BYTES", 0)
+        monkeypatch.setattr(L, "CHUNK_TOKENS", 96)
+    torch.manual_seed(3)
+    T, D, V = 201, 128, 640
+    hidden, weight = _rand(T, D).requires_grad_(True), _rand(V, D, scale=0.1).requires_grad_(True)
+    targets = torch.randint(0, V, (T,), device="cuda")
+    h64, w64 = (t.detach().double().requires_grad_(True) for t in (hidden, weight))
+    (3 * torch.nn.functional.cross_entropy(h64 @ w64.t(), targets)).backward()
+    loss = ops.lm_head_cross_entropy(hidden, weight, targets)
+    for _ in range(2):
+        hidden.grad = weight.grad = None
+        (3 * loss).backward(retain_graph=True)
+        # bf16 logits, dlogits and results: three roundings of 2^-9
+        assert _rel(hidden.grad, h64.grad) < 8e-3 and _rel(weight.grad, w64.grad) < 8e-3
+    weight.main_grad = torch.ones(V, D, device="cuda")
+    hidden.grad = None
+    (3 * ops.lm_head_cross_entropy(hidden, weight, targets)).backward()
+    assert _rel(weight.main_grad - 1, w64.grad) < 8e-3 and _rel(hidden.grad, h64.grad) < 8e-3
+    native.check_status()
+
+
 def test_cross_entropy_and_lm_head(native):
     from b200moe import ops
     T, D, V = 512, 256, 32000
