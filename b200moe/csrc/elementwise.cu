@@ -264,6 +264,56 @@ __global__ void __launch_bounds__(256) column_sum_kernel(const float* __restrict
   }
 }
 
+// ------------------------------------------------------------------ router softmax / top-2
+constexpr int ROUTER_MAX_E = 64;
+
+// Softmax over E <= MAXE experts and the renormalised weights of the two largest, one thread per row.
+template <int MAXE>
+__device__ __forceinline__ void top2_row(const float* __restrict__ logits, float* __restrict__ weights,
+                                         long long* __restrict__ idx, float* __restrict__ probs, int E) {
+  float p[MAXE];
+  float mx = -INFINITY;
+  for (int e = 0; e < E; ++e) {
+    p[e] = logits[e];
+    mx = fmaxf(mx, p[e]);
+  }
+  float sum = 0.f;
+  for (int e = 0; e < E; ++e) {
+    p[e] = __expf(p[e] - mx);
+    sum += p[e];
+  }
+  const float inv = 1.f / sum;
+  int a = 0, b = -1;
+  float pa = -1.f, pb = -1.f;
+  for (int e = 0; e < E; ++e) {
+    p[e] *= inv;
+    probs[e] = p[e];
+    if (p[e] > pa) {           // strict: ties keep the lower index first, like topk
+      pb = pa; b = a;
+      pa = p[e]; a = e;
+    } else if (p[e] > pb) {
+      pb = p[e]; b = e;
+    }
+  }
+  if (b < 0) {                 // only reachable with non-finite logits: keep the indices valid
+    b = a == 0 ? 1 : 0;
+    pb = p[b];
+  }
+  const float s = pa + pb;
+  weights[0] = pa / s;
+  weights[1] = pb / s;
+  idx[0] = a;
+  idx[1] = b;
+}
+
+__global__ void router_top2_fwd_kernel(const float* __restrict__ logits, float* __restrict__ weights,
+                                       long long* __restrict__ idx, float* __restrict__ probs, int T, int E) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= T) return;
+  const size_t row = static_cast<size_t>(t) * E;
+  top2_row<ROUTER_MAX_E>(logits + row, weights + 2 * static_cast<size_t>(t), idx + 2 * static_cast<size_t>(t), probs + row, E);
+}
+
 // ------------------------------------------------------------------ skinny linear (router: N <= 16 outputs)
 constexpr int SKINNY_MAX_N = 16;
 
@@ -292,12 +342,15 @@ __device__ __forceinline__ float warp_sum_scatter(float (&v)[32], int lane) {
   return v[0];
 }
 
-// logits[t, n] = sum_k x[t,k] w[n,k]; weights in shared memory.  NN: N rounded up to 8 or 16.
-template <int NN>
+// logits[t, n] = sum_k x[t,k] w[n,k]; weights in shared memory.  NN: N rounded up to 8 or 16.  With TOP2 the router's
+// softmax and choice follow in the same launch (four lanes, a token each).
+template <int NN, bool TOP2>
 __global__ void __launch_bounds__(256) skinny_nt_kernel(const __nv_bfloat16* __restrict__ x,
                                                         const __nv_bfloat16* __restrict__ w, float* __restrict__ out,
-                                                        int T, int N, int K) {
+                                                        float* __restrict__ weights, long long* __restrict__ idx,
+                                                        float* __restrict__ probs, int T, int N, int K) {
   extern __shared__ __nv_bfloat16 ws[];
+  __shared__ float chosen[TOP2 ? 8 : 1][SKINNY_TOKENS][NN];
   skinny_stage(ws, w, N * K);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int t0 = (blockIdx.x * 8 + warp) * SKINNY_TOKENS; t0 < T; t0 += gridDim.x * 8 * SKINNY_TOKENS) {
@@ -339,6 +392,13 @@ __global__ void __launch_bounds__(256) skinny_nt_kernel(const __nv_bfloat16* __r
       const float sum = warp_sum_scatter(acc[h], lane);
       const int t = t0 + lane / 8, n = h * 8 + lane % 8;
       if (t < T && n < N) out[static_cast<size_t>(t) * N + n] = sum;
+      if (TOP2) chosen[warp][lane / 8][n] = sum;
+    }
+    if (TOP2) {
+      __syncwarp();
+      const size_t t = t0 + lane;
+      if (lane < SKINNY_TOKENS && t < T) top2_row<NN>(chosen[warp][lane], weights + 2 * t, idx + 2 * t, probs + t * N, N);
+      __syncwarp();
     }
   }
 }
@@ -429,48 +489,7 @@ __global__ void __launch_bounds__(256) skinny_tn_kernel(const float* __restrict_
   }
 }
 
-// ------------------------------------------------------------------ router softmax / top-2
-constexpr int ROUTER_MAX_E = 64;
-
-__global__ void router_top2_fwd_kernel(const float* __restrict__ logits, float* __restrict__ weights,
-                                       long long* __restrict__ idx, float* __restrict__ probs, int T, int E) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= T) return;
-  float p[ROUTER_MAX_E];
-  float mx = -INFINITY;
-  for (int e = 0; e < E; ++e) {
-    p[e] = logits[static_cast<size_t>(t) * E + e];
-    mx = fmaxf(mx, p[e]);
-  }
-  float sum = 0.f;
-  for (int e = 0; e < E; ++e) {
-    p[e] = __expf(p[e] - mx);
-    sum += p[e];
-  }
-  const float inv = 1.f / sum;
-  int a = 0, b = -1;
-  float pa = -1.f, pb = -1.f;
-  for (int e = 0; e < E; ++e) {
-    p[e] *= inv;
-    probs[static_cast<size_t>(t) * E + e] = p[e];
-    if (p[e] > pa) {           // strict: ties keep the lower index first, like topk
-      pb = pa; b = a;
-      pa = p[e]; a = e;
-    } else if (p[e] > pb) {
-      pb = p[e]; b = e;
-    }
-  }
-  if (b < 0) {                 // only reachable with non-finite logits: keep the indices valid
-    b = a == 0 ? 1 : 0;
-    pb = p[b];
-  }
-  const float s = pa + pb;
-  weights[2 * t] = pa / s;
-  weights[2 * t + 1] = pb / s;
-  idx[2 * t] = a;
-  idx[2 * t + 1] = b;
-}
-
+// ------------------------------------------------------------------ router backward
 __global__ void router_top2_bwd_kernel(const float* __restrict__ dweights, const float* __restrict__ probs,
                                        const long long* __restrict__ idx, const float* __restrict__ weights,
                                        float* __restrict__ dlogits, int T, int E) {
@@ -875,22 +894,36 @@ int b2_rmsnorm_bwd(const void* dy, const void* x, const float* w, const float* r
   return ok();
 }
 
+}  // extern "C"
+
 // One CTA covers 32 tokens per turn; at most two per SM, so that the weights are staged once for many tokens.
 static int skinny_grid(int T) { return min((T + 31) / 32, sm_count_ew() * 2); }
 
-int b2_skinny_nt(const void* x, const void* w, float* out, int T, int N, int K, cudaStream_t s) {
-  if (N > SKINNY_MAX_N || K % 8 || (N * K) % 8) return -10;
+template <bool TOP2>
+static int launch_skinny_nt(const void* x, const void* w, float* out, float* weights, long long* idx, float* probs, int T,
+                            int N, int K, cudaStream_t s) {
   const size_t smem = static_cast<size_t>(N) * K * 2;
   if (smem > 200 * 1024) return -11;
   static bool set = false;
   if (!set) {
-    cudaFuncSetAttribute(skinny_nt_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(skinny_nt_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(skinny_nt_kernel<8, TOP2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(skinny_nt_kernel<16, TOP2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     set = true;
   }
-  if (N <= 8) skinny_nt_kernel<8><<<skinny_grid(T), 256, smem, s>>>((const bf16*)x, (const bf16*)w, out, T, N, K);
-  else skinny_nt_kernel<16><<<skinny_grid(T), 256, smem, s>>>((const bf16*)x, (const bf16*)w, out, T, N, K);
+  auto kernel = N <= 8 ? skinny_nt_kernel<8, TOP2> : skinny_nt_kernel<16, TOP2>;
+  kernel<<<skinny_grid(T), 256, smem, s>>>((const bf16*)x, (const bf16*)w, out, weights, idx, probs, T, N, K);
   return ok();
+}
+extern "C" {
+int b2_skinny_nt(const void* x, const void* w, float* out, int T, int N, int K, cudaStream_t s) {
+  if (N > SKINNY_MAX_N || K % 8 || (N * K) % 8) return -10;
+  return launch_skinny_nt<false>(x, w, out, nullptr, nullptr, nullptr, T, N, K, s);
+}
+// Router in one launch: logits[T,N] = x w^T, their softmax ``probs``, the two largest (idx) and their weights.
+int b2_router_fwd(const void* x, const void* w, float* logits, float* weights, long long* idx, float* probs, int T, int N,
+                  int K, cudaStream_t s) {
+  if (N < 2 || N > SKINNY_MAX_N || K % 8 || (N * K) % 8) return -10;
+  return launch_skinny_nt<true>(x, w, logits, weights, idx, probs, T, N, K, s);
 }
 int b2_skinny_nn(const float* dy, const void* w, void* dx, int T, int N, int K, cudaStream_t s) {
   if (N > SKINNY_MAX_N || K % 8) return -10;

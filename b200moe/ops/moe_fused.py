@@ -35,67 +35,128 @@ def _wgrad(dy, x, param, offs, num_experts):
     return native.gemm_tn(dy, x, out_dtype=param.dtype, expert_offsets=offs, num_experts=num_experts)
 
 
+def _experts_forward(x, weights, idx, w1, w2, w3, recompute, budget, wants_grad, residual=None):
+    """Plan, gather, gate/up, down projection and combine.  Returns ``(out, recompute, ledger, saved)``."""
+    tokens, dim = x.shape
+    experts = w1.shape[0]
+    cap = capacity_rows(tokens * 2, experts)
+    slot_row, row_slot, offs, tile_expert, meta, _ = native.moe_plan(idx, experts, cap)
+    x_perm = native.moe_gather(x, row_slot, meta, cap)
+    tiles = meta[0:1]
+    # what this call keeps for its backward pass: the permuted input and the expert outputs always, the
+    # gate/up pre-activations while the stage's activation budget has room for them
+    ledger = None
+    if budget is not None and wants_grad:
+        ledger = (cap * dim * 4, cap * w1.shape[1] * 4)
+        kept = budget.enter(*ledger)
+        recompute = recompute or not kept
+        ledger += (not recompute,)
+    h, gate, up = native.gemm_swiglu(x_perm, w1, w3, tile_expert, tiles, save_gate_up=not recompute, align256=True)
+    y_perm = native.gemm_nt(h, w2, tile_expert=tile_expert, num_m_tiles=tiles, num_experts=experts, align256=True)
+    out = native.moe_combine(y_perm, slot_row, weights, tokens, residual=residual)
+    saved = [x_perm, y_perm, weights, offs, tile_expert, meta, slot_row, row_slot]
+    if not recompute:
+        saved += [gate, up]
+    return out, recompute, ledger, saved
+
+
+def _experts_backward(dout, saved, w1, w2, w3, recompute):
+    """Returns ``(dx_perm, dweights, dw1, dw2, dw3)``."""
+    x_perm, y_perm, weights, offs, tile_expert, meta, slot_row, row_slot = saved[:8]
+    tokens, cap, experts, ffn = weights.shape[0], x_perm.shape[0], w1.shape[0], w1.shape[1]
+    tiles = meta[0:1]
+    if recompute:
+        _, gate, up = native.gemm_swiglu(x_perm, w1, w3, tile_expert, tiles, save_gate_up=True, align256=True)
+    else:
+        gate, up = saved[8:10]
+    dweights = torch.empty(tokens, 2, dtype=torch.float32, device=dout.device)   # every slot has its row
+    dy_perm = native.moe_gather(dout, row_slot, meta, cap, scale=weights.view(-1), y_perm=y_perm,
+                                dweights=dweights.view(-1))
+    dgu, h = native.gemm_nn_swiglu_bwd(dy_perm, w2, gate, up, tile_expert=tile_expert, num_m_tiles=tiles,
+                                       num_experts=experts, align256=True, live_rows=meta[1:2])
+    del gate, up
+    dx_perm = native.gemm_nn(dgu, w1, w2=w3, tile_expert=tile_expert, num_m_tiles=tiles, num_experts=experts,
+                             align256=True)
+    dw2 = _wgrad(dy_perm, h, w2, offs, experts)
+    dw1 = _wgrad(dgu[:, :ffn], x_perm, w1, offs, experts)
+    dw3 = _wgrad(dgu[:, ffn:], x_perm, w3, offs, experts)
+    return dx_perm, dweights, dw1, dw2, dw3
+
+
 class _MoEFused(torch.autograd.Function):
-    """The block when the expert group is this rank alone."""
+    """The experts for given routing weights, when the expert group is this rank alone."""
 
     @staticmethod
     def forward(ctx, x, weights, idx, w1, w2, w3, recompute, budget):
-        tokens, dim = x.shape
-        experts = w1.shape[0]
         x = x.contiguous()
         weights = weights.float().contiguous()
-        cap = capacity_rows(tokens * 2, experts)
-        slot_row, row_slot, offs, tile_expert, meta, _ = native.moe_plan(idx, experts, cap)
-        x_perm = native.moe_gather(x, row_slot, meta, cap)
-        tiles = meta[0:1]
-        # what this call keeps for its backward pass: the permuted input and the expert outputs always, the
-        # gate/up pre-activations while the stage's activation budget has room for them
-        ledger = None
-        if budget is not None and any(ctx.needs_input_grad):
-            ledger = (cap * dim * 4, cap * w1.shape[1] * 4)
-            kept = budget.enter(*ledger)
-            recompute = recompute or not kept
-            ledger += (not recompute,)
-        h, gate, up = native.gemm_swiglu(x_perm, w1, w3, tile_expert, tiles, save_gate_up=not recompute, align256=True)
-        y_perm = native.gemm_nt(h, w2, tile_expert=tile_expert, num_m_tiles=tiles, num_experts=experts, align256=True)
-        out = native.moe_combine(y_perm, slot_row, weights, tokens)
-        ctx.params = (w1, w2, w3)
-        ctx.meta_py = (tokens, dim, experts, cap, recompute)
-        ctx.budget, ctx.ledger = budget, ledger
-        saved = [x_perm, y_perm, weights, offs, tile_expert, meta, slot_row, row_slot]
-        if not recompute:
-            saved += [gate, up]
+        out, ctx.recompute, ctx.ledger, saved = _experts_forward(x, weights, idx, w1, w2, w3, recompute, budget,
+                                                                 any(ctx.needs_input_grad))
+        ctx.params, ctx.budget = (w1, w2, w3), budget
         ctx.save_for_backward(*saved)
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        w1, w2, w3 = ctx.params
-        tokens, dim, experts, cap, recompute = ctx.meta_py
-        saved = list(ctx.saved_tensors)
-        x_perm, y_perm, weights, offs, tile_expert, meta, slot_row, row_slot = saved[:8]
-        tiles = meta[0:1]
-        dout = dout.contiguous()
-        ffn = w1.shape[1]
-        if recompute:
-            _, gate, up = native.gemm_swiglu(x_perm, w1, w3, tile_expert, tiles, save_gate_up=True, align256=True)
-        else:
-            gate, up = saved[8:10]
-        dweights = torch.empty(tokens, 2, dtype=torch.float32, device=dout.device)   # every slot has its row
-        dy_perm = native.moe_gather(dout, row_slot, meta, cap, scale=weights.view(-1), y_perm=y_perm,
-                                    dweights=dweights.view(-1))
-        dgu, h = native.gemm_nn_swiglu_bwd(dy_perm, w2, gate, up, tile_expert=tile_expert, num_m_tiles=tiles,
-                                           num_experts=experts, align256=True, live_rows=meta[1:2])
-        del gate, up
-        dx_perm = native.gemm_nn(dgu, w1, w2=w3, tile_expert=tile_expert, num_m_tiles=tiles, num_experts=experts,
-                                 align256=True)
-        dw2 = _wgrad(dy_perm, h, w2, offs, experts)
-        dw1 = _wgrad(dgu[:, :ffn], x_perm, w1, offs, experts)
-        dw3 = _wgrad(dgu[:, ffn:], x_perm, w3, offs, experts)
-        dx = native.moe_combine(dx_perm, slot_row, None, tokens)
+        saved = ctx.saved_tensors
+        dx_perm, dweights, dw1, dw2, dw3 = _experts_backward(dout.contiguous(), saved, *ctx.params, ctx.recompute)
+        dx = native.moe_combine(dx_perm, saved[6], None, dweights.shape[0])
         if ctx.ledger is not None:
             ctx.budget.leave(*ctx.ledger)
         return dx, dweights, None, dw1, dw2, dw3, None, None
+
+
+class _MoELayer(torch.autograd.Function):
+    """Router and experts of one rank as one node: the router's product, softmax and choice are one launch, and so are
+    its backward, its share of ``dx``, the combine of the expert rows and the sum of both.  ``residual``, if given, is
+    added by the forward combine.  Also returns the logits (an auxiliary loss may send a gradient back through them)
+    and the chosen experts."""
+
+    @staticmethod
+    def forward(ctx, x, router_w, w1, w2, w3, residual, recompute, budget):
+        ctx.set_materialize_grads(False)
+        logits, weights, idx, probs = native.router_fwd(x, router_w)
+        out, ctx.recompute, ctx.ledger, saved = _experts_forward(x, weights, idx, w1, w2, w3, recompute, budget,
+                                                                 any(ctx.needs_input_grad), residual)
+        ctx.params, ctx.router_w, ctx.budget = (w1, w2, w3), router_w, budget
+        ctx.mark_non_differentiable(idx)
+        ctx.save_for_backward(x, probs, idx, *saved)
+        return out, logits, idx
+
+    @staticmethod
+    def backward(ctx, dout, dlogits_extra, _didx):
+        x, probs, idx, *saved = ctx.saved_tensors
+        router_w = ctx.router_w
+        dresidual = dout if ctx.needs_input_grad[5] else None
+        if dout is None:
+            dout = torch.zeros_like(x)
+        if dlogits_extra is not None:
+            dlogits_extra = dlogits_extra.float().contiguous()
+        dx_perm, dweights, dw1, dw2, dw3 = _experts_backward(dout.contiguous(), saved, *ctx.params, ctx.recompute)
+        dx, dlogits = native.moe_dx(dx_perm, saved[6], dweights, probs, idx, saved[2], router_w, dlogits_extra)
+        main_grad = getattr(router_w, "main_grad", None)
+        drouter = None
+        if main_grad is not None:
+            native.gemm_tn(dlogits, x, out=main_grad, accumulate=True)
+        elif ctx.needs_input_grad[1]:
+            drouter = native.gemm_tn(dlogits, x, out_dtype=router_w.dtype)
+        if ctx.ledger is not None:
+            ctx.budget.leave(*ctx.ledger)
+        return dx, drouter, dw1, dw2, dw3, dresidual, None, None
+
+
+def moe_layer_fused(x, router_w, w1, w2, w3, residual=None, recompute: bool = False, budget=None):
+    """``(out, logits, idx)`` of a routed layer on one rank, or ``None`` where the router has to run by itself: more
+    than 16 experts (or more router weights than a CTA stages), a weight that is still to be gathered, layouts that the
+    16-byte accesses do not take."""
+    experts, dim = router_w.shape
+    if not (2 <= experts <= 16 and experts == w1.shape[0] and dim == x.shape[1] and dim % 8 == 0
+            and experts * dim * 2 <= 200 * 1024 and x.shape[0] > 0
+            and getattr(router_w, "pending_gather", None) is None
+            and all(t.dtype == torch.bfloat16 and t.is_contiguous() and t.data_ptr() % 16 == 0
+                    for t in ((x, router_w) if residual is None else (x, router_w, residual)))):
+        return None
+    return _MoELayer.apply(x, router_w, w1, w2, w3, residual, recompute, budget)
 
 
 def moe_ffn_fused(x, weights, idx, w1, w2, w3, recompute: bool = False, budget=None):

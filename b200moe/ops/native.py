@@ -421,6 +421,18 @@ def router_top2_bwd(dweights, probs, idx, weights):
     return dlogits
 
 
+def router_fwd(x, w):
+    """Router product, softmax and top-2 in one launch (``w [E, D]`` bf16, E <= 16): ``(logits, weights, idx, probs)``."""
+    T, K = x.shape
+    E = w.shape[0]
+    logits, probs = torch.empty(2, T, E, dtype=torch.float32, device=x.device)
+    weights = torch.empty(T, 2, dtype=torch.float32, device=x.device)
+    idx = torch.empty(T, 2, dtype=torch.int64, device=x.device)
+    _call("b2_router_fwd", _p(_bf16(x)), _p(_bf16(w)), _p(logits), _p(weights), _p(idx), _p(probs), _I(T), _I(E), _I(K),
+          _stream())
+    return logits, weights, idx, probs
+
+
 # ------------------------------------------------------------------------------ loss
 def cross_entropy_fwd_bwd_(logits, targets):
     """Mean loss; ``logits`` (bf16 [T,V]) is overwritten with d(mean loss)/dlogits."""
@@ -634,6 +646,17 @@ def moe_combine(y_perm, slot_row, weights, tokens, residual=None):
     _call("b2_moe_combine", _p(_bf16(y_perm)), _p(slot_row), _p(weights), _p(residual), _p(out), _I(tokens), _I(D),
           _I(y_perm.shape[0]), _stream())
     return out
+
+
+def moe_dx(dy_perm, slot_row, dweights, probs, idx, weights, router_w, dlogits_extra=None):
+    """Input gradient of a routed layer: the two rows of each token plus the router's share; returns ``(dx, dlogits)``."""
+    T, E = probs.shape
+    D = dy_perm.shape[1]
+    dlogits = torch.empty(T, E, dtype=torch.float32, device=dy_perm.device)
+    dx = torch.empty(T, D, dtype=torch.bfloat16, device=dy_perm.device)
+    _call("b2_moe_dx", _p(_bf16(dy_perm)), _p(slot_row), _p(dweights), _p(probs), _p(idx), _p(weights), _p(dlogits_extra),
+          _p(_bf16(router_w)), _p(dlogits), _p(dx), _I(T), _I(E), _I(D), _I(dy_perm.shape[0]), _stream())
+    return dx, dlogits
 
 
 def swiglu_bwd(dh, gate, up, live_rows=None, want_h: bool = True):

@@ -427,6 +427,39 @@ def test_moe_block_with_fused_exchange_on_a_single_rank_group(native, tile_mode,
     native.check_status()
 
 
+@pytest.mark.parametrize("T,E", [(1, 2), (33, 8), (257, 9), (130, 16)])
+@pytest.mark.parametrize("aux", [False, True])
+def test_routed_layer_as_one_op_against_its_separate_steps(native, T, E, aux):
+    """Router, experts and the residual as one op against the separate router, top-2 and expert ops (a hook on the
+    router sends the layer there): token counts around the four-token groups, experts on both sides of eight.  The two
+    round the input gradient and the sum with the residual differently: three roundings of 2^-9."""
+    from b200moe.models.layers import MoELayerMulti
+    torch.manual_seed(T)
+    D, F = 128, 256
+    with torch.device("cuda"):
+        layer = MoELayerMulti(D, F, num_expert_per_node=E)
+    layer.router.compute_weight = layer.router.weight.detach().bfloat16().requires_grad_(True)
+    router = layer.router.compute_weight
+    x, residual, dy = _rand(T, D), _rand(T, D), _rand(T, D)
+    results = []
+    for separate in (False, True):
+        handle = layer.router.register_forward_hook(lambda *_: None) if separate else None
+        leaves = [t.clone().requires_grad_(True) for t in (x, residual)]
+        for p in (*layer.experts.parameters(), router):
+            p.grad = None
+        out = layer._forward(leaves[0], aux, leaves[1])
+        out, extra = out if aux else (out, None)
+        torch.autograd.backward([out] + ([extra] if aux else []), [dy] + ([torch.full_like(extra, 0.5)] if aux else []))
+        assert (type(out.grad_fn.next_functions[0][0]).__name__ == "_MoELayerBackward") or separate
+        results.append([out.detach(), *([extra.detach()] if aux else []), leaves[0].grad, leaves[1].grad, router.grad,
+                        *(p.grad for p in layer.experts.parameters())])
+        if handle:
+            handle.remove()
+    for got, want in zip(*results):
+        assert _rel(got, want) < 8e-3
+    native.check_status()
+
+
 def test_tiny_model_native_vs_torch_path(native):
     from b200moe import ops
     from b200moe.models import TransformerLMPipelined
