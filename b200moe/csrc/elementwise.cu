@@ -698,36 +698,61 @@ __device__ __forceinline__ void st8<__nv_bfloat16>(__nv_bfloat16* p, const float
   *reinterpret_cast<bf16x8*>(p) = pack8(f);
 }
 
+// Up to ADAMW_MAX tensors of the same types per launch; the table travels as a kernel argument.  Tensors are cut into
+// blocks of ADAMW_CHUNK elements that the CTAs take in turn, so that gains of a few thousand elements share a launch
+// with expert stacks (one launch per tensor left the chip idle between them).  Bound by memory traffic.
+constexpr int ADAMW_MAX = 48;
+constexpr int ADAMW_CHUNK = 8192;
+struct AdamwTensor {
+  void* p;
+  const void* g;
+  void* m;
+  void* v;
+  __nv_bfloat16* p_bf16;     // optional copy of the new p
+  long long n;
+};
+struct AdamwTable {
+  AdamwTensor t[ADAMW_MAX];
+  int first_chunk[ADAMW_MAX + 1];
+  int count;
+};
+
 // p <- p(1 - lr*wd); m, v moments; p <- p - a_t m/(sqrt(v)+eps).  Optional bf16 copy of the new p.
 // Eight elements per thread as 16/32-byte vectors; the last n % 8 elements go one by one.
 template <typename P, typename G, typename S>
-__global__ void adamw_kernel(P* __restrict__ p, const G* __restrict__ g, S* __restrict__ m, S* __restrict__ v,
-                             __nv_bfloat16* __restrict__ p_bf16, size_t n, float lr, float beta1, float beta2,
-                             float eps, float wd, float a_t, float grad_scale) {
-  const size_t vecs = n / 8;
+__global__ void __launch_bounds__(256) adamw_kernel(const __grid_constant__ AdamwTable table, float lr, float beta1,
+                                                    float beta2, float eps, float wd, float a_t, float grad_scale) {
   const float decay = 1.f - lr * wd;
-  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < vecs;
-       i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const size_t o = i * 8;
-    float pv[8], gv[8], mv[8], vv[8];
-    ld8(p + o, pv);
-    ld8(g + o, gv);
-    ld8(m + o, mv);
-    ld8(v + o, vv);
+  int which = 0;
+  for (int chunk = blockIdx.x; chunk < table.first_chunk[table.count]; chunk += gridDim.x) {
+    while (chunk >= table.first_chunk[which + 1]) ++which;
+    const AdamwTensor& t = table.t[which];
+    P* __restrict__ p = static_cast<P*>(t.p);
+    const G* __restrict__ g = static_cast<const G*>(t.g);
+    S* __restrict__ m = static_cast<S*>(t.m);
+    S* __restrict__ v = static_cast<S*>(t.v);
+    const size_t begin = static_cast<size_t>(chunk - table.first_chunk[which]) * ADAMW_CHUNK;
+    const size_t n = static_cast<size_t>(t.n);
+    const size_t end = begin + ADAMW_CHUNK < n ? begin + ADAMW_CHUNK : n;
+    for (size_t o = begin + threadIdx.x * 8; o + 8 <= end; o += 256 * 8) {
+      float pv[8], gv[8], mv[8], vv[8];
+      ld8(p + o, pv);
+      ld8(g + o, gv);
+      ld8(m + o, mv);
+      ld8(v + o, vv);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float gj = gv[j] * grad_scale;
-      mv[j] = beta1 * mv[j] + (1.f - beta1) * gj;
-      vv[j] = beta2 * vv[j] + (1.f - beta2) * gj * gj;
-      pv[j] = pv[j] * decay - a_t * mv[j] / (sqrtf(vv[j]) + eps);
+      for (int j = 0; j < 8; ++j) {
+        const float gj = gv[j] * grad_scale;
+        mv[j] = beta1 * mv[j] + (1.f - beta1) * gj;
+        vv[j] = beta2 * vv[j] + (1.f - beta2) * gj * gj;
+        pv[j] = pv[j] * decay - a_t * mv[j] / (sqrtf(vv[j]) + eps);
+      }
+      st8(p + o, pv);
+      st8(m + o, mv);
+      st8(v + o, vv);
+      if (t.p_bf16) st8(t.p_bf16 + o, pv);
     }
-    st8(p + o, pv);
-    st8(m + o, mv);
-    st8(v + o, vv);
-    if (p_bf16) st8(p_bf16 + o, pv);
-  }
-  if (blockIdx.x == 0) {
-    for (size_t i = vecs * 8 + threadIdx.x; i < n; i += blockDim.x) {
+    for (size_t i = begin + (end - begin) / 8 * 8 + threadIdx.x; i < end; i += 256) {   // only behind the last vector
       const float gj = ldf(g, i) * grad_scale;
       const float mj = beta1 * ldf(m, i) + (1.f - beta1) * gj;
       const float vj = beta2 * ldf(v, i) + (1.f - beta2) * gj * gj;
@@ -735,8 +760,31 @@ __global__ void adamw_kernel(P* __restrict__ p, const G* __restrict__ g, S* __re
       stf(p, i, pj);
       stf(m, i, mj);
       stf(v, i, vj);
-      if (p_bf16) p_bf16[i] = __float2bfloat16_rn(pj);
+      if (t.p_bf16) t.p_bf16[i] = __float2bfloat16_rn(pj);
     }
+  }
+}
+
+// Zeros into up to ZERO_MAX buffers in one launch: 64 KiB blocks in turn, 16-byte stores.  Write-bandwidth bound.
+constexpr int ZERO_MAX = 64;
+constexpr int ZERO_CHUNK = 65536;
+struct ZeroTable {
+  uint8_t* p[ZERO_MAX];
+  long long bytes[ZERO_MAX];
+  int first_chunk[ZERO_MAX + 1];
+  int count;
+};
+__global__ void __launch_bounds__(256) zero_kernel(const __grid_constant__ ZeroTable table) {
+  int which = 0;
+  for (int chunk = blockIdx.x; chunk < table.first_chunk[table.count]; chunk += gridDim.x) {
+    while (chunk >= table.first_chunk[which + 1]) ++which;
+    const size_t begin = static_cast<size_t>(chunk - table.first_chunk[which]) * ZERO_CHUNK;
+    const size_t left = static_cast<size_t>(table.bytes[which]) - begin;
+    const int bytes = left < ZERO_CHUNK ? static_cast<int>(left) : ZERO_CHUNK;
+    uint8_t* dst = table.p[which] + begin;
+#pragma unroll 4
+    for (int i = threadIdx.x * 16; i + 16 <= bytes; i += 256 * 16) *reinterpret_cast<uint4*>(dst + i) = make_uint4(0, 0, 0, 0);
+    for (int i = bytes / 16 * 16 + threadIdx.x; i < bytes; i += 256) dst[i] = 0;
   }
 }
 
@@ -997,27 +1045,63 @@ int b2_scale_bf16(void* x, const float* factor, long long n, cudaStream_t s) {
   return ok();
 }
 
-// dtype codes: 0 fp32, 1 bf16.  p_bf16 may be null.
-int b2_adamw(void* p, const void* g, void* m, void* v, void* p_bf16, long long n, int p_dt, int g_dt, int s_dt,
-             float lr, float beta1, float beta2, float eps, float wd, float a_t, float grad_scale, cudaStream_t s) {
-  const int grid = grid_for((n + 7) / 8, 256, 16);
-#define B2_ADAMW(P, G, S)                                                                                      \
-  adamw_kernel<P, G, S><<<grid, 256, 0, s>>>((P*)p, (const G*)g, (S*)m, (S*)v, (bf16*)p_bf16, n, lr, beta1, beta2, \
-                                             eps, wd, a_t, grad_scale)
+// ``count`` tensors of the same types: ``ptrs`` holds p, g, m, v and the optional bf16 copy (0 for none) of each, ``n``
+// the element counts.  dtype codes: 0 fp32, 1 bf16.
+int b2_adamw(const unsigned long long* ptrs, const long long* n, int count, int p_dt, int g_dt, int s_dt, float lr,
+             float beta1, float beta2, float eps, float wd, float a_t, float grad_scale, cudaStream_t s) {
   const int code = p_dt * 4 + g_dt * 2 + s_dt;
-  switch (code) {
-    case 0: B2_ADAMW(float, float, float); break;
-    case 1: B2_ADAMW(float, float, bf16); break;
-    case 2: B2_ADAMW(float, bf16, float); break;
-    case 3: B2_ADAMW(float, bf16, bf16); break;
-    case 4: B2_ADAMW(bf16, float, float); break;
-    case 5: B2_ADAMW(bf16, float, bf16); break;
-    case 6: B2_ADAMW(bf16, bf16, float); break;
-    case 7: B2_ADAMW(bf16, bf16, bf16); break;
-    default: return -10;
-  }
+  if (code < 0 || code > 7) return -10;
+  for (int base = 0; base < count; base += ADAMW_MAX) {
+    AdamwTable table;
+    table.count = min(ADAMW_MAX, count - base);
+    long long chunks = 0;
+    for (int i = 0; i < table.count; ++i) {
+      const unsigned long long* q = ptrs + 5 * (base + i);
+      table.t[i] = {reinterpret_cast<void*>(q[0]), reinterpret_cast<const void*>(q[1]), reinterpret_cast<void*>(q[2]),
+                    reinterpret_cast<void*>(q[3]), reinterpret_cast<bf16*>(q[4]), n[base + i]};
+      table.first_chunk[i] = static_cast<int>(chunks);
+      chunks += (n[base + i] + ADAMW_CHUNK - 1) / ADAMW_CHUNK;
+      if (chunks > 0x7fffffffLL) return -11;
+    }
+    table.first_chunk[table.count] = static_cast<int>(chunks);
+    if (chunks == 0) continue;
+    const int grid = static_cast<int>(min(chunks, static_cast<long long>(sm_count_ew()) * 16));
+#define B2_ADAMW(P, G, S) adamw_kernel<P, G, S><<<grid, 256, 0, s>>>(table, lr, beta1, beta2, eps, wd, a_t, grad_scale)
+    switch (code) {
+      case 0: B2_ADAMW(float, float, float); break;
+      case 1: B2_ADAMW(float, float, bf16); break;
+      case 2: B2_ADAMW(float, bf16, float); break;
+      case 3: B2_ADAMW(float, bf16, bf16); break;
+      case 4: B2_ADAMW(bf16, float, float); break;
+      case 5: B2_ADAMW(bf16, float, bf16); break;
+      case 6: B2_ADAMW(bf16, bf16, float); break;
+      default: B2_ADAMW(bf16, bf16, bf16); break;
+    }
 #undef B2_ADAMW
-  return ok();
+    if (ok()) return -1;
+  }
+  return 0;
+}
+// ``ptrs``: 16-byte aligned buffers of ``bytes`` bytes each.
+int b2_zero(const unsigned long long* ptrs, const long long* bytes, int count, cudaStream_t s) {
+  for (int base = 0; base < count; base += ZERO_MAX) {
+    ZeroTable table;
+    table.count = min(ZERO_MAX, count - base);
+    long long chunks = 0;
+    for (int i = 0; i < table.count; ++i) {
+      if (ptrs[base + i] % 16) return -10;
+      table.p[i] = reinterpret_cast<uint8_t*>(ptrs[base + i]);
+      table.bytes[i] = bytes[base + i];
+      table.first_chunk[i] = static_cast<int>(chunks);
+      chunks += (bytes[base + i] + ZERO_CHUNK - 1) / ZERO_CHUNK;
+      if (chunks > 0x7fffffffLL) return -11;
+    }
+    table.first_chunk[table.count] = static_cast<int>(chunks);
+    if (chunks == 0) continue;
+    zero_kernel<<<static_cast<int>(min(chunks, static_cast<long long>(sm_count_ew()) * 8)), 256, 0, s>>>(table);
+    if (ok()) return -1;
+  }
+  return 0;
 }
 int b2_cast_f32_bf16(const float* src, void* dst, long long n, cudaStream_t s) {
   cast_f32_bf16_kernel<<<grid_for(n, 256, 32), 256, 0, s>>>(src, (bf16*)dst, n);

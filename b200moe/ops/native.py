@@ -461,12 +461,37 @@ def scale_(x, factor):
 _DT = {torch.float32: 0, torch.bfloat16: 1}
 
 
-def adamw_(p, g, m, v, lr, beta1, beta2, eps, weight_decay, a_t, grad_scale=1.0, p_bf16=None):
-    for t in (p, g, m, v):
-        if not t.is_contiguous():
+def adamw_many_(tensors, lr, beta1, beta2, eps, weight_decay, a_t, grad_scale=1.0):
+    """One update of each ``(p, g, m, v, bf16 copy of the new p or None)``; all of the same types, 48 per launch."""
+    ptrs, numels = [], []
+    for p, g, m, v, copy in tensors:
+        if not (p.is_contiguous() and g.is_contiguous() and m.is_contiguous() and v.is_contiguous()):
             raise ValueError("adamw_ needs contiguous tensors")
-    _call("b2_adamw", _p(p), _p(g), _p(m), _p(v), _p(p_bf16), _L(p.numel()), _I(_DT[p.dtype]), _I(_DT[g.dtype]),
-          _I(_DT[m.dtype]), _F(lr), _F(beta1), _F(beta2), _F(eps), _F(weight_decay), _F(a_t), _F(grad_scale), _stream())
+        ptrs += (p.data_ptr(), g.data_ptr(), m.data_ptr(), v.data_ptr(), 0 if copy is None else copy.data_ptr())
+        numels.append(p.numel())
+    p, g, m = tensors[0][:3]
+    count = len(numels)
+    _call("b2_adamw", (ctypes.c_ulonglong * (5 * count))(*ptrs), (_L * count)(*numels), _I(count), _I(_DT[p.dtype]),
+          _I(_DT[g.dtype]), _I(_DT[m.dtype]), _F(lr), _F(beta1), _F(beta2), _F(eps), _F(weight_decay), _F(a_t),
+          _F(grad_scale), _stream(), n=(count + 47) // 48)
+
+
+def adamw_(p, g, m, v, lr, beta1, beta2, eps, weight_decay, a_t, grad_scale=1.0, p_bf16=None):
+    adamw_many_([(p, g, m, v, p_bf16)], lr, beta1, beta2, eps, weight_decay, a_t, grad_scale)
+
+
+def zero_many_(tensors):
+    """Zeros into contiguous tensors (64 per launch).  Buffers that 16-byte stores cannot take are left to PyTorch."""
+    fast = []
+    for t in tensors:
+        if t.is_contiguous() and t.data_ptr() % 16 == 0:
+            fast.append(t)
+        else:
+            t.zero_()
+    count = len(fast)
+    if count:
+        _call("b2_zero", (ctypes.c_ulonglong * count)(*[t.data_ptr() for t in fast]),
+              (_L * count)(*[t.numel() * t.element_size() for t in fast]), _I(count), _stream(), n=(count + 63) // 64)
 
 
 def cast_f32_bf16(src, dst):

@@ -90,11 +90,13 @@ class AdamW(torch.optim.Optimizer):
 
     @torch.no_grad()
     def step(self, closure=None, **kwargs):
+        from ..ops import native, use_native
         for group in self.param_groups:
             lr, beta1, beta2 = group["lr"], group["beta1"], group["beta2"]
             t, eps, decay = group["t"], group["epsilon"], group["lambda_"]
             a_t = lr * math.sqrt(1 - beta2 ** t) / (1 - beta1 ** t)
             done_flats = set()
+            batches: dict = {}          # updates on the GPU kernels, by device, types and gradient factor
             for p in group["params"]:
                 grad = self._grad_of(p)
                 if grad is None:
@@ -109,8 +111,14 @@ class AdamW(torch.optim.Optimizer):
                             adamw_update_(flat.master, flat.shard_grad, flat.m, flat.v,
                                           lr, beta1, beta2, eps, decay, a_t)
                     continue
-                adamw_update_(p.data, grad, m, v, lr, beta1, beta2, eps, decay, a_t,
-                              grad_scale=getattr(p, "_grad_scale", 1.0))
+                scale = getattr(p, "_grad_scale", 1.0)
+                if use_native(p, "adamw"):
+                    key = (p.device, p.dtype, grad.dtype, m.dtype, v.dtype, scale)
+                    batches.setdefault(key, []).append((p.data, grad, m, v, None))
+                    continue
+                adamw_update_(p.data, grad, m, v, lr, beta1, beta2, eps, decay, a_t, grad_scale=scale)
+            for (*_, scale), tensors in batches.items():
+                native.adamw_many_(tensors, lr, beta1, beta2, eps, decay, a_t, scale)
             group["t"] = t + 1
 
     def load_state_dict(self, state_dict):

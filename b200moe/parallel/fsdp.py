@@ -318,11 +318,14 @@ class FSDPWrapperPipelined(nn.Module):
             budget.reset()      # start of a step: no activation of the previous one is alive
         if self.comm is not None and getattr(self, "fused", False):
             self.comm.new_step()
-        self.flat.full_g.zero_()
-        for p in self.sharded_params + self.replicated_params:
-            p.grad = None
-        for p in self.expert_params:
-            p.main_grad.zero_()
+        accumulators = [self.flat.full_g, *(p.main_grad for p in self.expert_params)]
+        from ..ops import native, use_native
+        if all(use_native(t, "adamw") and t.device == accumulators[0].device for t in accumulators):
+            native.zero_many_(accumulators)      # one launch
+        else:
+            for t in accumulators:
+                t.zero_()
+        for p in self.sharded_params + self.replicated_params + self.expert_params:
             p.grad = None
 
     def accumulate_full_gradients(self):

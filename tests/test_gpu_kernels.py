@@ -285,6 +285,44 @@ def test_lm_head_forms_its_gradients_in_the_forward_pass_when_the_loss_factor_is
         assert _rel(w.main_grad, wr.grad) < 3e-2, announced
 
 
+def test_many_tensors_per_optimizer_launch_and_zero_fill(native):
+    """Sizes around the vector, the block and the 48-tensor table, mixed types and gradient factors: the update against
+    the same arithmetic on the CPU, and the zero fill against a guard element on either side."""
+    from b200moe.optim import AdamW
+    torch.manual_seed(7)
+    sizes = [1, 7, 8, 9, 8191, 8192, 8193, 16391] + [130] * 45
+    gpu, cpu = [], []
+    for i, n in enumerate(sizes):
+        dtype = torch.bfloat16 if i % 3 == 0 else torch.float32
+        p = torch.nn.Parameter(torch.randn(n, device="cuda").to(dtype))
+        p.grad = torch.randn(n, device="cuda").to(dtype)
+        q = torch.nn.Parameter(p.detach().cpu().clone())
+        q.grad = p.grad.cpu().clone()
+        if i % 5 == 0:
+            p._grad_scale = q._grad_scale = 0.5
+        gpu.append(p)
+        cpu.append(q)
+    a, b = AdamW(gpu, lr=1e-2), AdamW(cpu, lr=1e-2)
+    before = native.launch_count()
+    a.step()
+    assert native.launch_count() - before == 4          # two types, two factors
+    a.step()
+    b.step()
+    b.step()
+    for p, q in zip(gpu, cpu):
+        tol = 8e-3 if p.dtype == torch.bfloat16 else 1e-6
+        assert _rel(p.detach().cpu(), q.detach()) < tol
+        # the kernel forms 1 - beta2 in fp32: 0.999 is off by up to 2^-25, which is 3e-5 of 0.001
+        assert _rel(a.state[p]["v"].cpu(), b.state[q]["v"]) < 4e-5
+    spans = [torch.ones(n + 8, device="cuda", dtype=torch.bfloat16) for n in (1, 7, 8, 40000, 32760, 32768, 65537)] * 10
+    spans = [t.clone() for t in spans]
+    native.zero_many_([t[8:-1] if t.numel() > 9 else t[8:] for t in spans] + [spans[0][1:3]])
+    for i, t in enumerate(spans):
+        assert t[8:-1].abs().sum() == 0 and (t.numel() <= 9 or t[-1] == 1)
+        assert t[:8].sum() == (6 if i == 0 else 8)
+    native.check_status()
+
+
 def test_embedding_rope_adamw(native):
     from b200moe import ops
     from b200moe.ops import functional as Fn
