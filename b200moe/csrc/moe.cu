@@ -180,8 +180,47 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const __nv_bfloat16* _
   }
 }
 
+// Balance loss of top-2 routing, E * sum_e (counts[e] / A) * (sum_t probs[t,e]) * (2 / A) with A = 2 T assignments, one
+// CTA: a short reduction over T x E probabilities.  (As PyTorch operations: some twenty launches forward and backward
+// per layer, and a bincount that waits for the device.)
+__device__ __forceinline__ float aux_factor(int T, int E) {
+  const float assignments = fmaxf(2.f * T, 1.f);
+  return E * 2.f / (assignments * assignments);
+}
+__global__ void __launch_bounds__(1024) moe_aux_kernel(const float* __restrict__ probs, const int* __restrict__ counts,
+                                                       float* __restrict__ aux, int T, int E) {
+  __shared__ float partial[32];
+  float sum = 0.f;
+  const long long total = static_cast<long long>(T) * E;
+  // a thread's stride is a multiple of E, so it stays in one column
+  const int threads = 1024 / E * E;
+  if (static_cast<int>(threadIdx.x) < threads) {
+    float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+    long long i = threadIdx.x;
+    for (; i + 3LL * threads < total; i += 4LL * threads) {
+      s0 += probs[i];
+      s1 += probs[i + threads];
+      s2 += probs[i + 2LL * threads];
+      s3 += probs[i + 3LL * threads];
+    }
+    for (; i < total; i += threads) s0 += probs[i];
+    sum = ((s0 + s1) + (s2 + s3)) * counts[threadIdx.x % E];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0) partial[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    sum = partial[threadIdx.x];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (threadIdx.x == 0) *aux = sum * aux_factor(T, E);
+  }
+}
+
 // Input gradient of a routed layer on one GPU, in one launch:
-//   dlogits[t] = backward of softmax, top-2 and renormalisation for dweights[t] (+ dlogits_in[t])
+//   dlogits[t] = backward of softmax, top-2 and renormalisation for dweights[t]
+//                (+ daux * d(balance loss)/dlogits[t], which needs the probabilities and the experts' slot counts only)
 //   dx[t] = dy[slot_row[2t]] + dy[slot_row[2t+1]] + dlogits[t] Wr
 // Memory bound (two rows read, one written per token).  A warp works on four tokens at a time, so that an unpacked
 // router weight (shared memory) serves four of them.  Router backward, its input gradient, the combine and the sum of
@@ -192,7 +231,7 @@ __global__ void __launch_bounds__(256) moe_dx_kernel(const __nv_bfloat16* __rest
                                                      const float* __restrict__ dweights,
                                                      const float* __restrict__ probs, const long long* __restrict__ idx,
                                                      const float* __restrict__ weights,
-                                                     const float* __restrict__ dlogits_in,
+                                                     const float* __restrict__ daux, const int* __restrict__ counts,
                                                      const __nv_bfloat16* __restrict__ w, float* __restrict__ dlogits,
                                                      __nv_bfloat16* __restrict__ dx, int T, int N, int D, int rows) {
   extern __shared__ __nv_bfloat16 dx_ws[];
@@ -201,6 +240,7 @@ __global__ void __launch_bounds__(256) moe_dx_kernel(const __nv_bfloat16* __rest
     *reinterpret_cast<vec16*>(dx_ws + i) = *reinterpret_cast<const vec16*>(w + i);
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const float aux_scale = daux ? *daux * aux_factor(T, N) : 0.f;
   for (int t0 = (blockIdx.x * 8 + warp) * DX_TOKENS; t0 < T; t0 += gridDim.x * 8 * DX_TOKENS) {
     if (lane < DX_TOKENS && t0 + lane < T) {
       const size_t t = t0 + lane;
@@ -211,10 +251,14 @@ __global__ void __launch_bounds__(256) moe_dx_kernel(const __nv_bfloat16* __rest
       const float inner = da * weights[2 * t] + db * weights[2 * t + 1];
       const float dpa = (da - inner) / s, dpb = (db - inner) / s;
       const float dot = dpa * pa + dpb * pb;
+      float balance = 0.f;
+      if (daux)
+        for (int e = 0; e < N; ++e) balance += counts[e] * probs[t * N + e];
       for (int e = 0; e < N; ++e) {
         const float dp = e == a ? dpa : (e == b ? dpb : 0.f);
-        float g = probs[t * N + e] * (dp - dot);
-        if (dlogits_in) g += dlogits_in[t * N + e];
+        const float p = probs[t * N + e];
+        float g = p * (dp - dot);
+        if (daux) g += aux_scale * p * (counts[e] - balance);
         grads[warp][lane][e] = g;
         dlogits[t * N + e] = g;
       }
@@ -331,10 +375,17 @@ int b2_moe_combine(const void* y_perm, const int* slot_row, const float* weights
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-// See moe_dx_kernel.  N <= 16 experts; dlogits_in may be null.
+// probs fp32 [T,E], counts int32 [E] -> aux, one fp32 value.
+int b2_moe_aux(const float* probs, const int* counts, float* aux, int T, int E, cudaStream_t s) {
+  if (E < 1 || E > 1024) return -10;
+  moe_aux_kernel<<<1, 1024, 0, s>>>(probs, counts, aux, T, E);
+  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+// See moe_dx_kernel.  N <= 16 experts; daux (device scalar: gradient of the balance loss) and counts may be null.
 int b2_moe_dx(const void* dy, const int* slot_row, const float* dweights, const float* probs, const long long* idx,
-              const float* weights, const float* dlogits_in, const void* w, float* dlogits, void* dx, int T, int N, int D,
-              int rows, cudaStream_t s) {
+              const float* weights, const float* daux, const int* counts, const void* w, float* dlogits, void* dx, int T,
+              int N, int D, int rows, cudaStream_t s) {
   if (N < 2 || N > 16 || D % 8) return -10;
   const size_t smem = static_cast<size_t>(N) * D * 2;
   if (smem > 200 * 1024) return -11;
@@ -346,7 +397,7 @@ int b2_moe_dx(const void* dy, const int* slot_row, const float* dweights, const 
   }
   auto kernel = N <= 8 ? moe_dx_kernel<8> : moe_dx_kernel<16>;
   kernel<<<min((T + 31) / 32, sm_count_moe() * 2), 256, smem, s>>>((const bf16*)dy, slot_row, dweights, probs, idx, weights,
-                                                                   dlogits_in, (const bf16*)w, dlogits, (bf16*)dx, T, N, D, rows);
+                                                                   daux, counts, (const bf16*)w, dlogits, (bf16*)dx, T, N, D, rows);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

@@ -275,7 +275,7 @@ class MoELayerMulti(nn.Module):
     def forward(self, x, return_aux_loss=False):
         return self._forward(x, return_aux_loss, None)
 
-    def _fused(self, flat, residual):
+    def _fused(self, flat, residual, balance):
         """Router and experts as one op: one rank, and nobody watches the router's calls."""
         if not (self.world_size == 1 and ops.use_native(flat, "moe") and type(self.router) is LinearLayer
                 and type(self.experts) is GroupedPositionWiseFFLayer and not _hooked(self.router)):
@@ -283,23 +283,20 @@ class MoELayerMulti(nn.Module):
         from ..ops.moe_fused import moe_layer_fused
         router = self.router.compute_weight if self.router.compute_weight is not None else self.router.weight
         return moe_layer_fused(flat, router, self.experts.w1, self.experts.w2, self.experts.w3, residual,
-                               recompute=self.recompute, budget=self.budget)
+                               recompute=self.recompute, budget=self.budget, balance=balance)
 
     def _forward(self, x, return_aux_loss, residual):
         """The layer's output, plus ``residual`` where one is given (added by the combine kernel of the fused op)."""
         shape, in_dtype = x.shape, x.dtype
         flat = x.reshape(-1, shape[-1]).to(self.dtype)
         same = residual is not None and residual.dtype == in_dtype == self.dtype and residual.shape == shape
-        fused = self._fused(flat, residual.reshape(-1, shape[-1]) if same else None)
+        fused = self._fused(flat, residual.reshape(-1, shape[-1]) if same else None, return_aux_loss)
         if fused is not None:
-            out, logits, idx = fused
+            out, aux = fused if return_aux_loss else (fused, None)
             out = out.view(shape).to(in_dtype)
             if residual is not None and not same:
                 out = residual + out
-            if not return_aux_loss:
-                return out
-            from ..ops.moe import aux_loss_from
-            return out, aux_loss_from(logits, idx, self.num_expert_per_node, self.k, None)
+            return (out, aux) if return_aux_loss else out
         experts_total = self.world_size * self.num_expert_per_node
         ep_ctx = None
         if self.comm is not None and self.world_size > 1 and flat.is_cuda:

@@ -36,11 +36,12 @@ def _wgrad(dy, x, param, offs, num_experts):
 
 
 def _experts_forward(x, weights, idx, w1, w2, w3, recompute, budget, wants_grad, residual=None):
-    """Plan, gather, gate/up, down projection and combine.  Returns ``(out, recompute, ledger, saved)``."""
+    """Plan, gather, gate/up, down projection and combine.  Returns ``(out, recompute, ledger, saved)``; the last of
+    ``saved`` are the experts' slot counts."""
     tokens, dim = x.shape
     experts = w1.shape[0]
     cap = capacity_rows(tokens * 2, experts)
-    slot_row, row_slot, offs, tile_expert, meta, _ = native.moe_plan(idx, experts, cap)
+    slot_row, row_slot, offs, tile_expert, meta, counts = native.moe_plan(idx, experts, cap)
     x_perm = native.moe_gather(x, row_slot, meta, cap)
     tiles = meta[0:1]
     # what this call keeps for its backward pass: the permuted input and the expert outputs always, the
@@ -57,7 +58,7 @@ def _experts_forward(x, weights, idx, w1, w2, w3, recompute, budget, wants_grad,
     saved = [x_perm, y_perm, weights, offs, tile_expert, meta, slot_row, row_slot]
     if not recompute:
         saved += [gate, up]
-    return out, recompute, ledger, saved
+    return out, recompute, ledger, saved + [counts]
 
 
 def _experts_backward(dout, saved, w1, w2, w3, recompute):
@@ -93,7 +94,7 @@ class _MoEFused(torch.autograd.Function):
         out, ctx.recompute, ctx.ledger, saved = _experts_forward(x, weights, idx, w1, w2, w3, recompute, budget,
                                                                  any(ctx.needs_input_grad))
         ctx.params, ctx.budget = (w1, w2, w3), budget
-        ctx.save_for_backward(*saved)
+        ctx.save_for_backward(*saved[:-1])
         return out
 
     @staticmethod
@@ -109,31 +110,32 @@ class _MoEFused(torch.autograd.Function):
 class _MoELayer(torch.autograd.Function):
     """Router and experts of one rank as one node: the router's product, softmax and choice are one launch, and so are
     its backward, its share of ``dx``, the combine of the expert rows and the sum of both.  ``residual``, if given, is
-    added by the forward combine.  Also returns the logits (an auxiliary loss may send a gradient back through them)
-    and the chosen experts."""
+    added by the forward combine.  With ``balance`` the balance loss is a second output, one kernel over the router's
+    probabilities; its gradient joins the router's in the ``dx`` kernel."""
 
     @staticmethod
-    def forward(ctx, x, router_w, w1, w2, w3, residual, recompute, budget):
+    def forward(ctx, x, router_w, w1, w2, w3, residual, recompute, budget, balance):
         ctx.set_materialize_grads(False)
-        logits, weights, idx, probs = native.router_fwd(x, router_w)
+        _, weights, idx, probs = native.router_fwd(x, router_w)
         out, ctx.recompute, ctx.ledger, saved = _experts_forward(x, weights, idx, w1, w2, w3, recompute, budget,
                                                                  any(ctx.needs_input_grad), residual)
         ctx.params, ctx.router_w, ctx.budget = (w1, w2, w3), router_w, budget
-        ctx.mark_non_differentiable(idx)
-        ctx.save_for_backward(x, probs, idx, *saved)
-        return out, logits, idx
+        counts = saved.pop()
+        ctx.save_for_backward(x, probs, idx, counts, *saved)
+        return (out, native.moe_aux(probs, counts)) if balance else out
 
     @staticmethod
-    def backward(ctx, dout, dlogits_extra, _didx):
-        x, probs, idx, *saved = ctx.saved_tensors
+    def backward(ctx, dout, daux=None):
+        x, probs, idx, counts, *saved = ctx.saved_tensors
         router_w = ctx.router_w
         dresidual = dout if ctx.needs_input_grad[5] else None
         if dout is None:
             dout = torch.zeros_like(x)
-        if dlogits_extra is not None:
-            dlogits_extra = dlogits_extra.float().contiguous()
+        if daux is not None:
+            daux = daux.to(device=x.device, dtype=torch.float32)
         dx_perm, dweights, dw1, dw2, dw3 = _experts_backward(dout.contiguous(), saved, *ctx.params, ctx.recompute)
-        dx, dlogits = native.moe_dx(dx_perm, saved[6], dweights, probs, idx, saved[2], router_w, dlogits_extra)
+        dx, dlogits = native.moe_dx(dx_perm, saved[6], dweights, probs, idx, saved[2], router_w, daux,
+                                    counts)
         main_grad = getattr(router_w, "main_grad", None)
         drouter = None
         if main_grad is not None:
@@ -142,12 +144,13 @@ class _MoELayer(torch.autograd.Function):
             drouter = native.gemm_tn(dlogits, x, out_dtype=router_w.dtype)
         if ctx.ledger is not None:
             ctx.budget.leave(*ctx.ledger)
-        return dx, drouter, dw1, dw2, dw3, dresidual, None, None
+        return dx, drouter, dw1, dw2, dw3, dresidual, None, None, None
 
 
-def moe_layer_fused(x, router_w, w1, w2, w3, residual=None, recompute: bool = False, budget=None):
-    """``(out, logits, idx)`` of a routed layer on one rank, or ``None`` where the router has to run by itself: more
-    than 16 experts (or more router weights than a CTA stages), a weight that is still to be gathered, layouts that the
+def moe_layer_fused(x, router_w, w1, w2, w3, residual=None, recompute: bool = False, budget=None,
+                    balance: bool = False):
+    """Output of a routed layer on one rank (with ``balance``: and its balance loss), or ``None`` where the router has
+    to run by itself: more than 16 experts (or more router weights than a CTA stages), a weight that is still to be gathered, layouts that the
     16-byte accesses do not take."""
     experts, dim = router_w.shape
     if not (2 <= experts <= 16 and experts == w1.shape[0] and dim == x.shape[1] and dim % 8 == 0
@@ -156,7 +159,7 @@ def moe_layer_fused(x, router_w, w1, w2, w3, residual=None, recompute: bool = Fa
             and all(t.dtype == torch.bfloat16 and t.is_contiguous() and t.data_ptr() % 16 == 0
                     for t in ((x, router_w) if residual is None else (x, router_w, residual)))):
         return None
-    return _MoELayer.apply(x, router_w, w1, w2, w3, residual, recompute, budget)
+    return _MoELayer.apply(x, router_w, w1, w2, w3, residual, recompute, budget, balance)
 
 
 def moe_ffn_fused(x, weights, idx, w1, w2, w3, recompute: bool = False, budget=None):

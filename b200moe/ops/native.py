@@ -673,13 +673,21 @@ def moe_combine(y_perm, slot_row, weights, tokens, residual=None):
     return out
 
 
-def moe_dx(dy_perm, slot_row, dweights, probs, idx, weights, router_w, dlogits_extra=None):
-    """Input gradient of a routed layer: the two rows of each token plus the router's share; returns ``(dx, dlogits)``."""
+def moe_aux(probs, counts):
+    """Balance loss of top-2 routing from the router's probabilities ``[T, E]`` and the experts' slot counts."""
+    aux = torch.empty((), dtype=torch.float32, device=probs.device)
+    _call("b2_moe_aux", _p(probs), _p(counts), _p(aux), _I(probs.shape[0]), _I(probs.shape[1]), _stream())
+    return aux
+
+
+def moe_dx(dy_perm, slot_row, dweights, probs, idx, weights, router_w, daux=None, counts=None):
+    """Input gradient of a routed layer: the two rows of each token plus the router's share, that of the balance loss
+    (``daux``: its gradient, fp32 device scalar) included; returns ``(dx, dlogits)``."""
     T, E = probs.shape
     D = dy_perm.shape[1]
     dlogits = torch.empty(T, E, dtype=torch.float32, device=dy_perm.device)
     dx = torch.empty(T, D, dtype=torch.bfloat16, device=dy_perm.device)
-    _call("b2_moe_dx", _p(_bf16(dy_perm)), _p(slot_row), _p(dweights), _p(probs), _p(idx), _p(weights), _p(dlogits_extra),
+    _call("b2_moe_dx", _p(_bf16(dy_perm)), _p(slot_row), _p(dweights), _p(probs), _p(idx), _p(weights), _p(daux), _p(counts),
           _p(_bf16(router_w)), _p(dlogits), _p(dx), _I(T), _I(E), _I(D), _I(dy_perm.shape[0]), _stream())
     return dx, dlogits
 
