@@ -84,7 +84,11 @@ struct GemmParams {
   const int* num_m_tiles;      // device scalar: live 128-row tiles, or null (= ceil(M/128))
   int group_align256;          // grouped problems: every expert segment is a multiple of 256 rows
   const int* expert_offsets;   // [E] cumulative row ends (SCHED_WGRAD)
+  const int* expert_counts;    // optional [E]: rows of each segment that count; the reduction leaves out the zero rows
+                               // of its padding (a tenth of 10006 rows in eight segments of whole 256-row tiles)
   void* d;                     // output
+  void* d2;                    // optional (EPI_ACC_*): rows from m_split on go to rows [0, M - m_split) of this one
+  int m_split;
   void* d_gate;                // optional gate pre-activation (SwiGLU)
   void* d_up;                  // optional up pre-activation (SwiGLU)
   void* h;                     // EPI_SWIGLU_BWD: [M, N]; d_gate and d_up are inputs there
@@ -127,7 +131,7 @@ __device__ __forceinline__ TileCoord decode_tile(const GemmParams& p, long long 
     t.m_tile = first_m + in_group % rows_in_group;
     t.n_tile = in_group / rows_in_group;
     const int begin = t.expert == 0 ? 0 : p.expert_offsets[t.expert - 1];
-    const int end = p.expert_offsets[t.expert];
+    const int end = p.expert_counts ? begin + p.expert_counts[t.expert] : p.expert_offsets[t.expert];
     t.k_begin = begin;
     t.k_blocks = (end - begin + BK - 1) / BK;
   } else {
@@ -459,7 +463,8 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
         const long long col_base = static_cast<long long>(t.n_tile) * BN;
         const long long expert_off = SCHED == SCHED_WGRAD ? t.expert * p.d_expert_stride : 0;
         const int q = lane & 3;
-        const bool add = (EPI == EPI_ACC_F32 || EPI == EPI_ACC_BF16) && p.beta != 0.f;
+        constexpr bool ACC = EPI == EPI_ACC_F32 || EPI == EPI_ACC_BF16;
+        const bool add = ACC && p.beta != 0.f;
         constexpr bool SCALED = EPI == EPI_ACC_F32 || EPI == EPI_ACC_BF16 || EPI == EPI_STORE_BF16 || EPI == EPI_STORE_F32;
         const float alpha = SCALED && p.alpha ? *p.alpha : 1.f;
 #pragma unroll 1
@@ -474,12 +479,14 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
             for (int it = 0; it < 4; ++it) {
               const long long rr = row0 + it * 8 + (lane >> 2);
               if (rr >= p.M) continue;
-              const long long off = expert_off + rr * p.ldd + col;
+              const bool low = !ACC || !p.d2 || rr < p.m_split;
+              const long long off = expert_off + (low ? rr : rr - p.m_split) * p.ldd + col;
+              const void* out = low ? p.d : p.d2;
               if (EPI == EPI_ACC_F32 && add) {
-                old[it][0] = reinterpret_cast<const uint4*>(reinterpret_cast<const float*>(p.d) + off)[0];
-                old[it][OLD - 1] = reinterpret_cast<const uint4*>(reinterpret_cast<const float*>(p.d) + off)[1];
+                old[it][0] = reinterpret_cast<const uint4*>(reinterpret_cast<const float*>(out) + off)[0];
+                old[it][OLD - 1] = reinterpret_cast<const uint4*>(reinterpret_cast<const float*>(out) + off)[1];
               } else if (EPI == EPI_ACC_BF16 && add) {
-                old[it][0] = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.d) + off);
+                old[it][0] = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(out) + off);
               } else if (EPI == EPI_ROPE && col < p.rope_cols) {
                 // four adjacent pairs (2j, 2j+1) of a head: table entries [position][(col mod 128)/2 + j]
                 const size_t tab = static_cast<size_t>(static_cast<int>(rr) % p.rope_seq) * 64 + ((col & 127) >> 1);
@@ -516,7 +523,9 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
 #pragma unroll
               for (int i = 0; i < 8; ++i) x[i] *= alpha;
             }
-            const long long off = expert_off + (row0 + r) * p.ldd + col;
+            const bool low = !ACC || !p.d2 || row0 + r < p.m_split;
+            const long long off = expert_off + (low ? row0 + r : row0 + r - p.m_split) * p.ldd + col;
+            void* const out = low ? p.d : p.d2;
             if (EPI == EPI_ACC_F32 || EPI == EPI_STORE_F32) {
               if (add) {
 #pragma unroll
@@ -525,7 +534,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
                   x[4 + i] += __uint_as_float(w1[i]);
                 }
               }
-              float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.d) + off);
+              float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + off);
               dst[0] = make_float4(x[0], x[1], x[2], x[3]);
               dst[1] = make_float4(x[4], x[5], x[6], x[7]);
             } else if (EPI == EPI_SWIGLU_BWD) {
@@ -564,7 +573,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
                   x[2 * j + 1] = x0 * sv + x1 * cv;
                 }
               }
-              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.d) + off) =
+              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(out) + off) =
                   make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]), pack_bf16(x[6], x[7]));
             }
           }
@@ -882,16 +891,21 @@ int b2_gemm_nn_push(const void* a, const void* w, const void* w2, int M, int N, 
 // dw[e][M,N] (+)= a[rows_e, M]^T * b[rows_e, N]   (both MN-major; rows_e from cumulative offsets, or all R rows
 // when expert_offsets is null).  out_kind: 1 fp32 (+= if beta), 2 bf16 (+= if beta).  ``alpha`` (optional device scalar)
 // multiplies the product before it is added.
-int b2_gemm_tn(const void* a, const void* b, void* d, int M, int N, int R, long long lda, long long ldb,
-               long long ldd, int num_experts, const int* expert_offsets, int out_kind, float beta,
-               const float* alpha, int* status, cudaStream_t stream) {
-  if (N % 32 || M % 8) return -10;
+// With d2 the rows [m_split, M) of the product go to d2 (two weight gradients that share b, in one launch).
+// ``expert_counts`` (optional): rows of each segment that count; the rest of the segment holds zeros.
+int b2_gemm_tn(const void* a, const void* b, void* d, void* d2, int m_split, int M, int N, int R, long long lda,
+               long long ldb, long long ldd, int num_experts, const int* expert_offsets, const int* expert_counts,
+               int out_kind, float beta, const float* alpha, int* status, cudaStream_t stream) {
+  if (N % 32 || M % 8 || (d2 && (m_split < 1 || m_split >= M))) return -10;
   GemmParams p{};
+  p.d2 = d2;
+  p.m_split = m_split;
+  p.expert_counts = expert_counts;
   p.alpha = alpha;
   if (make_map(&p.map_a, a, M, R, lda, 64)) return -11;
   if (make_map(&p.map_b, b, N, R, ldb, 64)) return -12;
   p.M = M; p.N = N; p.K = R; p.num_experts = num_experts; p.b_expert_rows = 0; p.k_split = 0;
-  p.expert_offsets = expert_offsets; p.d = d; p.ldd = ldd; p.d_expert_stride = static_cast<long long>(M) * ldd;
+  p.expert_offsets = expert_offsets; p.d = d; p.ldd = ldd; p.d_expert_stride = static_cast<long long>(d2 ? m_split : M) * ldd;
   p.beta = beta; p.status = status;
   if (expert_offsets) {
     if (out_kind == 1) return launch<1, 1, EPI_ACC_F32, SCHED_WGRAD>(p, sm_count(), stream);

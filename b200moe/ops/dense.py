@@ -112,13 +112,20 @@ class _SwiGLUFFN(torch.autograd.Function):
         dy2d = dy.reshape(-1, dy.shape[-1]).contiguous()
         dgu, h = native.gemm_nn_swiglu_bwd(dy2d, w2, gate, up)
         dx = native.gemm_nn(dgu, w1, w2=w3).view_as(x) if ctx.needs_input_grad[0] else None
-        grads = []
-        for i, (weight, left, right) in enumerate(((w1, dgu[:, :ffn], x2d), (w3, dgu[:, ffn:], x2d), (w2, dy2d, h))):
-            main_grad = getattr(weight, "main_grad", None)
-            if main_grad is not None:
-                native.gemm_tn(left, right, out=main_grad, accumulate=True)
-            grads.append(native.gemm_tn(left, right, out_dtype=weight.dtype)
-                         if main_grad is None and ctx.needs_input_grad[i + 1] else None)
+        grads = [None, None, None]
+        accumulators = [getattr(w, "main_grad", None) for w in ctx.weights]
+        first = 0
+        if accumulators[0] is accumulators[1] is None and all(ctx.needs_input_grad[1:3]):
+            grads[0], grads[1] = torch.empty_like(w1), torch.empty_like(w3)
+            native.gemm_tn_two(dgu, x2d, grads[0], grads[1], False)      # both weights read x: one launch
+            first = 2
+        products = ((dgu[:, :ffn], x2d), (dgu[:, ffn:], x2d), (dy2d, h))
+        for i in range(first, 3):
+            left, right = products[i]
+            if accumulators[i] is not None:
+                native.gemm_tn(left, right, out=accumulators[i], accumulate=True)
+            elif ctx.needs_input_grad[i + 1]:
+                grads[i] = native.gemm_tn(left, right, out_dtype=ctx.weights[i].dtype)
         return dx, *grads
 
 

@@ -27,12 +27,28 @@ def capacity_rows(slots: int, num_experts: int) -> int:
     return (slots + num_experts * (ALIGN - 1) + ALIGN - 1) // ALIGN * ALIGN
 
 
-def _wgrad(dy, x, param, offs, num_experts):
+def _wgrad(dy, x, param, offs, num_experts, counts=None):
     main = getattr(param, "main_grad", None)
     if main is not None:
-        native.gemm_tn(dy, x, out=main, accumulate=True, expert_offsets=offs, num_experts=num_experts)
+        native.gemm_tn(dy, x, out=main, accumulate=True, expert_offsets=offs, num_experts=num_experts, counts=counts)
         return None
-    return native.gemm_tn(dy, x, out_dtype=param.dtype, expert_offsets=offs, num_experts=num_experts)
+    return native.gemm_tn(dy, x, out_dtype=param.dtype, expert_offsets=offs, num_experts=num_experts, counts=counts)
+
+
+def _wgrad_gate_up(dgu, x, w1, w3, offs, num_experts, counts):
+    """Gradients of the gate and up weights, in one launch where their accumulators are alike."""
+    ffn = w1.shape[1]
+    one, two = getattr(w1, "main_grad", None), getattr(w3, "main_grad", None)
+    if one is None and two is None and w1.dtype == w3.dtype == torch.bfloat16:
+        grads = torch.empty(w1.shape, dtype=w1.dtype, device=dgu.device), torch.empty_like(w3, dtype=w3.dtype)
+        native.gemm_tn_two(dgu, x, *grads, False, offs, num_experts, counts)
+        return grads
+    if (one is not None and two is not None and one.dtype == two.dtype and one.shape == two.shape
+            and one.is_contiguous() and two.is_contiguous()):
+        native.gemm_tn_two(dgu, x, one, two, True, offs, num_experts, counts)
+        return None, None
+    return (_wgrad(dgu[:, :ffn], x, w1, offs, num_experts, counts),
+            _wgrad(dgu[:, ffn:], x, w3, offs, num_experts, counts))
 
 
 def _experts_forward(x, weights, idx, w1, w2, w3, recompute, budget, wants_grad, residual=None):
@@ -61,10 +77,10 @@ def _experts_forward(x, weights, idx, w1, w2, w3, recompute, budget, wants_grad,
     return out, recompute, ledger, saved + [counts]
 
 
-def _experts_backward(dout, saved, w1, w2, w3, recompute):
+def _experts_backward(dout, saved, counts, w1, w2, w3, recompute):
     """Returns ``(dx_perm, dweights, dw1, dw2, dw3)``."""
     x_perm, y_perm, weights, offs, tile_expert, meta, slot_row, row_slot = saved[:8]
-    tokens, cap, experts, ffn = weights.shape[0], x_perm.shape[0], w1.shape[0], w1.shape[1]
+    tokens, cap, experts = weights.shape[0], x_perm.shape[0], w1.shape[0]
     tiles = meta[0:1]
     if recompute:
         _, gate, up = native.gemm_swiglu(x_perm, w1, w3, tile_expert, tiles, save_gate_up=True, align256=True)
@@ -78,9 +94,9 @@ def _experts_backward(dout, saved, w1, w2, w3, recompute):
     del gate, up
     dx_perm = native.gemm_nn(dgu, w1, w2=w3, tile_expert=tile_expert, num_m_tiles=tiles, num_experts=experts,
                              align256=True)
-    dw2 = _wgrad(dy_perm, h, w2, offs, experts)
-    dw1 = _wgrad(dgu[:, :ffn], x_perm, w1, offs, experts)
-    dw3 = _wgrad(dgu[:, ffn:], x_perm, w3, offs, experts)
+    # the reduction stops at each expert's own rows: its padding rows are zeros
+    dw2 = _wgrad(dy_perm, h, w2, offs, experts, counts)
+    dw1, dw3 = _wgrad_gate_up(dgu, x_perm, w1, w3, offs, experts, counts)
     return dx_perm, dweights, dw1, dw2, dw3
 
 
@@ -94,13 +110,13 @@ class _MoEFused(torch.autograd.Function):
         out, ctx.recompute, ctx.ledger, saved = _experts_forward(x, weights, idx, w1, w2, w3, recompute, budget,
                                                                  any(ctx.needs_input_grad))
         ctx.params, ctx.budget = (w1, w2, w3), budget
-        ctx.save_for_backward(*saved[:-1])
+        ctx.save_for_backward(*saved)
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        saved = ctx.saved_tensors
-        dx_perm, dweights, dw1, dw2, dw3 = _experts_backward(dout.contiguous(), saved, *ctx.params, ctx.recompute)
+        *saved, counts = ctx.saved_tensors
+        dx_perm, dweights, dw1, dw2, dw3 = _experts_backward(dout.contiguous(), saved, counts, *ctx.params, ctx.recompute)
         dx = native.moe_combine(dx_perm, saved[6], None, dweights.shape[0])
         if ctx.ledger is not None:
             ctx.budget.leave(*ctx.ledger)
@@ -133,7 +149,7 @@ class _MoELayer(torch.autograd.Function):
             dout = torch.zeros_like(x)
         if daux is not None:
             daux = daux.to(device=x.device, dtype=torch.float32)
-        dx_perm, dweights, dw1, dw2, dw3 = _experts_backward(dout.contiguous(), saved, *ctx.params, ctx.recompute)
+        dx_perm, dweights, dw1, dw2, dw3 = _experts_backward(dout.contiguous(), saved, counts, *ctx.params, ctx.recompute)
         dx, dlogits = native.moe_dx(dx_perm, saved[6], dweights, probs, idx, saved[2], router_w, daux,
                                     counts)
         main_grad = getattr(router_w, "main_grad", None)

@@ -325,9 +325,9 @@ def gemm_nn_swiglu_bwd(dy, w, gate, up, tile_expert=None, num_m_tiles=None, num_
 
 
 def gemm_tn(dy, x, out=None, accumulate: bool = False, out_dtype=None, expert_offsets=None, num_experts: int = 1,
-            alpha=None):
+            alpha=None, counts=None):
     """``out[e] (+)= dy[rows_e]ᵀ @ x[rows_e]`` -> ``[E?, N_out, K_in]``; fp32 or bf16 output.  ``alpha``: fp32 device
-    scalar that multiplies the product."""
+    scalar that multiplies the product.  ``counts``: int32 ``[E]`` rows of each segment that are not zero padding."""
     R, M = dy.shape
     N = x.shape[1]
     if M <= 16 and expert_offsets is None and alpha is None:
@@ -349,11 +349,25 @@ def gemm_tn(dy, x, out=None, accumulate: bool = False, out_dtype=None, expert_of
         accumulate = False
     kind = 1 if out.dtype == torch.float32 else 2
     assert dy.stride(-1) == 1 and x.stride(-1) == 1 and out.is_contiguous()
-    _call("b2_gemm_tn", _p(_bf16(dy)), _p(_bf16(x)), _p(out), _I(M), _I(N), _I(R), _L(dy.stride(0)), _L(x.stride(0)),
-          _L(N), _I(num_experts), _p(expert_offsets), _I(kind), _F(1.0 if accumulate else 0.0),
+    _call("b2_gemm_tn", _p(_bf16(dy)), _p(_bf16(x)), _p(out), _p(None), _I(0), _I(M), _I(N), _I(R), _L(dy.stride(0)),
+          _L(x.stride(0)), _L(N), _I(num_experts), _p(expert_offsets), _p(counts), _I(kind), _F(1.0 if accumulate else 0.0),
           _p(alpha), _p(status_word(dy.device)), _stream(),
           tag=f"{'grouped ' if expert_offsets is not None else ''}{M}x{N} {'fp32' if kind == 1 else 'bf16'}")
     return out if want is None or want == out.dtype else out.to(want)
+
+
+def gemm_tn_two(dy, x, out, out2, accumulate: bool, expert_offsets=None, num_experts: int = 1, counts=None):
+    """``[out[e]; out2[e]] (+)= dy[rows_e]ᵀ @ x[rows_e]``: the gradients of two weights that share their input, ``dy``
+    holding both halves side by side.  One launch: ``x`` is read once, and twice the tiles fill the last wave."""
+    R, M = dy.shape
+    N = x.shape[1]
+    assert dy.stride(-1) == 1 and x.stride(-1) == 1 and out.is_contiguous() and out2.is_contiguous()
+    assert out.shape == out2.shape and out.dtype == out2.dtype and 2 * out.shape[-2] == M and out.shape[-1] == N
+    kind = 1 if out.dtype == torch.float32 else 2
+    _call("b2_gemm_tn", _p(_bf16(dy)), _p(_bf16(x)), _p(out), _p(out2), _I(M // 2), _I(M), _I(N), _I(R),
+          _L(dy.stride(0)), _L(x.stride(0)), _L(N), _I(num_experts), _p(expert_offsets), _p(counts), _I(kind),
+          _F(1.0 if accumulate else 0.0), _p(None), _p(status_word(dy.device)), _stream(),
+          tag=f"{'grouped ' if expert_offsets is not None else ''}{M}x{N} {'fp32' if kind == 1 else 'bf16'}")
 
 
 def gemm_swiglu(x, w1, w3, tile_expert=None, num_m_tiles=None, save_gate_up: bool = True, align256: bool = False):

@@ -129,8 +129,8 @@ def test_grouped_expert_gemms(native, tile_mode, counts, pad):
     native.check_status()
 
 
-@pytest.mark.parametrize("tokens,dim,ffn,launches", [(1, 64, 128, 7), (129, 192, 384, 7), (300, 512, 640, 7),
-                                                     (5500, 64, 384, 8)])
+@pytest.mark.parametrize("tokens,dim,ffn,launches", [(1, 64, 128, 6), (129, 192, 384, 6), (300, 512, 640, 6),
+                                                     (5500, 64, 384, 7)])
 def test_dense_swiglu_layer_on_the_fused_kernels(native, tile_mode, tokens, dim, ffn, launches):
     """Rows and widths around the tile edges, in every tile kind, forward and all gradients against 64 bits; a hook on
     one projection sends the same layer through the three separate products."""
@@ -158,6 +158,39 @@ def test_dense_swiglu_layer_on_the_fused_kernels(native, tile_mode, tokens, dim,
         for got, want in zip((x.grad, layer.w1.weight.grad, layer.w3.weight.grad, layer.w2.weight.grad), wanted):
             assert _rel(got, want) < 1.2e-2
     assert calls
+    native.check_status()
+
+
+@pytest.mark.parametrize("counts", [[100, 0, 300, 17], [256, 1, 64, 65], [0, 0, 640, 0]])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_grouped_weight_gradients_of_two_weights_over_live_rows(native, tile_mode, counts, dtype):
+    """Two accumulators from one launch (their border inside a 256-row tile), the reduction cut at each expert's count:
+    what lies in the padding behind the last started 64 rows is not read."""
+    torch.manual_seed(1)
+    E, F, D = len(counts), 160, 96
+    offs, _, _, rows = _segments(counts, 256)
+    dy, x = _rand(rows, 2 * F, scale=0.1), _rand(rows, D, scale=0.1)
+    start, live = 0, torch.zeros(rows, dtype=torch.bool, device="cuda")
+    for e, c in enumerate(counts):
+        end = int(offs[e])
+        live[start:start + c] = True
+        dy[start + c:end] = 0
+        x[start + c:end] = 0
+        x[min(start + (c + 63) // 64 * 64, end):end] = float("nan")
+        start = end
+    base = [torch.randn(E, F, D, device="cuda").to(dtype) for _ in range(2)]
+    got = [t.clone() for t in base]
+    count = torch.tensor(counts, dtype=torch.int32, device="cuda")
+    native.gemm_tn_two(dy, x, *got, True, offs, E, count)
+    third = native.gemm_tn(dy[:, :F], x, out=base[0].clone(), accumulate=True, expert_offsets=offs, num_experts=E, counts=count)
+    assert torch.equal(third, got[0])
+    start = 0
+    for e, c in enumerate(counts):
+        want = dy[start:start + c].double().t() @ x[start:start + c].double()
+        for half in range(2):
+            assert _rel(got[half][e].double(), base[half][e].double() + want[half * F:(half + 1) * F]) < (
+                1e-5 if dtype == torch.float32 else 4e-3)
+        start = int(offs[e])
     native.check_status()
 
 
