@@ -461,7 +461,7 @@ def cross_entropy_scaled_(logits, targets, loss, loss_scale: float, grad_scale: 
     ``grad_scale · (softmax − onehot)``; rows up to 32768 entries are read once and written once."""
     T, V = logits.shape
     _call("b2_cross_entropy2", _p(_bf16(logits)), _p(targets.contiguous()), _p(loss), _I(T), _I(V), _F(loss_scale),
-          _F(grad_scale), _stream())
+          _F(grad_scale), _p(status_word(logits.device)), _stream())
     return loss
 
 

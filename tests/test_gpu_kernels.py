@@ -282,6 +282,26 @@ def test_lm_head_without_a_known_factor_keeps_or_rebuilds_its_logits(native, kee
     native.check_status()
 
 
+@pytest.mark.parametrize("T,V", [(1, 8), (149, 8192), (300, 8200), (297, 16384), (150, 16392), (600, 32000), (149, 32768),
+                                 (3, 32776)])
+def test_cross_entropy_row_sizes(native, T, V):
+    """Row sizes around those that select the kernel (2 and 4 vectors per thread, rows through shared memory, streaming
+    beyond), more rows than CTAs, the first and the last entry as targets: against 64 bits.  Loss: fp32 sums; gradient:
+    stored as bf16."""
+    torch.manual_seed(V)
+    logits = _rand(T, V, scale=2.0)
+    targets = torch.randint(0, V, (T,), device="cuda")
+    targets[0], targets[-1] = 0, V - 1
+    l64 = logits.double().requires_grad_(True)
+    want = torch.nn.functional.cross_entropy(l64, targets, reduction="sum") / T
+    want.backward()
+    loss = torch.zeros((), device="cuda")
+    native.cross_entropy_scaled_(logits, targets, loss, 1.0 / T, 1.0 / T)
+    assert abs(float(loss) - float(want)) < 1e-5 * abs(float(want))
+    assert _rel(logits.double(), l64.grad) < 4e-3
+    native.check_status()
+
+
 def test_cross_entropy_and_lm_head(native):
     from b200moe import ops
     T, D, V = 512, 256, 32000
