@@ -675,12 +675,14 @@ enum TileKind : int { TILE_128 = 0, TILE_256 = 1, TILE_PAIR = 2 };
 
 // 256-row tiles (one CTA with two sub-tiles, or a CTA pair) need whole 256-row tiles of one expert: the caller says
 // whether its segments are padded to 256 rows.
-// CTA pairs wherever their tiles reach half of the machine's pairs or more.  Whole passes, us, single-CTA kinds -> pairs:
-// three-layer dense SwiGLU stack 11374 -> 10544, 5003-token expert layer 11142 -> 10905, one-block step of 2 x 16384
-// tokens 109651 -> 104820, head and loss of 6001 tokens 3519 -> 3307; the eight-block step that runs against the 1000 W
-// power cap for ten seconds 10649 -> 10669 ms, which is the same.  (With the four-warp epilogue pairs lost 7 % there.)
-// Below that the single-CTA kinds: 256x256 for long K, where the exposed epilogue is amortised, else 128x256.  The
-// expert-parallel return (EPI_PUSH) stays with those: its time depends on the links, which one GPU does not show.
+// 256x256 on one CTA for long reductions over many tiles: the exposed epilogue is amortised, and it takes the least energy
+// per operation (down projection of 11 000 expert rows, K 14336: 0.96 ms against 1.02-1.10 ms on pairs; its dx, K 28672:
+// 1.82 against 1.96-2.15).  Otherwise CTA pairs wherever their tiles reach half of the machine's pairs: whole passes, us,
+// single-CTA kinds -> pairs: three-layer dense SwiGLU stack 11374 -> 10544, one-block step of 2 x 16384 tokens 109651 ->
+// 104820, head and loss of 6001 tokens 3519 -> 3307.  The eight-block step that runs against the 1000 W power cap for ten
+// seconds, ms: single-CTA kinds only 10510, pairs for everything large 10540, this rule 10237.  Below that 128x256 on one
+// CTA.  The expert-parallel return (EPI_PUSH) stays with the single-CTA kinds: its time depends on the links, which one
+// GPU does not show.
 template <int SCHED, int EPI>
 static TileKind choose_tile(const GemmParams& p, int sms, bool pair_available) {
   const long long k_eff = SCHED == SCHED_WGRAD ? p.K / (p.num_experts > 0 ? p.num_experts : 1) : p.K;
@@ -693,8 +695,8 @@ static TileKind choose_tile(const GemmParams& p, int sms, bool pair_available) {
   if (pair_available && g_tile_mode == 3) return TILE_PAIR;
   if (g_tile_mode == 3) return TILE_128;
   const bool pairs = g_tile_mode == 4 || (g_tile_mode == 0 && EPI != EPI_PUSH);
-  if (pair_available && pairs && tiles256 >= sms / 2) return TILE_PAIR;
-  return tiles256 >= 2LL * sms && k_eff >= 6144 ? TILE_256 : TILE_128;
+  if (tiles256 >= 2LL * sms && k_eff >= 6144) return TILE_256;
+  return pair_available && pairs && tiles256 >= sms / 2 ? TILE_PAIR : TILE_128;
 }
 
 template <int A_MN, int B_MN, int EPI, int SCHED>
