@@ -149,6 +149,8 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const __nv_bfloat16* __
 }
 
 // out[t] = (residual[t] +) w0 * y[slot_row[2t]] + w1 * y[slot_row[2t+1]]   (weights null => 1); one warp per token.
+// The weighted sum is rounded to bf16 before the residual is added: the layer's output followed by the block's sum, bit
+// for bit (a router further on turns another rounding into another choice between experts that are nearly tied).
 __global__ void __launch_bounds__(256) moe_combine_kernel(const __nv_bfloat16* __restrict__ y_perm,
                                                           const int* __restrict__ slot_row,
                                                           const float* __restrict__ weights,
@@ -171,8 +173,12 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const __nv_bfloat16* _
       for (int i = 0; i < 4; ++i) {
         const float2 fa = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&va.v[i]));
         const float2 fb = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&vb.v[i]));
-        const float2 fr = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&vr.v[i]));
-        const __nv_bfloat162 r = __floats2bfloat162_rn(fr.x + w0 * fa.x + w1 * fb.x, fr.y + w0 * fa.y + w1 * fb.y);
+        __nv_bfloat162 r = __floats2bfloat162_rn(__fmaf_rn(w1, fb.x, w0 * fa.x), __fmaf_rn(w1, fb.y, w0 * fa.y));
+        if (residual) {
+          const float2 fr = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&vr.v[i]));
+          const float2 f = __bfloat1622float2(r);
+          r = __floats2bfloat162_rn(fr.x + f.x, fr.y + f.y);
+        }
         o.v[i] = *reinterpret_cast<const uint32_t*>(&r);
       }
       *reinterpret_cast<vec16*>(out + static_cast<size_t>(t) * D + c) = o;

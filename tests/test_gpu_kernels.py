@@ -448,6 +448,16 @@ def test_moe_plan_gather_combine(native, T, E):
     assert _rel(out, x.float() * w.sum(1, keepdim=True)) < 5e-3
 
 
+def test_combine_with_a_residual_rounds_like_the_sum_of_two_tensors(native):
+    """A block's output decides the next router's choices, so the fused sum has to be the separate one bit for bit."""
+    T, D = 1001, 264
+    y, residual, w = _rand(2 * T, D), _rand(T, D), torch.rand(T, 2, device="cuda")
+    slot_row = torch.randperm(2 * T, device="cuda").int()
+    for weights in (w, None):
+        fused = native.moe_combine(y, slot_row, weights, T, residual=residual)
+        assert torch.equal(fused, residual + native.moe_combine(y, slot_row, weights, T))
+
+
 @pytest.mark.parametrize("recompute", [False, True])
 def test_moe_block_matches_torch_path(native, recompute):
     from b200moe import ops
