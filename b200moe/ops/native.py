@@ -525,7 +525,16 @@ def embedding_bwd(flat_ids, dy2d, main_grad):
           _I(flat_ids.numel()), _I(dy2d.shape[1]), _stream())
 
 
+def _rope_table(table, seq: int, half: int):
+    """A rotary table as the kernels read it: fp32, ``half`` entries for each of ``seq`` positions, 16-byte aligned."""
+    if table.dtype != torch.float32 or table.numel() < seq * half:
+        raise ValueError(f"rotary tables must be fp32 [>= {seq}, {half}]")
+    table = table.contiguous()
+    return table if table.data_ptr() % 16 == 0 else table.clone()
+
+
 def rope_inplace(buf, first_elem_offset, tokens, seq, heads, head_dim, pitch, cos, sin, sign):
+    cos, sin = _rope_table(cos, seq, head_dim // 2), _rope_table(sin, seq, head_dim // 2)
     ptr = ctypes.c_void_p(buf.data_ptr() + first_elem_offset * buf.element_size())
     _call("b2_rope", ptr, _p(cos), _p(sin), _I(tokens), _I(seq), _I(heads), _I(head_dim), _L(pitch), _F(sign), _stream())
 
@@ -618,6 +627,7 @@ def attention_fwd(q, k, v, cos=None, sin=None, causal=True):
     Hkv = k.shape[2]
     f16 = q.dtype == k.dtype == v.dtype == torch.float16 and cos is None
     if cos is not None:
+        cos, sin = _rope_table(cos, S, 64), _rope_table(sin, S, 64)
         q, k = (t if _pitched(_bf16(t)) else t.clone(memory_format=torch.contiguous_format) for t in (q, k))
         qr, kr = (torch.empty(t.shape, dtype=torch.bfloat16, device=t.device) for t in (q, k))
         _call("b2_rope_copy", _p(q), _p(k), _p(qr), _p(kr), _p(cos), _p(sin), _I(B * S), _I(S), _I(Hq), _I(Hkv),

@@ -219,3 +219,27 @@ def test_fsdp_first_use_gather_needs_the_fused_backend():
     assert wrapped._lazy == [] and not any(e.get("lazy") for e in wrapped.flat.entries)
     with pytest.raises(ValueError):
         FSDPWrapperPipelined(model, None, None, gather="sometimes")
+
+
+def test_rotary_tables_that_the_kernels_would_read_past_are_refused(monkeypatch):
+    """Refused before anything is launched: tables shorter than the sequence or of a narrower type.  A table that
+    starts off a 16-byte boundary is copied."""
+    from b200moe.ops import native
+    launched = []
+    monkeypatch.setattr(native, "_call", lambda name, *args, **kw: launched.append((name, args)))
+    monkeypatch.setattr(native, "_stream", lambda: None)
+    S, hd = 130, 128
+    cos, sin = Fn.rope_tables(10000.0, hd, S)
+    q, k = torch.zeros(1, S, 4, hd, dtype=torch.bfloat16), torch.zeros(1, S, 1, hd, dtype=torch.bfloat16)
+    for bad in (cos[:S - 1], cos.bfloat16()):
+        for pair in ((bad, sin), (cos, bad)):
+            with pytest.raises(ValueError):
+                native.attention_fwd(q, k, k, *pair)
+            with pytest.raises(ValueError):
+                native.rope_inplace(q, 0, S, S, 4, hd, 4 * hd, *pair, 1.0)
+    assert launched == []
+    shifted = torch.cat((torch.zeros(1), cos.reshape(-1)))[1:].view(S, -1)
+    native.rope_inplace(q, 0, S, S, 4, hd, 4 * hd, shifted, sin, 1.0)
+    (name, args), = launched
+    assert name == "b2_rope" and args[1].value % 16 == 0 and args[1].value != shifted.data_ptr()
+    assert args[2].value == sin.data_ptr()
