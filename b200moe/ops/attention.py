@@ -140,6 +140,18 @@ def attention_backend() -> str:
     return os.environ.get("B200MOE_ATTENTION", "native")
 
 
+def library_attention(q, k, v, cos, sin):
+    """``rope_attention`` through PyTorch's library kernels: the A/B baseline, head sizes the kernels do not take, and
+    the attention layer's sequences that are no multiple of 128."""
+    qh, kh, vh = (t.transpose(1, 2) for t in (q, k, v))
+    if cos is not None:
+        seq = qh.shape[-2]
+        qh = Fn.apply_rope_ref(qh, cos[:seq], sin[:seq])
+        kh = Fn.apply_rope_ref(kh, cos[:seq], sin[:seq])
+    out = F.scaled_dot_product_attention(qh, kh, vh, is_causal=True, enable_gqa=True)
+    return out.transpose(1, 2)
+
+
 def rope_attention(q, k, v, cos, sin):
     """Returns ``[B, S, Hq, head_dim]``.  ``cos``/``sin`` are ``[S_max, hd/2]``
     fp32 tables or ``None`` for no rotation."""
@@ -147,14 +159,7 @@ def rope_attention(q, k, v, cos, sin):
             q.shape[1] % 128 == 0 or _ragged_ok(q, k, v, cos, sin)):
         return _RopeAttention.apply(q, k, v, cos, sin)
     if q.is_cuda:
-        # library attention on the GPU (A/B baseline only)
-        qh, kh, vh = (t.transpose(1, 2) for t in (q, k, v))
-        if cos is not None:
-            seq = qh.shape[-2]
-            qh = Fn.apply_rope_ref(qh, cos[:seq], sin[:seq])
-            kh = Fn.apply_rope_ref(kh, cos[:seq], sin[:seq])
-        out = F.scaled_dot_product_attention(qh, kh, vh, is_causal=True, enable_gqa=True)
-        return out.transpose(1, 2)
+        return library_attention(q, k, v, cos, sin)
     return Fn.attention_ref(q, k, v, cos, sin, causal=True)
 
 

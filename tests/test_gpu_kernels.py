@@ -817,6 +817,34 @@ def test_projection_with_rope_in_the_gemm_epilogue_then_attention(native, tile):
         native.set_gemm_tile_mode(0)
 
 
+@pytest.mark.parametrize("S", [100, 129])
+@pytest.mark.parametrize("fused", [True, False])
+def test_attention_layer_of_ragged_sequences_rounds_like_the_library(native, S, fused):
+    """Bit for bit the projection, the rotation and the library's attention one by one, with and without a fused
+    projection weight: routers behind the layer turn another rounding into other choices."""
+    from b200moe import ops
+    from b200moe.models.layers import MultiHeadLayerLL, ROPELayer
+    from b200moe.ops.attention import library_attention, rope_qk_
+    torch.manual_seed(S)
+    B, D, Hq, Hkv, hd = 2, 512, 4, 1, 128
+    with torch.device("cuda"):
+        layer = MultiHeadLayerLL(D, Hq, RoPE=ROPELayer(10000, hd, 256))
+    for p in (layer.q_proj, layer.k_proj, layer.v_proj, layer.output_proj):
+        p.compute_weight = p.weight.detach().bfloat16()
+    q, k, v, out = (p.compute_weight for p in (layer.q_proj, layer.k_proj, layer.v_proj, layer.output_proj))
+    x, cos, sin = _rand(B, S, D), layer.RoPE.cos, layer.RoPE.sin
+    if fused:
+        layer.qkv_weight = torch.cat((q, k, v))
+        qkv = rope_qk_(ops.linear(x.view(B * S, D), layer.qkv_weight), S, Hq + 2 * Hkv, Hq + Hkv, hd, cos, sin)
+        heads = qkv.view(B, S, Hq + 2 * Hkv, hd).split((Hq, Hkv, Hkv), dim=2)
+        attended = library_attention(*heads, None, None)
+    else:
+        heads = [ops.linear(x, w).view(B, S, -1, hd) for w in (q, k, v)]
+        attended = library_attention(*heads, cos, sin)
+    assert torch.equal(layer(x), ops.linear(attended.reshape(B, S, D), out))
+    native.check_status()
+
+
 @pytest.mark.parametrize("M,K,world,segments", [(1000, 512, 2, [1536]), (300, 256, 2, [1984]),
                                                 (2048, 1024, 4, [2048]), (700, 512, 2, [1024, 256, 256]),
                                                 (513, 256, 4, [1024, 512, 512, 96 * 4])])
