@@ -40,6 +40,13 @@ def use_native(t: torch.Tensor, op: str = "") -> bool:
     return native.has(op)
 
 
+def backward_follows(*tensors) -> bool:
+    """Whether a call on ``tensors`` (``None`` among them) can be differentiated.  Asked by the callers of autograd
+    functions: inside ``forward`` grad mode is off, and ``ctx.needs_input_grad`` repeats the inputs' ``requires_grad``
+    even under ``no_grad``."""
+    return torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in tensors)
+
+
 from .dense import linear, linear_rope, swiglu_ffn, embedding, rmsnorm, add_rmsnorm  # noqa: E402
 from .attention import rope_attention  # noqa: E402
 from .loss import lm_head_cross_entropy  # noqa: E402

@@ -13,7 +13,7 @@ from __future__ import annotations
 
 import torch
 
-from . import functional as Fn, native, use_native
+from . import backward_follows, functional as Fn, native, use_native
 
 
 class _Linear(torch.autograd.Function):
@@ -94,9 +94,8 @@ class _SwiGLUFFN(torch.autograd.Function):
     gradients."""
 
     @staticmethod
-    def forward(ctx, x, w1, w3, w2):
+    def forward(ctx, x, w1, w3, w2, keep):
         x2d = x.reshape(-1, x.shape[-1])
-        keep = any(ctx.needs_input_grad)
         h, gate, up = native.gemm_swiglu(x2d, w1.unsqueeze(0), w3.unsqueeze(0), save_gate_up=keep)
         y = native.gemm_nt(h, w2)
         ctx.weights = (w1, w3, w2)
@@ -126,7 +125,7 @@ class _SwiGLUFFN(torch.autograd.Function):
                 native.gemm_tn(left, right, out=accumulators[i], accumulate=True)
             elif ctx.needs_input_grad[i + 1]:
                 grads[i] = native.gemm_tn(left, right, out_dtype=ctx.weights[i].dtype)
-        return dx, *grads
+        return dx, *grads, None
 
 
 def swiglu_ffn(x, w1, w3, w2):
@@ -143,7 +142,7 @@ def swiglu_ffn(x, w1, w3, w2):
     ffn, dim = w1.shape
     if w3.shape != w1.shape or w2.shape != (dim, ffn) or ffn % 128 or dim % 64 or x.shape[-1] != dim:
         return None
-    return _SwiGLUFFN.apply(x, *weights)
+    return _SwiGLUFFN.apply(x, *weights, backward_follows(x, *weights))
 
 
 class _Embedding(torch.autograd.Function):

@@ -243,3 +243,23 @@ def test_rotary_tables_that_the_kernels_would_read_past_are_refused(monkeypatch)
     (name, args), = launched
     assert name == "b2_rope" and args[1].value % 16 == 0 and args[1].value != shifted.data_ptr()
     assert args[2].value == sin.data_ptr()
+
+
+def test_dense_swiglu_keeps_gate_and_up_only_where_a_backward_pass_can_follow(monkeypatch):
+    from b200moe.ops import dense, native
+    kept = []
+
+    def gemm_swiglu(x, w1, w3, save_gate_up=True):
+        kept.append(save_gate_up)
+        return (x.new_zeros(x.shape[0], w1.shape[1]),) * 3
+
+    monkeypatch.setattr(dense, "use_native", lambda *_: True)
+    monkeypatch.setattr(native, "gemm_swiglu", gemm_swiglu)
+    monkeypatch.setattr(native, "gemm_nt", lambda x, w: x.new_zeros(x.shape[0], w.shape[0]))
+    x = torch.zeros(3, 64, dtype=torch.bfloat16)
+    weights = [torch.zeros(s, dtype=torch.bfloat16, requires_grad=True) for s in ((128, 64), (128, 64), (64, 128))]
+    assert ops.swiglu_ffn(x, *weights).requires_grad
+    with torch.no_grad():
+        ops.swiglu_ffn(x, *weights)
+    assert not ops.swiglu_ffn(x, *(w.detach() for w in weights)).requires_grad
+    assert kept == [True, False, False]
