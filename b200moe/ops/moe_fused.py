@@ -17,7 +17,7 @@ from __future__ import annotations
 
 import torch
 
-from . import native
+from . import backward_follows, native
 
 ALIGN = 256       # expert segments are padded to 256 rows (whole 256x256 GEMM tiles)
 
@@ -68,11 +68,12 @@ def _experts_forward(x, weights, idx, w1, w2, w3, recompute, budget, wants_grad,
         kept = budget.enter(*ledger)
         recompute = recompute or not kept
         ledger += (not recompute,)
-    h, gate, up = native.gemm_swiglu(x_perm, w1, w3, tile_expert, tiles, save_gate_up=not recompute, align256=True)
+    keep = wants_grad and not recompute
+    h, gate, up = native.gemm_swiglu(x_perm, w1, w3, tile_expert, tiles, save_gate_up=keep, align256=True)
     y_perm = native.gemm_nt(h, w2, tile_expert=tile_expert, num_m_tiles=tiles, num_experts=experts, align256=True)
     out = native.moe_combine(y_perm, slot_row, weights, tokens, residual=residual)
     saved = [x_perm, y_perm, weights, offs, tile_expert, meta, slot_row, row_slot]
-    if not recompute:
+    if keep:
         saved += [gate, up]
     return out, recompute, ledger, saved + [counts]
 
@@ -104,11 +105,11 @@ class _MoEFused(torch.autograd.Function):
     """The experts for given routing weights, when the expert group is this rank alone."""
 
     @staticmethod
-    def forward(ctx, x, weights, idx, w1, w2, w3, recompute, budget):
+    def forward(ctx, x, weights, idx, w1, w2, w3, recompute, budget, wants_grad):
         x = x.contiguous()
         weights = weights.float().contiguous()
         out, ctx.recompute, ctx.ledger, saved = _experts_forward(x, weights, idx, w1, w2, w3, recompute, budget,
-                                                                 any(ctx.needs_input_grad))
+                                                                 wants_grad)
         ctx.params, ctx.budget = (w1, w2, w3), budget
         ctx.save_for_backward(*saved)
         return out
@@ -120,7 +121,7 @@ class _MoEFused(torch.autograd.Function):
         dx = native.moe_combine(dx_perm, saved[6], None, dweights.shape[0])
         if ctx.ledger is not None:
             ctx.budget.leave(*ctx.ledger)
-        return dx, dweights, None, dw1, dw2, dw3, None, None
+        return dx, dweights, None, dw1, dw2, dw3, None, None, None
 
 
 class _MoELayer(torch.autograd.Function):
@@ -130,11 +131,11 @@ class _MoELayer(torch.autograd.Function):
     probabilities; its gradient joins the router's in the ``dx`` kernel."""
 
     @staticmethod
-    def forward(ctx, x, router_w, w1, w2, w3, residual, recompute, budget, balance):
+    def forward(ctx, x, router_w, w1, w2, w3, residual, recompute, budget, balance, wants_grad):
         ctx.set_materialize_grads(False)
         _, weights, idx, probs = native.router_fwd(x, router_w)
         out, ctx.recompute, ctx.ledger, saved = _experts_forward(x, weights, idx, w1, w2, w3, recompute, budget,
-                                                                 any(ctx.needs_input_grad), residual)
+                                                                 wants_grad, residual)
         ctx.params, ctx.router_w, ctx.budget = (w1, w2, w3), router_w, budget
         counts = saved.pop()
         ctx.save_for_backward(x, probs, idx, counts, *saved)
@@ -160,7 +161,7 @@ class _MoELayer(torch.autograd.Function):
             drouter = native.gemm_tn(dlogits, x, out_dtype=router_w.dtype)
         if ctx.ledger is not None:
             ctx.budget.leave(*ctx.ledger)
-        return dx, drouter, dw1, dw2, dw3, dresidual, None, None, None
+        return dx, drouter, dw1, dw2, dw3, dresidual, None, None, None, None
 
 
 def moe_layer_fused(x, router_w, w1, w2, w3, residual=None, recompute: bool = False, budget=None,
@@ -175,13 +176,14 @@ def moe_layer_fused(x, router_w, w1, w2, w3, residual=None, recompute: bool = Fa
             and all(t.dtype == torch.bfloat16 and t.is_contiguous() and t.data_ptr() % 16 == 0
                     for t in ((x, router_w) if residual is None else (x, router_w, residual)))):
         return None
-    return _MoELayer.apply(x, router_w, w1, w2, w3, residual, recompute, budget, balance)
+    return _MoELayer.apply(x, router_w, w1, w2, w3, residual, recompute, budget, balance,
+                           backward_follows(x, router_w, w1, w2, w3, residual))
 
 
 def moe_ffn_fused(x, weights, idx, w1, w2, w3, recompute: bool = False, budget=None):
     """The block on one rank.  ``budget`` (``parallel.memory.ActivationBudget``): when given, the call keeps its
     gate/up pre-activations only while the budget has room and rebuilds them in the backward pass otherwise."""
-    return _MoEFused.apply(x, weights, idx, w1, w2, w3, recompute, budget)
+    return _MoEFused.apply(x, weights, idx, w1, w2, w3, recompute, budget, backward_follows(x, weights, w1, w2, w3))
 
 
 # ----------------------------------------------------------------------------- expert-parallel path (comm/ep.py)
@@ -209,14 +211,13 @@ class _MoEPull(torch.autograd.Function):
     weight-gradient GEMMs, combine."""
 
     @staticmethod
-    def forward(ctx, x, weights, idx, w1, w2, w3, recompute, epc, key, budget, slot):
+    def forward(ctx, x, weights, idx, w1, w2, w3, recompute, epc, key, budget, slot, wants_grad):
         from ..comm import ep as E
         g = epc.g
         tokens, dim = x.shape
         ffn = w1.shape[1]
         weights = weights.float().contiguous()
         offs, seg_live_end, tile_expert, meta, seq = epc.plan(idx, weights, key)
-        wants_grad = any(ctx.needs_input_grad)
         cap_saved, ledger = 0, None
         if wants_grad and not recompute:
             cap_saved = epc.expected_rows(key)
@@ -282,7 +283,7 @@ class _MoEPull(torch.autograd.Function):
         dx, dweights = epc.combine(epc.ret_b, E.SIG_RET_B, ret_seq, with_scalars=True)
         if ctx.ledger is not None:
             ctx.budget.leave(*ctx.ledger)
-        return dx, dweights, None, dw1, dw2, dw3, None, None, None, None, None
+        return dx, dweights, None, dw1, dw2, dw3, None, None, None, None, None, None
 
 
 def moe_ffn_pull(x, weights_of, w1, w2, w3, epc, recompute: bool = False, key=None, budget=None):
@@ -293,7 +294,7 @@ def moe_ffn_pull(x, weights_of, w1, w2, w3, epc, recompute: bool = False, key=No
     staged = _StageIn.apply(x.contiguous(), epc, slot)
     weights, idx = weights_of(staged)
     out = _MoEPull.apply(staged, weights, idx, w1, w2, w3, recompute, epc, key if key is not None else id(w1), budget,
-                         slot)
+                         slot, backward_follows(staged, weights, w1, w2, w3))
     if not (torch.is_grad_enabled() and (x.requires_grad or weights.requires_grad)):
         epc.release(slot)          # no backward pass will come for this call
     return out, weights, idx

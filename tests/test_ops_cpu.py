@@ -263,3 +263,41 @@ def test_dense_swiglu_keeps_gate_and_up_only_where_a_backward_pass_can_follow(mo
         ops.swiglu_ffn(x, *weights)
     assert not ops.swiglu_ffn(x, *(w.detach() for w in weights)).requires_grad
     assert kept == [True, False, False]
+
+
+@pytest.mark.parametrize("form", ["layer", "experts"])
+def test_routed_experts_charge_the_budget_only_where_a_backward_pass_can_follow(monkeypatch, form):
+    """Evaluation and the first forward pass of a recomputed block keep no gate and up, and leave the activation budget
+    as it was: no backward pass comes that would give the charge back."""
+    from b200moe.ops import moe_fused, native
+    from b200moe.parallel.memory import ActivationBudget
+    T, D, F, E = 5, 8, 16, 2
+    kept = []
+
+    def gemm_swiglu(x, w1, w3, tile_expert, tiles, save_gate_up, align256):
+        kept.append(save_gate_up)
+        return x.new_zeros(x.shape[0], F), x.new_zeros(1), x.new_zeros(1)
+
+    table = torch.zeros(4, dtype=torch.int32)
+    monkeypatch.setattr(native, "router_fwd", lambda x, w: (None, torch.ones(T, 2), torch.zeros(T, 2), torch.ones(T, E)))
+    monkeypatch.setattr(native, "moe_plan", lambda *_: (table,) * 6)
+    monkeypatch.setattr(native, "moe_gather", lambda x, row_slot, meta, cap: x.new_zeros(cap, D))
+    monkeypatch.setattr(native, "gemm_swiglu", gemm_swiglu)
+    monkeypatch.setattr(native, "gemm_nt", lambda h, w, **_: h.new_zeros(h.shape[0], D))
+    monkeypatch.setattr(native, "moe_combine", lambda y, slot_row, w, tokens, residual=None: y.new_zeros(tokens, D))
+    budget = ActivationBudget(1 << 30)
+    x = torch.zeros(T, D, dtype=torch.bfloat16)
+    w1, w3, w2, router = (torch.zeros(s, dtype=torch.bfloat16, requires_grad=True)
+                          for s in ((E, F, D), (E, F, D), (E, D, F), (E, D)))
+
+    def call():
+        if form == "layer":
+            return moe_fused.moe_layer_fused(x, router, w1, w2, w3, budget=budget)
+        return moe_fused.moe_ffn_fused(x, torch.ones(T, 2), torch.zeros(T, 2), w1, w2, w3, budget=budget)
+
+    with torch.no_grad():
+        call()
+    assert (budget.used, budget.live_calls, budget.granted, budget.refused) == (0, 0, 0, 0)
+    assert call().requires_grad
+    assert budget.live_calls == 1 and budget.used > 0
+    assert kept == [False, True]
