@@ -24,7 +24,7 @@ from __future__ import annotations
 
 import torch
 
-from . import functional as Fn, native, use_native
+from . import backward_follows, functional as Fn, native, use_native
 
 CHUNK_TOKENS = 4096
 # 16384 tokens of a 32000-entry vocabulary: 1.05 GB of 180.  Keeping instead of rebuilding saves one of four products
@@ -39,15 +39,15 @@ def _chunks(total: int, size: int):
 
 class _LMHeadCE(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, hidden, weight, targets, grad_scale):
+    def forward(ctx, hidden, weight, targets, grad_scale, wants_grad):
         h2d = hidden.reshape(-1, hidden.shape[-1])
         flat_targets = targets.reshape(-1).contiguous()
         tokens = h2d.shape[0]
         main_grad = getattr(weight, "main_grad", None)
-        eager = grad_scale is not None and main_grad is not None and ctx.needs_input_grad[0]
+        eager = wants_grad and grad_scale is not None and main_grad is not None and ctx.needs_input_grad[0]
         loss = torch.zeros((), dtype=torch.float32, device=hidden.device)
         ctx.weight, ctx.shape, ctx.eager, ctx.grad_scale = weight, hidden.shape, eager, grad_scale
-        ctx.kept = (not eager and any(ctx.needs_input_grad) and 0 < tokens * weight.shape[0] * 2 <= KEEP_BYTES)
+        ctx.kept = not eager and wants_grad and 0 < tokens * weight.shape[0] * 2 <= KEEP_BYTES
         if ctx.kept:
             logits = native.gemm_nt(h2d, weight)
             native.cross_entropy_scaled_(logits, flat_targets, loss, 1.0 / tokens, 1.0 / tokens)
@@ -73,7 +73,7 @@ class _LMHeadCE(torch.autograd.Function):
         if ctx.eager:
             (dh,) = ctx.saved_tensors
             native.scale_(dh, dloss / ctx.grad_scale)
-            return dh.view(ctx.shape), None, None, None
+            return dh.view(ctx.shape), None, None, None, None
         if ctx.kept:
             h2d, dlogits = ctx.saved_tensors
             scale = dloss.to(device=h2d.device, dtype=torch.float32)
@@ -84,7 +84,7 @@ class _LMHeadCE(torch.autograd.Function):
                 native.gemm_tn(dlogits, h2d, out=main_grad, accumulate=True, alpha=scale)
             elif ctx.needs_input_grad[1]:
                 dw = native.gemm_tn(dlogits, h2d, out_dtype=weight.dtype, alpha=scale)
-            return None if dh is None else dh.view(ctx.shape), dw, None, None
+            return None if dh is None else dh.view(ctx.shape), dw, None, None, None
         h2d, flat_targets = ctx.saved_tensors
         tokens = h2d.shape[0]
         main_grad = getattr(weight, "main_grad", None)
@@ -99,7 +99,7 @@ class _LMHeadCE(torch.autograd.Function):
             native.scale_(logits, dloss)
             native.gemm_nn(logits, weight, out=dh[lo:hi])
             native.gemm_tn(logits, h2d[lo:hi], out=main_grad if main_grad is not None else dw, accumulate=True)
-        return dh.view(ctx.shape), (dw.to(weight.dtype) if dw is not None else None), None, None
+        return dh.view(ctx.shape), (dw.to(weight.dtype) if dw is not None else None), None, None, None
 
 
 def lm_head_cross_entropy(hidden: torch.Tensor, weight: torch.Tensor, targets: torch.Tensor,
@@ -108,6 +108,6 @@ def lm_head_cross_entropy(hidden: torch.Tensor, weight: torch.Tensor, targets: t
     back-propagate into the returned loss, when it is known in advance (see the module text)."""
     from .dense import linear
     if use_native(hidden, "lmhead_ce"):
-        return _LMHeadCE.apply(hidden, weight, targets, grad_scale)
+        return _LMHeadCE.apply(hidden, weight, targets, grad_scale, backward_follows(hidden, weight))
     logits = linear(hidden, weight)
     return Fn.cross_entropy(logits.reshape(-1, logits.shape[-1]), targets.reshape(-1))

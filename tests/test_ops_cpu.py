@@ -301,3 +301,25 @@ def test_routed_experts_charge_the_budget_only_where_a_backward_pass_can_follow(
     assert call().requires_grad
     assert budget.live_calls == 1 and budget.used > 0
     assert kept == [False, True]
+
+
+def test_head_keeps_whole_logits_only_where_a_backward_pass_can_follow(monkeypatch):
+    from b200moe.ops import loss, native
+    rows = []
+
+    def gemm_nt(h, w):
+        rows.append(h.shape[0])
+        return h.new_zeros(h.shape[0], w.shape[0])
+
+    monkeypatch.setattr(loss, "use_native", lambda *_: True)
+    monkeypatch.setattr(loss, "CHUNK_TOKENS", 4)
+    monkeypatch.setattr(native, "gemm_nt", gemm_nt)
+    monkeypatch.setattr(native, "cross_entropy_scaled_", lambda *_: None)
+    hidden, targets = torch.zeros(10, 8), torch.zeros(10, dtype=torch.long)
+    weight = torch.zeros(16, 8, requires_grad=True)
+    with torch.no_grad():
+        ops.lm_head_cross_entropy(hidden, weight, targets)
+    assert rows == [4, 4, 2]
+    rows.clear()
+    assert ops.lm_head_cross_entropy(hidden, weight, targets).requires_grad
+    assert rows == [10]
