@@ -283,9 +283,11 @@ class MoELayerMulti(nn.Module):
         return self._forward(x, return_aux_loss, None)
 
     def _fused(self, flat, residual, balance):
-        """Router and experts as one op: one rank, and nobody watches the router's calls."""
-        if not (self.world_size == 1 and ops.use_native(flat, "moe") and type(self.router) is LinearLayer
-                and type(self.experts) is GroupedPositionWiseFFLayer and not _hooked(self.router)):
+        """Router and experts as one op: one rank, the kernels of every step switched on, and nobody watches the
+        router's calls."""
+        if not (self.world_size == 1 and all(ops.use_native(flat, op) for op in ("moe", "router", "gemm"))
+                and type(self.router) is LinearLayer and type(self.experts) is GroupedPositionWiseFFLayer
+                and not _hooked(self.router)):
             return None
         from ..ops.moe_fused import moe_layer_fused
         router = self.router.compute_weight if self.router.compute_weight is not None else self.router.weight

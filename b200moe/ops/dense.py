@@ -134,8 +134,8 @@ def swiglu_ffn(x, w1, w3, w2):
     take 128 gate columns beside 128 up columns, and reduce in steps of 64).  4096 x 4096 -> 14336, forward and
     backward: 3.8 ms of products instead of 3.45 ms plus 1.6 ms of elementwise passes over the hidden layer."""
     weights = (w1, w3, w2)
-    if not (use_native(x, "gemm") and x.dtype == torch.bfloat16 and x.numel() > 0 and x.data_ptr() % 16 == 0
-            and x.is_contiguous() and all(
+    if not (use_native(x, "gemm") and use_native(x, "swiglu") and x.dtype == torch.bfloat16 and x.numel() > 0
+            and x.data_ptr() % 16 == 0 and x.is_contiguous() and all(
                 w.dtype == torch.bfloat16 and w.dim() == 2 and w.is_contiguous() and w.data_ptr() % 16 == 0
                 and w.device == x.device and getattr(w, "pending_gather", None) is None for w in weights)):
         return None

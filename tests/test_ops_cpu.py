@@ -323,3 +323,18 @@ def test_head_keeps_whole_logits_only_where_a_backward_pass_can_follow(monkeypat
     rows.clear()
     assert ops.lm_head_cross_entropy(hidden, weight, targets).requires_grad
     assert rows == [10]
+
+
+@pytest.mark.parametrize("disabled", ["", "moe", "router", "gemm", "swiglu"])
+def test_switching_off_an_op_family_leaves_the_fused_layers_that_replace_it(monkeypatch, disabled):
+    from b200moe.models.layers import MoELayerMulti
+    from b200moe.ops import dense, moe_fused
+    monkeypatch.setattr(ops, "use_native", lambda t, op="": op != disabled)
+    monkeypatch.setattr(dense, "use_native", lambda t, op="": op != disabled)
+    monkeypatch.setattr(moe_fused, "moe_layer_fused", lambda *_, **__: "fused")
+    monkeypatch.setattr(dense._SwiGLUFFN, "apply", lambda *_: "fused")
+    layer = MoELayerMulti(64, 128, num_expert_per_node=2)
+    x = torch.zeros(3, 64, dtype=torch.bfloat16)
+    assert (layer._fused(x, None, False) is None) == (disabled in ("moe", "router", "gemm"))
+    weights = [torch.zeros(s, dtype=torch.bfloat16) for s in ((128, 64), (128, 64), (64, 128))]
+    assert (ops.swiglu_ffn(x, *weights) is None) == (disabled in ("gemm", "swiglu"))
