@@ -51,6 +51,7 @@ def _second_order(q, k, v, dout, cos, sin, causal):
 class _RopeAttention(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, cos, sin):
+        native._bf16(q)           # the forward kernel takes fp16 too, the gradients do not
         out, lse, q_rot, k_rot = native.attention_fwd(q, k, v, cos, sin)
         ctx.ragged = q.shape[1] % 128 != 0
         ctx.save_for_backward(q_rot, k_rot, v, out, lse, cos, sin, *((q, k) if ctx.ragged else ()))

@@ -338,3 +338,15 @@ def test_switching_off_an_op_family_leaves_the_fused_layers_that_replace_it(monk
     assert (layer._fused(x, None, False) is None) == (disabled in ("moe", "router", "gemm"))
     weights = [torch.zeros(s, dtype=torch.bfloat16) for s in ((128, 64), (128, 64), (64, 128))]
     assert (ops.swiglu_ffn(x, *weights) is None) == (disabled in ("gemm", "swiglu"))
+
+
+def test_differentiable_attention_refuses_fp16_before_it_runs(monkeypatch):
+    """The fp16 kernel has no backward pass: an error in the forward call, not later."""
+    from b200moe.ops import attention, native
+    monkeypatch.setattr(attention, "use_native", lambda *_: True)
+    monkeypatch.setattr(native, "attention_fwd", lambda q, k, v, cos, sin: (q, q.new_zeros(1), q, k))
+    q = torch.zeros(1, 128, 1, 128, dtype=torch.float16, requires_grad=True)
+    with pytest.raises(TypeError):
+        ops.rope_attention(q, q, q, None, None)
+    q = torch.zeros(1, 128, 1, 128, dtype=torch.bfloat16, requires_grad=True)
+    assert ops.rope_attention(q, q, q, None, None).requires_grad
