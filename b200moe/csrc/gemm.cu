@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
     // bytes per lane at 32 rows into one instruction: half sectors, 32 lines.  Instead each warp passes 32 rows x 32
     // fp32 columns through shared memory (16-byte units, XOR-swizzled by row: conflict-free both ways), after which
     // four lanes hold 32 consecutive columns of a row.  Products with a short reduction are bound by this part; before
-    // (four warps, straight stores) and after, us: bf16 store 8192 x 3584 K 1024 60 -> 53, SwiGLU 4096 x 14336 K 4096
+    // (four warps, straight stores) and after, us: bf16 store 8192 x 3584 K 1024 55 -> 47, SwiGLU 4096 x 14336 K 4096
     // 756 -> 711 and 4096 x 1536 K 1024 45 -> 34, fp32 accumulate 4096 x 14336 K 4096 412 -> 375 and K 512 183 -> 130.
     uint4* const staged = reinterpret_cast<uint4*>(smem + STAGES * STAGE_BYTES + 256) + (warp - 2) * 256;
     auto swz = [](int r) { return (r & 1) | ((r & 2) << 1) | ((r & 4) >> 1); };
@@ -467,8 +467,49 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
         const bool add = ACC && p.beta != 0.f;
         constexpr bool SCALED = EPI == EPI_ACC_F32 || EPI == EPI_ACC_BF16 || EPI == EPI_STORE_BF16 || EPI == EPI_STORE_F32;
         const float alpha = SCALED && p.alpha ? *p.alpha : 1.f;
+        if (EPI == EPI_STORE_BF16 || (EPI == EPI_ACC_BF16 && !add)) {
+          // Nothing is added to the product: it is rounded before it is staged, 64 columns of a row in 128 bytes.  In fp32 a
+          // tile passes 128 KiB each way, 2048 cycles of the shared memory, which a launch with a short reduction or a
+          // single tile shows: us, 6144 x 4096 K 100 26.7 -> 22.2, 1024 x 1024 K 1024 10.7 -> 9.7, 100 x 512 K 512 8.0 ->
+          // 7.1 (stored straight from the accumulator's layout: 22.1, 10.2 and 7.2).
+          const int q8 = lane & 7;
 #pragma unroll 1
-        for (int c = half * 128; c < half * 128 + 128; c += 32) {
+          for (int c = half * 128; c < half * 128 + 128; c += 64) {
+            if (col_base + c >= p.N) break;
+            uint32_t v[2][32];
+            if (!empty_k) {
+              tmem_ld_32x32(taddr + c, v[0]);
+              tmem_ld_32x32(taddr + c + 32, v[1]);
+              tmem_ld_wait();
+            } else {
+#pragma unroll
+              for (int i = 0; i < 64; ++i) v[i >> 5][i & 31] = 0;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              uint32_t w[4];
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                const int e = (i & 3) * 8 + 2 * k;
+                w[k] = pack_bf16(__uint_as_float(v[i >> 2][e]) * alpha, __uint_as_float(v[i >> 2][e + 1]) * alpha);
+              }
+              staged[lane * 8 + (i ^ swz(lane))] = make_uint4(w[0], w[1], w[2], w[3]);
+            }
+            __syncwarp();
+            const long long col = col_base + c + q8 * 8;     // N is a multiple of 32 (checked on the host)
+#pragma unroll
+            for (int it = 0; it < 8; ++it) {
+              const int r = it * 4 + (lane >> 3);
+              if (row0 + r >= p.M || col >= p.N) continue;
+              const bool low = !ACC || !p.d2 || row0 + r < p.m_split;
+              const long long off = expert_off + (low ? row0 + r : row0 + r - p.m_split) * p.ldd + col;
+              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(low ? p.d : p.d2) + off) = staged[r * 8 + (q8 ^ swz(r))];
+            }
+            __syncwarp();
+          }
+        }
+#pragma unroll 1
+        for (int c = half * 128; EPI != EPI_STORE_BF16 && (EPI != EPI_ACC_BF16 || add) && c < half * 128 + 128; c += 32) {
           const long long col = col_base + c + q * 8;     // N is a multiple of 32 (checked on the host)
           if (col_base + c >= p.N) break;
           // what the epilogue reads from global memory, all of the chunk in flight before the accumulator arrives

@@ -73,6 +73,20 @@ def _segments(counts, pad=128):
     return (torch.tensor(offs, **dev), torch.tensor(tiles, **dev), torch.tensor([len(tiles), row, 0, 0], **dev), row)
 
 
+@pytest.mark.parametrize("R,M,N", [(64, 8, 32), (100, 136, 96), (129, 264, 288), (64, 520, 352)])
+def test_bf16_products_are_the_fp32_ones_rounded_once(native, tile_mode, R, M, N):
+    """Columns that end inside the 64 of a staged row, rows that end inside a warp's 32: bit for bit the fp32 result
+    of the same tiles, rounded; with a factor, and cut into two outputs."""
+    dy, x, alpha = _rand(R, M), _rand(R, N), torch.tensor(0.37, device="cuda")
+    exact = native.gemm_tn(dy, x, out_dtype=torch.float32, alpha=alpha)
+    assert torch.equal(native.gemm_tn(dy, x, out_dtype=torch.bfloat16, alpha=alpha), exact.bfloat16())
+    halves = [torch.empty(1, M // 2, N, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    native.gemm_tn_two(dy, x, *halves, False)
+    whole = native.gemm_tn(dy, x, out_dtype=torch.float32, alpha=torch.ones((), device="cuda"))
+    assert torch.equal(torch.cat(halves, 1)[0], whole.view(M, N).bfloat16())
+    native.check_status()
+
+
 @pytest.mark.parametrize("pad", [128, 256])
 @pytest.mark.parametrize("counts", [[128, 256], [100, 0, 300, 17], [0, 0, 640, 0], [384] * 4])
 def test_grouped_expert_gemms(native, tile_mode, counts, pad):
