@@ -729,15 +729,19 @@ static TileKind choose_tile(const GemmParams& p, int sms, bool pair_available) {
   const long long k_eff = SCHED == SCHED_WGRAD ? p.K / (p.num_experts > 0 ? p.num_experts : 1) : p.K;
   const bool legal = SCHED == SCHED_WGRAD ||
                      (p.tile_expert == nullptr ? p.num_m_tiles == nullptr : p.group_align256 != 0);
-  const long long tiles256 = static_cast<long long>((p.M + 255) / 256) * ((p.N + BN - 1) / BN) *
-                             (SCHED == SCHED_WGRAD ? p.num_experts : 1);
+  const long long columns = static_cast<long long>((p.N + BN - 1) / BN) * (SCHED == SCHED_WGRAD ? p.num_experts : 1);
+  const long long tiles256 = (p.M + 255) / 256 * columns, tiles128 = (p.M + 127) / 128 * columns;
   if (!legal || g_tile_mode == 1) return TILE_128;
   if (g_tile_mode == 2) return TILE_256;
   if (pair_available && g_tile_mode == 3) return TILE_PAIR;
   if (g_tile_mode == 3) return TILE_128;
   const bool pairs = g_tile_mode == 4 || (g_tile_mode == 0 && EPI != EPI_PUSH);
   if (tiles256 >= 2LL * sms && k_eff >= 6144) return TILE_256;
-  return pair_available && pairs && tiles256 >= sms / 2 ? TILE_PAIR : TILE_128;
+  // Where the second half of the last row of pair tiles lies behind the matrix, pairs may need a wave more: not where it
+  // is more than the tenth that they gain per wave.  Loss of one token, 32000 entries, width 4096: 75 us on 125 pair
+  // tiles (two waves of 74), 61 on 125 single ones (one of 148); 100 tokens, width 512: 22.8 and 16.0.
+  const long long waves256 = (tiles256 + sms / 2 - 1) / (sms / 2), waves128 = (tiles128 + sms - 1) / sms;
+  return pair_available && pairs && tiles256 >= sms / 2 && 10 * waves256 <= 11 * waves128 ? TILE_PAIR : TILE_128;
 }
 
 template <int A_MN, int B_MN, int EPI, int SCHED>
