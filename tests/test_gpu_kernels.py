@@ -390,6 +390,24 @@ def test_many_tensors_per_optimizer_launch_and_zero_fill(native):
     native.check_status()
 
 
+@pytest.mark.parametrize("total", [2047, 4097, 19_500_001])
+def test_optimizer_blocks_of_both_sizes(native, total):
+    """Blocks of 2048 elements, and of 8192 where they fill the machine (from 16 per SM): every element updated once, the
+    remainder behind the last vector too.  fp32 arithmetic in another order: four roundings of 2^-24."""
+    shapes = [total - total // 3, total // 3]
+    p, g, m, v = ([torch.randn(n, device="cuda") for n in shapes] for _ in range(4))
+    v = [t.abs() for t in v]
+    want = []
+    for a, b, c, d in zip(p, g, m, v):
+        mean, square = 0.9 * c + 0.1 * b, 0.999 * d + 0.001 * b * b
+        want.append((a * (1 - 1e-3 * 0.1) - 2e-3 * mean / (square.sqrt() + 1e-8), mean, square))
+    native.adamw_many_([(*t, None) for t in zip(p, g, m, v)], 1e-3, 0.9, 0.999, 1e-8, 0.1, 2e-3)
+    for got, exact in zip(zip(p, m, v), want):
+        for a, b in zip(got, exact):
+            assert torch.allclose(a, b, rtol=1e-4, atol=1e-6)     # 1 - beta2 formed in fp32: 3e-5 of 0.001
+    native.check_status()
+
+
 def test_embedding_rope_adamw(native):
     from b200moe import ops
     from b200moe.ops import functional as Fn
