@@ -8,7 +8,8 @@
 // it into bf16 P in place, and P feeds the next MMA straight from TMEM (A operand in
 // tensor memory), so P never touches shared memory.
 //
-// Forward, one CTA per (256 queries, head, batch): see attn_fwd_kernel.
+// Forward, one CTA per (256 queries, head, batch), or per 128 queries in grids of one wave: see attn_fwd_kernel and
+//   attn_fwd_one_tile_kernel.
 // Backward dK/dV, one CTA per (128 keys, kv head, batch): loops over the 4 query heads
 //   of the group and their causal query tiles with S^T = K Q^T, dP^T = V dO^T, so P^T
 //   and dS^T are A operands in TMEM; dV and dK accumulate in TMEM over the whole loop
@@ -125,6 +126,12 @@ __device__ __forceinline__ f32x2 mul_f32x2(f32x2 a, f32x2 b) {
   return r;
 }
 
+__device__ __forceinline__ float sum_f32x2(f32x2 v) {
+  float a, b;
+  split_f32x2(v, a, b);
+  return a + b;
+}
+
 #define ATTN_FAIL(code)            \
   {                                \
     *abort_flag = 1;               \
@@ -147,6 +154,47 @@ __device__ __forceinline__ AttnWork attn_work(const AttnParams& p, int tiles, in
   const int rest = static_cast<int>(blockIdx.x) - set * per_set;
   const int count = min(p.set_heads, heads - set * p.set_heads);
   return {rest / count, set * p.set_heads + rest % count};
+}
+
+// Probabilities of 64 scores of one row: exponentials, stored in 16 bits as pairs over the first 32 of the 64 score
+// columns at ``ts`` (which the thread has read before), and their sum.  Both forward kernels call it, so the order of the
+// sum (eight partial sums: no long add chain) is the same in both, and which of them runs does not change a bit of the
+// result.  CHUNK columns are stored at a time: 64 leave no bubble before a store, 32 need fewer registers.
+template <int F16, int CHUNK>
+__device__ __forceinline__ float probabilities64(const uint32_t (&lo)[32], const uint32_t (&hi)[32], uint32_t ts,
+                                                 float scale_log2, float neg) {
+  const f32x2 scale2 = make_f32x2(scale_log2, scale_log2), neg2 = make_f32x2(neg, neg);
+  f32x2 sum2[4] = {0, 0, 0, 0};
+  uint32_t packed[CHUNK / 2];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    float x0, x1;
+    split_f32x2(fma_f32x2(bits_f32x2(&(i < 16 ? lo : hi)[(i & 15) * 2]), scale2, neg2), x0, x1);
+    const float p0 = ex2(x0), p1 = ex2(x1);
+    sum2[i & 3] = add_f32x2(sum2[i & 3], make_f32x2(p0, p1));
+    packed[i % (CHUNK / 2)] = F16 ? pack_f16(p0, p1) : pack_bf16(p0, p1);
+    if constexpr (CHUNK == 32) {
+      if (i % 16 == 15) tmem_st_32x16(ts + i / 16 * 16, packed);
+    }
+  }
+  if constexpr (CHUNK == 64) tmem_st_32x32(ts, packed);
+  return sum_f32x2(add_f32x2(add_f32x2(sum2[0], sum2[1]), add_f32x2(sum2[2], sum2[3])));
+}
+
+// Stores 32 output columns of one row, normalised.
+template <int F16>
+__device__ __forceinline__ void store_out32(uint8_t* dst, const uint32_t (&o)[32], float inv) {
+  uint4* d4 = reinterpret_cast<uint4*>(dst);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    uint32_t w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float a = __uint_as_float(o[8 * i + 2 * k]) * inv, e = __uint_as_float(o[8 * i + 2 * k + 1]) * inv;
+      w[k] = F16 ? pack_f16(a, e) : pack_bf16(a, e);
+    }
+    d4[i] = make_uint4(w[0], w[1], w[2], w[3]);
+  }
 }
 
 // One CTA per (two adjacent 128-query tiles, head, batch): the tiles ping-pong, so the tensor core works on one while
@@ -278,7 +326,8 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_fwd_kernel(const __grid_
     const int n = t ? n1 : n0;
     const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
     const uint32_t ts = tmem + t * 128 + lane_base, to = tmem + 256 + t * 128 + lane_base;
-    float m_ref = -INFINITY, l = 0.f;
+    float m_ref = -INFINITY;
+    float l[2] = {0.f, 0.f};                              // row sums of the two column halves
     for (int j = 0; j < n && !*abort_flag; ++j) {
       if (!mbar_wait(&bars->s_full[t], j & 1)) { ATTN_FAIL(206); break; }
       tc_fence_after();
@@ -303,7 +352,8 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_fwd_kernel(const __grid_
       if (__any_sync(0xffffffffu, need)) {
         const float alpha = ex2((m_ref - mx) * p.scale_log2);   // 0 on the first tile
         m_ref = mx;
-        l *= alpha;
+        l[0] *= alpha;
+        l[1] *= alpha;
         if (j > 0) {
 #pragma unroll 1
           for (int c = 0; c < 8; ++c) {
@@ -317,38 +367,20 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_fwd_kernel(const __grid_
         }
       }
       const float neg = -m_ref * p.scale_log2;
-      const f32x2 scale2 = make_f32x2(p.scale_log2, p.scale_log2), neg2 = make_f32x2(neg, neg);
-      f32x2 sum2[4] = {0, 0, 0, 0};          // independent partial sums: no long add chain
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf) {
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          uint32_t packed[16];
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const int k = hf * 64 + c * 32 + 2 * i;
-            float x0, x1;
-            split_f32x2(fma_f32x2(make_f32x2(score(k), score(k + 1)), scale2, neg2), x0, x1);
-            const float p0 = ex2(x0), p1 = ex2(x1);
-            sum2[i & 3] = add_f32x2(sum2[i & 3], make_f32x2(p0, p1));
-            packed[i] = F16 ? pack_f16(p0, p1) : pack_bf16(p0, p1);
-          }
-          tmem_st_32x16(ts + hf * 32 + c * 16, packed);      // pairs over the score columns read above
-        }
+        l[hf] += probabilities64<F16, 32>(raw[2 * hf], raw[2 * hf + 1], ts + hf * 32, p.scale_log2, neg);
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(hf ? &bars->p_hi[t] : &bars->p_lo[t]);
       }
-      float s0, s1;
-      split_f32x2(add_f32x2(add_f32x2(sum2[0], sum2[1]), add_f32x2(sum2[2], sum2[3])), s0, s1);
-      l += s0 + s1;
     }
     // epilogue: normalise and store this thread's query row
     if (n > 0 && !*abort_flag) {
       if (!mbar_wait(&bars->o_done[t], 0)) ATTN_FAIL(208);
       tc_fence_after();
-      const float inv = 1.f / l;
+      const float sum = l[0] + l[1], inv = 1.f / sum;
       const int pos = qt * TQ + r;
       uint8_t* dst = static_cast<uint8_t*>(p.out) + ((static_cast<size_t>(b) * p.S + pos) * p.Hq + h) * HD * 2;
 #pragma unroll 1
@@ -356,22 +388,213 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_fwd_kernel(const __grid_
         uint32_t o[32];
         tmem_ld_32x32(to + c * 32, o);
         tmem_ld_wait();
-        if (pos < p.S) {
-          uint4* d4 = reinterpret_cast<uint4*>(dst + c * 64);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            uint32_t w[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const float a = __uint_as_float(o[8 * i + 2 * k]) * inv, e = __uint_as_float(o[8 * i + 2 * k + 1]) * inv;
-              w[k] = F16 ? pack_f16(a, e) : pack_bf16(a, e);
-            }
-            d4[i] = make_uint4(w[0], w[1], w[2], w[3]);
-          }
-        }
+        if (pos < p.S) store_out32<F16>(dst + c * 64, o, inv);
         __syncwarp();
       }
-      if (pos < p.S) p.lse[static_cast<size_t>(work.head) * p.S + pos] = m_ref * p.scale + logf(l);
+      if (pos < p.S) p.lse[static_cast<size_t>(work.head) * p.S + pos] = m_ref * p.scale + logf(sum);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 9) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 512);
+  }
+}
+
+// The same for grids of at most one CTA per SM: one CTA per (128 queries, head, batch), a row's 128 score columns shared by
+// two threads (a warpgroup per 64 columns) that exchange their row maxima, scores of two key tiles in flight.  A tile's
+// chain is half as long as with a row per thread, and where the two-tile form would leave half of the SMs idle that is
+// all that counts: 32 heads of 512 tokens (128 CTAs) 9.9 us against 13.6, 4 heads of 4096 40.2 against 60.0; with 160
+// CTAs, a second wave, 15.7 against 13.7.  Results are the same bit for bit.
+struct FwdOneBars {
+  uint64_t q_full, k_full[2], v_full[2], k_empty[2], v_empty[2], s_full[2], p_full[2], o_done, row_ready;
+};
+struct FwdOneSmem {
+  uint8_t q[TILE_BYTES], k[2][TILE_BYTES], v[2][TILE_BYTES];
+  float row_max[2][2][TQ], row_sum[2][TQ];      // [buffer][half][row], [half][row]
+  FwdOneBars bars;
+  uint32_t tmem_slot;
+  int abort_flag;
+};
+
+template <int F16>
+__global__ void __launch_bounds__(ATTN_THREADS, 1) attn_fwd_one_tile_kernel(const __grid_constant__ AttnParams p) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  FwdOneSmem& sm = *reinterpret_cast<FwdOneSmem*>(smem_raw);
+  FwdOneBars* bars = &sm.bars;
+  volatile int* abort_flag = &sm.abort_flag;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int kv_tiles = (p.S + TK - 1) / TK;
+  const AttnWork work = attn_work(p, kv_tiles, p.B * p.Hq);
+  const int qt = kv_tiles - 1 - work.tile;
+  const int b = work.head / p.Hq, h = work.head - b * p.Hq;
+  const int hk = h / (p.Hq / p.Hkv);
+  const int n_kv = p.causal ? qt + 1 : kv_tiles;
+
+  if (threadIdx.x == 0) {
+    mbar_init(&bars->q_full, 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&bars->k_full[s], 1);
+      mbar_init(&bars->v_full[s], 1);
+      mbar_init(&bars->k_empty[s], 1);
+      mbar_init(&bars->v_empty[s], 1);
+      mbar_init(&bars->s_full[s], 1);
+      mbar_init(&bars->p_full[s], 8);
+    }
+    mbar_init(&bars->o_done, 1);
+    mbar_init(&bars->row_ready, 8);
+    sm.abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 9) {
+    tmem_alloc(&sm.tmem_slot, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = sm.tmem_slot;       // S / P of even and odd key tiles, O: 128 columns each
+  const uint32_t t_o = tmem + 256;
+
+  if (warp == 8) {
+    if (elect_one()) {
+      mbar_expect_tx(&bars->q_full, TILE_BYTES);
+      load_tile(sm.q, &p.map_q, &bars->q_full, h * HD, qt * TQ, b);
+      for (int j = 0; j < n_kv && !*abort_flag; ++j) {
+        const int s = j & 1;
+        const uint32_t ph = ((j >> 1) & 1) ^ 1;
+        if (!mbar_wait(&bars->k_empty[s], ph)) { ATTN_FAIL(201); break; }
+        mbar_expect_tx(&bars->k_full[s], TILE_BYTES);
+        load_tile(sm.k[s], &p.map_k, &bars->k_full[s], hk * HD, j * TK, b);
+        if (!mbar_wait(&bars->v_empty[s], ph)) { ATTN_FAIL(202); break; }
+        mbar_expect_tx(&bars->v_full[s], TILE_BYTES);
+        load_tile(sm.v[s], &p.map_v, &bars->v_full[s], hk * HD, j * TK, b);
+      }
+    }
+  } else if (warp == 9) {
+    if (elect_one()) {
+      constexpr uint32_t idesc_qk = attn_idesc<F16>(0);
+      constexpr uint32_t idesc_pv = attn_idesc<F16>(1);
+      const uint32_t q_addr = smem_u32(sm.q);
+      auto issue_s = [&](int j) {
+        const int s = j & 1;
+        if (!mbar_wait(&bars->k_full[s], (j >> 1) & 1)) return false;
+        tc_fence_after();
+        const uint32_t k_addr = smem_u32(sm.k[s]);
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks)
+          umma_bf16_ss(tmem + s * 128, desc_kmajor(q_addr, ks), desc_kmajor(k_addr, ks), idesc_qk, ks != 0);
+        umma_commit(&bars->k_empty[s]);
+        umma_commit(&bars->s_full[s]);
+        return true;
+      };
+      bool ok = mbar_wait(&bars->q_full, 0) && issue_s(0) && (n_kv < 2 || issue_s(1));
+      if (!ok) ATTN_FAIL(203);
+      for (int j = 0; j < n_kv && ok && !*abort_flag; ++j) {
+        const int s = j & 1;
+        if (!mbar_wait(&bars->p_full[s], (j >> 1) & 1) || !mbar_wait(&bars->v_full[s], (j >> 1) & 1)) {
+          ATTN_FAIL(205);
+          break;
+        }
+        tc_fence_after();
+        const uint32_t v_addr = smem_u32(sm.v[s]);
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks)
+          umma_bf16_ts(t_o, tmem + s * 128 + (ks >> 2) * 64 + (ks & 3) * 8, desc_mnmajor(v_addr, ks), idesc_pv,
+                       (j | ks) != 0);
+        umma_commit(&bars->v_empty[s]);
+        umma_commit(&bars->o_done);
+        if (j + 2 < n_kv && !issue_s(j + 2)) { ATTN_FAIL(204); break; }     // behind the product that reads its P
+      }
+    }
+  } else {
+    const int half = warp >> 2;                           // which 64 key columns this thread handles
+    const int quad = warp & 3;
+    const int r = quad * 32 + lane;                       // query row inside the tile
+    const int col0 = half * 64;
+    const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
+    const uint32_t to = t_o + lane_base + col0;
+    float m_ref = -INFINITY, l = 0.f;
+    for (int j = 0; j < n_kv && !*abort_flag; ++j) {
+      const int s = j & 1;
+      if (!mbar_wait(&bars->s_full[s], (j >> 1) & 1)) { ATTN_FAIL(206); break; }
+      tc_fence_after();
+      const uint32_t ts = tmem + s * 128 + lane_base + col0;
+      uint32_t raw[2][32];
+      tmem_ld_32x32(ts, raw[0]);
+      tmem_ld_32x32(ts + 32, raw[1]);
+      tmem_ld_wait();
+      // keys that the row does not see: after the query (causal, diagonal tile) or behind the sequence
+      const bool diagonal = p.causal && j == qt;
+      if (diagonal || (j + 1) * TK > p.S) {
+        const int limit = (diagonal ? r + 1 : p.S - j * TK) - col0;
+#pragma unroll
+        for (int i = 0; i < 64; ++i)
+          if (i >= limit) raw[i >> 5][i & 31] = 0xff800000u;   // -inf
+      }
+      float mpart[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int i = 0; i < 64; i += 2)
+        mpart[(i >> 1) & 3] = fmaxf(fmaxf(mpart[(i >> 1) & 3], __uint_as_float(raw[i >> 5][i & 31])),
+                                    __uint_as_float(raw[i >> 5][(i & 31) + 1]));
+      float mx = fmaxf(fmaxf(mpart[0], mpart[1]), fmaxf(mpart[2], mpart[3]));
+      // exchange with the thread that owns the other 64 columns; two buffers, since that thread may be a tile ahead
+      sm.row_max[s][half][r] = mx;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->row_ready);
+      if (!mbar_wait(&bars->row_ready, j & 1)) { ATTN_FAIL(209); break; }
+      mx = fmaxf(fmaxf(mx, sm.row_max[s][half ^ 1][r]), m_ref);
+      const bool need = (mx - m_ref) * p.scale_log2 > 8.f;      // also true on the first tile (m_ref = -inf)
+      const bool any = __any_sync(0xffffffffu, need);
+      float alpha = 1.f;
+      if (any) {
+        alpha = ex2((m_ref - mx) * p.scale_log2);               // 0 on the first tile
+        m_ref = mx;
+        l *= alpha;
+      }
+      l += probabilities64<F16, 64>(raw[0], raw[1], ts, p.scale_log2, -m_ref * p.scale_log2);
+      if (j > 0) {
+        if (!mbar_wait(&bars->o_done, (j - 1) & 1)) { ATTN_FAIL(207); break; }
+        tc_fence_after();
+        if (any) {
+#pragma unroll 1
+          for (int c = 0; c < 2; ++c) {
+            uint32_t o[32];
+            tmem_ld_32x32(to + c * 32, o);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+            tmem_st_32x32(to + c * 32, o);
+          }
+        }
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->p_full[s]);
+    }
+    // epilogue: add the two halves of the row sum, normalise and store this thread's 64 columns
+    if (!*abort_flag) {
+      sm.row_sum[half][r] = l;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->row_ready);
+      if (!mbar_wait(&bars->row_ready, n_kv & 1)) ATTN_FAIL(210);
+      const float sum = sm.row_sum[0][r] + sm.row_sum[1][r], inv = 1.f / sum;
+      if (!mbar_wait(&bars->o_done, (n_kv - 1) & 1)) ATTN_FAIL(208);
+      tc_fence_after();
+      const int pos = qt * TQ + r;
+      uint8_t* dst = static_cast<uint8_t*>(p.out) + (((static_cast<size_t>(b) * p.S + pos) * p.Hq + h) * HD + col0) * 2;
+#pragma unroll 1
+      for (int c = 0; c < 2; ++c) {
+        uint32_t o[32];
+        tmem_ld_32x32(to + c * 32, o);
+        tmem_ld_wait();
+        if (pos < p.S) store_out32<F16>(dst + c * 64, o, inv);
+        __syncwarp();
+      }
+      if (half == 0 && pos < p.S) p.lse[static_cast<size_t>(work.head) * p.S + pos] = m_ref * p.scale + logf(sum);
     }
   }
   tc_fence_before();
@@ -921,18 +1144,28 @@ static int heads_per_set(int heads, long long bytes_per_head) {
 
 // The dynamic windows start 1024-byte aligned (the kernels have no static shared memory).
 constexpr int FWD_SMEM = 6 * TILE_BYTES + 512;
+constexpr int FWD_ONE_SMEM = sizeof(FwdOneSmem);
 constexpr int BWD_SMEM = sizeof(BwdSmem);
 static_assert(BWD_SMEM <= 227 * 1024, "shared memory of a backward CTA");
 
-template <int F16>
+static int sm_count_attn() {
+  static int sms = 0;
+  if (sms == 0) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      sms = 0;
+  }
+  return sms > 0 ? sms : 148;
+}
+
+template <void (*kernel)(AttnParams), int smem>
 static int launch_fwd(const AttnParams& p, long long ctas, cudaStream_t stream) {
   static bool set = false;
   if (!set) {
-    if (cudaFuncSetAttribute(attn_fwd_kernel<F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, FWD_SMEM) != cudaSuccess)
-      return -3;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -3;
     set = true;
   }
-  attn_fwd_kernel<F16><<<static_cast<unsigned>(ctas), ATTN_THREADS, FWD_SMEM, stream>>>(p);
+  kernel<<<static_cast<unsigned>(ctas), ATTN_THREADS, smem, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
@@ -960,9 +1193,15 @@ int b2_attention_fwd_ex(const void* q, const void* k, const void* v, long long q
   p.set_heads = heads_per_set(B * Hq, 4LL * S * HD * Hkv / Hq);
   p.out = out; p.lse = lse; p.status = status;
   const long long tiles = (S + TQ - 1) / TQ;
-  const long long ctas = (tiles + 1) / 2 * B * Hq;
-  if (ctas > 0x7fffffffLL) return -10;
-  return f16 ? launch_fwd<1>(p, ctas, stream) : launch_fwd<0>(p, ctas, stream);
+  const long long heads = static_cast<long long>(B) * Hq;
+  if (tiles * heads > 0x7fffffffLL) return -10;
+  // one wave of one-tile CTAs, or heads of a single tile (nothing to ping-pong with): see attn_fwd_one_tile_kernel
+  if (tiles == 1 || tiles * heads <= sm_count_attn())
+    return f16 ? launch_fwd<attn_fwd_one_tile_kernel<1>, FWD_ONE_SMEM>(p, tiles * heads, stream)
+               : launch_fwd<attn_fwd_one_tile_kernel<0>, FWD_ONE_SMEM>(p, tiles * heads, stream);
+  const long long ctas = (tiles + 1) / 2 * heads;
+  return f16 ? launch_fwd<attn_fwd_kernel<1>, FWD_SMEM>(p, ctas, stream)
+             : launch_fwd<attn_fwd_kernel<0>, FWD_SMEM>(p, ctas, stream);
 }
 
 // Causal form (the one the model uses).

@@ -731,6 +731,26 @@ def test_attention_of_ragged_sequences(native, S, causal):
     native.check_status()
 
 
+@pytest.mark.parametrize("S", [1, 128, 129, 200, 256, 257, 387, 640])
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_attention_forward_does_not_depend_on_the_size_of_the_grid(native, S, causal, dtype):
+    """One sequence on the kernel for grids of one wave, and the same sequence in a batch that takes the kernel with two
+    query tiles per CTA: the same bits.  The next batch entry is not finite: a last tile must not read its rows."""
+    torch.manual_seed(S)
+    H = 2
+    B = torch.cuda.get_device_properties(0).multi_processor_count // (H * ((S + 127) // 128)) + 2
+    q, k, v = (torch.randn(B, S, H, 128, device="cuda").to(dtype) for _ in range(3))
+    q[:, :, 0] *= 4                                   # row maxima that grow by more than the rescaling threshold
+    for t in (q, k, v):
+        t[1] = float("inf")
+    alone, alone_lse, _, _ = native.attention_fwd(q[:1], k[:1], v[:1], causal=causal)
+    batch, batch_lse, _, _ = native.attention_fwd(q, k, v, causal=causal)
+    assert bool(torch.isfinite(alone).all()) and bool(torch.isfinite(alone_lse).all())
+    assert torch.equal(batch[0], alone[0]) and torch.equal(batch_lse[0], alone_lse[0])
+    native.check_status()
+
+
 @pytest.mark.parametrize("S", [128, 384])
 @pytest.mark.parametrize("causal", [True, False])
 def test_flash_attention_in_fp16_keeps_fp16_precision(native, S, causal):
