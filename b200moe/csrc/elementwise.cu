@@ -877,9 +877,12 @@ __global__ void __launch_bounds__(256) adamw_kernel(const __grid_constant__ Adam
   }
 }
 
-// Zeros into up to ZERO_MAX buffers in one launch: 64 KiB blocks in turn, 16-byte stores.  Write-bandwidth bound.
+// Zeros into up to ZERO_MAX buffers in one launch: a CTA per 8 KiB, 32 bytes per thread, no loop.  Bound by the writes to
+// memory, which arrive in order this way: 5.9 GB in 783 us, 7.5 TB/s (a copy measures 6.45).  Eight persistent CTAs per SM
+// that take 64 KiB in turn, with 16-byte stores, need 978, with 32-byte stores 962; bulk copies of a zeroed buffer 927;
+// cudaMemset 805.
 constexpr int ZERO_MAX = 64;
-constexpr int ZERO_CHUNK = 65536;
+constexpr int ZERO_CHUNK = 8192;
 struct ZeroTable {
   uint8_t* p[ZERO_MAX];
   long long bytes[ZERO_MAX];
@@ -887,16 +890,25 @@ struct ZeroTable {
   int count;
 };
 __global__ void __launch_bounds__(256) zero_kernel(const __grid_constant__ ZeroTable table) {
-  int which = 0;
-  for (int chunk = blockIdx.x; chunk < table.first_chunk[table.count]; chunk += gridDim.x) {
-    while (chunk >= table.first_chunk[which + 1]) ++which;
-    const size_t begin = static_cast<size_t>(chunk - table.first_chunk[which]) * ZERO_CHUNK;
-    const size_t left = static_cast<size_t>(table.bytes[which]) - begin;
-    const int bytes = left < ZERO_CHUNK ? static_cast<int>(left) : ZERO_CHUNK;
-    uint8_t* dst = table.p[which] + begin;
-#pragma unroll 4
-    for (int i = threadIdx.x * 16; i + 16 <= bytes; i += 256 * 16) *reinterpret_cast<uint4*>(dst + i) = make_uint4(0, 0, 0, 0);
-    for (int i = bytes / 16 * 16 + threadIdx.x; i < bytes; i += 256) dst[i] = 0;
+  const int chunk = blockIdx.x;
+  int which = 0, end = table.count;          // the last buffer that starts at or before this chunk
+  while (end - which > 1) {
+    const int mid = (which + end) / 2;
+    if (table.first_chunk[mid] <= chunk) which = mid;
+    else end = mid;
+  }
+  const size_t at = static_cast<size_t>(chunk - table.first_chunk[which]) * ZERO_CHUNK + threadIdx.x * 32;
+  const size_t bytes = static_cast<size_t>(table.bytes[which]);
+  uint8_t* const dst = table.p[which] + at;
+  if (at + 32 <= bytes) {
+    if ((reinterpret_cast<uintptr_t>(dst) & 31) == 0) {
+      asm volatile("st.global.v8.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1};" ::"l"(dst), "r"(0) : "memory");
+    } else {
+      reinterpret_cast<uint4*>(dst)[0] = make_uint4(0, 0, 0, 0);
+      reinterpret_cast<uint4*>(dst)[1] = make_uint4(0, 0, 0, 0);
+    }
+  } else {
+    for (size_t i = at; i < bytes; ++i) dst[i - at] = 0;
   }
 }
 
@@ -1225,7 +1237,7 @@ int b2_zero(const unsigned long long* ptrs, const long long* bytes, int count, c
     }
     table.first_chunk[table.count] = static_cast<int>(chunks);
     if (chunks == 0) continue;
-    zero_kernel<<<static_cast<int>(min(chunks, static_cast<long long>(sm_count_ew()) * 8)), 256, 0, s>>>(table);
+    zero_kernel<<<static_cast<unsigned>(chunks), 256, 0, s>>>(table);
     if (ok()) return -1;
   }
   return 0;

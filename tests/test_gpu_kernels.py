@@ -390,6 +390,20 @@ def test_many_tensors_per_optimizer_launch_and_zero_fill(native):
     native.check_status()
 
 
+def test_zero_fill_of_whole_vectors_remainders_and_empty_buffers(native):
+    """Buffers on 32-byte and on 16-byte boundaries, empty ones between and behind them, ends inside a thread's 32 bytes
+    and around the 8 KiB of a CTA; guard bytes on either side stay."""
+    sizes = [0, 1, 31, 32, 33, 0, 0, 8191, 8192, 8193, 100_000, 0]
+    for shift in (32, 16):
+        spans = [torch.full((n + 96,), 7, dtype=torch.uint8, device="cuda") for n in sizes]
+        native.zero_many_([t[shift:shift + n] for t, n in zip(spans, sizes)])
+        for t, n in zip(spans, sizes):
+            assert not t[shift:shift + n].any()
+            assert bool((t[:shift] == 7).all()) and bool((t[shift + n:] == 7).all())
+    native.zero_many_([torch.empty(0, device="cuda")])
+    native.check_status()
+
+
 @pytest.mark.parametrize("total", [2047, 4097, 19_500_001])
 def test_optimizer_blocks_of_both_sizes(native, total):
     """Blocks of 2048 elements, and of 8192 where they fill the machine (from 16 per SM): every element updated once, the
