@@ -697,7 +697,10 @@ __global__ void __launch_bounds__(CE_THREADS, 2)
     const bool here = mbar_wait(&arrived, phase);
     phase ^= 1;
     if (__syncthreads_or(!here)) {            // a copy did not arrive in time: report and leave, all threads alike
-      if (threadIdx.x == 0) atomicExch(status, 5);
+      if (threadIdx.x == 0) {
+        atomicExch(status, 5);
+        mbar_wait(&arrived, phase ^ 1);       // it may still land in this CTA's memory: one more limit's time
+      }
       break;
     }
     const float picked =

@@ -215,6 +215,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
     if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
+      bool wrapped = false;       // every stage has been requested at least once
       for (long long tile = worker; tile < total_tiles && !*abort_flag; tile += num_workers) {
         const TileCoord t = decode_tile<SCHED, TM>(p, tile, m_tiles, n_tiles);
         const int m0 = t.m_tile * TILE_M + (PAIR ? static_cast<int>(cta) * BM : 0);
@@ -270,8 +271,15 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
           if (++stage == STAGES) {
             stage = 0;
             phase ^= 1;
+            wrapped = true;
           }
         }
+      }
+      // a CTA that gives up waits (with a limit) for its copies before its shared memory goes to another one; the
+      // leader's barriers count those of both CTAs of a pair
+      if (*abort_flag && cta == 0) {
+        for (int s = 0; s < STAGES; ++s)
+          if (wrapped || s < stage) mbar_wait(&full_bar[s], s < stage ? phase : phase ^ 1);
       }
     }
   } else if (warp == 1) {
