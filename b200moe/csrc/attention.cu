@@ -1243,13 +1243,6 @@ int b2_attention_fwd_ex(const void* q, const void* k, const void* v, long long q
              : launch_fwd<attn_fwd_kernel<0>, FWD_SMEM>(p, ctas, stream);
 }
 
-// Causal form (the one the model uses).
-int b2_attention_fwd(const void* q, const void* k, const void* v, long long q_pitch, long long k_pitch,
-                     long long v_pitch, void* out, float* lse, int B, int S, int Hq, int Hkv, float scale, int* status,
-                     cudaStream_t stream) {
-  return b2_attention_fwd_ex(q, k, v, q_pitch, k_pitch, v_pitch, out, lse, B, S, Hq, Hkv, scale, 1, 0, status, stream);
-}
-
 // Gradients.  dout, out: [B,S,Hq,128] contiguous; stats: fp32 scratch [B*Hq, 2, Sp] with Sp = S rounded up to 128; dq
 // [B,S,Hq,128], dk, dv [B,S,Hkv,128] with token pitches dq_pitch, dk_pitch, dv_pitch (they may be views into one fused
 // gradient buffer).  With rotary tables (fp32 [S, 64]) q and k are the ROTATED tensors the forward pass saw, and dq, dk

@@ -345,7 +345,7 @@ __device__ __forceinline__ float warp_sum_scatter(float (&v)[32], int lane) {
 }
 
 // logits[t, n] = sum_k x[t,k] w[n,k]; weights in shared memory.  NN: N rounded up to 8 or 16.  With TOP2 the router's
-// softmax and choice follow in the same launch (four lanes, a token each).
+// softmax and choice follow in the same launch (four lanes, a token each) and the product itself is not stored.
 template <int NN, bool TOP2>
 __global__ void __launch_bounds__(256) skinny_nt_kernel(const __nv_bfloat16* __restrict__ x,
                                                         const __nv_bfloat16* __restrict__ w, float* __restrict__ out,
@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(256) skinny_nt_kernel(const __nv_bfloat16* __r
     for (int h = 0; h < NN / 8; ++h) {
       const float sum = warp_sum_scatter(acc[h], lane);
       const int t = t0 + lane / 8, n = h * 8 + lane % 8;
-      if (t < T && n < N) out[static_cast<size_t>(t) * N + n] = sum;
+      if (!TOP2 && t < T && n < N) out[static_cast<size_t>(t) * N + n] = sum;
       if (TOP2) chosen[warp][lane / 8][n] = sum;
     }
     if (TOP2) {
@@ -1094,11 +1094,11 @@ int b2_skinny_nt(const void* x, const void* w, float* out, int T, int N, int K, 
   if (N > SKINNY_MAX_N || K % 8 || (N * K) % 8) return -10;
   return launch_skinny_nt<false>(x, w, out, nullptr, nullptr, nullptr, T, N, K, s);
 }
-// Router in one launch: logits[T,N] = x w^T, their softmax ``probs``, the two largest (idx) and their weights.
-int b2_router_fwd(const void* x, const void* w, float* logits, float* weights, long long* idx, float* probs, int T, int N,
-                  int K, cudaStream_t s) {
+// Router in one launch: the softmax ``probs`` [T,N] of x w^T, the two largest (idx) and their weights.
+int b2_router_fwd(const void* x, const void* w, float* weights, long long* idx, float* probs, int T, int N, int K,
+                  cudaStream_t s) {
   if (N < 2 || N > SKINNY_MAX_N || K % 8 || (N * K) % 8) return -10;
-  return launch_skinny_nt<true>(x, w, logits, weights, idx, probs, T, N, K, s);
+  return launch_skinny_nt<true>(x, w, nullptr, weights, idx, probs, T, N, K, s);
 }
 int b2_skinny_nn(const float* dy, const void* w, void* dx, int T, int N, int K, cudaStream_t s) {
   if (N > SKINNY_MAX_N || K % 8) return -10;
@@ -1147,13 +1147,8 @@ int b2_swiglu_bwd(const void* dh, const void* gate, const void* up, void* dgu, v
   return ok();
 }
 
-// loss must be zeroed by the caller; scale is usually 1/T (mean over tokens).
-int b2_cross_entropy(void* logits, const long long* targets, float* loss, int T, int V, float scale, cudaStream_t s) {
-  if (V % 8) return -10;
-  cross_entropy_kernel<<<min(T, sm_count_ew() * 4), CE_THREADS, 0, s>>>((bf16*)logits, targets, loss, T, V, scale);
-  return ok();
-}
-// Loss and gradient scaled separately; rows up to 32768 entries stay in registers (one read, one write).
+// ``loss`` (zeroed by the caller) += loss_scale * sum of the rows' losses, logits <- grad_scale * gradient; rows up to
+// 32768 entries are read once and written once.
 int b2_cross_entropy2(void* logits, const long long* targets, float* loss, int T, int V, float loss_scale,
                       float grad_scale, int* status, cudaStream_t s) {
   if (V % 8) return -10;

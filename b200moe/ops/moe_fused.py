@@ -133,7 +133,7 @@ class _MoELayer(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, router_w, w1, w2, w3, residual, recompute, budget, balance, wants_grad):
         ctx.set_materialize_grads(False)
-        _, weights, idx, probs = native.router_fwd(x, router_w)
+        weights, idx, probs = native.router_fwd(x, router_w)
         out, ctx.recompute, ctx.ledger, saved = _experts_forward(x, weights, idx, w1, w2, w3, recompute, budget,
                                                                  wants_grad, residual)
         ctx.params, ctx.router_w, ctx.budget = (w1, w2, w3), router_w, budget
@@ -167,8 +167,8 @@ class _MoELayer(torch.autograd.Function):
 def moe_layer_fused(x, router_w, w1, w2, w3, residual=None, recompute: bool = False, budget=None,
                     balance: bool = False):
     """Output of a routed layer on one rank (with ``balance``: and its balance loss), or ``None`` where the router has
-    to run by itself: more than 16 experts (or more router weights than a CTA stages), a weight that is still to be gathered, layouts that the
-    16-byte accesses do not take."""
+    to run by itself: more than 16 experts (or more router weights than a CTA stages), a weight that is still to be
+    gathered, layouts that the 16-byte accesses do not take."""
     experts, dim = router_w.shape
     if not (2 <= experts <= 16 and experts == w1.shape[0] and dim == x.shape[1] and dim % 8 == 0
             and experts * dim * 2 <= 200 * 1024 and x.shape[0] > 0

@@ -28,9 +28,9 @@ _has = {}            # op family -> whether the library has it
 
 _FAMILIES = {
     "gemm": "b2_gemm_nt", "rmsnorm": "b2_rmsnorm_fwd", "router": "b2_router_top2_fwd",
-    "lmhead_ce": "b2_cross_entropy", "adamw": "b2_adamw", "embedding": "b2_embedding_fwd",
-    "rope": "b2_rope", "moe": "b2_moe_plan", "attention": "b2_attention_fwd", "comm": "b2_comm_allreduce",
-    "swiglu": "b2_swiglu_bwd",
+    "lmhead_ce": "b2_cross_entropy2", "adamw": "b2_adamw", "embedding": "b2_embedding_fwd",
+    "rope": "b2_rope", "moe": "b2_moe_plan", "attention": "b2_attention_fwd_ex", "comm": "b2_comm_allreduce",
+    "swiglu": "b2_swiglu_bwd", "zero": "b2_zero",
 }
 
 
@@ -239,9 +239,11 @@ def _bf16(t):
 
 # ------------------------------------------------------------------------------ GEMM
 def set_gemm_tile_mode(mode: int) -> None:
-    """0: automatic (the default): 256x256 tiles on CTA pairs (``cta_group::2``) for problems that fill the machine,
-    else the single-CTA kinds; 1: always 128x256 CTA tiles; 2: single-CTA 256x256 tiles wherever legal; 3: CTA pairs
-    wherever legal; 4: like 0, the expert-parallel return included; 5: automatic among the single-CTA kinds.  The environment variable ``B200MOE_GEMM_TILE_MODE`` sets it at load time."""
+    """0: automatic (the default): 256x256 tiles on one CTA for reductions of 6144 and more over at least two such tiles
+    per SM, else on CTA pairs (``cta_group::2``) where they fill the machine, else 128x256 tiles; 1: always 128x256 CTA
+    tiles; 2: single-CTA 256x256 tiles wherever legal; 3: CTA pairs wherever legal; 4: like 0, the expert-parallel return
+    included; 5: automatic among the single-CTA kinds.  The environment variable ``B200MOE_GEMM_TILE_MODE`` sets it at
+    load time."""
     require().b2_gemm_set_tile_mode(_I(mode))
 
 
@@ -295,7 +297,8 @@ def gemm_nn(dy, w, w2=None, tile_expert=None, num_m_tiles=None, num_experts: int
     assert dy.stride(-1) == 1 and w.is_contiguous() and out.stride(-1) == 1 and out.shape == (M, N)
     _call("b2_gemm_nn", _p(_bf16(dy)), _p(_bf16(w)), _p(w2), _p(_bf16(out)), _I(M), _I(N), _I(K), _I(k_split),
           _L(dy.stride(0)), _L(N), _L(out.stride(0)), _I(num_experts), _p(tile_expert), _p(num_m_tiles), _I(int(align256)),
-          _p(alpha), _p(status_word(dy.device)), _stream(), tag=f"{'grouped ' if tile_expert is not None else ''}N={N} K={K}")
+          _p(alpha), _p(status_word(dy.device)), _stream(),
+          tag=f"{'grouped ' if tile_expert is not None else ''}N={N} K={K}")
     return out
 
 
@@ -436,26 +439,17 @@ def router_top2_bwd(dweights, probs, idx, weights):
 
 
 def router_fwd(x, w):
-    """Router product, softmax and top-2 in one launch (``w [E, D]`` bf16, E <= 16): ``(logits, weights, idx, probs)``."""
+    """Router product, softmax and top-2 in one launch (``w [E, D]`` bf16, E <= 16): ``(weights, idx, probs)``."""
     T, K = x.shape
     E = w.shape[0]
-    logits, probs = torch.empty(2, T, E, dtype=torch.float32, device=x.device)
+    probs = torch.empty(T, E, dtype=torch.float32, device=x.device)
     weights = torch.empty(T, 2, dtype=torch.float32, device=x.device)
     idx = torch.empty(T, 2, dtype=torch.int64, device=x.device)
-    _call("b2_router_fwd", _p(_bf16(x)), _p(_bf16(w)), _p(logits), _p(weights), _p(idx), _p(probs), _I(T), _I(E), _I(K),
-          _stream())
-    return logits, weights, idx, probs
+    _call("b2_router_fwd", _p(_bf16(x)), _p(_bf16(w)), _p(weights), _p(idx), _p(probs), _I(T), _I(E), _I(K), _stream())
+    return weights, idx, probs
 
 
 # ------------------------------------------------------------------------------ loss
-def cross_entropy_fwd_bwd_(logits, targets):
-    """Mean loss; ``logits`` (bf16 [T,V]) is overwritten with d(mean loss)/dlogits."""
-    T, V = logits.shape
-    loss = torch.zeros((), dtype=torch.float32, device=logits.device)
-    _call("b2_cross_entropy", _p(_bf16(logits)), _p(targets.contiguous()), _p(loss), _I(T), _I(V), _F(1.0 / T), _stream())
-    return loss
-
-
 def cross_entropy_scaled_(logits, targets, loss, loss_scale: float, grad_scale: float):
     """Adds ``loss_scale · Σ_rows CE`` to ``loss`` (fp32 scalar tensor) and overwrites ``logits`` (bf16 [T,V]) with
     ``grad_scale · (softmax − onehot)``; rows up to 32768 entries are read once and written once."""

@@ -320,7 +320,7 @@ class FSDPWrapperPipelined(nn.Module):
             self.comm.new_step()
         accumulators = [self.flat.full_g, *(p.main_grad for p in self.expert_params)]
         from ..ops import native, use_native
-        if all(use_native(t, "adamw") and t.device == accumulators[0].device for t in accumulators):
+        if all(use_native(t, "zero") and t.device == accumulators[0].device for t in accumulators):
             native.zero_many_(accumulators)      # one launch
         else:
             for t in accumulators:

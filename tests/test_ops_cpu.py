@@ -279,7 +279,7 @@ def test_routed_experts_charge_the_budget_only_where_a_backward_pass_can_follow(
         return x.new_zeros(x.shape[0], F), x.new_zeros(1), x.new_zeros(1)
 
     table = torch.zeros(4, dtype=torch.int32)
-    monkeypatch.setattr(native, "router_fwd", lambda x, w: (None, torch.ones(T, 2), torch.zeros(T, 2), torch.ones(T, E)))
+    monkeypatch.setattr(native, "router_fwd", lambda x, w: (torch.ones(T, 2), torch.zeros(T, 2), torch.ones(T, E)))
     monkeypatch.setattr(native, "moe_plan", lambda *_: (table,) * 6)
     monkeypatch.setattr(native, "moe_gather", lambda x, row_slot, meta, cap: x.new_zeros(cap, D))
     monkeypatch.setattr(native, "gemm_swiglu", gemm_swiglu)
