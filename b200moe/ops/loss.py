@@ -1,24 +1,25 @@
-"""LM head fused with the cross-entropy loss, in token chunks.
+"""LM head fused with the cross-entropy loss.
 
 The reference materialises fp32 logits ``[tokens, vocab]`` and runs max, exp,
 sum, log, gather, mean as separate ops (implementation/nnfunctions.py:56-64,
-layers.py:415-417).  Here no full logits tensor ever exists.  The tokens are
-processed in chunks: the head GEMM writes the bf16 logits of one chunk, one
-kernel (row in registers: one read, one write) turns them into the chunk's
-loss and, in place, into ``dlogits``, and two more GEMMs consume that buffer at
-once: ``dh = dlogits W`` and ``dW += dlogitsᵀ h``.  What is kept for the backward
-pass is ``dh`` ``[tokens, d_model]``, a thirty-second of the logits' size.
+layers.py:415-417).  Here the head GEMM writes bf16 logits, one kernel (rows up
+to 32768 entries read once and written once) turns them into the loss and, in
+place, into ``dlogits``, and two more GEMMs consume those: ``dh = dlogits W``
+and ``dW += dlogitsᵀ h``.
 
-Because the gradients are formed during the forward pass, the factor that the
-caller will back-propagate into the loss has to be known then: ``grad_scale``
-(the pipeline step passes ``1 / microbatches``).  The backward pass multiplies
+Where the factor that the caller will back-propagate into the loss is known
+(``grad_scale``; the pipeline step passes ``1 / microbatches``) and the weight
+has a ``main_grad`` buffer, all of it happens in the forward pass, a chunk of
+tokens at a time: no full logits tensor exists, and what is kept for the
+backward pass is ``dh`` ``[tokens, d_model]``.  The backward pass multiplies
 ``dh`` by ``dloss / grad_scale``, which is one when the caller keeps its word;
-the weight gradient has already been accumulated with ``grad_scale``.  Without
-``grad_scale`` (or without a ``main_grad`` buffer on the weight) nothing is known
-yet: up to ``KEEP_BYTES`` the forward pass then keeps ``d(mean loss)/dlogits``
-as bf16 and the backward pass is two products over all tokens whose epilogues
-multiply by ``dloss``; beyond that the logits of each chunk are rebuilt in the
-backward pass.  The value returned is the mean over tokens, like the reference.
+the weight gradient has already been accumulated with ``grad_scale``.
+
+Where it is not known, the forward pass keeps ``d(mean loss)/dlogits`` of as many
+tokens as ``KEEP_BYTES`` hold, and the backward pass is two products over them
+whose epilogues multiply by ``dloss``; the logits of the chunks beyond are
+rebuilt.  Where no backward pass can follow, only the loss is formed, chunk by
+chunk.  The value returned is the mean over tokens, like the reference.
 """
 from __future__ import annotations
 
@@ -27,14 +28,21 @@ import torch
 from . import backward_follows, functional as Fn, native, use_native
 
 CHUNK_TOKENS = 4096
-# 16384 tokens of a 32000-entry vocabulary: 1.05 GB of 180.  Keeping instead of rebuilding saves one of four products
-# and a pass over the logits (6001 tokens, width 2048: 3307 -> 2115 us); above, the chunked form bounds the memory.
+# Keeping logits saves one of four products and a pass over them for each token kept (6001 tokens, width 2048, 32000
+# entries: 3307 us rebuilt, 2054 kept).  1 GiB is what a planned stage sets aside for the head's transients
+# (parallel.memory: two logits tensors of a microbatch) at 8192 tokens of 32000 entries.
 KEEP_BYTES = 1 << 30
 
 
-def _chunks(total: int, size: int):
-    for lo in range(0, total, size):
+def _chunks(first: int, total: int, size: int):
+    for lo in range(first, total, size):
         yield lo, min(total, lo + size)
+
+
+def _kept_tokens(tokens: int, vocab: int) -> int:
+    """How many of ``tokens`` rows of bf16 logits ``KEEP_BYTES`` hold: all, or as many whole chunks as fit."""
+    fit = KEEP_BYTES // (2 * vocab)
+    return tokens if tokens <= fit else fit // CHUNK_TOKENS * CHUNK_TOKENS
 
 
 class _LMHeadCE(torch.autograd.Function):
@@ -47,14 +55,13 @@ class _LMHeadCE(torch.autograd.Function):
         eager = wants_grad and grad_scale is not None and main_grad is not None and ctx.needs_input_grad[0]
         loss = torch.zeros((), dtype=torch.float32, device=hidden.device)
         ctx.weight, ctx.shape, ctx.eager, ctx.grad_scale = weight, hidden.shape, eager, grad_scale
-        ctx.kept = not eager and wants_grad and 0 < tokens * weight.shape[0] * 2 <= KEEP_BYTES
+        ctx.kept = _kept_tokens(tokens, weight.shape[0]) if wants_grad and not eager else 0
+        kept = None
         if ctx.kept:
-            logits = native.gemm_nt(h2d, weight)
-            native.cross_entropy_scaled_(logits, flat_targets, loss, 1.0 / tokens, 1.0 / tokens)
-            ctx.save_for_backward(h2d, logits)
-            return loss
+            kept = native.gemm_nt(h2d[:ctx.kept], weight)
+            native.cross_entropy_scaled_(kept, flat_targets[:ctx.kept], loss, 1.0 / tokens, 1.0 / tokens)
         dh = torch.empty_like(h2d) if eager else None
-        for lo, hi in _chunks(tokens, CHUNK_TOKENS):
+        for lo, hi in _chunks(ctx.kept, tokens, CHUNK_TOKENS):
             logits = native.gemm_nt(h2d[lo:hi], weight)
             native.cross_entropy_scaled_(logits, flat_targets[lo:hi], loss, 1.0 / tokens,
                                          (grad_scale if eager else 1.0) / tokens)
@@ -64,7 +71,7 @@ class _LMHeadCE(torch.autograd.Function):
         if eager:
             ctx.save_for_backward(dh)
         else:
-            ctx.save_for_backward(h2d, flat_targets)
+            ctx.save_for_backward(h2d, flat_targets, kept)
         return loss
 
     @staticmethod
@@ -74,32 +81,34 @@ class _LMHeadCE(torch.autograd.Function):
             (dh,) = ctx.saved_tensors
             native.scale_(dh, dloss / ctx.grad_scale)
             return dh.view(ctx.shape), None, None, None, None
-        if ctx.kept:
-            h2d, dlogits = ctx.saved_tensors
-            scale = dloss.to(device=h2d.device, dtype=torch.float32)
-            dh = native.gemm_nn(dlogits, weight, alpha=scale) if ctx.needs_input_grad[0] else None
-            main_grad = getattr(weight, "main_grad", None)
-            dw = None
-            if main_grad is not None:
-                native.gemm_tn(dlogits, h2d, out=main_grad, accumulate=True, alpha=scale)
-            elif ctx.needs_input_grad[1]:
-                dw = native.gemm_tn(dlogits, h2d, out_dtype=weight.dtype, alpha=scale)
-            return None if dh is None else dh.view(ctx.shape), dw, None, None, None
-        h2d, flat_targets = ctx.saved_tensors
+        h2d, flat_targets, kept = ctx.saved_tensors
         tokens = h2d.shape[0]
+        scale = dloss.to(device=h2d.device, dtype=torch.float32)
         main_grad = getattr(weight, "main_grad", None)
-        dh = torch.empty_like(h2d)
-        dw = None
-        if main_grad is None and ctx.needs_input_grad[1]:
+        wants_dw = main_grad is not None or ctx.needs_input_grad[1]
+        whole = 0 < tokens == ctx.kept
+        dh = torch.empty_like(h2d) if ctx.needs_input_grad[0] else None
+        dw = main_grad
+        if wants_dw and main_grad is None and not whole:
             dw = torch.zeros(weight.shape, dtype=torch.float32, device=weight.device)
+        if ctx.kept:
+            if dh is not None:
+                native.gemm_nn(kept, weight, out=dh[:ctx.kept], alpha=scale)
+            if wants_dw and dw is None:
+                dw = native.gemm_tn(kept, h2d, out_dtype=weight.dtype, alpha=scale)
+            elif wants_dw:
+                native.gemm_tn(kept, h2d[:ctx.kept], out=dw, accumulate=True, alpha=scale)
         scratch = torch.zeros((), dtype=torch.float32, device=h2d.device)
-        for lo, hi in _chunks(tokens, CHUNK_TOKENS):
+        for lo, hi in _chunks(ctx.kept, tokens, CHUNK_TOKENS):
             logits = native.gemm_nt(h2d[lo:hi], weight)
             native.cross_entropy_scaled_(logits, flat_targets[lo:hi], scratch, 1.0 / tokens, 1.0 / tokens)
             native.scale_(logits, dloss)
-            native.gemm_nn(logits, weight, out=dh[lo:hi])
-            native.gemm_tn(logits, h2d[lo:hi], out=main_grad if main_grad is not None else dw, accumulate=True)
-        return dh.view(ctx.shape), (dw.to(weight.dtype) if dw is not None else None), None, None, None
+            if dh is not None:
+                native.gemm_nn(logits, weight, out=dh[lo:hi])
+            if wants_dw:
+                native.gemm_tn(logits, h2d[lo:hi], out=dw, accumulate=True)
+        return (None if dh is None else dh.view(ctx.shape), None if main_grad is not None or dw is None
+                else dw.to(weight.dtype), None, None, None)
 
 
 def lm_head_cross_entropy(hidden: torch.Tensor, weight: torch.Tensor, targets: torch.Tensor,

@@ -296,6 +296,34 @@ def test_lm_head_without_a_known_factor_keeps_or_rebuilds_its_logits(native, kee
     native.check_status()
 
 
+@pytest.mark.parametrize("kept", [64, 128, 192])
+def test_lm_head_keeps_the_chunks_that_fit_and_rebuilds_the_rest(native, kept, monkeypatch):
+    """The same results as with all logits kept, up to the roundings of the rebuilt chunks (logits times the factor in
+    bf16) and of a weight gradient that is added up in fp32: four of 2^-9."""
+    from b200moe import ops
+    from b200moe.ops import loss as L
+    torch.manual_seed(3)
+    T, D, V = 201, 128, 640
+    targets, results = torch.randint(0, V, (T,), device="cuda"), []
+    hidden, weight = _rand(T, D).requires_grad_(True), _rand(V, D, scale=0.1).requires_grad_(True)
+    for limit in (L.KEEP_BYTES, 2 * V * (kept + 5)):
+        monkeypatch.setattr(L, "KEEP_BYTES", limit)
+        monkeypatch.setattr(L, "CHUNK_TOKENS", 64)
+        assert L._kept_tokens(T, V) == (T if not results else kept)
+        hidden.grad = weight.grad = None
+        loss = ops.lm_head_cross_entropy(hidden, weight, targets)
+        (3 * loss).backward()
+        weight.main_grad = torch.ones(V, D, device="cuda")
+        first = [loss.detach(), hidden.grad, weight.grad]
+        hidden.grad = None
+        (3 * ops.lm_head_cross_entropy(hidden, weight, targets)).backward()
+        results.append(first + [hidden.grad, weight.main_grad - 1])
+        del weight.main_grad
+    for got, want in zip(*results):
+        assert _rel(got, want) < 8e-3
+    native.check_status()
+
+
 @pytest.mark.parametrize("T,V", [(1, 8), (149, 8192), (300, 8200), (297, 16384), (150, 16392), (600, 32000), (149, 32768),
                                  (3, 32776)])
 def test_cross_entropy_row_sizes(native, T, V):
