@@ -265,23 +265,21 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_fwd_kernel(const __grid_
       mbar_expect_tx(&bars->q_full, (n1 ? 2 : 1) * TILE_BYTES);
       load_tile(sQ, &p.map_q, &bars->q_full, h * HD, qt0 * TQ, b);
       if (n1) load_tile(sQ + TILE_BYTES, &p.map_q, &bars->q_full, h * HD, (qt0 + 1) * TQ, b);
-      int keys = 0, values = 0;           // tiles requested
-      for (int j = 0; j < n_kv && !*abort_flag; ++j) {
+      int j = 0, key_ahead = 0;
+      for (; j < n_kv && !*abort_flag; ++j) {
         const int s = j & 1;
         const uint32_t ph = ((j >> 1) & 1) ^ 1;
         if (!mbar_wait(&bars->k_empty[s], ph)) { ATTN_FAIL(201); break; }
         mbar_expect_tx(&bars->k_full[s], TILE_BYTES);
         load_tile(sK + s * TILE_BYTES, &p.map_k, &bars->k_full[s], hk * HD, j * TK, b);
-        ++keys;
-        if (!mbar_wait(&bars->v_empty[s], ph)) { ATTN_FAIL(202); break; }
+        if (!mbar_wait(&bars->v_empty[s], ph)) { ATTN_FAIL(202); key_ahead = 1; break; }
         mbar_expect_tx(&bars->v_full[s], TILE_BYTES);
         load_tile(sV + s * TILE_BYTES, &p.map_v, &bars->v_full[s], hk * HD, j * TK, b);
-        ++values;
       }
       if (*abort_flag) {
         mbar_wait(&bars->q_full, 0);
-        drain_ring<2>(bars->k_full, keys);
-        drain_ring<2>(bars->v_full, values);
+        drain_ring<2>(bars->k_full, j + key_ahead);
+        drain_ring<2>(bars->v_full, j);
       }
     }
   } else if (warp == 9) {
@@ -477,23 +475,21 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_fwd_one_tile_kernel(cons
     if (elect_one()) {
       mbar_expect_tx(&bars->q_full, TILE_BYTES);
       load_tile(sm.q, &p.map_q, &bars->q_full, h * HD, qt * TQ, b);
-      int keys = 0, values = 0;           // tiles requested
-      for (int j = 0; j < n_kv && !*abort_flag; ++j) {
+      int j = 0, key_ahead = 0;
+      for (; j < n_kv && !*abort_flag; ++j) {
         const int s = j & 1;
         const uint32_t ph = ((j >> 1) & 1) ^ 1;
         if (!mbar_wait(&bars->k_empty[s], ph)) { ATTN_FAIL(201); break; }
         mbar_expect_tx(&bars->k_full[s], TILE_BYTES);
         load_tile(sm.k[s], &p.map_k, &bars->k_full[s], hk * HD, j * TK, b);
-        ++keys;
-        if (!mbar_wait(&bars->v_empty[s], ph)) { ATTN_FAIL(202); break; }
+        if (!mbar_wait(&bars->v_empty[s], ph)) { ATTN_FAIL(202); key_ahead = 1; break; }
         mbar_expect_tx(&bars->v_full[s], TILE_BYTES);
         load_tile(sm.v[s], &p.map_v, &bars->v_full[s], hk * HD, j * TK, b);
-        ++values;
       }
       if (*abort_flag) {
         mbar_wait(&bars->q_full, 0);
-        drain_ring<2>(bars->k_full, keys);
-        drain_ring<2>(bars->v_full, values);
+        drain_ring<2>(bars->k_full, j + key_ahead);
+        drain_ring<2>(bars->v_full, j);
       }
     }
   } else if (warp == 9) {
@@ -790,8 +786,8 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dkv_kernel(const __g
       mbar_expect_tx(&bars->fixed_full, 2 * TILE_BYTES);
       load_tile(sm.fixed[0], &p.map_k, &bars->fixed_full, hk * HD, kt * TK, b);
       load_tile(sm.fixed[1], &p.map_v, &bars->fixed_full, hk * HD, kt * TK, b);
-      int first = 0, second = 0;          // tiles requested for the two rings
-      for (int it = 0; it < iters && !*abort_flag; ++it) {
+      int it = 0, a_ahead = 0;
+      for (; it < iters && !*abort_flag; ++it) {
         const int s3 = slot3(it), s2 = it & 1;
         const int hq = hk * group + it / per_head;
         const int qi = q_first + it % per_head;
@@ -800,17 +796,15 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dkv_kernel(const __g
         mbar_expect_tx(&bars->a_full[s3], TILE_BYTES + TQ * 4);
         load_tile(sm.a[s3], &p.map_q, &bars->a_full[s3], hq * HD, qi * TQ, b);
         bulk_load(sm.a_stat[s3], stat + q_tiles * TQ, &bars->a_full[s3], TQ * 4);
-        ++first;
-        if (!mbar_wait(&bars->b_empty[s2], ((it >> 1) & 1) ^ 1)) { ATTN_FAIL(212); break; }
+        if (!mbar_wait(&bars->b_empty[s2], ((it >> 1) & 1) ^ 1)) { ATTN_FAIL(212); a_ahead = 1; break; }
         mbar_expect_tx(&bars->b_full[s2], TILE_BYTES + TQ * 4);
         load_tile(sm.b[s2], &p.map_do, &bars->b_full[s2], hq * HD, qi * TQ, b);
         bulk_load(sm.b_stat[s2], stat, &bars->b_full[s2], TQ * 4);
-        ++second;
       }
       if (*abort_flag) {
         mbar_wait(&bars->fixed_full, 0);
-        drain_ring<3>(bars->a_full, first);
-        drain_ring<2>(bars->b_full, second);
+        drain_ring<3>(bars->a_full, it + a_ahead);
+        drain_ring<2>(bars->b_full, it);
       }
     }
   } else if (warp == 9) {
@@ -1002,22 +996,20 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dq_kernel(const __gr
       mbar_expect_tx(&bars->fixed_full, 2 * TILE_BYTES);
       load_tile(sm.fixed[0], &p.map_q, &bars->fixed_full, h * HD, qt * TQ, b);
       load_tile(sm.fixed[1], &p.map_do, &bars->fixed_full, h * HD, qt * TQ, b);
-      int first = 0, second = 0;          // tiles requested for the two rings
-      for (int j = 0; j < n_kv && !*abort_flag; ++j) {
+      int j = 0, a_ahead = 0;
+      for (; j < n_kv && !*abort_flag; ++j) {
         const int s3 = slot3(j), s2 = j & 1;
         if (!mbar_wait(&bars->a_empty[s3], phase3(j) ^ 1)) { ATTN_FAIL(221); break; }
         mbar_expect_tx(&bars->a_full[s3], TILE_BYTES);
         load_tile(sm.a[s3], &p.map_k, &bars->a_full[s3], hk * HD, j * TK, b);
-        ++first;
-        if (!mbar_wait(&bars->b_empty[s2], ((j >> 1) & 1) ^ 1)) { ATTN_FAIL(222); break; }
+        if (!mbar_wait(&bars->b_empty[s2], ((j >> 1) & 1) ^ 1)) { ATTN_FAIL(222); a_ahead = 1; break; }
         mbar_expect_tx(&bars->b_full[s2], TILE_BYTES);
         load_tile(sm.b[s2], &p.map_v, &bars->b_full[s2], hk * HD, j * TK, b);
-        ++second;
       }
       if (*abort_flag) {
         mbar_wait(&bars->fixed_full, 0);
-        drain_ring<3>(bars->a_full, first);
-        drain_ring<2>(bars->b_full, second);
+        drain_ring<3>(bars->a_full, j + a_ahead);
+        drain_ring<2>(bars->b_full, j);
       }
     }
   } else if (warp == 9) {
