@@ -878,6 +878,78 @@ def test_fused_qkv_attention_with_rope(native):
     native.check_status()
 
 
+@pytest.mark.parametrize("S", [100, 129, 387])
+@pytest.mark.parametrize("in_epilogue", [False, True])
+def test_fused_projection_and_attention_of_ragged_sequences(native, S, in_epilogue, monkeypatch):
+    """The rotation by position = row mod S (in place, or in the projection's epilogue), and attention on strided slices
+    of one buffer, where the rows behind a sequence belong to the next one: every row of the output and of the one
+    gradient buffer (filled with NaN first) against 64 bits.  Bound per row: bf16 inputs, probabilities, products and
+    results, as for whole tiles, against the mean row."""
+    from b200moe import ops
+    from b200moe.ops import functional as Fn
+    from b200moe.ops.attention import fused_qkv_attention
+    torch.manual_seed(S)
+    B, Hq, Hkv, hd, D = 3, 4, 1, 128, 256
+    total = Hq + 2 * Hkv
+    cos, sin = Fn.rope_tables(10000.0, hd, 512, device="cuda")
+    x, w, g = _rand(B * S, D), _rand(total * hd, D, scale=D ** -0.5), _rand(B, S, Hq, hd)
+    if in_epilogue:
+        qkv = ops.linear_rope(x, w, cos, sin, (Hq + Hkv) * hd, S)
+    else:
+        qkv = native.gemm_nt(x, w)
+    leaf = qkv.detach().requires_grad_(True)
+    plain = native.gemm_nt(x, w).double().requires_grad_(True)
+    heads = [t.transpose(1, 2) for t in plain.view(B, S, total, hd).split((Hq, Hkv, Hkv), dim=2)]
+
+    def turn(t):
+        a, b, c, s_ = t[..., 0::2], t[..., 1::2], cos[:S].double(), sin[:S].double()
+        return torch.stack((a * c - b * s_, a * s_ + b * c), -1).flatten(-2)
+
+    scores = turn(heads[0]) @ turn(heads[1]).repeat_interleave(Hq // Hkv, 1).mT / math.sqrt(hd)
+    hidden = torch.ones(S, S, dtype=torch.bool, device="cuda").triu(1)
+    ref = (scores.masked_fill(hidden, -math.inf).softmax(-1) @ heads[2].repeat_interleave(Hq // Hkv, 1)).transpose(1, 2)
+    ref.backward(g.double())
+    empty_like = torch.empty_like
+    monkeypatch.setattr(torch, "empty_like", lambda t, **kw: empty_like(t, **kw).fill_(float("nan")))
+    out = fused_qkv_attention(leaf * 1.0, B, S, Hq, Hkv, hd, cos, sin, pre_rotated=in_epilogue)
+    out.backward(g)
+    for got, want in ((out.reshape(B * S, -1), ref.reshape(B * S, -1)), (leaf.grad, plain.grad)):
+        rows = want.norm(dim=1)
+        assert bool(torch.isfinite(got).all())
+        assert float(((got.double() - want).norm(dim=1) / (rows + rows.mean())).max()) < 2e-2
+    native.check_status()
+
+
+@pytest.mark.parametrize("causal", [True, False])
+def test_second_derivatives_of_ragged_attention(native, causal):
+    """``create_graph=True`` at a length that is no multiple of 128: gradients of the gradients through the formula, where
+    the library has a differentiable backward pass for it.  Bounds as for the gradients."""
+    from torch.nn.attention import SDPBackend, sdpa_kernel
+    from b200moe.ops.attention import attention
+    torch.manual_seed(9)
+    B, S, H, hd = 1, 100, 2, 128
+    leaves = [_rand(B, S, H, hd).requires_grad_(True) for _ in range(3)]
+    dout, mix = _rand(B, S, H, hd), [_rand(B, S, H, hd) for _ in range(3)]
+
+    def second(inputs, forward, weight):
+        first = torch.autograd.grad(forward(*inputs), inputs, weight, create_graph=True)
+        return torch.autograd.grad(sum((f * m.to(f.dtype)).sum() for f, m in zip(first, mix)), inputs)
+
+    def formula(q, k, v):
+        q, k, v = (t.transpose(1, 2) for t in (q, k, v))
+        scores = q @ k.mT / math.sqrt(hd)
+        if causal:
+            scores = scores.masked_fill(torch.ones(S, S, dtype=torch.bool, device="cuda").triu(1), -math.inf)
+        return (scores.softmax(-1) @ v).transpose(1, 2)
+
+    with sdpa_kernel(SDPBackend.MATH):
+        got = second(leaves, lambda *t: attention(*t, causal=causal), dout)
+    want = second([t.detach().double().requires_grad_(True) for t in leaves], formula, dout.double())
+    for a, b in zip(got, want):
+        assert _rel(a, b) < 2e-2
+    native.check_status()
+
+
 @pytest.mark.parametrize("tile", [0, 3], ids=["tiles_auto", "tiles_cta_pair"])
 def test_projection_with_rope_in_the_gemm_epilogue_then_attention(native, tile):
     """q/k/v projection whose epilogue rotates q and k, attention on the rotated tensors, and a backward pass whose
