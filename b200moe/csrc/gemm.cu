@@ -726,12 +726,12 @@ enum TileKind : int { TILE_128 = 0, TILE_256 = 1, TILE_PAIR = 2 };
 // whether its segments are padded to 256 rows.
 // 256x256 on one CTA for long reductions over many tiles: the exposed epilogue is amortised, and it takes the least energy
 // per operation (down projection of 11 000 expert rows, K 14336: 0.96 ms against 1.02-1.10 ms on pairs; its dx, K 28672:
-// 1.82 against 1.96-2.15).  Otherwise CTA pairs wherever their tiles reach half of the machine's pairs: whole passes, us,
-// single-CTA kinds -> pairs: three-layer dense SwiGLU stack 11374 -> 10544, one-block step of 2 x 16384 tokens 109651 ->
-// 104820, head and loss of 6001 tokens 3519 -> 3307.  The eight-block step that runs against the 1000 W power cap for ten
-// seconds, ms: single-CTA kinds only 10510, pairs for everything large 10540, this rule 10237.  Below that 128x256 on one
-// CTA.  The expert-parallel return (EPI_PUSH) stays with the single-CTA kinds: its time depends on the links, which one
-// GPU does not show.
+// 1.82 against 1.96-2.15).  Otherwise CTA pairs wherever their tiles reach half of the machine's pairs.  Whole passes,
+// single-CTA kinds only -> this rule: three-layer dense SwiGLU stack 11.28 -> 10.36 ms, one-block step of 2 x 16384 tokens
+// 107.5 -> 103.0, head and loss of 6001 tokens 2.17 -> 2.07.  The eight-block step that runs against the 1000 W power cap
+// for ten seconds, ms: single-CTA kinds only 10510, pairs for everything large 10540, this rule 10237.  Below that 128x256
+// on one CTA.  The expert-parallel return (EPI_PUSH) stays with the single-CTA kinds: its time depends on the links, which
+// one GPU does not show.
 template <int SCHED, int EPI>
 static TileKind choose_tile(const GemmParams& p, int sms, bool pair_available) {
   const long long k_eff = SCHED == SCHED_WGRAD ? p.K / (p.num_experts > 0 ? p.num_experts : 1) : p.K;

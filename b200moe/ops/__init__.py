@@ -53,6 +53,7 @@ from .loss import lm_head_cross_entropy  # noqa: E402
 from .moe import router_top2, moe_ffn, DispatchPlan  # noqa: E402
 
 __all__ = [
-    "Fn", "set_native", "native_enabled", "use_native", "linear", "linear_rope", "swiglu_ffn", "embedding", "rmsnorm", "add_rmsnorm",
+    "Fn", "set_native", "native_enabled", "use_native", "backward_follows", "linear", "linear_rope", "swiglu_ffn",
+    "embedding", "rmsnorm", "add_rmsnorm",
     "rope_attention", "lm_head_cross_entropy", "router_top2", "moe_ffn", "DispatchPlan",
 ]

@@ -135,8 +135,8 @@ def fused_qkv_attention(qkv2d, batch, seq, hq, hkv, hd, cos, sin, pre_rotated: b
 
 
 def attention_backend() -> str:
-    """``native`` (this repository's tcgen05 kernels, the default) or ``library`` (cuDNN through PyTorch, for A/B runs); chosen by the
-    environment variable ``B200MOE_ATTENTION``."""
+    """``native`` (this repository's tcgen05 kernels, the default) or ``library`` (cuDNN through PyTorch, for A/B runs);
+    chosen by the environment variable ``B200MOE_ATTENTION``."""
     import os
     return os.environ.get("B200MOE_ATTENTION", "native")
 
@@ -206,8 +206,9 @@ def flash_attention_forward(q, k, v, causal: bool = False):
     entry point of the reference's hand-written kernel (implementation/kernels/flash_attention.cu:390-448, fp16,
     ``mma.sync``/``wmma``, 32 queries per CTA).  Here every (batch, head) pair is a batch entry of the tcgen05
     forward kernel with one head — ``[B, H, S, 128]`` is read in place as ``[B·H, S, 1, 128]`` — so no transposed
-    copy is made.  The kernel exists for both types (fp16 inputs went through bf16 before: three casts in, one out, 8
-    bits of mantissa instead of 11); shapes it does not cover (head_dim ≠ 128, ``S % 128 ≠ 0``, CPU) take the PyTorch formula, like the reference's scalar fallback kernel."""
+    copy is made.  bf16, and fp16 with its 11 bits of mantissa, run in their own type where ``S`` is a multiple of 128;
+    other lengths (which the kernel would take, but this entry point never sent there), head sizes and devices take the
+    PyTorch formula, like the reference's scalar fallback kernel."""
     B, H, S, hd = q.shape
     want = q.dtype
     if q.is_cuda and want in (torch.float16, torch.bfloat16):

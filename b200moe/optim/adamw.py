@@ -14,8 +14,8 @@ Differences in mechanism: the arithmetic runs in fp32 whatever the storage
 types; a parameter may carry ``main_grad`` (its gradient accumulator, possibly
 of another dtype) which is used instead of ``.grad``; parameters that are views
 of one flat buffer (``p._flat``) are updated with one launch over the whole
-buffer; on CUDA the update is one fused kernel per tensor or flat buffer
-instead of six elementwise launches.  Moment dtype: ``state_dtype`` argument,
+buffer; on CUDA the other tensors share launches of one fused kernel, up to 48
+of the same types each.  Moment dtype: ``state_dtype`` argument,
 or per parameter ``p._state_dtype``, default fp32.
 """
 from __future__ import annotations
