@@ -166,7 +166,8 @@ __device__ __forceinline__ AttnWork attn_work(const AttnParams& p, int tiles, in
 // Probabilities of 64 scores of one row: exponentials, stored in 16 bits as pairs over the first 32 of the 64 score
 // columns at ``ts`` (which the thread has read before), and their sum.  Both forward kernels call it, so the order of the
 // sum (eight partial sums: no long add chain) is the same in both, and which of them runs does not change a bit of the
-// result.  CHUNK columns are stored at a time: 64 leave no bubble before a store, 32 need fewer registers.
+// result (for the two-tile kernel a second sum per row and tile, 82.0 -> 82.3 us at 32 heads of 2048 tokens, every key).
+// CHUNK columns are stored at a time: 64 leave no bubble before a store, 32 need fewer registers.
 template <int F16, int CHUNK>
 __device__ __forceinline__ float probabilities64(const uint32_t (&lo)[32], const uint32_t (&hi)[32], uint32_t ts,
                                                  float scale_log2, float neg) {
