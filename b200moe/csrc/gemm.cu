@@ -75,6 +75,7 @@ enum Schedule : int {
 struct GemmParams {
   CUtensorMap map_a;
   CUtensorMap map_b;
+  CUtensorMap map_d, map_d2;   // fp32 results: d, d2 as the epilogue's bulk stores address them
   CUtensorMap map_b2;          // second B: up-projection (SwiGLU) or K-continuation (k >= k_split)
   int M, N, K;                 // problem per expert for SCHED_WGRAD (K unused there)
   int num_experts;             // >= 1
@@ -159,7 +160,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
   constexpr int TILE_M = BM * TM;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES + EPI_STAGING);
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* tmem_full = empty_bar + STAGES;
   uint64_t* tmem_empty = tmem_full + 2;
@@ -356,8 +357,8 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
     // fp32 columns through shared memory (16-byte units, XOR-swizzled by row: conflict-free both ways), after which
     // four lanes hold 32 consecutive columns of a row.  Products with a short reduction are bound by this part; before
     // (four warps, straight stores) and after, us: bf16 store 8192 x 3584 K 1024 55 -> 47, SwiGLU 4096 x 14336 K 4096
-    // 756 -> 711 and 4096 x 1536 K 1024 45 -> 34, fp32 accumulate 4096 x 14336 K 4096 412 -> 375 and K 512 183 -> 130.
-    uint4* const staged = reinterpret_cast<uint4*>(smem + STAGES * STAGE_BYTES + 256) + (warp - 2) * 256;
+    // 756 -> 711 and 4096 x 1536 K 1024 45 -> 34.
+    uint4* const staged = reinterpret_cast<uint4*>(smem + STAGES * STAGE_BYTES) + (warp - 2) * 256;
     auto swz = [](int r) { return (r & 1) | ((r & 2) << 1) | ((r & 4) >> 1); };
     int acc = 0;
     uint32_t acc_phase = 0;
@@ -427,7 +428,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
         // 128 columns of its 32 rows in shared memory (16-byte units XOR-swizzled by row: conflict-free both ways) and
         // writes them out two rows per instruction, 256 contiguous bytes per row.
         const long long col_base = static_cast<long long>(t.n_tile) * BN;
-        uint4* stage = reinterpret_cast<uint4*>(smem + STAGES * STAGE_BYTES + 256) + (warp - 2) * (32 * 16);
+        uint4* stage = reinterpret_cast<uint4*>(smem + STAGES * STAGE_BYTES) + (warp - 2) * (32 * 16);
         int tag = -1, dest = -1;
         float w = 1.f;
         if (row_ok) {
@@ -471,7 +472,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
         const long long col_base = static_cast<long long>(t.n_tile) * BN;
         const long long expert_off = SCHED == SCHED_WGRAD ? t.expert * p.d_expert_stride : 0;
         const int q = lane & 3;
-        constexpr bool ACC = EPI == EPI_ACC_F32 || EPI == EPI_ACC_BF16;
+        constexpr bool ACC = EPI == EPI_ACC_F32 || EPI == EPI_ACC_BF16, F32 = EPI == EPI_ACC_F32 || EPI == EPI_STORE_F32;
         const bool add = ACC && p.beta != 0.f;
         constexpr bool SCALED = EPI == EPI_ACC_F32 || EPI == EPI_ACC_BF16 || EPI == EPI_STORE_BF16 || EPI == EPI_STORE_F32;
         const float alpha = SCALED && p.alpha ? *p.alpha : 1.f;
@@ -516,12 +517,61 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
             __syncwarp();
           }
         }
+        if (F32) {
+          // fp32 results leave as 32 x 32 boxes that the memory system writes or adds: a warp stages its rows of 32 columns
+          // (16-byte units, XOR-swizzled by row as the tensor map has it) and one lane sends them off.  Each value is added once per launch, so
+          // results do not depend on the order of the tiles (an fp32 subnormal counts as zero in that addition).  Before, the
+          // warp read the old values, added and stored: twice the traffic through the SM, beside the operands of the next
+          // tile.  us, before -> now: 8 experts of 3584 x 1024, 1024 rows each 82.7 -> 72.7, both halves in one launch 140.6 ->
+          // 130.6 (470 MB of results alone are 73), 768 x 512 K 1024 15.1 -> 12.6, 6144 x 4096 K 16384 575 -> 558.  Reading
+          // the old values a chunk ahead instead, or 16 contiguous bytes per lane, gave nothing.
 #pragma unroll 1
-        for (int c = half * 128; EPI != EPI_STORE_BF16 && (EPI != EPI_ACC_BF16 || add) && c < half * 128 + 128; c += 32) {
+          for (int c = half * 128; c < half * 128 + 128; c += 32) {
+            if (col_base + c >= p.N || row0 >= p.M || (add && empty_k)) break;
+            uint32_t v[32];
+            if (!empty_k) {
+              tmem_ld_32x32(taddr + c, v);
+              tmem_ld_wait();
+            } else {
+#pragma unroll
+              for (int i = 0; i < 32; ++i) v[i] = 0;
+            }
+            if (ACC && p.d2 && row0 < p.m_split && row0 + 32 > p.m_split) {
+              // rows of both results in one warp (a cut that is no multiple of 32): each lane its own row
+              if (row_ok) {
+                float* dst = reinterpret_cast<float*>(row < p.m_split ? p.d : p.d2) + expert_off +
+                             (row < p.m_split ? row : row - p.m_split) * p.ldd + col_base + c;
+#pragma unroll
+                for (int i = 0; i < 32; ++i) dst[i] = (add ? dst[i] : 0.f) + __uint_as_float(v[i]) * alpha;
+              }
+              continue;
+            }
+            if (lane == 0) bulk_wait_read();      // the previous box has left the staging buffer
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              staged[lane * 8 + (i ^ (lane & 7))] = make_uint4(
+                  __float_as_uint(__uint_as_float(v[4 * i]) * alpha), __float_as_uint(__uint_as_float(v[4 * i + 1]) * alpha),
+                  __float_as_uint(__uint_as_float(v[4 * i + 2]) * alpha), __float_as_uint(__uint_as_float(v[4 * i + 3]) * alpha));
+            fence_async_shared();
+            __syncwarp();
+            if (lane == 0) {
+              const int col = static_cast<int>(col_base) + c, r = static_cast<int>(row0);
+              const bool low = !ACC || !p.d2 || r < p.m_split;
+              const CUtensorMap* map = low ? &p.map_d : &p.map_d2;
+              const int expert = SCHED == SCHED_WGRAD ? t.expert : 0;
+              if (add) tma_add_3d(map, staged, col, low ? r : r - p.m_split, expert);
+              else tma_store_3d(map, staged, col, low ? r : r - p.m_split, expert);
+              bulk_commit();
+            }
+          }
+        }
+#pragma unroll 1
+        for (int c = half * 128; !F32 && EPI != EPI_STORE_BF16 && (EPI != EPI_ACC_BF16 || add) && c < half * 128 + 128; c += 32) {
           const long long col = col_base + c + q * 8;     // N is a multiple of 32 (checked on the host)
           if (col_base + c >= p.N) break;
           // what the epilogue reads from global memory, all of the chunk in flight before the accumulator arrives
-          constexpr int OLD = EPI == EPI_ACC_BF16 ? 1 : (EPI == EPI_ACC_F32 || EPI == EPI_ROPE || EPI == EPI_SWIGLU_BWD) ? 2 : 0;
+          constexpr int OLD = EPI == EPI_ACC_BF16 ? 1 : (EPI == EPI_ROPE || EPI == EPI_SWIGLU_BWD) ? 2 : 0;
           uint4 old[4][OLD ? OLD : 1];
           if (OLD) {
 #pragma unroll
@@ -531,10 +581,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
               const bool low = !ACC || !p.d2 || rr < p.m_split;
               const long long off = expert_off + (low ? rr : rr - p.m_split) * p.ldd + col;
               const void* out = low ? p.d : p.d2;
-              if (EPI == EPI_ACC_F32 && add) {
-                old[it][0] = reinterpret_cast<const uint4*>(reinterpret_cast<const float*>(out) + off)[0];
-                old[it][OLD - 1] = reinterpret_cast<const uint4*>(reinterpret_cast<const float*>(out) + off)[1];
-              } else if (EPI == EPI_ACC_BF16 && add) {
+              if (EPI == EPI_ACC_BF16 && add) {
                 old[it][0] = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(out) + off);
               } else if (EPI == EPI_ROPE && col < p.rope_cols) {
                 // four adjacent pairs (2j, 2j+1) of a head: table entries [position][(col mod 128)/2 + j]
@@ -575,18 +622,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
             const bool low = !ACC || !p.d2 || row0 + r < p.m_split;
             const long long off = expert_off + (low ? row0 + r : row0 + r - p.m_split) * p.ldd + col;
             void* const out = low ? p.d : p.d2;
-            if (EPI == EPI_ACC_F32 || EPI == EPI_STORE_F32) {
-              if (add) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                  x[i] += __uint_as_float(w0[i]);
-                  x[4 + i] += __uint_as_float(w1[i]);
-                }
-              }
-              float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + off);
-              dst[0] = make_float4(x[0], x[1], x[2], x[3]);
-              dst[1] = make_float4(x[4], x[5], x[6], x[7]);
-            } else if (EPI == EPI_SWIGLU_BWD) {
+            if (EPI == EPI_SWIGLU_BWD) {
               uint32_t og[4], ou[4], oh[4];
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
@@ -641,6 +677,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
         acc_phase ^= 1;
       }
     }
+    if ((EPI == EPI_ACC_F32 || EPI == EPI_STORE_F32) && lane == 0) bulk_wait();      // this warp's stores are done
   }
 
   if (EPI == EPI_PUSH) __threadfence_system();   // my rows are in the peers' memory before the flag below
@@ -819,6 +856,7 @@ int b2_gemm_nt(const void* a, const void* w, void* d, int M, int N, int K, long 
   if (make_map(&p.map_b, w, K, static_cast<long long>(num_experts) * N, ldw, kind == TILE_PAIR ? BN / 2 : BN))
     return -12;
   if (epi == EPI_STORE_BF16) return launch<0, 0, EPI_STORE_BF16, SCHED_FLAT>(p, kind, sms, stream);
+  if (make_out_map(&p.map_d, d, N, M, 1, ldd, M * ldd)) return -14;
   return launch<0, 0, EPI_STORE_F32, SCHED_FLAT>(p, kind, sms, stream);
 }
 
@@ -962,6 +1000,11 @@ int b2_gemm_tn(const void* a, const void* b, void* d, void* d2, int m_split, int
   p.M = M; p.N = N; p.K = R; p.num_experts = num_experts; p.b_expert_rows = 0; p.k_split = 0;
   p.expert_offsets = expert_offsets; p.d = d; p.ldd = ldd; p.d_expert_stride = static_cast<long long>(d2 ? m_split : M) * ldd;
   p.beta = beta; p.status = status;
+  if (out_kind == 1) {
+    const long long low = d2 ? m_split : M;
+    if (make_out_map(&p.map_d, d, N, low, num_experts, ldd, low * ldd)) return -14;
+    if (d2 && make_out_map(&p.map_d2, d2, N, M - m_split, num_experts, ldd, low * ldd)) return -14;
+  }
   if (expert_offsets) {
     if (out_kind == 1) return launch<1, 1, EPI_ACC_F32, SCHED_WGRAD>(p, sm_count(), stream);
     if (out_kind == 2) return launch<1, 1, EPI_ACC_BF16, SCHED_WGRAD>(p, sm_count(), stream);

@@ -50,4 +50,20 @@ static inline int make_map(CUtensorMap* map, const void* base, long long inner, 
   return r == CUDA_SUCCESS ? 0 : -2;
 }
 
+// fp32 result [experts, rows, cols] with row pitch ``pitch_elems`` and expert pitch ``expert_elems``, as the epilogue's
+// stores address it: boxes of 32 rows x 32 columns, 128B swizzle.
+static inline int make_out_map(CUtensorMap* map, const void* base, long long cols, long long rows, long long experts,
+                               long long pitch_elems, long long expert_elems) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return -1;
+  cuuint64_t dims[3] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(experts)};
+  cuuint64_t strides[2] = {static_cast<cuuint64_t>(pitch_elems) * 4, static_cast<cuuint64_t>(expert_elems) * 4};
+  cuuint32_t box[3] = {32, 32, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -2;
+}
+
 }  // namespace b2

@@ -62,6 +62,23 @@ def test_gemm_tn_accumulates(native, tile_mode, R, M, N, dtype):
     native.check_status()
 
 
+@pytest.mark.parametrize("R,F,N", [(64, 4, 32), (100, 36, 96), (129, 264, 288)])
+@pytest.mark.parametrize("accumulate", [True, False])
+def test_fp32_results_cut_between_two_weights(native, tile_mode, R, F, N, accumulate):
+    """The bulk stores of fp32 results: rows behind the matrix, and a cut that lies inside a warp's 32 rows."""
+    dy, x = _rand(R, 2 * F, scale=0.1), _rand(R, N, scale=0.1)
+    guard = torch.randn(3, F, N, device="cuda")
+    got = guard.clone()
+    native.gemm_tn_two(dy, x, got[0], got[1], accumulate)
+    product = (dy.double().t() @ x.double()).view(2, F, N)
+    want = product + guard[:2].double() if accumulate else product
+    # products of bf16 are exact in fp32; R additions and the final one round to 2^-24 of the running sum each
+    bound = (R + 1) * 2.0 ** -24 * (dy.double().abs().t() @ x.double().abs()).view(2, F, N) + 2.0 ** -24 * guard[:2].abs()
+    assert bool(((got[:2].double() - want).abs() <= bound * 1.01 + 1e-30).all())
+    assert torch.equal(got[2], guard[2])
+    native.check_status()
+
+
 def _segments(counts, pad=128):
     padded = [(c + pad - 1) // pad * pad for c in counts]
     offs, tiles, row = [], [], 0
