@@ -24,10 +24,9 @@
 namespace b2 {
 
 constexpr int BM = 128;
-constexpr int BN = 256;
+constexpr int BN = 256;                    // columns of a tile; 128 and 64 for small products (``NT`` below)
 constexpr int BK = 64;
 constexpr int A_SUB_BYTES = BM * BK * 2;   // 16 KiB per 128-row sub-tile of A
-constexpr int B_BYTES = BN * BK * 2;       // 32 KiB
 // MT = 128-row sub-tiles of A per CTA tile.  MT=1: 128x256 tile, 4 stages, accumulator double-buffered in
 // TMEM (epilogue overlaps the next main loop).  MT=2: 256x256 tile (two MMAs per k-step share the B tile in
 // shared memory, a third fewer operand bytes per FLOP), 3 stages, both accumulators fill TMEM.
@@ -35,9 +34,11 @@ constexpr int B_BYTES = BN * BK * 2;       // 32 KiB
 // own 128 rows of A and 128 rows/columns of B (32 KiB per stage, 6 stages), the even CTA issues the MMAs for both,
 // and each CTA's tensor memory holds its 128 rows x 256 columns, double-buffered: the operand traffic of a 256x256
 // tile with the epilogue overlap of a 128x256 one.
-template <int MT, int PAIR = 0> struct Cfg {
-  static constexpr int STAGES = PAIR ? 6 : (MT == 2 ? 3 : 4);
+// NT = columns of the tile.  128 and 64 (MT = 1, no pair) are for products whose 128x256 tiles leave SMs without work.
+template <int MT, int PAIR = 0, int NT = BN> struct Cfg {
+  static constexpr int STAGES = PAIR ? 6 : MT == 2 ? 3 : NT == 256 ? 4 : NT == 128 ? 6 : 8;
   static constexpr int A_BYTES = MT * A_SUB_BYTES;
+  static constexpr int B_BYTES = NT * BK * 2;
   static constexpr int B_STAGE_BYTES = PAIR ? B_BYTES / 2 : B_BYTES;
   static constexpr int STAGE_BYTES = A_BYTES + B_STAGE_BYTES;
   static constexpr int NACC = MT == 2 ? 1 : 2;
@@ -49,7 +50,7 @@ template <int MT, int PAIR = 0> struct Cfg {
 constexpr int EPI_STAGING = 32 * 1024;
 template <int EPI> constexpr int epi_warps() { return EPI == 5 /*EPI_PUSH*/ ? 4 : 8; }
 template <int EPI> constexpr int gemm_threads() { return 64 + 32 * epi_warps<EPI>(); }
-template <int EPI, int MT, int PAIR = 0> constexpr int smem_bytes() { return Cfg<MT, PAIR>::SMEM + EPI_STAGING; }
+template <int EPI, int MT, int PAIR = 0, int NT = BN> constexpr int smem_bytes() { return Cfg<MT, PAIR, NT>::SMEM + EPI_STAGING; }
 constexpr int GROUP_M = 8;
 
 enum Epilogue : int {
@@ -149,14 +150,15 @@ __device__ __forceinline__ TileCoord decode_tile(const GemmParams& p, long long 
   return t;
 }
 
-template <int A_MN, int B_MN, int EPI, int SCHED, int MT, int PAIR>
+template <int A_MN, int B_MN, int EPI, int SCHED, int MT, int PAIR, int NT = BN>
 __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(const __grid_constant__ GemmParams p) {
   static_assert(!PAIR || MT == 1, "a CTA of a pair holds one 128-row sub-tile");
-  constexpr int STAGES = Cfg<MT, PAIR>::STAGES;
-  constexpr int A_BYTES = Cfg<MT, PAIR>::A_BYTES;
-  constexpr int STAGE_BYTES = Cfg<MT, PAIR>::STAGE_BYTES;
-  constexpr int NACC = Cfg<MT, PAIR>::NACC;
-  constexpr int TM = Cfg<MT, PAIR>::TM;
+  static_assert(NT == BN || (MT == 1 && !PAIR && EPI != EPI_PUSH), "narrow tiles: one CTA, 128 rows");
+  constexpr int STAGES = Cfg<MT, PAIR, NT>::STAGES;
+  constexpr int A_BYTES = Cfg<MT, PAIR, NT>::A_BYTES;
+  constexpr int STAGE_BYTES = Cfg<MT, PAIR, NT>::STAGE_BYTES;
+  constexpr int NACC = Cfg<MT, PAIR, NT>::NACC;
+  constexpr int TM = Cfg<MT, PAIR, NT>::TM;
   constexpr int TILE_M = BM * TM;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -175,7 +177,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
   const int worker = PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
   const int num_workers = PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
   const int m_tiles = p.num_m_tiles ? (*p.num_m_tiles + TM - 1) / TM : (p.M + TILE_M - 1) / TILE_M;
-  const int n_tiles = (p.N + BN - 1) / BN;
+  const int n_tiles = (p.N + NT - 1) / NT;
   const long long total_tiles = static_cast<long long>(m_tiles) * n_tiles * (SCHED == SCHED_WGRAD ? p.num_experts : 1);
 
   if (threadIdx.x == 0) {
@@ -220,7 +222,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
       for (long long tile = worker; tile < total_tiles && !*abort_flag; tile += num_workers) {
         const TileCoord t = decode_tile<SCHED, TM>(p, tile, m_tiles, n_tiles);
         const int m0 = t.m_tile * TILE_M + (PAIR ? static_cast<int>(cta) * BM : 0);
-        const int n0 = t.n_tile * BN + (PAIR ? static_cast<int>(cta) * (BN / 2) : 0);
+        const int n0 = t.n_tile * NT + (PAIR ? static_cast<int>(cta) * (NT / 2) : 0);
         for (int kb = 0; kb < t.k_blocks; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1)) {
             *abort_flag = 1;
@@ -252,22 +254,22 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
           }
           // ---- B
           if (EPI == EPI_SWIGLU) {
-            // gate rows then up rows of the same 128 output features (K-major)
-            const int row = t.expert * p.b_expert_rows + t.n_tile * 128;
+            // gate rows then up rows of the same NT / 2 output features (K-major)
+            const int row = t.expert * p.b_expert_rows + t.n_tile * (NT / 2);
             if (PAIR) {
               load(sb, cta == 0 ? &p.map_b : &p.map_b2, k0, row);      // leader: gate rows, peer: up rows
             } else {
               load(sb, &p.map_b, k0, row);
-              load(sb + 16384, &p.map_b2, k0, row);
+              load(sb + NT * 64, &p.map_b2, k0, row);
             }
           } else if (B_MN) {
             const bool second = p.k_split > 0 && k0 >= p.k_split;
             const CUtensorMap* map = second ? &p.map_b2 : &p.map_b;
             const int krow = (SCHED == SCHED_WGRAD ? 0 : t.expert * p.b_expert_rows) + (second ? k0 - p.k_split : k0);
 #pragma unroll
-            for (int c = 0; c < (PAIR ? BN / 128 : BN / 64); ++c) load(sb + c * 8192, map, n0 + c * 64, krow);
+            for (int c = 0; c < (PAIR ? NT / 128 : NT / 64); ++c) load(sb + c * 8192, map, n0 + c * 64, krow);
           } else {
-            load(sb, &p.map_b, k0, t.expert * p.b_expert_rows + n0);     // box of 256 rows (128 in pair mode)
+            load(sb, &p.map_b, k0, t.expert * p.b_expert_rows + n0);     // box of NT rows (128 in pair mode)
           }
           if (++stage == STAGES) {
             stage = 0;
@@ -286,7 +288,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (the leader of a pair)
     if (cta == 0 && elect_one()) {
-      constexpr uint32_t idesc = umma_idesc_bf16(PAIR ? 2 * BM : BM, BN, A_MN, B_MN);
+      constexpr uint32_t idesc = umma_idesc_bf16(PAIR ? 2 * BM : BM, NT, A_MN, B_MN);
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -308,7 +310,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
           break;
         }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + (MT == 2 ? 0 : acc * BN);
+        const uint32_t d_tmem = tmem_base + (MT == 2 ? 0 : acc * NT);
         bool failed = false;
         for (int kb = 0; kb < t.k_blocks; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase)) {
@@ -325,8 +327,8 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
             for (int i = 0; i < MT; ++i) {
               const uint32_t sai = sa + i * A_SUB_BYTES;
               const uint64_t da = A_MN ? umma_smem_desc(sai + k * 2048, 8192, 1024) : umma_smem_desc(sai + k * 32, 16, 1024);
-              if (PAIR) umma_bf16_ss_pair(d_tmem + i * BN, da, db, idesc, (kb | k) != 0);
-              else umma_bf16_ss(d_tmem + i * BN, da, db, idesc, (kb | k) != 0);
+              if (PAIR) umma_bf16_ss_pair(d_tmem + i * NT, da, db, idesc, (kb | k) != 0);
+              else umma_bf16_ss(d_tmem + i * NT, da, db, idesc, (kb | k) != 0);
             }
           }
           commit(&empty_bar[stage]);   // frees the stage once these MMAs have read it
@@ -360,10 +362,44 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
     // 756 -> 711 and 4096 x 1536 K 1024 45 -> 34.
     uint4* const staged = reinterpret_cast<uint4*>(smem + STAGES * STAGE_BYTES) + (warp - 2) * 256;
     auto swz = [](int r) { return (r & 1) | ((r & 2) << 1) | ((r & 4) >> 1); };
+    constexpr bool ACC = EPI == EPI_ACC_F32 || EPI == EPI_ACC_BF16, F32 = EPI == EPI_ACC_F32 || EPI == EPI_STORE_F32;
+    const bool add = ACC && p.beta != 0.f;
+    const int q = lane & 3;
+    // What the epilogue reads from global memory for 32 columns of the warp's rows.  A tile of 64 columns has one such chunk
+    // per warp, which is requested before the wait for the product (1024 x 768 K 512 with rotation 6.2 -> 5.5 us); wider
+    // tiles request a chunk as they come to it, the product of the next tile hides it.
+    constexpr int OLD = EPI == EPI_ACC_BF16 ? 1 : (EPI == EPI_ROPE || EPI == EPI_SWIGLU_BWD) ? 2 : 0;
+    constexpr bool EARLY = NT == 64;
+    uint4 old[4][OLD ? OLD : 1];
+    auto fetch_old = [&](const TileCoord& t, int sub, int c) {
+      const long long col = static_cast<long long>(t.n_tile) * NT + c + q * 8;
+      if ((ACC && !add) || col >= p.N) return;
+      const long long expert_off = SCHED == SCHED_WGRAD ? t.expert * p.d_expert_stride : 0;
+      const long long first = static_cast<long long>(t.m_tile) * TILE_M + (PAIR ? static_cast<int>(cta) : sub) * BM + quad * 32;
+#pragma unroll
+      for (int it = 0; it < 4; ++it) {
+        const long long rr = first + it * 8 + (lane >> 2);
+        if (rr >= p.M) continue;
+        if (EPI == EPI_ACC_BF16) {
+          const bool low = !p.d2 || rr < p.m_split;
+          old[it][0] = *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(low ? p.d : p.d2) + expert_off +
+                                                       (low ? rr : rr - p.m_split) * p.ldd + col);
+        } else if (EPI == EPI_ROPE && col < p.rope_cols) {
+          // four adjacent pairs (2j, 2j+1) of a head: table entries [position][(col mod 128)/2 + j]
+          const size_t tab = static_cast<size_t>(static_cast<int>(rr) % p.rope_seq) * 64 + ((col & 127) >> 1);
+          old[it][0] = *reinterpret_cast<const uint4*>(p.rope_cos + tab);
+          old[it][OLD - 1] = *reinterpret_cast<const uint4*>(p.rope_sin + tab);
+        } else if (EPI == EPI_SWIGLU_BWD) {
+          old[it][0] = *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(p.d_gate) + rr * p.N + col);
+          old[it][OLD - 1] = *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(p.d_up) + rr * p.N + col);
+        }
+      }
+    };
     int acc = 0;
     uint32_t acc_phase = 0;
     for (long long tile = worker; tile < total_tiles && !*abort_flag; tile += num_workers) {
       const TileCoord t = decode_tile<SCHED, TM>(p, tile, m_tiles, n_tiles);
+      if (OLD && EARLY) fetch_old(t, 0, half * (NT / 2));
       if (!mbar_wait(&tmem_full[acc], acc_phase)) {
         *abort_flag = 1;
         atomicExch(p.status, 4);
@@ -373,7 +409,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
       const bool empty_k = t.k_blocks == 0;   // an expert without rows contributes nothing
 #pragma unroll 1
       for (int sub = 0; sub < MT; ++sub) {
-      const uint32_t taddr = tmem_base + (MT == 2 ? sub * BN : acc * BN) + (static_cast<uint32_t>(quad * 32) << 16);
+      const uint32_t taddr = tmem_base + (MT == 2 ? sub * NT : acc * NT) + (static_cast<uint32_t>(quad * 32) << 16);
       const long long row = static_cast<long long>(t.m_tile) * TILE_M + (PAIR ? static_cast<int>(cta) : sub) * BM + row_in_tile;
       const bool row_ok = row < p.M;
       const long long row0 = row - lane;
@@ -381,13 +417,13 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
         // 16 gate and 16 up columns at a time; afterwards two lanes per row, eight features each
         __nv_bfloat16* h = reinterpret_cast<__nv_bfloat16*>(p.d);
         const long long half_n = p.N / 2;
-        const long long col0 = static_cast<long long>(t.n_tile) * 128;
+        const long long col0 = static_cast<long long>(t.n_tile) * (NT / 2);
         const int q = lane & 1;
 #pragma unroll 1
-        for (int c = half * 64; c < half * 64 + 64; c += 16) {
+        for (int c = half * (NT / 4); c < (half + 1) * (NT / 4); c += 16) {
           uint32_t g[16], u[16];
           tmem_ld_32x16(taddr + c, g);
-          tmem_ld_32x16(taddr + 128 + c, u);
+          tmem_ld_32x16(taddr + NT / 2 + c, u);
           tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -469,21 +505,18 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
           __syncwarp();
         }
       } else {
-        const long long col_base = static_cast<long long>(t.n_tile) * BN;
+        const long long col_base = static_cast<long long>(t.n_tile) * NT;
         const long long expert_off = SCHED == SCHED_WGRAD ? t.expert * p.d_expert_stride : 0;
-        const int q = lane & 3;
-        constexpr bool ACC = EPI == EPI_ACC_F32 || EPI == EPI_ACC_BF16, F32 = EPI == EPI_ACC_F32 || EPI == EPI_STORE_F32;
-        const bool add = ACC && p.beta != 0.f;
         constexpr bool SCALED = EPI == EPI_ACC_F32 || EPI == EPI_ACC_BF16 || EPI == EPI_STORE_BF16 || EPI == EPI_STORE_F32;
         const float alpha = SCALED && p.alpha ? *p.alpha : 1.f;
-        if (EPI == EPI_STORE_BF16 || (EPI == EPI_ACC_BF16 && !add)) {
+        if (NT >= 128 && (EPI == EPI_STORE_BF16 || (EPI == EPI_ACC_BF16 && !add))) {
           // Nothing is added to the product: it is rounded before it is staged, 64 columns of a row in 128 bytes.  In fp32 a
           // tile passes 128 KiB each way, 2048 cycles of the shared memory, which a launch with a short reduction or a
           // single tile shows: us, 6144 x 4096 K 100 26.7 -> 22.2, 1024 x 1024 K 1024 10.7 -> 9.7, 100 x 512 K 512 8.0 ->
           // 7.1 (stored straight from the accumulator's layout: 22.1, 10.2 and 7.2).
           const int q8 = lane & 7;
 #pragma unroll 1
-          for (int c = half * 128; c < half * 128 + 128; c += 64) {
+          for (int c = half * (NT / 2); c < (half + 1) * (NT / 2); c += 64) {
             if (col_base + c >= p.N) break;
             uint32_t v[2][32];
             if (!empty_k) {
@@ -526,7 +559,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
           // 130.6 (470 MB of results alone are 73), 768 x 512 K 1024 15.1 -> 12.6, 6144 x 4096 K 16384 575 -> 558.  Reading
           // the old values a chunk ahead instead, or 16 contiguous bytes per lane, gave nothing.
 #pragma unroll 1
-          for (int c = half * 128; c < half * 128 + 128; c += 32) {
+          for (int c = half * (NT / 2); c < (half + 1) * (NT / 2); c += 32) {
             if (col_base + c >= p.N || row0 >= p.M || (add && empty_k)) break;
             uint32_t v[32];
             if (!empty_k) {
@@ -567,33 +600,10 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
           }
         }
 #pragma unroll 1
-        for (int c = half * 128; !F32 && EPI != EPI_STORE_BF16 && (EPI != EPI_ACC_BF16 || add) && c < half * 128 + 128; c += 32) {
+        for (int c = half * (NT / 2); !F32 && (NT < 128 || (EPI != EPI_STORE_BF16 && (EPI != EPI_ACC_BF16 || add))) && c < (half + 1) * (NT / 2); c += 32) {
           const long long col = col_base + c + q * 8;     // N is a multiple of 32 (checked on the host)
           if (col_base + c >= p.N) break;
-          // what the epilogue reads from global memory, all of the chunk in flight before the accumulator arrives
-          constexpr int OLD = EPI == EPI_ACC_BF16 ? 1 : (EPI == EPI_ROPE || EPI == EPI_SWIGLU_BWD) ? 2 : 0;
-          uint4 old[4][OLD ? OLD : 1];
-          if (OLD) {
-#pragma unroll
-            for (int it = 0; it < 4; ++it) {
-              const long long rr = row0 + it * 8 + (lane >> 2);
-              if (rr >= p.M) continue;
-              const bool low = !ACC || !p.d2 || rr < p.m_split;
-              const long long off = expert_off + (low ? rr : rr - p.m_split) * p.ldd + col;
-              const void* out = low ? p.d : p.d2;
-              if (EPI == EPI_ACC_BF16 && add) {
-                old[it][0] = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(out) + off);
-              } else if (EPI == EPI_ROPE && col < p.rope_cols) {
-                // four adjacent pairs (2j, 2j+1) of a head: table entries [position][(col mod 128)/2 + j]
-                const size_t tab = static_cast<size_t>(static_cast<int>(rr) % p.rope_seq) * 64 + ((col & 127) >> 1);
-                old[it][0] = *reinterpret_cast<const uint4*>(p.rope_cos + tab);
-                old[it][OLD - 1] = *reinterpret_cast<const uint4*>(p.rope_sin + tab);
-              } else if (EPI == EPI_SWIGLU_BWD) {
-                old[it][0] = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.d_gate) + rr * p.N + col);
-                old[it][OLD - 1] = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(p.d_up) + rr * p.N + col);
-              }
-            }
-          }
+          if (OLD && !EARLY) fetch_old(t, sub, c);
           uint32_t v[32];
           if (!empty_k) {
             tmem_ld_32x32(taddr + c, v);
@@ -617,7 +627,7 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
             if (row0 + r >= p.M) continue;
             if (SCALED) {
 #pragma unroll
-              for (int i = 0; i < 8; ++i) x[i] *= alpha;
+              for (int i = 0; i < 8; ++i) x[i] = __fmul_rn(x[i], alpha);     // rounded before the addition on every tile kind
             }
             const bool low = !ACC || !p.d2 || row0 + r < p.m_split;
             const long long off = expert_off + (low ? row0 + r : row0 + r - p.m_split) * p.ldd + col;
@@ -645,8 +655,8 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                   const float2 prev = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w0[j]));
-                  x[2 * j] += prev.x;
-                  x[2 * j + 1] += prev.y;
+                  x[2 * j] = __fadd_rn(x[2 * j], prev.x);
+                  x[2 * j + 1] = __fadd_rn(x[2 * j + 1], prev.y);
                 }
               }
               if (EPI == EPI_ROPE && col < p.rope_cols) {
@@ -700,16 +710,20 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
 }
 
 // ------------------------------------------------------------------ host side
-template <int A_MN, int B_MN, int EPI, int SCHED, int MT>
+template <int A_MN, int B_MN, int EPI, int SCHED, int MT, int NT = BN>
 static int launch_mt(const GemmParams& p, int sms, cudaStream_t stream) {
-  auto kernel = gemm_tcgen05_kernel<A_MN, B_MN, EPI, SCHED, MT, 0>;
+  auto kernel = gemm_tcgen05_kernel<A_MN, B_MN, EPI, SCHED, MT, 0, NT>;
+  constexpr int smem = smem_bytes<EPI, MT, 0, NT>();
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<EPI, MT>()) != cudaSuccess)
-      return -3;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -3;
     configured = true;
   }
-  kernel<<<sms, gemm_threads<EPI>(), smem_bytes<EPI, MT>(), stream>>>(p);
+  const long long tiles = static_cast<long long>((p.M + MT * BM - 1) / (MT * BM)) * ((p.N + NT - 1) / NT) *
+                          (SCHED == SCHED_WGRAD ? p.num_experts : 1);
+  // a CTA per tile where that is less than one per SM (the return of an expert group counts its CTAs: always all)
+  const int grid = EPI != EPI_PUSH && tiles < sms ? static_cast<int>(tiles < 1 ? 1 : tiles) : sms;
+  kernel<<<grid, gemm_threads<EPI>(), smem, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
@@ -757,7 +771,13 @@ static int launch_pair(const GemmParams& p, int sms, cudaStream_t stream) {
 static int g_tile_mode = 0;   // 0 auto, 1 force 128x256, 2 force 256x256 on one CTA, 3 force CTA pairs where legal, 4 auto
                               // (EPI_PUSH included), 5 auto among the single-CTA kinds
 
-enum TileKind : int { TILE_128 = 0, TILE_256 = 1, TILE_PAIR = 2 };
+enum TileKind : int { TILE_128 = 0, TILE_256 = 1, TILE_PAIR = 2, TILE_N128 = 3, TILE_N64 = 4 };
+
+// Rows of one box of a K-major B operand (SwiGLU: of each of its two weights).
+static int box_rows(TileKind kind, bool swiglu = false) {
+  if (swiglu) return kind == TILE_N64 ? 32 : kind == TILE_N128 ? 64 : 128;
+  return kind == TILE_N64 ? 64 : kind == TILE_N128 || kind == TILE_PAIR ? 128 : 256;
+}
 
 // 256-row tiles (one CTA with two sub-tiles, or a CTA pair) need whole 256-row tiles of one expert: the caller says
 // whether its segments are padded to 256 rows.
@@ -776,6 +796,21 @@ static TileKind choose_tile(const GemmParams& p, int sms, bool pair_available) {
                      (p.tile_expert == nullptr ? p.num_m_tiles == nullptr : p.group_align256 != 0);
   const long long columns = static_cast<long long>((p.N + BN - 1) / BN) * (SCHED == SCHED_WGRAD ? p.num_experts : 1);
   const long long tiles256 = (p.M + 255) / 256 * columns, tiles128 = (p.M + 127) / 128 * columns;
+  if (EPI != EPI_PUSH && (g_tile_mode == 6 || g_tile_mode == 7)) return g_tile_mode == 6 ? TILE_N128 : TILE_N64;
+  if (EPI != EPI_PUSH && (g_tile_mode == 0 || g_tile_mode == 4 || g_tile_mode == 5)) {
+    // Narrow tiles.  A step of 64 along k takes a CTA 0.27 us at 256 columns and 0.16 at 128 or 64 (its loads bound it), so
+    // tiles of 128 columns win where their waves are fewer than 1.6 times those of 256: one wave instead of one, up to three
+    // instead of two.  64 columns take as long as 128 along k and half as long in the epilogue: where they make one wave.
+    // Grouped rows: an expert's padding to 256 rows is half of that on average.  us, 256 -> 128 -> 64 columns: 1024 x 512 K
+    // 512 7.3, 5.6, 5.3; 2048 x 1024 K 1024 10.0, 7.4, 9.6 (two waves); 4096 x 1536 K 1024 16.3, 14.8, 20.7; fp32 gradient
+    // 768 x 512 K 1024 12.4, 8.4, 6.9, 1024 x 1024 K 4096 25.7, 16.3, 14.6; but 4096 x 1024 K 1024 10.4, 11.1, 15.0.
+    const long long rows = p.num_m_tiles ? max(128, p.M - 128 * p.num_experts) : p.M;
+    const long long groups = SCHED == SCHED_WGRAD ? p.num_experts : 1;
+    const auto waves = [&](int width) { return ((rows + 127) / 128 * ((p.N + width - 1) / width) * groups + sms - 1) / sms; };
+    const long long w256 = waves(256), w128 = waves(128);
+    if (waves(64) == 1) return TILE_N64;
+    if (w128 == 1 || (w256 == 2 && w128 == 3)) return TILE_N128;
+  }
   if (!legal || g_tile_mode == 1) return TILE_128;
   if (g_tile_mode == 2) return TILE_256;
   if (pair_available && g_tile_mode == 3) return TILE_PAIR;
@@ -798,6 +833,10 @@ static bool pair_available(int sms) {
 
 template <int A_MN, int B_MN, int EPI, int SCHED>
 static int launch(const GemmParams& p, TileKind kind, int sms, cudaStream_t stream) {
+  if constexpr (EPI != EPI_PUSH) {
+    if (kind == TILE_N128) return launch_mt<A_MN, B_MN, EPI, SCHED, 1, 128>(p, sms, stream);
+    if (kind == TILE_N64) return launch_mt<A_MN, B_MN, EPI, SCHED, 1, 64>(p, sms, stream);
+  }
   if (kind == TILE_PAIR) return launch_pair<A_MN, B_MN, EPI, SCHED>(p, sms, stream);
   if (kind == TILE_256) return launch_mt<A_MN, B_MN, EPI, SCHED, 2>(p, sms, stream);
   return launch_mt<A_MN, B_MN, EPI, SCHED, 1>(p, sms, stream);
@@ -833,7 +872,8 @@ using namespace b2;
 extern "C" {
 
 // 0 automatic, 1 always 128x256 tiles, 2 single-CTA 256x256 tiles wherever they are legal, 3 CTA pairs wherever legal,
-// 4 automatic for the expert-parallel return too, 5 automatic among the single-CTA kinds.
+// 4 automatic for the expert-parallel return too, 5 automatic among the single-CTA kinds, 6 and 7 tiles of 128 and of 64
+// columns.
 void b2_gemm_set_tile_mode(int mode) { g_tile_mode = mode; }
 
 // y[M,N] = a[M,K] * w[e][N,K]^T      (a K-major, w K-major)
@@ -853,8 +893,7 @@ int b2_gemm_nt(const void* a, const void* w, void* d, int M, int N, int K, long 
   const TileKind kind = choose_tile<SCHED_FLAT, EPI_STORE_BF16>(p, sms, pairs);
   if (make_map(&p.map_a, a, K, M, lda, BM)) return -11;
   // a CTA of a pair stages 128 of the tile's 256 weight rows
-  if (make_map(&p.map_b, w, K, static_cast<long long>(num_experts) * N, ldw, kind == TILE_PAIR ? BN / 2 : BN))
-    return -12;
+  if (make_map(&p.map_b, w, K, static_cast<long long>(num_experts) * N, ldw, box_rows(kind))) return -12;
   if (epi == EPI_STORE_BF16) return launch<0, 0, EPI_STORE_BF16, SCHED_FLAT>(p, kind, sms, stream);
   if (make_out_map(&p.map_d, d, N, M, 1, ldd, M * ldd)) return -14;
   return launch<0, 0, EPI_STORE_F32, SCHED_FLAT>(p, kind, sms, stream);
@@ -866,13 +905,15 @@ int b2_gemm_swiglu(const void* a, const void* w1, const void* w3, void* h, void*
                    int* status, cudaStream_t stream) {
   if (F % 128 || K % 8) return -10;
   GemmParams p{};
-  if (make_map(&p.map_a, a, K, M, lda, BM)) return -11;
-  if (make_map(&p.map_b, w1, K, static_cast<long long>(num_experts) * F, K, 128)) return -12;
-  if (make_map(&p.map_b2, w3, K, static_cast<long long>(num_experts) * F, K, 128)) return -12;
   p.M = M; p.N = 2 * F; p.K = K; p.num_experts = num_experts; p.b_expert_rows = F; p.k_split = 0;
   p.tile_expert = tile_expert; p.num_m_tiles = num_m_tiles; p.d = h; p.d_gate = gate; p.d_up = up; p.ldd = F;
   p.status = status; p.group_align256 = group_align256;
-  return launch<0, 0, EPI_SWIGLU, SCHED_FLAT>(p, sm_count(), stream);
+  const int sms = sm_count();
+  const TileKind kind = choose_tile<SCHED_FLAT, EPI_SWIGLU>(p, sms, pair_available<0, 0, EPI_SWIGLU, SCHED_FLAT>(sms));
+  if (make_map(&p.map_a, a, K, M, lda, BM)) return -11;
+  if (make_map(&p.map_b, w1, K, static_cast<long long>(num_experts) * F, K, box_rows(kind, true))) return -12;
+  if (make_map(&p.map_b2, w3, K, static_cast<long long>(num_experts) * F, K, box_rows(kind, true))) return -12;
+  return launch<0, 0, EPI_SWIGLU, SCHED_FLAT>(p, kind, sms, stream);
 }
 
 // dx[M,N] = a[M,K] * w[e][K,N]     (w MN-major: its rows are the reduction index).
@@ -924,7 +965,7 @@ int b2_gemm_nt_rope(const void* a, const void* w, void* d, int M, int N, int K, 
   const int sms = sm_count();
   const TileKind kind = choose_tile<SCHED_FLAT, EPI_ROPE>(p, sms, pair_available<0, 0, EPI_ROPE, SCHED_FLAT>(sms));
   if (make_map(&p.map_a, a, K, M, lda, BM)) return -11;
-  if (make_map(&p.map_b, w, K, N, K, kind == TILE_PAIR ? BN / 2 : BN)) return -12;
+  if (make_map(&p.map_b, w, K, N, K, box_rows(kind))) return -12;
   return launch<0, 0, EPI_ROPE, SCHED_FLAT>(p, kind, sms, stream);
 }
 
@@ -957,7 +998,7 @@ int b2_gemm_nt_push(const void* a, const void* w, int M, int N, int K, long long
   const int sms = sm_count();
   const TileKind kind = choose_tile<SCHED_FLAT, EPI_PUSH>(p, sms, pair_available<0, 0, EPI_PUSH, SCHED_FLAT>(sms));
   if (make_map(&p.map_a, a, K, M, lda, BM)) return -11;
-  if (make_map(&p.map_b, w, K, static_cast<long long>(num_experts) * N, K, kind == TILE_PAIR ? BN / 2 : BN))
+  if (make_map(&p.map_b, w, K, static_cast<long long>(num_experts) * N, K, box_rows(kind)))
     return -12;
   return launch<0, 0, EPI_PUSH, SCHED_FLAT>(p, kind, sms, stream);
 }

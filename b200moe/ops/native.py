@@ -239,10 +239,11 @@ def _bf16(t):
 
 # ------------------------------------------------------------------------------ GEMM
 def set_gemm_tile_mode(mode: int) -> None:
-    """0: automatic (the default): 256x256 tiles on one CTA for reductions of 6144 and more over at least two such tiles
-    per SM, else on CTA pairs (``cta_group::2``) where they fill the machine, else 128x256 tiles; 1: always 128x256 CTA
-    tiles; 2: single-CTA 256x256 tiles wherever legal; 3: CTA pairs wherever legal; 4: like 0, the expert-parallel return
-    included; 5: automatic among the single-CTA kinds.  The environment variable ``B200MOE_GEMM_TILE_MODE`` sets it at
+    """0: automatic (the default): 128x64 or 128x128 tiles for products of one or two waves, 256x256 tiles on one CTA for
+    reductions of 6144 and more over at least two such tiles per SM, else on CTA pairs (``cta_group::2``) where they fill
+    the machine, else 128x256 tiles; 1: always 128x256 CTA tiles; 2: single-CTA 256x256 tiles wherever legal; 3: CTA pairs
+    wherever legal; 4: like 0, the expert-parallel return included; 5: automatic among the single-CTA kinds; 6, 7: 128x128
+    and 128x64 tiles.  The environment variable ``B200MOE_GEMM_TILE_MODE`` sets it at
     load time."""
     require().b2_gemm_set_tile_mode(_I(mode))
 

@@ -62,6 +62,71 @@ def test_gemm_tn_accumulates(native, tile_mode, R, M, N, dtype):
     native.check_status()
 
 
+@pytest.mark.parametrize("mode", [6, 7], ids=["128x128", "128x64"])
+@pytest.mark.parametrize("M,N,K", [(1, 32, 64), (129, 96, 128), (200, 320, 576), (300, 2080, 64), (2100, 1312, 192)])
+def test_narrow_tiles_give_the_bits_of_wide_ones(native, mode, M, N, K):
+    """Every product on tiles of 128 and 64 columns (rows and columns behind the last tile; one tile, several waves): each
+    element is the same chain of additions as on 128x256 tiles."""
+    x, w, wt = _rand(M, K), _rand(N, K, scale=0.1), _rand(K, N, scale=0.1)
+    F = 128 * (N // 128 + 1)
+    w1, w3 = _rand(1, F, K, scale=0.1), _rand(1, F, K, scale=0.1)
+    gate, up, left, right = _rand(M, N), _rand(M, N), _rand(K, 8 * (M // 8 + 1)), _rand(K, N)
+    base = torch.randn(left.shape[1], N, device="cuda")
+    cos, sin = torch.rand(M, 64, device="cuda"), torch.rand(M, 64, device="cuda")
+    half = torch.full((), 0.375, device="cuda")
+
+    def products():
+        sums = [base.clone(), base.bfloat16()]
+        for out in sums:
+            native.gemm_tn(left, right, out=out, accumulate=True, alpha=half)
+        return [native.gemm_nt(x, w), native.gemm_nt(x, w, out_dtype=torch.float32),
+                native.gemm_nt_rope(x, w, cos, sin, N // 128 * 128, M), native.gemm_nn(x, wt, alpha=half),
+                native.gemm_nn(torch.cat((x, x), 1), wt, w2=wt), *native.gemm_swiglu(x, w1, w3),
+                *(native.gemm_nn_swiglu_bwd(x, wt, gate, up) if M * N <= 1 << 21 else ()), *sums,
+                native.gemm_tn(left, right, out_dtype=torch.bfloat16)]
+
+    try:
+        native.set_gemm_tile_mode(1)
+        want = products()
+        native.set_gemm_tile_mode(mode)
+        got = products()
+    finally:
+        native.set_gemm_tile_mode(0)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    assert _rel(got[0], x.float() @ w.float().t()) < 6e-3
+    native.check_status()
+
+
+@pytest.mark.parametrize("mode", [6, 7], ids=["128x128", "128x64"])
+@pytest.mark.parametrize("counts", [[100, 0, 300, 17], [256, 1, 64, 65]])
+def test_grouped_products_on_narrow_tiles(native, mode, counts):
+    offs, tile_expert, meta, rows = _segments(counts, 256)
+    E, D, F = len(counts), 192, 384
+    x, dy = torch.zeros(rows, D, device="cuda").bfloat16(), torch.zeros(rows, F, device="cuda").bfloat16()
+    for e, n in enumerate(counts):
+        lo = 0 if e == 0 else int(offs[e - 1])
+        x[lo:lo + n], dy[lo:lo + n] = _rand(n, D), _rand(n, F)
+    w1, w3, w2 = _rand(E, F, D, scale=0.1), _rand(E, F, D, scale=0.1), _rand(E, D, F, scale=0.1)
+    count, base = torch.tensor(counts, device="cuda", dtype=torch.int32), torch.randn(E, F, D, device="cuda")
+
+    def products():
+        h, gate, up = native.gemm_swiglu(x, w1, w3, tile_expert, meta[:1], align256=True)
+        out = native.gemm_nt(h, w2, tile_expert=tile_expert, num_m_tiles=meta[:1], num_experts=E, align256=True)
+        dx = native.gemm_nn(dy, w1, tile_expert=tile_expert, num_m_tiles=meta[:1], num_experts=E, align256=True)
+        dw = native.gemm_tn(dy, x, out=base.clone(), accumulate=True, expert_offsets=offs, num_experts=E, counts=count)
+        return h, gate, up, out, dx, dw
+
+    try:
+        native.set_gemm_tile_mode(1)
+        want = products()
+        native.set_gemm_tile_mode(mode)
+        got = products()
+    finally:
+        native.set_gemm_tile_mode(0)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    native.check_status()
+
+
 @pytest.mark.parametrize("R,F,N", [(64, 4, 32), (100, 36, 96), (129, 264, 288)])
 @pytest.mark.parametrize("accumulate", [True, False])
 def test_fp32_results_cut_between_two_weights(native, tile_mode, R, F, N, accumulate):
