@@ -64,13 +64,191 @@ __device__ __forceinline__ float block_max(float v, float* scratch) {
 }
 
 // ------------------------------------------------------------------ RMSNorm
-constexpr int NORM_THREADS = 256;
-constexpr int NORM_MAX_CHUNKS = 4;  // D <= 256 * 8 * 4 = 8192
+// Both directions are bound by memory traffic.  Eight warps work on the rows, W of them on one row (so that narrow rows keep
+// every lane busy: 512 columns are one warp's), a ninth brings blocks of 8 / W consecutive rows into a ring in shared memory
+// by bulk copies: the next blocks arrive while the present one is reduced, whatever the registers hold.  us, one CTA per row
+// with loads through registers -> now: backward with residual and column sum 1024 x 512 11.9 -> 6.2, 4096 x 1024 22 -> 14,
+// 16384 x 4096 164 -> 109 (4.9 TB/s); forward 16384 x 4096 72 -> 53, with the sum 123 -> 98.
+constexpr int NORM_THREADS = 256;      // the warps that work on the rows
+constexpr int NORM_VECS = 2;           // 16-byte vectors of a row per thread, 4 beyond 4096 columns
+constexpr int NORM_MAX_D = 8192;
+constexpr int NORM_RING = 4;
 
-// y = (x [+ delta]) * rstd * w ; optionally writes the sum.  One CTA per row (grid-stride); CH = 8-element
-// vectors per thread (compile time, so the row stays in registers as packed bf16).
+struct NormBars {
+  uint64_t full[NORM_RING], empty[NORM_RING];
+};
+
+// The producer warp: blocks ``blockIdx.x``, ``+ gridDim.x``, ... of up to R rows of each tensor (null ones are left out).
+template <int R, int TENSORS>
+__device__ __forceinline__ void norm_producer(const __nv_bfloat16* const (&src)[TENSORS], uint8_t* ring, int ring_stages,
+                                              NormBars& bars, int* status, int rows, int D) {
+  if ((threadIdx.x & 31) != 0) return;
+  const int blocks = (rows + R - 1) / R;
+  const uint32_t row_bytes = D * 2, slot = R * row_bytes;
+  int count = 0;
+  for (int block = blockIdx.x; block < blocks; block += gridDim.x, ++count) {
+    const int s = count % ring_stages;
+    if (!mbar_wait(&bars.empty[s], ((count / ring_stages) & 1) ^ 1)) {
+      atomicExch(status, 6);
+      break;
+    }
+    const uint32_t bytes = min(R, rows - block * R) * row_bytes;
+    uint32_t tensors = 0;
+#pragma unroll
+    for (int i = 0; i < TENSORS; ++i) tensors += src[i] != nullptr;
+    mbar_expect_tx(&bars.full[s], tensors * bytes);
+#pragma unroll
+    for (int i = 0; i < TENSORS; ++i)
+      if (src[i])
+        bulk_load(ring + (static_cast<size_t>(s) * TENSORS + i) * slot, src[i] + static_cast<size_t>(block) * R * D, &bars.full[s], bytes);
+  }
+  // copies of a CTA whose other warps gave up land before it exits
+  for (int i = max(0, count - ring_stages); i < count; ++i) mbar_wait(&bars.full[i % ring_stages], (i / ring_stages) & 1);
+}
+
+__device__ __forceinline__ void norm_init(NormBars& bars) {
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < NORM_RING; ++s) {
+      mbar_init(&bars.full[s], 1);
+      mbar_init(&bars.empty[s], NORM_THREADS / 32);
+    }
+    mbar_fence_init();
+  }
+  __syncthreads();
+}
+
+// Waits for a block.  A warp whose wait ran out reports and goes on without waiting: the warps of a row meet at barriers.
+__device__ __forceinline__ bool norm_arrived(bool so_far, uint64_t& bar, uint32_t parity, int* status) {
+  if (!so_far) return false;
+  if (mbar_wait(&bar, parity)) return true;
+  if ((threadIdx.x & 31) == 0) atomicExch(status, 6);
+  return false;
+}
+
+// Sum over one row, whose W warps hold V x 256 columns each: the sums of 256 (W = 8: of the V parts of a thread together)
+// columns are formed by shuffles and added in the order of the columns.  ``scratch`` alternates between two halves, so that
+// one barrier per row is enough.
+template <int W, int V>
+__device__ __forceinline__ float norm_row_sum(float (&part)[V], float (*scratch)[8], int slot, int warp_in_row, int lane) {
+  if (W == 8) {
+    float v = part[0];
+    v = warp_sum(v);
+    if (lane == 0) scratch[0][warp_in_row] = v;
+  } else {
+#pragma unroll
+    for (int c = 0; c < V; ++c) part[c] = warp_sum(part[c]);
+    if (W == 1) {
+      float total = 0.f;
+#pragma unroll
+      for (int c = 0; c < V; ++c) total += part[c];
+      return total;
+    }
+    if (lane == 0) {
+#pragma unroll
+      for (int c = 0; c < V; ++c) scratch[slot][c * W + warp_in_row] = part[c];
+    }
+  }
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + slot), "r"(W * 32) : "memory");
+  float total = 0.f;
+#pragma unroll
+  for (int i = 0; i < (W == 8 ? 8 : W * V); ++i) total += scratch[slot][i];
+  return total;
+}
+
+// y = (x [+ delta]) * rstd * w ; optionally writes the sum.
+template <int W, int V>
+__global__ void __launch_bounds__(NORM_THREADS + 32) rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x,
+                                                                       const __nv_bfloat16* __restrict__ delta,
+                                                                       const float* __restrict__ w,
+                                                                       __nv_bfloat16* __restrict__ sum_out,
+                                                                       __nv_bfloat16* __restrict__ y,
+                                                                       float* __restrict__ rstd, int* __restrict__ status,
+                                                                       int rows, int D, float eps, int ring_stages) {
+  constexpr int R = 8 / W;
+  extern __shared__ __align__(128) uint8_t norm_ring[];
+  __shared__ NormBars bars;
+  __shared__ float scratch[2][R][8];
+  norm_init(bars);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp == NORM_THREADS / 32) {
+    const __nv_bfloat16* const src[2] = {x, delta};
+    norm_producer<R, 2>(src, norm_ring, ring_stages, bars, status, rows, D);
+    return;
+  }
+  const int slot = warp / W, in_row = warp % W;
+  float wv[V][8];
+#pragma unroll
+  for (int c = 0; c < V; ++c) {
+    const int col = ((c * W + in_row) * 32 + lane) * 8;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) wv[c][i] = col < D ? w[col + i] : 0.f;
+  }
+  const int blocks = (rows + R - 1) / R;
+  int count = 0;
+  bool here = true;
+  for (int block = blockIdx.x; block < blocks; block += gridDim.x, ++count) {
+    const int s = count % ring_stages;
+    const int row = block * R + slot;
+    const bool live = row < rows;
+    const size_t base = static_cast<size_t>(row) * D;
+    const __nv_bfloat16* in = reinterpret_cast<const __nv_bfloat16*>(norm_ring) + (static_cast<size_t>(s) * 2 * R + slot) * D;
+    here = norm_arrived(here, bars.full[s], (count / ring_stages) & 1, status);
+    bf16x8 raw[V], add[V];
+#pragma unroll
+    for (int c = 0; c < V; ++c) {
+      const int col = ((c * W + in_row) * 32 + lane) * 8;
+      if (live && col < D) {
+        raw[c] = *reinterpret_cast<const bf16x8*>(in + col);
+        if (delta) add[c] = *reinterpret_cast<const bf16x8*>(in + static_cast<size_t>(R) * D + col);
+      }
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&bars.empty[s]);
+    float part[V];
+#pragma unroll
+    for (int c = 0; c < V; ++c) part[c] = 0.f;
+#pragma unroll
+    for (int c = 0; c < V; ++c) {
+      const int col = ((c * W + in_row) * 32 + lane) * 8;
+      if (live && col < D) {
+        float v[8];
+        unpack8(raw[c], v);
+        if (delta) {
+          float d[8];
+          unpack8(add[c], d);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) v[i] += d[i];
+          // the sum is rounded to bf16 once; the norm sees the rounded value, like the unfused path
+          raw[c] = pack8(v);
+          *reinterpret_cast<bf16x8*>(sum_out + base + col) = raw[c];
+          unpack8(raw[c], v);
+        }
+        float& ss = part[W == 8 ? 0 : c];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) ss += v[i] * v[i];
+      }
+    }
+    const float total = norm_row_sum<W, V>(part, scratch[count & 1], slot, in_row, lane);
+    const float r = rsqrtf(total / D + eps);
+    if (live && in_row == 0 && lane == 0) rstd[row] = r;
+#pragma unroll
+    for (int c = 0; c < V; ++c) {
+      const int col = ((c * W + in_row) * 32 + lane) * 8;
+      if (live && col < D) {
+        float v[8], o[8];
+        unpack8(raw[c], v);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) o[i] = v[i] * r * wv[c][i];
+        *reinterpret_cast<bf16x8*>(y + base + col) = pack8(o);
+      }
+    }
+  }
+}
+
+// The same for few rows, one CTA per row (grid-stride), straight from global memory: a ring has nothing to read ahead where
+// a CTA has one block of rows (200 x 512: 1.8 us here, 2.6 there).  CH = 8-element vectors per thread.  Same sums, same bits.
 template <int CH>
-__global__ void __launch_bounds__(NORM_THREADS) rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x,
+__global__ void __launch_bounds__(NORM_THREADS) rmsnorm_fwd_row_kernel(const __nv_bfloat16* __restrict__ x,
                                                                   const __nv_bfloat16* __restrict__ delta,
                                                                   const float* __restrict__ w,
                                                                   __nv_bfloat16* __restrict__ sum_out,
@@ -127,143 +305,152 @@ __global__ void __launch_bounds__(NORM_THREADS) rmsnorm_fwd_kernel(const __nv_bf
 }
 
 // dx = rstd * (dy*w - xhat * mean(dy*w*xhat)) [+ residual]; dw partial per CTA.
-// One CTA per row (grid-stride).  The loads of the CTA's next row are issued before the current row is reduced and
-// stored, so each thread keeps two rows' worth of 16-byte loads in flight across the block-wide reduction.
-template <int CH>
-struct NormRow {
-  bf16x8 dy[CH], x[CH];
-  float r;
-};
-
-template <int CH>
-__device__ __forceinline__ void norm_row_load(NormRow<CH>& row, const __nv_bfloat16* __restrict__ dy,
-                                              const __nv_bfloat16* __restrict__ x, const float* __restrict__ rstd,
-                                              int index, int D) {
-  const size_t base = static_cast<size_t>(index) * D;
+template <int W, int V>
+__global__ void __launch_bounds__(NORM_THREADS + 32, V == 2 ? 2 : 1)
+    rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+                       const float* __restrict__ w, const float* __restrict__ rstd,
+                       const __nv_bfloat16* __restrict__ residual, __nv_bfloat16* __restrict__ dx,
+                       float* __restrict__ dw_partial, int* __restrict__ status, int rows, int D, int ring_stages) {
+  constexpr int R = 8 / W;
+  extern __shared__ __align__(128) uint8_t norm_ring[];
+  __shared__ NormBars bars;
+  __shared__ float scratch[2][R][8];
+  norm_init(bars);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool worker = warp < NORM_THREADS / 32;
+  const int slot = warp / W, in_row = warp % W;
+  float dw_acc[V][8];
+  if (!worker) {
+    const __nv_bfloat16* const src[3] = {dy, x, residual};
+    norm_producer<R, 3>(src, norm_ring, ring_stages, bars, status, rows, D);
+    __syncwarp();
+  } else {
+    float wv[V][8];
 #pragma unroll
-  for (int c = 0; c < CH; ++c) {
-    const int col = (c * NORM_THREADS + threadIdx.x) * 8;
-    if (col < D) {
-      row.dy[c] = *reinterpret_cast<const bf16x8*>(dy + base + col);
-      row.x[c] = *reinterpret_cast<const bf16x8*>(x + base + col);
-    }
-  }
-  row.r = rstd[index];
-}
-
-template <int CH>
-__device__ __forceinline__ void norm_row_finish(const NormRow<CH>& row, float (&dw_acc)[CH][8],
-                                                const float (&wv)[CH][8],
-                                                const __nv_bfloat16* __restrict__ residual,
-                                                __nv_bfloat16* __restrict__ dx, int index, int D, float* scratch) {
-  const size_t base = static_cast<size_t>(index) * D;
-  const float r = row.r;
-  float dot = 0.f;
-#pragma unroll
-  for (int c = 0; c < CH; ++c) {
-    const int col = (c * NORM_THREADS + threadIdx.x) * 8;
-    if (col < D) {
-      float dyv[8], xv[8];
-      unpack8(row.dy[c], dyv);
-      unpack8(row.x[c], xv);
+    for (int c = 0; c < V; ++c) {
+      const int col = ((c * W + in_row) * 32 + lane) * 8;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const float xh = xv[i] * r;
-        dw_acc[c][i] += dyv[i] * xh;
-        dot += dyv[i] * wv[c][i] * xh;
+        dw_acc[c][i] = 0.f;
+        wv[c][i] = col < D ? w[col + i] : 0.f;
+      }
+    }
+    const int blocks = (rows + R - 1) / R;
+    int count = 0;
+    bool here = true;
+    float next_r = static_cast<int>(blockIdx.x) * R + slot < rows ? rstd[blockIdx.x * R + slot] : 0.f;
+    for (int block = blockIdx.x; block < blocks; block += gridDim.x, ++count) {
+      const int s = count % ring_stages;
+      const int row = block * R + slot, after = row + static_cast<int>(gridDim.x) * R;
+      const bool live = row < rows;
+      const float r = next_r;
+      if (after < rows) next_r = rstd[after];
+      const __nv_bfloat16* in = reinterpret_cast<const __nv_bfloat16*>(norm_ring) + (static_cast<size_t>(s) * 3 * R + slot) * D;
+      here = norm_arrived(here, bars.full[s], (count / ring_stages) & 1, status);
+      bf16x8 a[V], b[V], res[V];
+#pragma unroll
+      for (int c = 0; c < V; ++c) {
+        const int col = ((c * W + in_row) * 32 + lane) * 8;
+        if (live && col < D) {
+          a[c] = *reinterpret_cast<const bf16x8*>(in + col);
+          b[c] = *reinterpret_cast<const bf16x8*>(in + static_cast<size_t>(R) * D + col);
+          if (residual) res[c] = *reinterpret_cast<const bf16x8*>(in + static_cast<size_t>(2 * R) * D + col);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars.empty[s]);
+      float part[V];
+#pragma unroll
+      for (int c = 0; c < V; ++c) part[c] = 0.f;
+#pragma unroll
+      for (int c = 0; c < V; ++c) {
+        const int col = ((c * W + in_row) * 32 + lane) * 8;
+        if (live && col < D) {
+          float dyv[8], xv[8];
+          unpack8(a[c], dyv);
+          unpack8(b[c], xv);
+          float& dot = part[W == 8 ? 0 : c];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float xh = xv[i] * r;
+            dw_acc[c][i] += dyv[i] * xh;
+            dot += dyv[i] * wv[c][i] * xh;
+          }
+        }
+      }
+      const float mean = norm_row_sum<W, V>(part, scratch[count & 1], slot, in_row, lane) / D;
+#pragma unroll
+      for (int c = 0; c < V; ++c) {
+        const int col = ((c * W + in_row) * 32 + lane) * 8;
+        if (live && col < D) {
+          float dyv[8], xv[8], o[8];
+          unpack8(a[c], dyv);
+          unpack8(b[c], xv);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) o[i] = r * (dyv[i] * wv[c][i] - xv[i] * r * mean);
+          if (residual) {
+            float add[8];
+            unpack8(res[c], add);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] += add[i];
+          }
+          *reinterpret_cast<bf16x8*>(dx + static_cast<size_t>(row) * D + col) = pack8(o);
+        }
       }
     }
   }
-  const float mean = block_sum<NORM_THREADS>(dot, scratch) / D;
+  // the rows that the CTA worked on at the same time are added up in the ring, whose copies have all been taken
+  float* const sums = reinterpret_cast<float*>(norm_ring);
+  __syncthreads();
+  if (W < 8) {
+    if (worker) {
 #pragma unroll
-  for (int c = 0; c < CH; ++c) {
-    const int col = (c * NORM_THREADS + threadIdx.x) * 8;
-    if (col < D) {
-      float dyv[8], xv[8], o[8];
-      unpack8(row.dy[c], dyv);
-      unpack8(row.x[c], xv);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) o[i] = r * (dyv[i] * wv[c][i] - xv[i] * r * mean);
-      if (residual) {
-        float res[8];
-        unpack8(*reinterpret_cast<const bf16x8*>(residual + base + col), res);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] += res[i];
+      for (int c = 0; c < V; ++c) {
+        const int col = ((c * W + in_row) * 32 + lane) * 8;
+        if (col < D) {
+          float4* const dst = reinterpret_cast<float4*>(sums + static_cast<size_t>(slot) * D + col);
+          dst[0] = make_float4(dw_acc[c][0], dw_acc[c][1], dw_acc[c][2], dw_acc[c][3]);
+          dst[1] = make_float4(dw_acc[c][4], dw_acc[c][5], dw_acc[c][6], dw_acc[c][7]);
+        }
       }
-      *reinterpret_cast<bf16x8*>(dx + base + col) = pack8(o);
+    }
+    __syncthreads();
+    for (int col = threadIdx.x; col < D; col += NORM_THREADS + 32) {
+      float total = 0.f;
+#pragma unroll
+      for (int k = 0; k < R; ++k) total += sums[static_cast<size_t>(k) * D + col];
+      dw_partial[static_cast<size_t>(blockIdx.x) * D + col] = total;
+    }
+  } else if (worker) {
+#pragma unroll
+    for (int c = 0; c < V; ++c) {
+      const int col = ((c * W + in_row) * 32 + lane) * 8;
+      if (col < D) {
+        float4* const dst = reinterpret_cast<float4*>(dw_partial + static_cast<size_t>(blockIdx.x) * D + col);
+        dst[0] = make_float4(dw_acc[c][0], dw_acc[c][1], dw_acc[c][2], dw_acc[c][3]);
+        dst[1] = make_float4(dw_acc[c][4], dw_acc[c][5], dw_acc[c][6], dw_acc[c][7]);
+      }
     }
   }
 }
 
-template <int CH>
-__global__ void __launch_bounds__(NORM_THREADS) rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy,
-                                                                  const __nv_bfloat16* __restrict__ x,
-                                                                  const float* __restrict__ w,
-                                                                  const float* __restrict__ rstd,
-                                                                  const __nv_bfloat16* __restrict__ residual,
-                                                                  __nv_bfloat16* __restrict__ dx,
-                                                                  float* __restrict__ dw_partial, int rows, int D) {
-  __shared__ float scratch[NORM_THREADS / 32];
-  float dw_acc[CH][8];
-  float wv[CH][8];
-#pragma unroll
-  for (int c = 0; c < CH; ++c) {
-    const int col = (c * NORM_THREADS + threadIdx.x) * 8;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      dw_acc[c][i] = 0.f;
-      wv[c][i] = col < D ? w[col + i] : 0.f;
-    }
-  }
-  NormRow<CH> a, b;
-  int row = blockIdx.x;
-  if (row < rows) norm_row_load(a, dy, x, rstd, row, D);
-  while (row < rows) {
-    const int next = row + gridDim.x;
-    if (next < rows) norm_row_load(b, dy, x, rstd, next, D);
-    norm_row_finish(a, dw_acc, wv, residual, dx, row, D, scratch);
-    if (next >= rows) break;
-    const int after = next + gridDim.x;
-    if (after < rows) norm_row_load(a, dy, x, rstd, after, D);
-    norm_row_finish(b, dw_acc, wv, residual, dx, next, D, scratch);
-    row = after;
-  }
-#pragma unroll
-  for (int c = 0; c < CH; ++c) {
-    const int col = (c * NORM_THREADS + threadIdx.x) * 8;
-    if (col < D) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) dw_partial[static_cast<size_t>(blockIdx.x) * D + col + i] = dw_acc[c][i];
-    }
-  }
-}
-
-// out[col] = sum over parts of partial[part][col].  One CTA per 32 columns: lane = column (coalesced 128-byte
-// reads), the eight warps take every eighth part, shared memory adds the eight partial sums.
-__global__ void __launch_bounds__(256) column_sum_kernel(const float* __restrict__ partial, float* __restrict__ out,
-                                                        int parts, int D) {
-  __shared__ float acc[8][33];
+// out[col] = sum over parts of partial[part][col].  One CTA per 32 columns: lane = column (coalesced 128-byte reads), the
+// 32 warps take every 32nd part (eight warps in four chains each were 7.6 us at 296 parts of 512 columns, this 2.5),
+// shared memory adds the 32 partial sums.
+__global__ void __launch_bounds__(1024) column_sum_kernel(const float* __restrict__ partial, float* __restrict__ out,
+                                                         int parts, int D) {
+  __shared__ float acc[32][33];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col = blockIdx.x * 32 + lane;
-  float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+  float s = 0.f;
   if (col < D) {
-    int p = warp;
-    for (; p + 24 < parts; p += 32) {
-      s0 += partial[static_cast<size_t>(p) * D + col];
-      s1 += partial[static_cast<size_t>(p + 8) * D + col];
-      s2 += partial[static_cast<size_t>(p + 16) * D + col];
-      s3 += partial[static_cast<size_t>(p + 24) * D + col];
-    }
-    for (; p < parts; p += 8) s0 += partial[static_cast<size_t>(p) * D + col];
+#pragma unroll 10
+    for (int p = warp; p < parts; p += 32) s += partial[static_cast<size_t>(p) * D + col];
   }
-  acc[warp][lane] = (s0 + s1) + (s2 + s3);
+  acc[warp][lane] = s;
   __syncthreads();
-  if (warp == 0 && col < D) {
-    float s = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) s += acc[i][lane];
-    out[col] = s;
-  }
+  s = warp_sum(acc[lane][warp]);             // transposed: warp = column, lane = part
+  if (lane == 0 && blockIdx.x * 32 + warp < D) out[blockIdx.x * 32 + warp] = s;
 }
 
 // ------------------------------------------------------------------ router softmax / top-2
@@ -1030,6 +1217,33 @@ static inline int grid_for(size_t work, int threads, int per_sm = 16) {
 }
 static inline int ok() { return cudaGetLastError() == cudaSuccess ? 0 : -1; }
 
+constexpr int NORM_FWD_CTAS = 3;
+constexpr int NORM_SMEM = 110 * 1024;        // two CTAs per SM
+template <int N> struct Int { static constexpr int value = N; };
+static inline int norm_rows_at_once(int D) { return D <= 512 ? 8 : D <= 1024 ? 4 : D <= 2048 ? 2 : 1; }
+// ``launch(W, V, shared memory, ring stages)`` for rows of D columns and ``tensors`` tensors in the ring.
+template <typename F>
+static int launch_norm(int D, int tensors, F launch) {
+  const int slot = norm_rows_at_once(D) * D * 2 * tensors;
+  const int stages = min(NORM_RING, NORM_SMEM / slot);
+  // (backward: the sums of the rows at once, four bytes a column, fit into two stages)
+  const int smem = max(stages, 1) * slot;
+  if (D <= 512) return launch(Int<1>{}, Int<NORM_VECS>{}, smem, stages);
+  if (D <= 1024) return launch(Int<2>{}, Int<NORM_VECS>{}, smem, stages);
+  if (D <= 2048) return launch(Int<4>{}, Int<NORM_VECS>{}, smem, stages);
+  if (D <= 4096) return launch(Int<8>{}, Int<NORM_VECS>{}, smem, stages);
+  return launch(Int<8>{}, Int<4>{}, smem, stages);
+}
+template <int W, int V, int KIND, typename K>
+static int norm_smem(K kernel) {
+  static bool set = false;
+  if (!set) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, NORM_SMEM) != cudaSuccess) return -3;
+    set = true;
+  }
+  return 0;
+}
+
 }  // namespace b2
 
 using namespace b2;
@@ -1037,35 +1251,47 @@ typedef __nv_bfloat16 bf16;
 
 extern "C" {
 
+// bf16 tensors: 16-byte aligned, rows of D elements one after the other.  status: device word, set if a copy did not arrive.
 int b2_rmsnorm_fwd(const void* x, const void* delta, const float* w, void* sum_out, void* y, float* rstd, int rows,
-                   int D, float eps, cudaStream_t s) {
-  if (D % 8 || D > NORM_THREADS * 8 * NORM_MAX_CHUNKS) return -10;
-  const int grid = min(rows, sm_count_ew() * 8);
-#define B2_NORM_FWD(CH)                                                                                         \
-  rmsnorm_fwd_kernel<CH><<<grid, NORM_THREADS, 0, s>>>((const bf16*)x, (const bf16*)delta, w, (bf16*)sum_out, \
-                                                       (bf16*)y, rstd, rows, D, eps)
-  if (D <= 2048) B2_NORM_FWD(1);
-  else if (D <= 4096) B2_NORM_FWD(2);
-  else B2_NORM_FWD(4);
-#undef B2_NORM_FWD
-  return ok();
+                   int D, float eps, int* status, cudaStream_t s) {
+  if (D % 8 || D > NORM_MAX_D) return -10;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(delta)) % 16) return -12;
+  const int at_once = norm_rows_at_once(D);
+  if ((rows + at_once - 1) / at_once <= sm_count_ew() * NORM_FWD_CTAS) {
+    auto kernel = D <= 2048 ? rmsnorm_fwd_row_kernel<1> : D <= 4096 ? rmsnorm_fwd_row_kernel<2> : rmsnorm_fwd_row_kernel<4>;
+    kernel<<<min(rows, sm_count_ew() * 8), NORM_THREADS, 0, s>>>((const bf16*)x, (const bf16*)delta, w, (bf16*)sum_out, (bf16*)y,
+                                                                 rstd, rows, D, eps);
+    return ok();
+  }
+  return launch_norm(D, 2, [&](auto W, auto V, int smem, int stages) {
+    auto kernel = rmsnorm_fwd_kernel<decltype(W)::value, decltype(V)::value>;
+    if (const int rc = norm_smem<decltype(W)::value, decltype(V)::value, 0>(kernel)) return rc;
+    kernel<<<sm_count_ew() * NORM_FWD_CTAS, NORM_THREADS + 32, smem, s>>>((const bf16*)x, (const bf16*)delta, w, (bf16*)sum_out, (bf16*)y, rstd, status,
+                                                 rows, D, eps, stages);
+    return ok();
+  });
 }
 
-// dw_partial: fp32 [parts, D] scratch with parts = b2_rmsnorm_bwd_parts(rows); dw: fp32 [D] (overwritten).
+// dw_partial: fp32 [parts, D] scratch with parts = b2_rmsnorm_bwd_parts(rows, D); dw: fp32 [D] (overwritten).
 // two CTAs are resident per SM (registers): one wave, and as few partial rows as possible for the column sum
-int b2_rmsnorm_bwd_parts(int rows) { return min(rows, sm_count_ew() * 2); }
+int b2_rmsnorm_bwd_parts(int rows, int D) {
+  const int R = norm_rows_at_once(D);
+  return min((rows + R - 1) / R, sm_count_ew() * 2);
+}
 int b2_rmsnorm_bwd(const void* dy, const void* x, const float* w, const float* rstd, const void* residual, void* dx,
-                   float* dw_partial, float* dw, int rows, int D, cudaStream_t s) {
-  if (D % 8 || D > NORM_THREADS * 8 * NORM_MAX_CHUNKS) return -10;
-  const int parts = b2_rmsnorm_bwd_parts(rows);
-#define B2_NORM_BWD(CH)                                                                                       \
-  rmsnorm_bwd_kernel<CH><<<parts, NORM_THREADS, 0, s>>>((const bf16*)dy, (const bf16*)x, w, rstd,             \
-                                                        (const bf16*)residual, (bf16*)dx, dw_partial, rows, D)
-  if (D <= 2048) B2_NORM_BWD(1);
-  else if (D <= 4096) B2_NORM_BWD(2);
-  else B2_NORM_BWD(4);
-#undef B2_NORM_BWD
-  column_sum_kernel<<<(D + 31) / 32, 256, 0, s>>>(dw_partial, dw, parts, D);
+                   float* dw_partial, float* dw, int rows, int D, int* status, cudaStream_t s) {
+  if (D % 8 || D > NORM_MAX_D) return -10;
+  if ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(residual)) % 16) return -12;
+  const int parts = b2_rmsnorm_bwd_parts(rows, D);
+  const int rc = launch_norm(D, 3, [&](auto W, auto V, int smem, int stages) {
+    auto kernel = rmsnorm_bwd_kernel<decltype(W)::value, decltype(V)::value>;
+    if (const int rc = norm_smem<decltype(W)::value, decltype(V)::value, 1>(kernel)) return rc;
+    kernel<<<parts, NORM_THREADS + 32, smem, s>>>((const bf16*)dy, (const bf16*)x, w, rstd, (const bf16*)residual, (bf16*)dx,
+                                                  dw_partial, status, rows, D, stages);
+    return ok();
+  });
+  if (rc) return rc;
+  column_sum_kernel<<<(D + 31) / 32, 1024, 0, s>>>(dw_partial, dw, parts, D);
   return ok();
 }
 

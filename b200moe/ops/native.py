@@ -393,7 +393,7 @@ def rmsnorm_fwd(x, weight, eps):
     y = torch.empty_like(x2)
     rstd = torch.empty(x2.shape[0], dtype=torch.float32, device=x.device)
     _call("b2_rmsnorm_fwd", _p(x2), _p(None), _p(weight), _p(None), _p(y), _p(rstd), _I(x2.shape[0]), _I(x2.shape[1]),
-          _F(eps), _stream())
+          _F(eps), _p(status_word(x.device)), _stream())
     return y.view(x.shape), rstd
 
 
@@ -402,7 +402,7 @@ def add_rmsnorm_fwd(x, delta, weight, eps):
     summed, y = torch.empty_like(x2), torch.empty_like(x2)
     rstd = torch.empty(x2.shape[0], dtype=torch.float32, device=x.device)
     _call("b2_rmsnorm_fwd", _p(x2), _p(d2), _p(weight), _p(summed), _p(y), _p(rstd), _I(x2.shape[0]), _I(x2.shape[1]),
-          _F(eps), _stream())
+          _F(eps), _p(status_word(x.device)), _stream())
     return summed.view(x.shape), y.view(x.shape), rstd
 
 
@@ -410,13 +410,13 @@ def rmsnorm_bwd(dy, x, weight, rstd, residual_grad=None):
     x2 = x.reshape(-1, x.shape[-1])
     dy2 = _bf16(dy).reshape(-1, x.shape[-1])
     rows, D = x2.shape
-    parts = require().b2_rmsnorm_bwd_parts(_I(rows))
+    parts = require().b2_rmsnorm_bwd_parts(_I(rows), _I(D))
     partial = torch.empty(parts, D, dtype=torch.float32, device=x.device)
     dx = torch.empty_like(x2)
     dw = torch.empty(D, dtype=torch.float32, device=x.device)
     res = None if residual_grad is None else _bf16(residual_grad).reshape(-1, D).contiguous()
     _call("b2_rmsnorm_bwd", _p(dy2), _p(x2), _p(weight), _p(rstd), _p(res), _p(dx), _p(partial), _p(dw), _I(rows), _I(D),
-          _stream(), n=2)
+          _p(status_word(x.device)), _stream(), n=2)
     return dx.view(x.shape), dw
 
 

@@ -315,6 +315,30 @@ def test_rmsnorm_forward_backward(native):
         assert _rel(w.grad, wr2.grad) < 8e-3
 
 
+@pytest.mark.parametrize("rows,D", [(1, 8), (3563, 512), (1800, 520), (1777, 1024), (893, 2048), (451, 2056), (450, 8192)])
+def test_rmsnorm_row_blocks(native, rows, D):
+    """Blocks of eight to one rows through the ring, the last one cut short; the one-CTA-per-row form of few rows."""
+    x, delta, dy, res = (_rand(rows, D) for _ in range(4))
+    w = torch.rand(D, device="cuda") + 0.5
+    summed, y, rstd = native.add_rmsnorm_fwd(x, delta, w, 1e-5)
+    few = native.add_rmsnorm_fwd(x[-3:], delta[-3:], w, 1e-5)
+    assert all(torch.equal(a[-3:], b) for a, b in zip((summed, y, rstd), few))
+    assert torch.equal(summed, (x.float() + delta.float()).bfloat16())
+    s64, w64, dy64 = summed.double(), w.double(), dy.double()
+    r64 = (s64.square().mean(1) + 1e-5).rsqrt()
+    # rstd: D additions and a few operations in fp32; y: one more rounding to bf16
+    assert bool(((rstd.double() / r64 - 1).abs() <= (D + 8) * 2.0 ** -24).all())
+    assert bool(((y.double() - s64 * r64[:, None] * w64).abs() <= 2.0 ** -8 * (s64 * r64[:, None] * w64).abs() + 1e-30).all())
+    for residual in (None, res):
+        dx, dw = native.rmsnorm_bwd(dy, summed, w, rstd, residual_grad=residual)
+        xhat, g = s64 * r64[:, None], dy64 * w64
+        want = r64[:, None] * (g - xhat * (g * xhat).mean(1, keepdim=True)) + (0 if residual is None else residual.double())
+        assert _rel(dx, want) < 4e-3
+        bound = (rows + 8) * 2.0 ** -23 * (dy64 * xhat).abs().sum(0)
+        assert bool(((dw.double() - (dy64 * xhat).sum(0)).abs() <= bound + 1e-30).all())
+    native.check_status()
+
+
 def test_router_linear_and_top2(native):
     from b200moe import ops
     from b200moe.ops import functional as Fn
