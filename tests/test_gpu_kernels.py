@@ -628,6 +628,40 @@ def test_moe_plan_gather_combine(native, T, E):
     assert _rel(out, x.float() * w.sum(1, keepdim=True)) < 5e-3
 
 
+@pytest.mark.parametrize("T,E", [(1279, 8), (1280, 8), (5003, 16), (3000, 49), (2000, 1)])
+def test_moe_plan_of_many_slots(native, T, E):
+    """One CTA and a cluster of eight, runs of slots that end inside a warp, more experts than lanes."""
+    from b200moe.ops.moe_fused import capacity_rows
+    idx = torch.randint(0, E, (T, 2), device="cuda")
+    slot_row, row_slot, offs, tile_expert, meta, counts = native.moe_plan(idx, E, capacity_rows(T * 2, E))
+    flat = idx.reshape(-1)
+    order = torch.argsort(flat, stable=True)
+    want = torch.bincount(flat, minlength=E)
+    ends = ((want + 255) // 256 * 256).cumsum(0)
+    starts = ends - (want + 255) // 256 * 256
+    rank = torch.arange(2 * T, device="cuda") - (want.cumsum(0) - want)[flat[order]]
+    assert torch.equal(counts.long(), want) and torch.equal(offs.long(), ends)
+    assert torch.equal(slot_row[order].long(), starts[flat[order]] + rank)
+    live = int(ends[-1])
+    rows = torch.full((live,), -1, device="cuda")
+    rows[slot_row.long()] = torch.arange(2 * T, device="cuda")
+    assert torch.equal(row_slot[:live].long(), rows) and meta[:3].tolist() == [live // 128, live, 0]
+    assert torch.equal(tile_expert[:live // 128].long(), torch.repeat_interleave(torch.arange(E, device="cuda"), (ends - starts) // 128))
+
+
+@pytest.mark.parametrize("offset", [0, 1, 4])
+def test_embedding_gradient_on_and_off_a_16_byte_boundary(native, offset):
+    T, V, D = 301, 40, 72
+    ids, dy = torch.randint(0, V, (T,), device="cuda"), _rand(T, D)
+    grad = torch.zeros(V * D + 8, device="cuda")
+    native.embedding_bwd(ids, dy, grad[offset:offset + V * D].view(V, D))
+    want = torch.zeros(V, D, device="cuda", dtype=torch.float64).index_add_(0, ids, dy.double())
+    scale = torch.zeros(V, D, device="cuda", dtype=torch.float64).index_add_(0, ids, dy.double().abs())
+    got = grad[offset:offset + V * D].view(V, D)
+    assert bool(((got.double() - want).abs() <= T * 2.0 ** -24 * scale).all())
+    assert not grad[:offset].any() and not grad[offset + V * D:].any()
+
+
 def test_combine_with_a_residual_rounds_like_the_sum_of_two_tensors(native):
     """A block's output decides the next router's choices, so the fused sum has to be the separate one bit for bit."""
     T, D = 1001, 264
