@@ -69,6 +69,41 @@ def _compile(name: str, verbose: bool) -> str:
     return obj
 
 
+def _build_nodes(verbose: bool) -> None:
+    """The C++ autograd nodes (csrc/nodes.cpp), compiled against the installed PyTorch; one file for both libraries, which
+    it binds to at run time.  Skipped where PyTorch is not there (the package's Python nodes do without)."""
+    try:
+        import torch
+        from torch.utils import cpp_extension
+    except ImportError:
+        if verbose:
+            print("[b200moe.build] no PyTorch here: C++ autograd nodes not built")
+        return
+    import sysconfig
+    source, target = os.path.join(SRC, "nodes.cpp"), os.path.join(HERE, "_C", "b200moe_nodes.so")
+    with open(source, "rb") as f:
+        digest = hashlib.sha256(f.read() + torch.__version__.encode() + sys.version.encode()).hexdigest()
+    stamp = target + ".sha"
+    if os.path.exists(target) and os.path.exists(stamp) and open(stamp).read() == digest:
+        return
+    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cuda = os.path.dirname(os.path.dirname(nvcc()))
+    include = [*cpp_extension.include_paths(), os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    os.makedirs(os.path.dirname(target), exist_ok=True)
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           "-DTORCH_EXTENSION_NAME=b200moe_nodes", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *(f"-I{path}" for path in include), source, "-o", target, f"-L{lib}", "-lc10", "-lc10_cuda", "-ltorch",
+           "-ltorch_cpu", "-ltorch_python", "-ldl"]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode:
+        sys.stderr.write(proc.stdout + proc.stderr)
+        raise RuntimeError("g++ failed for nodes.cpp")
+    with open(stamp, "w") as f:
+        f.write(digest)
+    if verbose:
+        print("[b200moe.build] compiled nodes.cpp")
+
+
 def build_all(verbose: bool = False, force: bool = False) -> str:
     os.makedirs(OUT, exist_ok=True)
     if force:
@@ -77,7 +112,9 @@ def build_all(verbose: bool = False, force: bool = False) -> str:
                 os.unlink(os.path.join(OUT, name))
     names = _sources()
     with ThreadPoolExecutor(max_workers=min(8, len(names) or 1)) as pool:
+        nodes = pool.submit(_build_nodes, verbose)
         objects = list(pool.map(lambda n: _compile(n, verbose), names))
+        nodes.result()
     newest = max(os.path.getmtime(o) for o in objects)
     if not os.path.exists(LIB) or os.path.getmtime(LIB) < newest:
         cmd = [nvcc(), "-shared", "-o", LIB, *objects, "-Xcompiler", "-fPIC", "-lcudart"]

@@ -72,9 +72,10 @@ def _trunc_normal(shape, std, device=None, dtype=None):
 def _hooked(module) -> bool:
     """Whether somebody watches calls of ``module`` (its own or global hooks), so that it has to be called."""
     from torch.nn.modules import module as m
-    own = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks")
-    return "forward" in module.__dict__ or any(getattr(module, name, None) for name in own) or any(
-        getattr(m, "_global" + name, None) for name in own)
+    own = module.__dict__
+    return bool("forward" in own or own["_forward_hooks"] or own["_forward_pre_hooks"] or own["_backward_hooks"]
+                or own["_backward_pre_hooks"] or m._global_forward_hooks or m._global_forward_pre_hooks
+                or m._global_backward_hooks or m._global_backward_pre_hooks)
 
 
 class LinearLayer(nn.Module):
@@ -282,12 +283,16 @@ class MoELayerMulti(nn.Module):
     def forward(self, x, return_aux_loss=False):
         return self._forward(x, return_aux_loss, None)
 
+    def _one_op(self, x) -> bool:
+        """Whether router and experts run as one op: one rank, the kernels of every step switched on, and nobody watches
+        the router's calls."""
+        router = self._modules["router"]
+        return (self.world_size == 1 and ops.use_native(x, "moe") and ops.use_native(x, "router")
+                and ops.use_native(x, "gemm") and type(router) is LinearLayer
+                and type(self._modules["experts"]) is GroupedPositionWiseFFLayer and not _hooked(router))
+
     def _fused(self, flat, residual, balance):
-        """Router and experts as one op: one rank, the kernels of every step switched on, and nobody watches the
-        router's calls."""
-        if not (self.world_size == 1 and all(ops.use_native(flat, op) for op in ("moe", "router", "gemm"))
-                and type(self.router) is LinearLayer and type(self.experts) is GroupedPositionWiseFFLayer
-                and not _hooked(self.router)):
+        if not self._one_op(flat):
             return None
         from ..ops.moe_fused import moe_layer_fused
         router = self.router.compute_weight if self.router.compute_weight is not None else self.router.weight
@@ -296,6 +301,13 @@ class MoELayerMulti(nn.Module):
 
     def _forward(self, x, return_aux_loss, residual):
         """The layer's output, plus ``residual`` where one is given (added by the combine kernel of the fused op)."""
+        if self.budget is None and x.is_cuda and x.dtype == self.dtype == torch.bfloat16 and self._one_op(x):
+            from ..ops.moe_fused import moe_layer_node
+            router, experts = self._modules["router"], self._modules["experts"]
+            out = moe_layer_node(x, router.compute_weight if router.compute_weight is not None else router.weight, experts.w1,
+                                 experts.w2, experts.w3, residual, self.recompute, return_aux_loss)
+            if out is not None:
+                return tuple(out) if return_aux_loss else out
         shape, in_dtype = x.shape, x.dtype
         flat = x.reshape(-1, shape[-1]).to(self.dtype)
         same = residual is not None and residual.dtype == in_dtype == self.dtype and residual.shape == shape
@@ -405,9 +417,28 @@ class TransformerLayer(nn.Module):
         self.ffn = MoELayerMulti(d_model, d_ff, num_expert_per_node=num_expert_per_node, dp_group=dp_group,
                                  dtype=moe_compute_dtype)
 
+    def _attention_half(self, x):
+        """``(x + attn(ln1(x)), ln2 of it)`` as one call, or ``None``: nobody watches the calls of the modules that it
+        stands for, and the operands are what the fused path of ``MultiHeadLayerLL.forward`` takes."""
+        modules = self._modules
+        ln1, attn, ln2 = modules["ln1"], modules["attn"], modules["ln2"]
+        if not (x.is_cuda and type(attn) is MultiHeadLayerLL and attn.qkv_weight is not None and attn.use_rope
+                and type(ln1) is type(ln2) is RMSNormLayer and type(attn.output_proj) is LinearLayer):
+            return None
+        out = attn.output_proj
+        if attn.head_dim != 128 or out.compute_weight is None or _hooked(ln1) or _hooked(attn) or _hooked(out):
+            return None
+        from ..ops.block import attn_half
+        return attn_half(x, ln1.weight, attn.qkv_weight, attn.RoPE.cos, attn.RoPE.sin, out.compute_weight, ln2.weight,
+                         (attn.num_heads, attn.num_kv_heads), ln1.eps, ln2.eps)
+
     def forward(self, x, return_aux_loss=False):
-        attn_out = self.attn(self.ln1(x))
-        x, normed = ops.add_rmsnorm(x, attn_out, self.ln2.weight, self.ln2.eps)
+        half = self._attention_half(x)
+        if half is not None:
+            x, normed = half
+        else:
+            attn_out = self.attn(self.ln1(x))
+            x, normed = ops.add_rmsnorm(x, attn_out, self.ln2.weight, self.ln2.eps)
         if type(self.ffn) is MoELayerMulti and not _hooked(self.ffn):
             return self.ffn._forward(normed, return_aux_loss, x)
         if return_aux_loss:

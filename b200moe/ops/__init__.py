@@ -40,6 +40,19 @@ def use_native(t: torch.Tensor, op: str = "") -> bool:
     return native.has(op)
 
 
+def cpp_nodes(*tensors):
+    """The C++ autograd nodes for these operands, or ``None``: they take plain tensors outside of every transformation that
+    looks through Python nodes (function transforms, forward-mode differentiation, tracing)."""
+    from torch.autograd import forward_ad
+    from . import native
+    if (any(type(t) is not torch.Tensor and type(t) is not torch.nn.Parameter for t in tensors)
+            or torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0
+            or torch.compiler.is_compiling() or torch.jit.is_tracing() or torch.overrides._get_current_function_mode_stack()
+            or torch.utils._python_dispatch._get_current_dispatch_mode() is not None):
+        return None
+    return native.nodes()
+
+
 def backward_follows(*tensors) -> bool:
     """Whether a call on ``tensors`` (``None`` among them) can be differentiated.  Asked by the callers of autograd
     functions: inside ``forward`` grad mode is off, and ``ctx.needs_input_grad`` repeats the inputs' ``requires_grad``

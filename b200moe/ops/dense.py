@@ -13,7 +13,7 @@ from __future__ import annotations
 
 import torch
 
-from . import backward_follows, functional as Fn, native, use_native
+from . import backward_follows, cpp_nodes, functional as Fn, native, use_native
 
 
 class _Linear(torch.autograd.Function):
@@ -174,6 +174,12 @@ class _Embedding(torch.autograd.Function):
 
 def embedding(ids: torch.Tensor, table: torch.Tensor) -> torch.Tensor:
     """Row gather ``table[ids]``; the backward pass scatter-adds in fp32."""
+    grad = getattr(table, "main_grad", None)
+    if grad is not None and use_native(table, "embedding"):
+        nodes = cpp_nodes(ids, table, grad)
+        out = nodes.embedding(ids, table, grad) if nodes else None
+        if out is not None:
+            return out
     return _Embedding.apply(ids, table)
 
 
@@ -194,7 +200,9 @@ class _RMSNorm(torch.autograd.Function):
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5) -> torch.Tensor:
     """``x · rsqrt(mean(x²) + eps) · weight`` evaluated in fp32, cast back."""
     if use_native(x, "rmsnorm"):
-        return _RMSNorm.apply(x, weight, eps)
+        nodes = cpp_nodes(x, weight)
+        out = nodes.rmsnorm(x, weight, eps, native.status_word(x.device)) if nodes else None
+        return _RMSNorm.apply(x, weight, eps) if out is None else out
     return Fn.rmsnorm_ref(x, weight, eps)
 
 

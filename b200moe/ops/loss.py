@@ -25,7 +25,7 @@ from __future__ import annotations
 
 import torch
 
-from . import backward_follows, functional as Fn, native, use_native
+from . import backward_follows, cpp_nodes, functional as Fn, native, use_native
 
 CHUNK_TOKENS = 4096
 # Keeping logits saves one of four products and a pass over them for each token kept (6001 tokens, width 2048, 32000
@@ -117,6 +117,13 @@ def lm_head_cross_entropy(hidden: torch.Tensor, weight: torch.Tensor, targets: t
     back-propagate into the returned loss, when it is known in advance (see the module text)."""
     from .dense import linear
     if use_native(hidden, "lmhead_ce"):
+        grad = getattr(weight, "main_grad", None)
+        if grad is not None and grad_scale is not None:
+            nodes = cpp_nodes(hidden, weight, targets, grad)
+            loss = nodes.head(hidden, weight, targets, grad, grad_scale, CHUNK_TOKENS, native.status_word(hidden.device)) \
+                if nodes else None
+            if loss is not None:
+                return loss
         return _LMHeadCE.apply(hidden, weight, targets, grad_scale, backward_follows(hidden, weight))
     logits = linear(hidden, weight)
     return Fn.cross_entropy(logits.reshape(-1, logits.shape[-1]), targets.reshape(-1))

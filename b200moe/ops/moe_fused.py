@@ -17,7 +17,7 @@ from __future__ import annotations
 
 import torch
 
-from . import backward_follows, native
+from . import backward_follows, cpp_nodes, native
 
 ALIGN = 256       # expert segments are padded to 256 rows (whole 256x256 GEMM tiles)
 
@@ -162,6 +162,20 @@ class _MoELayer(torch.autograd.Function):
         if ctx.ledger is not None:
             ctx.budget.leave(*ctx.ledger)
         return dx, drouter, dw1, dw2, dw3, dresidual, None, None, None, None
+
+
+def moe_layer_node(x, router_w, w1, w2, w3, residual=None, recompute: bool = False, balance: bool = False):
+    """The routed layer of ``x [..., D]`` as a C++ node (``csrc/nodes.cpp: MoELayer``; the steps of ``_MoELayer``, which
+    stays for callers with an activation budget, for weights without gradient buffers and for what the node does not take):
+    its output, with ``balance`` and its balance loss, or ``None``."""
+    grouter = getattr(router_w, "main_grad", None)
+    g1, g3, g2 = getattr(w1, "main_grad", None), getattr(w3, "main_grad", None), getattr(w2, "main_grad", None)
+    if (grouter is None or g1 is None or g2 is None or g3 is None or getattr(router_w, "pending_gather", None) is not None):
+        return None
+    nodes = cpp_nodes(x, router_w, w1, w3, w2, grouter, g1, g3, g2, *(() if residual is None else (residual,)))
+    done = nodes.moe_layer(x, router_w, w1, w3, w2, residual, grouter, g1, g3, g2, native.status_word(x.device), ALIGN,
+                           recompute, balance) if nodes else None
+    return done if balance or done is None else done[0]
 
 
 def moe_layer_fused(x, router_w, w1, w2, w3, residual=None, recompute: bool = False, budget=None,

@@ -75,7 +75,7 @@ def available_ops() -> list:
 
 
 def launch_count() -> int:
-    return _launches
+    return _launches + (_nodes.launches() if _nodes else 0)
 
 
 def count_launch(n: int = 1) -> None:
@@ -96,6 +96,30 @@ _raw_device = getattr(torch._C, "_cuda_getDevice", None)
 
 def _stream():
     return ctypes.c_void_p(_raw_stream(_raw_device()))
+
+
+_nodes = None        # the C++ autograd nodes (csrc/nodes.cpp), False where they were not built
+
+
+def nodes():
+    """The C++ autograd nodes, bound to this library; ``None`` where the extension was not built (the nodes in Python then
+    issue the same launches) and while launches are timed or marked one by one."""
+    global _nodes
+    if _nodes is None:
+        import importlib.machinery
+        import importlib.util
+        path = os.path.join(_HERE, "_C", "b200moe_nodes.so")
+        _nodes = False
+        if require() is not None and os.path.exists(path):
+            loader = importlib.machinery.ExtensionFileLoader("b200moe_nodes", path)
+            module = importlib.util.module_from_spec(importlib.util.spec_from_loader("b200moe_nodes", loader))
+            loader.exec_module(module)
+            module.bind(_LIB_PATH)
+            _nodes = module
+        else:
+            import warnings
+            warnings.warn(f"{path} not found: small layers run at the speed of Python; run `python -m b200moe.build`")
+    return _nodes if _nodes and _timed is None and not _nvtx else None
 
 
 def status_word(device=None) -> torch.Tensor:
@@ -303,6 +327,11 @@ def gemm_nn(dy, w, w2=None, tile_expert=None, num_m_tiles=None, num_experts: int
     return out
 
 
+def swiglu_bwd_in_product(M: int, F: int, K: int) -> bool:
+    """Whether ``gemm_nn_swiglu_bwd`` is one launch."""
+    return bool(require().b2_swiglu_bwd_in_product(_L(M), _I(F), _I(K)))
+
+
 def gemm_nn_swiglu_bwd(dy, w, gate, up, tile_expert=None, num_m_tiles=None, num_experts: int = 1,
                        align256: bool = False, live_rows=None):
     """``dh = dy [M,K] @ w[e] [K,F]`` and the SwiGLU backward of it: returns ``dgu [M,2F]`` (gradients of the gate and up
@@ -314,7 +343,7 @@ def gemm_nn_swiglu_bwd(dy, w, gate, up, tile_expert=None, num_m_tiles=None, num_
     1024: 114 us against 130 us; 4096 x 1536, K 1024: 34 against 40)."""
     M, K = dy.shape
     F = w.shape[-1]
-    if K < 2048 and M * F > 1 << 21:
+    if not swiglu_bwd_in_product(M, F, K):
         dh = gemm_nn(dy, w, tile_expert=tile_expert, num_m_tiles=num_m_tiles, num_experts=num_experts,
                      align256=align256)
         return swiglu_bwd(dh, gate, up, live_rows=live_rows)

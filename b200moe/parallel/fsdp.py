@@ -369,7 +369,10 @@ class FSDPWrapperPipelined(nn.Module):
                 for p in self.expert_params:
                     dist.all_reduce(p.main_grad, op=dist.ReduceOp.AVG, group=ddp_group)
         for e in flat.entries:
-            e["param"].grad = flat.shard_view(flat.shard_grad, e)
+            view = e.get("grad")           # the same views of the same buffer every step
+            if view is None:
+                view = e["grad"] = flat.shard_view(flat.shard_grad, e)
+            e["param"].grad = view
 
     def finish_gradient_synchronization(self):
         """Kept for API parity; all reductions above complete before returning."""

@@ -1,0 +1,174 @@
+"""The C++ autograd nodes against the Python nodes that they stand for."""
+import os
+
+import pytest
+import torch
+
+from b200moe.ops import native
+
+
+def _nodes():
+    module = native.nodes()
+    if module is None:
+        pytest.skip("built without PyTorch")
+    return module
+
+
+# ------------------------------------------------------------------------------ CPU
+def test_nodes_leave_what_they_do_not_take_to_the_general_way():
+    nodes = _nodes()
+    x, w, word = torch.zeros(2, 128, 512, dtype=torch.bfloat16), torch.ones(512), torch.zeros(1, dtype=torch.int32)
+    table, ids = torch.zeros(9, 512, dtype=torch.bfloat16), torch.zeros(3, dtype=torch.int64)
+    grad, cos = torch.zeros(9, 512), torch.zeros(128, 64)
+    assert nodes.rmsnorm(x, w, 1e-5, word) is None
+    assert nodes.embedding(ids, table, grad) is None
+    assert nodes.head(x, table, ids, grad, 1.0, 4096, word) is None
+    square, fused = torch.zeros(512, 512), torch.zeros(768, 512)
+    assert nodes.attn_half(x, w, fused.bfloat16(), fused, cos, cos, square.bfloat16(), square, w, word, 4, 1, 1e-5, 1e-5) is None
+    experts = torch.zeros(2, 128, 512, dtype=torch.bfloat16)
+    down = torch.zeros(2, 512, 128, dtype=torch.bfloat16)
+    assert nodes.moe_layer(x, table[:2], experts, experts, down, None, grad[:2], experts.float(), experts.float(), down.float(), word,
+                           256, False, False) is None
+    with pytest.raises(RuntimeError, match="cannot load"):
+        nodes.bind("/nonexistent/library.so")
+    nodes.bind(native._LIB_PATH)
+
+
+def test_transformations_that_look_through_nodes_get_the_python_ones():
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from b200moe import ops
+
+    class Other(torch.Tensor):
+        pass
+
+    class Watch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    _nodes()
+    x, seen = torch.zeros(2, 3), []
+    assert ops.cpp_nodes(x, torch.nn.Parameter(x)) is native.nodes()
+    assert ops.cpp_nodes(x, x.as_subclass(Other)) is None
+    torch.func.vmap(lambda t: seen.append(ops.cpp_nodes(x)) or t)(x)
+    torch.func.jvp(lambda t: seen.append(ops.cpp_nodes(x)) or t, (x,), (x,))
+    with Watch():
+        seen.append(ops.cpp_nodes(x))
+    with torch.device("cpu"):
+        seen.append(ops.cpp_nodes(x))
+    native.set_nvtx(True)
+    try:
+        seen.append(ops.cpp_nodes(x))
+    finally:
+        native.set_nvtx(False)
+    assert seen == [None] * 5
+
+
+# ------------------------------------------------------------------------------ GPU
+def _rel(a, b):
+    return float((a.double() - b.double()).norm() / (b.double().norm() + 1e-30))
+
+
+def _decoder(D=512, heads=4, experts=4, ffn=256, vocab=320, blocks=2, expert_grad=torch.float32):
+    from b200moe.models import TransformerLMPipelined
+    from b200moe.parallel import FSDPWrapperPipelined
+    torch.manual_seed(3)
+    with torch.device("cuda"):
+        model = TransformerLMPipelined(vocab, 256, D, blocks, heads, 0, 1, num_expert_per_node=experts, d_ff=ffn)
+    return FSDPWrapperPipelined(model, None, None, compute_dtype=torch.bfloat16, expert_grad_dtype=expert_grad)
+
+
+def _step(model, ids, aux=0.0, scale=0.5):
+    model.clear_grad_accumulators()
+    out = model.loss(ids[:, :-1].contiguous(), ids[:, 1:].contiguous(), return_aux_loss=aux > 0, grad_scale=scale)
+    loss, extra = out if aux else (out, None)
+    torch.autograd.backward([loss] + ([extra] if aux else []), [torch.full_like(loss, scale)] + ([torch.full_like(loss, aux)] if aux else []))
+    model.reduce_accumulated_gradients()
+    grads = {n: (p.main_grad if hasattr(p, "main_grad") else p.grad).clone() for n, p in model.named_parameters()}
+    return loss.detach().clone(), extra, grads
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("S,aux,expert_grad,recompute", [(128, 0.0, torch.float32, False), (256, 0.02, torch.bfloat16, False),
+                                                         (128, 0.02, torch.float32, True)])
+def test_training_step_on_cpp_nodes_matches_python_nodes(monkeypatch, S, aux, expert_grad, recompute):
+    _nodes()
+    model = _decoder(expert_grad=expert_grad)
+    for layer in model.module.layers:
+        layer.ffn.recompute = recompute
+    ids = torch.randint(0, 320, (3, S + 1), device="cuda")
+    before = native.launch_count()
+    loss, extra, got = _step(model, ids, aux)
+    launched = native.launch_count() - before
+    monkeypatch.setattr(native, "nodes", lambda: None)
+    before = native.launch_count()
+    want_loss, want_extra, want = _step(model, ids, aux)
+    assert launched == native.launch_count() - before > 50
+    # the same forward kernels; the loss is a sum of atomics
+    assert abs(float(loss - want_loss)) <= 1e-5 * float(want_loss)
+    assert extra is None or torch.equal(extra, want_extra)
+    # backward: the sum of a block's two input gradients is rounded once where it was rounded twice (2^-9 each)
+    assert got.keys() == want.keys() and all(_rel(got[n], want[n]) < 2e-2 for n in want)
+    with torch.no_grad():
+        logits = model(ids[:, :-1].contiguous())
+        monkeypatch.undo()
+        assert torch.equal(model(ids[:, :-1].contiguous()), logits)
+    native.check_status()
+
+
+@pytest.mark.gpu
+def test_cpp_nodes_under_saved_tensor_hooks_and_on_another_stream():
+    _nodes()
+    model = _decoder()
+    ids = torch.randint(0, 320, (2, 129), device="cuda")
+    _, _, want = _step(model, ids)
+    with torch.autograd.graph.save_on_cpu():
+        _, _, got = _step(model, ids)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        _, _, other = _step(model, ids)
+    torch.cuda.current_stream().wait_stream(side)
+    # sums of atomics (router, embedding) differ in their last bits
+    assert all(_rel(got[n], want[n]) < 1e-3 and _rel(other[n], want[n]) < 1e-3 for n in want)
+    native.check_status()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("which", ["ln1", "attn", "attn.output_proj", "ffn", "ffn.router"])
+def test_watched_modules_are_called(which):
+    model = _decoder(blocks=1)
+    ids = torch.randint(0, 320, (2, 128), device="cuda")
+    calls = []
+    layer = model.module.layers[0]
+    handle = layer.get_submodule(which).register_forward_hook(lambda *_: calls.append(1))
+    with torch.no_grad():
+        model(ids)
+        handle.remove()
+        model(ids)
+    assert calls == [1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,D,V,chunk", [(1, 64, 64, 4096), (300, 512, 320, 128), (257, 128, 32000, 256)])
+def test_head_node_in_chunks(monkeypatch, T, D, V, chunk):
+    from b200moe import ops
+    from b200moe.ops import loss as L
+    _nodes()
+    monkeypatch.setattr(L, "CHUNK_TOKENS", chunk)
+    hidden = torch.randn(T, D, device="cuda").bfloat16().requires_grad_(True)
+    weight = (torch.randn(V, D, device="cuda") * 0.05).bfloat16().requires_grad_(True)
+    weight.main_grad = torch.zeros(V, D, device="cuda")
+    targets = torch.randint(0, V, (T,), device="cuda")
+    out = []
+    for _ in range(2):
+        hidden.grad = None
+        weight.main_grad.zero_()
+        loss = ops.lm_head_cross_entropy(hidden, weight, targets, 0.25)
+        (loss * 0.5).backward()                       # another factor than announced: dh follows, dW keeps its word
+        out.append((loss.detach(), hidden.grad, weight.main_grad.clone()))
+        monkeypatch.setattr(native, "nodes", lambda: None)
+    for a, b in zip(*out):
+        assert _rel(a, b) < 1e-5
+    assert weight.grad is None
+    native.check_status()
