@@ -150,6 +150,13 @@ struct FwdBars {
   uint64_t q_full, k_full[2], v_full[2], k_empty[2], v_empty[2], s_full[2], p_lo[2], p_hi[2], o_done[2];
 };
 
+// The two-tile kernel's threads: two softmax warpgroups and one with the TMA and the MMA warp.  At launch each thread has 168
+// registers; the softmax threads, which hold 128 scores, take most of the third warpgroup's.
+constexpr int FWD_THREADS = 384, FWD_SOFTMAX_REGS = 208, FWD_PRODUCER_REGS = 88;
+static_assert(256 * FWD_SOFTMAX_REGS + 128 * FWD_PRODUCER_REGS <= 384 * 168, "registers of the forward CTA");
+template <int N> __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
 // Which tile a CTA works on.  CTAs are numbered so that the longest causal rows of a set of heads start first, and a
 // set holds as many heads as keep the tensors they re-read inside the L2 (p.set_heads, host side).
 struct AttnWork {
@@ -211,11 +218,14 @@ __device__ __forceinline__ void store_out32(uint8_t* dst, const uint32_t (&o)[32
 // fill tensor memory; P overwrites S.  MMA order O0(j) S0(j+1) O1(j) S1(j+1): a tile's next scores are issued behind
 // the product that still reads its probabilities, so "scores ready" also means "output of the previous key tile
 // accumulated", and the rare rescale of O (row maximum grew by more than 2^8) needs no further wait.
-// Bound by the chain scores -> exponentials -> product of each tile.  32/8 heads of 8192 tokens, causal: 447 us, 1230
-// TFLOP/s (one query tile per CTA with two threads per row: 622 us); 32 heads of 2048 tokens, every key, fp16: 77 us
-// (bf16 kernel 95 us plus 96 us of casts).
+// Bound by the chain scores -> exponentials -> product of each tile: of 2930 cycles per key tile 360 were the row maximum, now
+// formed beside the first half's exponentials, and 2048 are the products of both tiles.  32/8 heads of 8192 tokens, causal:
+// 447 -> 434 us, 1270 TFLOP/s (one query tile per CTA with two threads per row: 622 us); 32 heads of 2048 tokens, every key,
+// fp16: 70.7 -> 68.6 us (at 1.9 GHz; 78 -> 76 on a slower box).  The special-function unit is not the limit: an eighth to
+// half of the exponentials as polynomials on the FMA pipe took 1 to 18 % longer; nor do scores in two halves of 64 keys help,
+// whose products read their operands from shared memory half as often as they use them (2930 -> 3350 cycles).
 template <int F16>
-__global__ void __launch_bounds__(ATTN_THREADS, 1) attn_fwd_kernel(const __grid_constant__ AttnParams p) {
+__global__ void __launch_bounds__(FWD_THREADS, 1) attn_fwd_kernel(const __grid_constant__ AttnParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = smem_raw;
   uint8_t* sQ = smem;                       // 2 tiles
@@ -261,8 +271,9 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_fwd_kernel(const __grid_
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;         // S0 | S1 | O0 | O1, 128 columns each
 
-  if (warp == 8) {
-    if (elect_one()) {
+  if (warp >= 8) {
+    reg_dec<FWD_PRODUCER_REGS>();
+    if (warp == 8 && elect_one()) {
       mbar_expect_tx(&bars->q_full, (n1 ? 2 : 1) * TILE_BYTES);
       load_tile(sQ, &p.map_q, &bars->q_full, h * HD, qt0 * TQ, b);
       if (n1) load_tile(sQ + TILE_BYTES, &p.map_q, &bars->q_full, h * HD, (qt0 + 1) * TQ, b);
@@ -283,8 +294,7 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_fwd_kernel(const __grid_
         drain_ring<2>(bars->v_full, j);
       }
     }
-  } else if (warp == 9) {
-    if (elect_one()) {
+    if (warp == 9 && elect_one()) {
       constexpr uint32_t idesc_qk = attn_idesc<F16>(0);
       constexpr uint32_t idesc_pv = attn_idesc<F16>(1);
       auto issue_s = [&](int t, int j) {
@@ -333,6 +343,7 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_fwd_kernel(const __grid_
       }
     }
   } else {
+    reg_inc<FWD_SOFTMAX_REGS>();
     const int t = warp >> 2;                              // query tile of this warpgroup
     const int quad = warp & 3;
     const int r = quad * 32 + lane;                       // query row inside the tile
@@ -358,37 +369,43 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_fwd_kernel(const __grid_
         for (int i = 0; i < 128; ++i)
           if (i >= limit) raw[i >> 5][i & 31] = 0xff800000u;   // -inf
       }
-      float mpart[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      auto row_max = [&] {
+        float mpart[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-      for (int i = 0; i < 128; i += 2) mpart[(i >> 1) & 3] = fmaxf(fmaxf(mpart[(i >> 1) & 3], score(i)), score(i + 1));
-      const float mx = fmaxf(fmaxf(fmaxf(mpart[0], mpart[1]), fmaxf(mpart[2], mpart[3])), m_ref);
-      const bool need = (mx - m_ref) * p.scale_log2 > 8.f;      // also true on the first tile (m_ref = -inf)
-      if (__any_sync(0xffffffffu, need)) {
-        const float alpha = ex2((m_ref - mx) * p.scale_log2);   // 0 on the first tile
+        for (int i = 0; i < 128; i += 2) mpart[(i >> 1) & 3] = fmaxf(fmaxf(mpart[(i >> 1) & 3], score(i)), score(i + 1));
+        return fmaxf(fmaxf(fmaxf(mpart[0], mpart[1]), fmaxf(mpart[2], mpart[3])), m_ref);
+      };
+      if (j == 0) m_ref = row_max();
+      // The first half's exponentials do not wait for the row maximum, which is formed beside them: the reference rarely
+      // moves (by more than 2^8), and where it does they are formed again.
+      float low = probabilities64<F16, 32>(raw[0], raw[1], ts, p.scale_log2, -m_ref * p.scale_log2);
+      const float mx = row_max();
+      if (__any_sync(0xffffffffu, (mx - m_ref) * p.scale_log2 > 8.f)) {
+        const float alpha = ex2((m_ref - mx) * p.scale_log2);
         m_ref = mx;
         l[0] *= alpha;
         l[1] *= alpha;
-        if (j > 0) {
 #pragma unroll 1
-          for (int c = 0; c < 8; ++c) {
-            uint32_t o[16];
-            tmem_ld_32x16(to + c * 16, o);
-            tmem_ld_wait();
+        for (int c = 0; c < 8; ++c) {
+          uint32_t o[16];
+          tmem_ld_32x16(to + c * 16, o);
+          tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-            tmem_st_32x16(to + c * 16, o);
-          }
+          for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+          tmem_st_32x16(to + c * 16, o);
         }
+        low = probabilities64<F16, 32>(raw[0], raw[1], ts, p.scale_log2, -m_ref * p.scale_log2);
       }
-      const float neg = -m_ref * p.scale_log2;
-#pragma unroll
-      for (int hf = 0; hf < 2; ++hf) {
-        l[hf] += probabilities64<F16, 32>(raw[2 * hf], raw[2 * hf + 1], ts + hf * 32, p.scale_log2, neg);
+      auto publish = [&](uint64_t* bar) {
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(hf ? &bars->p_hi[t] : &bars->p_lo[t]);
-      }
+        if (lane == 0) mbar_arrive(bar);
+      };
+      l[0] += low;
+      publish(&bars->p_lo[t]);
+      l[1] += probabilities64<F16, 32>(raw[2], raw[3], ts + 32, p.scale_log2, -m_ref * p.scale_log2);
+      publish(&bars->p_hi[t]);
     }
     // epilogue: normalise and store this thread's query row
     if (n > 0 && !*abort_flag) {
@@ -1190,14 +1207,14 @@ static int sm_count_attn() {
   return sms > 0 ? sms : 148;
 }
 
-template <void (*kernel)(AttnParams), int smem>
+template <void (*kernel)(AttnParams), int smem, int threads = ATTN_THREADS>
 static int launch_fwd(const AttnParams& p, long long ctas, cudaStream_t stream) {
   static bool set = false;
   if (!set) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -3;
     set = true;
   }
-  kernel<<<static_cast<unsigned>(ctas), ATTN_THREADS, smem, stream>>>(p);
+  kernel<<<static_cast<unsigned>(ctas), threads, smem, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
@@ -1232,8 +1249,8 @@ int b2_attention_fwd_ex(const void* q, const void* k, const void* v, long long q
     return f16 ? launch_fwd<attn_fwd_one_tile_kernel<1>, FWD_ONE_SMEM>(p, tiles * heads, stream)
                : launch_fwd<attn_fwd_one_tile_kernel<0>, FWD_ONE_SMEM>(p, tiles * heads, stream);
   const long long ctas = (tiles + 1) / 2 * heads;
-  return f16 ? launch_fwd<attn_fwd_kernel<1>, FWD_SMEM>(p, ctas, stream)
-             : launch_fwd<attn_fwd_kernel<0>, FWD_SMEM>(p, ctas, stream);
+  return f16 ? launch_fwd<attn_fwd_kernel<1>, FWD_SMEM, FWD_THREADS>(p, ctas, stream)
+             : launch_fwd<attn_fwd_kernel<0>, FWD_SMEM, FWD_THREADS>(p, ctas, stream);
 }
 
 // Gradients.  dout, out: [B,S,Hq,128] contiguous; stats: fp32 scratch [B*Hq, 2, Sp] with Sp = S rounded up to 128; dq
