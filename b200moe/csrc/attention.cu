@@ -987,7 +987,7 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dkv_kernel(const __g
 }
 
 // ================================================================= backward: dQ
-// TMEM: S [0,128), dP / dS [128,256), dQ [256,384).  Thread layout as above with query rows: group g handles key columns
+// TMEM: S [0,128), dP / dS [128,256), dQ [256,384), Q and dO as A operands [384,448) and [448,512).  Thread layout as above with query rows: group g handles key columns
 // [64 g, 64 g + 64).  The ring of three holds K tiles, the ring of two V tiles.  P stays in registers, so the next
 // scores of a half are issued as soon as its warps have read the present ones (p_ready counts that).  MMA order:
 //   S0(j+1) | dQ1(j-1) dP1(j) | S1(j+1) | dQ0(j) dP0(j+1)
@@ -1007,7 +1007,7 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dq_kernel(const __gr
 
   bwd_init(sm, warp);
   const uint32_t tmem = sm.tmem_slot;
-  const uint32_t t_s = tmem, t_dp = tmem + 128, t_dq = tmem + 256;
+  const uint32_t t_s = tmem, t_dp = tmem + 128, t_dq = tmem + 256, t_q = tmem + 384, t_do = tmem + 448;
 
   if (warp == 8) {
     if (elect_one()) {
@@ -1034,19 +1034,18 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dq_kernel(const __gr
     if (elect_one()) {
       constexpr uint32_t idesc_kk = umma_idesc_bf16(128, HALF, 0, 0);
       constexpr uint32_t idesc_tn = umma_idesc_bf16(128, 128, 0, 1);
-      const uint32_t q_addr = smem_u32(sm.fixed[0]), do_addr = smem_u32(sm.fixed[1]);
       auto issue_s = [&](int j, int g) {           // S[q, key half] = Q K^T
         const uint32_t k_addr = smem_u32(sm.a[slot3(j)]) + g * HALF * 128;
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
-          umma_bf16_ss(t_s + g * HALF, desc_kmajor(q_addr, ks), desc_kmajor(k_addr, ks), idesc_kk, ks != 0);
+          umma_bf16_ts(t_s + g * HALF, t_q + ks * 8, desc_kmajor(k_addr, ks), idesc_kk, ks != 0);
         umma_commit(&bars->st_full[g]);
       };
       auto issue_dp = [&](int j, int g) {          // dP[q, key half] = dO V^T
         const uint32_t v_addr = smem_u32(sm.b[j & 1]) + g * HALF * 128;
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
-          umma_bf16_ss(t_dp + g * HALF, desc_kmajor(do_addr, ks), desc_kmajor(v_addr, ks), idesc_kk, ks != 0);
+          umma_bf16_ts(t_dp + g * HALF, t_do + ks * 8, desc_kmajor(v_addr, ks), idesc_kk, ks != 0);
         umma_commit(&bars->dpt_full[g]);
       };
       auto issue_dq = [&](int j, int g) {          // dQ[q, d] += dS[q, key half] K[key half, d]
@@ -1055,7 +1054,9 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dq_kernel(const __gr
         for (int ks = 0; ks < 4; ++ks)
           umma_bf16_ts(t_dq, t_dp + g * HALF + ks * 8, desc_mnmajor(k_addr, g * 4 + ks), idesc_tn, (j | g | ks) != 0);
       };
-      bool ok = mbar_wait(&bars->fixed_full, 0) && mbar_wait(&bars->a_full[0], 0) && mbar_wait(&bars->b_full[0], 0);
+      // Q and dO are in tensor memory once both groups have copied their tile (see below)
+      bool ok = mbar_wait(&bars->ds_ready[0], 0) && mbar_wait(&bars->ds_ready[1], 0) && mbar_wait(&bars->a_full[0], 0) &&
+                mbar_wait(&bars->b_full[0], 0);
       if (ok) {
         tc_fence_after();
         issue_s(0, 0);
@@ -1071,7 +1072,7 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dq_kernel(const __gr
           issue_s(j + 1, 0);
         }
         if (j > 0) {
-          if (!(ok = mbar_wait(&bars->ds_ready[1], ph ^ 1))) break;
+          if (!(ok = mbar_wait(&bars->ds_ready[1], ph))) break;
           tc_fence_after();
           issue_dq(j - 1, 1);
           umma_commit(&bars->a_empty[slot3(j - 1)]);
@@ -1083,7 +1084,7 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dq_kernel(const __gr
           tc_fence_after();
           issue_s(j + 1, 1);
         }
-        if (!(ok = mbar_wait(&bars->ds_ready[0], ph))) break;
+        if (!(ok = mbar_wait(&bars->ds_ready[0], ph ^ 1))) break;
         tc_fence_after();
         issue_dq(j, 0);
         if (more) {
@@ -1092,7 +1093,7 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dq_kernel(const __gr
           issue_dp(j + 1, 0);
         }
       }
-      if (ok && !*abort_flag && (ok = mbar_wait(&bars->ds_ready[1], (n_kv - 1) & 1))) {
+      if (ok && !*abort_flag && (ok = mbar_wait(&bars->ds_ready[1], n_kv & 1))) {
         tc_fence_after();
         issue_dq(n_kv - 1, 1);
         umma_commit(&bars->acc_done);
@@ -1110,6 +1111,26 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dq_kernel(const __gr
     const f32x2 scale2 = make_f32x2(p.scale_log2, p.scale_log2);
     const f32x2 nlse2 = make_f32x2(stat[0], stat[0]);
     const f32x2 ndelta2 = make_f32x2(stat[q_tiles * TQ], stat[q_tiles * TQ]);
+    // The A operands of both score products, the same for every key tile, move to tensor memory: group 0 copies Q, group 1
+    // dO, a row per thread (16-byte units of the 128-byte-swizzled tile).  From shared memory they were read again for every
+    // 64 keys, and the products with N = 64 waited for it (6 KiB per 32 cycles): 32/8 heads of 8192 tokens, causal, backward
+    // pass as a whole 1609 -> 1546 us, 128 heads of 640 tokens, every key, 158 -> 153.
+    if (!mbar_wait(&bars->fixed_full, 0)) ATTN_FAIL(224);
+    if (!*abort_flag) {
+      const uint8_t* row = sm.fixed[half] + r * 128;
+#pragma unroll
+      for (int atom = 0; atom < 2; ++atom) {
+        uint32_t w[32];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const uint4 x = *reinterpret_cast<const uint4*>(row + atom * ATOM_BYTES + ((u ^ (r & 7)) << 4));
+          w[4 * u] = x.x; w[4 * u + 1] = x.y; w[4 * u + 2] = x.z; w[4 * u + 3] = x.w;
+        }
+        tmem_st_32x32((half ? t_do : t_q) + lane_base + atom * 32, w);
+      }
+      tmem_st_wait();
+      arrive_half(&bars->ds_ready[half], lane);
+    }
     for (int j = 0; j < n_kv && !*abort_flag; ++j) {
       const uint32_t ph = j & 1;
       if (!mbar_wait(&bars->st_full[half], ph)) { ATTN_FAIL(225); break; }
