@@ -18,6 +18,7 @@
 //   and accumulates dQ += dS K in TMEM.
 // A sequence may have any length: its last tile reads zeros behind it and is masked.
 // Every barrier wait is bounded; a wait that runs out sets the status word.
+#include "chain.cuh"
 #include "ptx.cuh"
 #include "tensormap.cuh"
 
@@ -269,6 +270,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) attn_fwd_kernel(const __grid_c
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  chain_begin();
   const uint32_t tmem = *tmem_slot;         // S0 | S1 | O0 | O1, 128 columns each
 
   if (warp >= 8) {
@@ -486,6 +488,7 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_fwd_one_tile_kernel(cons
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  chain_begin();
   const uint32_t tmem = sm.tmem_slot;       // S / P of even and odd key tiles, O: 128 columns each
   const uint32_t t_o = tmem + 256;
 
@@ -650,6 +653,7 @@ __global__ void __launch_bounds__(256) attn_stats_kernel(const __nv_bfloat16* __
                                                          const __nv_bfloat16* __restrict__ out,
                                                          const float* __restrict__ lse, float* __restrict__ stats, int S,
                                                          int Sp, int Hq) {
+  chain_begin();
   const int sub = threadIdx.x & 15;
   const int blocks_per_head = Sp / 16;
   const int head = blockIdx.x / blocks_per_head;           // batch * Hq + h
@@ -754,6 +758,7 @@ __device__ __forceinline__ void bwd_init(BwdSmem& sm, int warp) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  chain_begin();
 }
 
 __device__ __forceinline__ void bwd_exit(BwdSmem& sm, int warp, uint32_t tmem) {
@@ -1235,7 +1240,7 @@ static int launch_fwd(const AttnParams& p, long long ctas, cudaStream_t stream) 
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -3;
     set = true;
   }
-  kernel<<<static_cast<unsigned>(ctas), threads, smem, stream>>>(p);
+  launch_next(kernel, static_cast<unsigned>(ctas), threads, smem, stream, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
@@ -1307,13 +1312,12 @@ int b2_attention_bwd_rope(const void* dout, const void* q, const void* k, const 
   }
   const long long tiles = (S + TQ - 1) / TQ, Sp = tiles * TQ;
   if (Sp / 16 * B * Hq > 0x7fffffffLL) return -10;
-  attn_stats_kernel<<<static_cast<unsigned>(Sp / 16 * B * Hq), 256, 0, stream>>>(
-      static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(out), lse, stats, S,
+  launch_next(attn_stats_kernel, static_cast<unsigned>(Sp / 16 * B * Hq), 256, 0, stream, static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(out), lse, stats, S,
       static_cast<int>(Sp), Hq);
   p.set_heads = heads_per_set(B * Hkv, 4LL * S * HD * (Hq / Hkv));
-  attn_bwd_dkv_kernel<<<static_cast<unsigned>(tiles * B * Hkv), ATTN_THREADS, BWD_SMEM, stream>>>(p);
+  launch_next(attn_bwd_dkv_kernel, static_cast<unsigned>(tiles * B * Hkv), ATTN_THREADS, BWD_SMEM, stream, p);
   p.set_heads = heads_per_set(B * Hq, 4LL * S * HD * Hkv / Hq);
-  attn_bwd_dq_kernel<<<static_cast<unsigned>(tiles * B * Hq), ATTN_THREADS, BWD_SMEM, stream>>>(p);
+  launch_next(attn_bwd_dq_kernel, static_cast<unsigned>(tiles * B * Hq), ATTN_THREADS, BWD_SMEM, stream, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 

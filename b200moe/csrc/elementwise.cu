@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "chain.cuh"
 #include "ptx.cuh"
 
 namespace b2 {
@@ -164,6 +165,7 @@ __global__ void __launch_bounds__(NORM_THREADS + 32) rmsnorm_fwd_kernel(const __
                                                                        __nv_bfloat16* __restrict__ y,
                                                                        float* __restrict__ rstd, int* __restrict__ status,
                                                                        int rows, int D, float eps, int ring_stages) {
+  chain_begin();
   constexpr int R = 8 / W;
   extern __shared__ __align__(128) uint8_t norm_ring[];
   __shared__ NormBars bars;
@@ -254,6 +256,7 @@ __global__ void __launch_bounds__(NORM_THREADS) rmsnorm_fwd_row_kernel(const __n
                                                                   __nv_bfloat16* __restrict__ sum_out,
                                                                   __nv_bfloat16* __restrict__ y,
                                                                   float* __restrict__ rstd, int rows, int D, float eps) {
+  chain_begin();
   __shared__ float scratch[NORM_THREADS / 32];
   float wv[CH][8];
 #pragma unroll
@@ -311,6 +314,7 @@ __global__ void __launch_bounds__(NORM_THREADS + 32, V == 2 ? 2 : 1)
                        const float* __restrict__ w, const float* __restrict__ rstd,
                        const __nv_bfloat16* __restrict__ residual, __nv_bfloat16* __restrict__ dx,
                        float* __restrict__ dw_partial, int* __restrict__ status, int rows, int D, int ring_stages) {
+  chain_begin();
   constexpr int R = 8 / W;
   extern __shared__ __align__(128) uint8_t norm_ring[];
   __shared__ NormBars bars;
@@ -439,6 +443,7 @@ __global__ void __launch_bounds__(NORM_THREADS + 32, V == 2 ? 2 : 1)
 // shared memory adds the 32 partial sums.
 __global__ void __launch_bounds__(1024) column_sum_kernel(const float* __restrict__ partial, float* __restrict__ out,
                                                          int parts, int D) {
+  chain_begin();
   __shared__ float acc[32][33];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col = blockIdx.x * 32 + lane;
@@ -497,6 +502,7 @@ __device__ __forceinline__ void top2_row(const float* __restrict__ logits, float
 
 __global__ void router_top2_fwd_kernel(const float* __restrict__ logits, float* __restrict__ weights,
                                        long long* __restrict__ idx, float* __restrict__ probs, int T, int E) {
+  chain_begin();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= T) return;
   const size_t row = static_cast<size_t>(t) * E;
@@ -538,6 +544,7 @@ __global__ void __launch_bounds__(256) skinny_nt_kernel(const __nv_bfloat16* __r
                                                         const __nv_bfloat16* __restrict__ w, float* __restrict__ out,
                                                         float* __restrict__ weights, long long* __restrict__ idx,
                                                         float* __restrict__ probs, int T, int N, int K) {
+  chain_begin();
   extern __shared__ __nv_bfloat16 ws[];
   __shared__ float chosen[TOP2 ? 8 : 1][SKINNY_TOKENS][NN];
   skinny_stage(ws, w, N * K);
@@ -597,6 +604,7 @@ template <int NN>
 __global__ void __launch_bounds__(256) skinny_nn_kernel(const float* __restrict__ dy,
                                                         const __nv_bfloat16* __restrict__ w,
                                                         __nv_bfloat16* __restrict__ dx, int T, int N, int K) {
+  chain_begin();
   extern __shared__ __nv_bfloat16 ws[];
   skinny_stage(ws, w, N * K);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -637,6 +645,7 @@ template <int NN>
 __global__ void __launch_bounds__(256) skinny_tn_kernel(const float* __restrict__ dy,
                                                         const __nv_bfloat16* __restrict__ x, float* __restrict__ dw,
                                                         int T, int N, int K, int tokens_per_cta) {
+  chain_begin();
   __shared__ float sums[8][8][32 + 1];       // [warp][column of the lane][lane], one output at a time
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int k = blockIdx.x * 256 + lane * 8;
@@ -682,6 +691,7 @@ __global__ void __launch_bounds__(256) skinny_tn_kernel(const float* __restrict_
 __global__ void router_top2_bwd_kernel(const float* __restrict__ dweights, const float* __restrict__ probs,
                                        const long long* __restrict__ idx, const float* __restrict__ weights,
                                        float* __restrict__ dlogits, int T, int E) {
+  chain_begin();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= T) return;
   const int a = static_cast<int>(idx[2 * t]), b = static_cast<int>(idx[2 * t + 1]);
@@ -704,6 +714,7 @@ __global__ void router_top2_bwd_kernel(const float* __restrict__ dweights, const
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dh, const __nv_bfloat16* __restrict__ gate,
                                   const __nv_bfloat16* __restrict__ up, __nv_bfloat16* __restrict__ dgu,
                                   __nv_bfloat16* __restrict__ h, const int* __restrict__ live_rows, int rows, int F) {
+  chain_begin();
   const int limit = live_rows ? min(rows, *live_rows) : rows;
   const size_t per_row = F / 8;
   const size_t total = static_cast<size_t>(limit) * per_row;
@@ -735,6 +746,7 @@ constexpr int CE_THREADS = 512;
 __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16* __restrict__ logits,
                                                                   const long long* __restrict__ targets,
                                                                   float* __restrict__ loss, int T, int V, float scale) {
+  chain_begin();
   __shared__ float scratch[CE_THREADS / 32];
   for (int t = blockIdx.x; t < T; t += gridDim.x) {
     __nv_bfloat16* row = logits + static_cast<size_t>(t) * V;
@@ -788,6 +800,7 @@ template <int CHUNKS>
 __global__ void __launch_bounds__(CE_THREADS, 2)
     cross_entropy_reg_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets,
                              float* __restrict__ loss, int T, int V, float loss_scale, float grad_scale) {
+  chain_begin();
   __shared__ float scratch[CE_THREADS / 32];
   float local_loss = 0.f;
   bf16x8 raw[CHUNKS];
@@ -862,6 +875,7 @@ __global__ void __launch_bounds__(CE_THREADS, 2)
     cross_entropy_bulk_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets,
                               float* __restrict__ loss, int* __restrict__ status, int T, int V, float loss_scale,
                               float grad_scale) {
+  chain_begin();
   extern __shared__ __align__(128) uint8_t ce_row[];
   __shared__ float scratch[CE_THREADS / 32];
   __shared__ uint64_t arrived;
@@ -949,6 +963,7 @@ __global__ void __launch_bounds__(CE_THREADS, 2)
 }
 
 __global__ void scale_bf16_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ factor, size_t n8) {
+  chain_begin();
   const float f = *factor;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n8;
        i += static_cast<size_t>(gridDim.x) * blockDim.x) {
@@ -1024,6 +1039,7 @@ struct AdamwTable {
 template <typename P, typename G, typename S>
 __global__ void __launch_bounds__(256) adamw_kernel(const __grid_constant__ AdamwTable table, float lr, float beta1,
                                                     float beta2, float eps, float wd, float a_t, float grad_scale) {
+  chain_begin();
   const float decay = 1.f - lr * wd;
   int which = 0;
   for (int chunk = blockIdx.x; chunk < table.first_chunk[table.count]; chunk += gridDim.x) {
@@ -1080,6 +1096,7 @@ struct ZeroTable {
   int count;
 };
 __global__ void __launch_bounds__(256) zero_kernel(const __grid_constant__ ZeroTable table) {
+  chain_begin();
   const int chunk = blockIdx.x;
   int which = 0, end = table.count;          // the last buffer that starts at or before this chunk
   while (end - which > 1) {
@@ -1103,6 +1120,7 @@ __global__ void __launch_bounds__(256) zero_kernel(const __grid_constant__ ZeroT
 }
 
 __global__ void cast_f32_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, size_t n) {
+  chain_begin();
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<size_t>(gridDim.x) * blockDim.x)
     dst[i] = __float2bfloat16_rn(src[i]);
@@ -1111,6 +1129,7 @@ __global__ void cast_f32_bf16_kernel(const float* __restrict__ src, __nv_bfloat1
 // ------------------------------------------------------------------ embedding
 __global__ void embedding_fwd_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ table,
                                      __nv_bfloat16* __restrict__ out, int T, int D) {
+  chain_begin();
   const int per_row = D / 8;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < static_cast<size_t>(T) * per_row;
        i += static_cast<size_t>(gridDim.x) * blockDim.x) {
@@ -1125,6 +1144,7 @@ __global__ void embedding_fwd_kernel(const long long* __restrict__ ids, const __
 template <bool VECTOR>
 __global__ void embedding_bwd_kernel(const long long* __restrict__ ids, const __nv_bfloat16* __restrict__ dy,
                                      float* __restrict__ grad, int T, int D) {
+  chain_begin();
   const int per_row = D / 8;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < static_cast<size_t>(T) * per_row;
        i += static_cast<size_t>(gridDim.x) * blockDim.x) {
@@ -1148,6 +1168,7 @@ __global__ void embedding_bwd_kernel(const long long* __restrict__ ids, const __
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ cos_t,
                             const float* __restrict__ sin_t, int tokens, int S, int H, int hd, long long pitch,
                             float sign) {
+  chain_begin();
   const int vec_per_head = hd / 8;
   const size_t total = static_cast<size_t>(tokens) * H * vec_per_head;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
@@ -1183,6 +1204,7 @@ __global__ void __launch_bounds__(256) rope_copy_kernel(const __nv_bfloat16* __r
                                                         const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                                                         int tokens, int S, int Hq, int Hkv, long long q_pitch,
                                                         long long k_pitch) {
+  chain_begin();
   const int per_token = (Hq + Hkv) * 16;       // 16-byte vectors
   const size_t total = static_cast<size_t>(tokens) * per_token;
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < total;
@@ -1268,14 +1290,14 @@ int b2_rmsnorm_fwd(const void* x, const void* delta, const float* w, void* sum_o
   const int at_once = norm_rows_at_once(D);
   if ((rows + at_once - 1) / at_once <= sm_count_ew() * NORM_FWD_CTAS) {
     auto kernel = D <= 2048 ? rmsnorm_fwd_row_kernel<1> : D <= 4096 ? rmsnorm_fwd_row_kernel<2> : rmsnorm_fwd_row_kernel<4>;
-    kernel<<<min(rows, sm_count_ew() * 8), NORM_THREADS, 0, s>>>((const bf16*)x, (const bf16*)delta, w, (bf16*)sum_out, (bf16*)y,
+    launch_next(kernel, min(rows, sm_count_ew() * 8), NORM_THREADS, 0, s, (const bf16*)x, (const bf16*)delta, w, (bf16*)sum_out, (bf16*)y,
                                                                  rstd, rows, D, eps);
     return ok();
   }
   return launch_norm(D, 2, [&](auto W, auto V, int smem, int stages) {
     auto kernel = rmsnorm_fwd_kernel<decltype(W)::value, decltype(V)::value>;
     if (const int rc = norm_smem<decltype(W)::value, decltype(V)::value, 0>(kernel)) return rc;
-    kernel<<<sm_count_ew() * NORM_FWD_CTAS, NORM_THREADS + 32, smem, s>>>((const bf16*)x, (const bf16*)delta, w, (bf16*)sum_out, (bf16*)y, rstd, status,
+    launch_next(kernel, sm_count_ew() * NORM_FWD_CTAS, NORM_THREADS + 32, smem, s, (const bf16*)x, (const bf16*)delta, w, (bf16*)sum_out, (bf16*)y, rstd, status,
                                                  rows, D, eps, stages);
     return ok();
   });
@@ -1295,12 +1317,12 @@ int b2_rmsnorm_bwd(const void* dy, const void* x, const float* w, const float* r
   const int rc = launch_norm(D, 3, [&](auto W, auto V, int smem, int stages) {
     auto kernel = rmsnorm_bwd_kernel<decltype(W)::value, decltype(V)::value>;
     if (const int rc = norm_smem<decltype(W)::value, decltype(V)::value, 1>(kernel)) return rc;
-    kernel<<<parts, NORM_THREADS + 32, smem, s>>>((const bf16*)dy, (const bf16*)x, w, rstd, (const bf16*)residual, (bf16*)dx,
+    launch_next(kernel, parts, NORM_THREADS + 32, smem, s, (const bf16*)dy, (const bf16*)x, w, rstd, (const bf16*)residual, (bf16*)dx,
                                                   dw_partial, status, rows, D, stages);
     return ok();
   });
   if (rc) return rc;
-  column_sum_kernel<<<(D + 31) / 32, 1024, 0, s>>>(dw_partial, dw, parts, D);
+  launch_next(column_sum_kernel, (D + 31) / 32, 1024, 0, s, dw_partial, dw, parts, D);
   return ok();
 }
 
@@ -1321,7 +1343,7 @@ static int launch_skinny_nt(const void* x, const void* w, float* out, float* wei
     set = true;
   }
   auto kernel = N <= 8 ? skinny_nt_kernel<8, TOP2> : skinny_nt_kernel<16, TOP2>;
-  kernel<<<skinny_grid(T), 256, smem, s>>>((const bf16*)x, (const bf16*)w, out, weights, idx, probs, T, N, K);
+  launch_next(kernel, skinny_grid(T), 256, smem, s, (const bf16*)x, (const bf16*)w, out, weights, idx, probs, T, N, K);
   return ok();
 }
 extern "C" {
@@ -1345,8 +1367,8 @@ int b2_skinny_nn(const float* dy, const void* w, void* dx, int T, int N, int K, 
     cudaFuncSetAttribute(skinny_nn_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     set = true;
   }
-  if (N <= 8) skinny_nn_kernel<8><<<skinny_grid(T), 256, smem, s>>>(dy, (const bf16*)w, (bf16*)dx, T, N, K);
-  else skinny_nn_kernel<16><<<skinny_grid(T), 256, smem, s>>>(dy, (const bf16*)w, (bf16*)dx, T, N, K);
+  if (N <= 8) launch_next(skinny_nn_kernel<8>, skinny_grid(T), 256, smem, s, dy, (const bf16*)w, (bf16*)dx, T, N, K);
+  else launch_next(skinny_nn_kernel<16>, skinny_grid(T), 256, smem, s, dy, (const bf16*)w, (bf16*)dx, T, N, K);
   return ok();
 }
 int b2_skinny_tn(const float* dy, const void* x, float* dw, int T, int N, int K, cudaStream_t s) {
@@ -1357,28 +1379,27 @@ int b2_skinny_tn(const float* dy, const void* x, float* dw, int T, int N, int K,
   const int splits = max(1, min((T + 63) / 64, sm_count_ew() * 2 / columns));
   const int per = (T + splits - 1) / splits;
   const dim3 grid(columns, (T + per - 1) / per);
-  if (N <= 8) skinny_tn_kernel<8><<<grid, 256, 0, s>>>(dy, (const bf16*)x, dw, T, N, K, per);
-  else skinny_tn_kernel<16><<<grid, 256, 0, s>>>(dy, (const bf16*)x, dw, T, N, K, per);
+  if (N <= 8) launch_next(skinny_tn_kernel<8>, grid, 256, 0, s, dy, (const bf16*)x, dw, T, N, K, per);
+  else launch_next(skinny_tn_kernel<16>, grid, 256, 0, s, dy, (const bf16*)x, dw, T, N, K, per);
   return ok();
 }
 
 int b2_router_top2_fwd(const float* logits, float* weights, long long* idx, float* probs, int T, int E,
                        cudaStream_t s) {
   if (E > ROUTER_MAX_E || E < 2) return -10;
-  router_top2_fwd_kernel<<<(T + 127) / 128, 128, 0, s>>>(logits, weights, idx, probs, T, E);
+  launch_next(router_top2_fwd_kernel, (T + 127) / 128, 128, 0, s, logits, weights, idx, probs, T, E);
   return ok();
 }
 int b2_router_top2_bwd(const float* dweights, const float* probs, const long long* idx, const float* weights,
                        float* dlogits, int T, int E, cudaStream_t s) {
-  router_top2_bwd_kernel<<<(T + 127) / 128, 128, 0, s>>>(dweights, probs, idx, weights, dlogits, T, E);
+  launch_next(router_top2_bwd_kernel, (T + 127) / 128, 128, 0, s, dweights, probs, idx, weights, dlogits, T, E);
   return ok();
 }
 
 int b2_swiglu_bwd(const void* dh, const void* gate, const void* up, void* dgu, void* h, const int* live_rows, int rows,
                   int F, cudaStream_t s) {
   if (F % 8) return -10;
-  swiglu_bwd_kernel<<<grid_for(static_cast<size_t>(rows) * F / 8, 256), 256, 0, s>>>(
-      (const bf16*)dh, (const bf16*)gate, (const bf16*)up, (bf16*)dgu, (bf16*)h, live_rows, rows, F);
+  launch_next(swiglu_bwd_kernel, grid_for(static_cast<size_t>(rows) * F / 8, 256), 256, 0, s, (const bf16*)dh, (const bf16*)gate, (const bf16*)up, (bf16*)dgu, (bf16*)h, live_rows, rows, F);
   return ok();
 }
 
@@ -1393,7 +1414,7 @@ int b2_cross_entropy2(void* logits, const long long* targets, float* loss, int T
     const int grid = min(T, sm_count_ew() * 2);
     if (V <= CE_THREADS * 32) {
       auto kernel = V <= CE_THREADS * 16 ? cross_entropy_reg_kernel<2> : cross_entropy_reg_kernel<4>;
-      kernel<<<grid, CE_THREADS, 0, s>>>((bf16*)logits, targets, loss, T, V, loss_scale, grad_scale);
+      launch_next(kernel, grid, CE_THREADS, 0, s, (bf16*)logits, targets, loss, T, V, loss_scale, grad_scale);
       return ok();
     }
     static bool set = false;
@@ -1402,16 +1423,16 @@ int b2_cross_entropy2(void* logits, const long long* targets, float* loss, int T
         return -3;
       set = true;
     }
-    cross_entropy_bulk_kernel<<<grid, CE_THREADS, V * 2, s>>>((bf16*)logits, targets, loss, status, T, V, loss_scale,
+    launch_next(cross_entropy_bulk_kernel, grid, CE_THREADS, V * 2, s, (bf16*)logits, targets, loss, status, T, V, loss_scale,
                                                               grad_scale);
     return ok();
   }
-  cross_entropy_kernel<<<min(T, sm_count_ew() * 4), CE_THREADS, 0, s>>>((bf16*)logits, targets, loss, T, V, loss_scale);
+  launch_next(cross_entropy_kernel, min(T, sm_count_ew() * 4), CE_THREADS, 0, s, (bf16*)logits, targets, loss, T, V, loss_scale);
   return ok();
 }
 int b2_scale_bf16(void* x, const float* factor, long long n, cudaStream_t s) {
   if (n % 8) return -10;
-  scale_bf16_kernel<<<grid_for(n / 8, 256), 256, 0, s>>>((bf16*)x, factor, n / 8);
+  launch_next(scale_bf16_kernel, grid_for(n / 8, 256), 256, 0, s, (bf16*)x, factor, n / 8);
   return ok();
 }
 
@@ -1438,7 +1459,7 @@ int b2_adamw(const unsigned long long* ptrs, const long long* n, int count, int 
     table.first_chunk[table.count] = static_cast<int>(chunks);
     if (chunks == 0) continue;
     const int grid = static_cast<int>(min(chunks, static_cast<long long>(sm_count_ew()) * 16));
-#define B2_ADAMW(P, G, S) adamw_kernel<P, G, S><<<grid, 256, 0, s>>>(table, lr, beta1, beta2, eps, wd, a_t, grad_scale)
+#define B2_ADAMW(P, G, S) launch_next(adamw_kernel<P, G, S>, grid, 256, 0, s, table, lr, beta1, beta2, eps, wd, a_t, grad_scale)
     switch (code) {
       case 0: B2_ADAMW(float, float, float); break;
       case 1: B2_ADAMW(float, float, bf16); break;
@@ -1470,33 +1491,33 @@ int b2_zero(const unsigned long long* ptrs, const long long* bytes, int count, c
     }
     table.first_chunk[table.count] = static_cast<int>(chunks);
     if (chunks == 0) continue;
-    zero_kernel<<<static_cast<unsigned>(chunks), 256, 0, s>>>(table);
+    launch_next(zero_kernel, static_cast<unsigned>(chunks), 256, 0, s, table);
     if (ok()) return -1;
   }
   return 0;
 }
 int b2_cast_f32_bf16(const float* src, void* dst, long long n, cudaStream_t s) {
-  cast_f32_bf16_kernel<<<grid_for(n, 256, 32), 256, 0, s>>>(src, (bf16*)dst, n);
+  launch_next(cast_f32_bf16_kernel, grid_for(n, 256, 32), 256, 0, s, src, (bf16*)dst, n);
   return ok();
 }
 
 int b2_embedding_fwd(const long long* ids, const void* table, void* out, int T, int D, cudaStream_t s) {
   if (D % 8) return -10;
-  embedding_fwd_kernel<<<grid_for(static_cast<size_t>(T) * D / 8, 256), 256, 0, s>>>(ids, (const bf16*)table,
+  launch_next(embedding_fwd_kernel, grid_for(static_cast<size_t>(T) * D / 8, 256), 256, 0, s, ids, (const bf16*)table,
                                                                                     (bf16*)out, T, D);
   return ok();
 }
 int b2_embedding_bwd(const long long* ids, const void* dy, float* grad, int T, int D, cudaStream_t s) {
   if (D % 8) return -10;
   auto kernel = reinterpret_cast<uintptr_t>(grad) % 16 == 0 ? embedding_bwd_kernel<true> : embedding_bwd_kernel<false>;
-  kernel<<<grid_for(static_cast<size_t>(T) * D / 8, 256), 256, 0, s>>>(ids, (const bf16*)dy, grad, T, D);
+  launch_next(kernel, grid_for(static_cast<size_t>(T) * D / 8, 256), 256, 0, s, ids, (const bf16*)dy, grad, T, D);
   return ok();
 }
 
 int b2_rope(void* x, const float* cos_t, const float* sin_t, int tokens, int S, int H, int hd, long long pitch,
             float sign, cudaStream_t s) {
   if (hd % 8 || pitch % 8) return -10;
-  rope_kernel<<<grid_for(static_cast<size_t>(tokens) * H * hd / 8, 256), 256, 0, s>>>((bf16*)x, cos_t, sin_t, tokens, S,
+  launch_next(rope_kernel, grid_for(static_cast<size_t>(tokens) * H * hd / 8, 256), 256, 0, s, (bf16*)x, cos_t, sin_t, tokens, S,
                                                                                      H, hd, pitch, sign);
   return ok();
 }
@@ -1504,8 +1525,7 @@ int b2_rope(void* x, const float* cos_t, const float* sin_t, int tokens, int S, 
 int b2_rope_copy(const void* q, const void* k, void* q_out, void* k_out, const float* cos_t, const float* sin_t,
                  int tokens, int S, int Hq, int Hkv, long long q_pitch, long long k_pitch, cudaStream_t s) {
   if (q_pitch % 8 || k_pitch % 8 || S < 1) return -10;
-  rope_copy_kernel<<<grid_for(static_cast<size_t>(tokens) * (Hq + Hkv) * 16, 256), 256, 0, s>>>(
-      (const bf16*)q, (const bf16*)k, (bf16*)q_out, (bf16*)k_out, cos_t, sin_t, tokens, S, Hq, Hkv, q_pitch, k_pitch);
+  launch_next(rope_copy_kernel, grid_for(static_cast<size_t>(tokens) * (Hq + Hkv) * 16, 256), 256, 0, s, (const bf16*)q, (const bf16*)k, (bf16*)q_out, (bf16*)k_out, cos_t, sin_t, tokens, S, Hq, Hkv, q_pitch, k_pitch);
   return ok();
 }
 

@@ -17,6 +17,7 @@
 // of tile i overlaps the main loop of tile i+1.  Shared memory holds a 4-stage
 // ring of {A 128x64, B 256x64} bf16 tiles in the 128-byte-swizzled layout that
 // both TMA and the MMA descriptors understand.
+#include "chain.cuh"
 #include "peer.cuh"
 #include "ptx.cuh"
 #include "tensormap.cuh"
@@ -176,10 +177,6 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
   const uint32_t cta = PAIR ? cluster_ctarank() : 0;
   const int worker = PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
   const int num_workers = PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
-  const int m_tiles = p.num_m_tiles ? (*p.num_m_tiles + TM - 1) / TM : (p.M + TILE_M - 1) / TILE_M;
-  const int n_tiles = (p.N + NT - 1) / NT;
-  const long long total_tiles = static_cast<long long>(m_tiles) * n_tiles * (SCHED == SCHED_WGRAD ? p.num_experts : 1);
-
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full_bar[s], 1);
@@ -212,6 +209,10 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_begin();
+  const int m_tiles = p.num_m_tiles ? (*p.num_m_tiles + TM - 1) / TM : (p.M + TILE_M - 1) / TILE_M;
+  const int n_tiles = (p.N + NT - 1) / NT;
+  const long long total_tiles = static_cast<long long>(m_tiles) * n_tiles * (SCHED == SCHED_WGRAD ? p.num_experts : 1);
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (every CTA)
@@ -723,7 +724,8 @@ static int launch_mt(const GemmParams& p, int sms, cudaStream_t stream) {
                           (SCHED == SCHED_WGRAD ? p.num_experts : 1);
   // a CTA per tile where that is less than one per SM (the return of an expert group counts its CTAs: always all)
   const int grid = EPI != EPI_PUSH && tiles < sms ? static_cast<int>(tiles < 1 ? 1 : tiles) : sms;
-  kernel<<<grid, gemm_threads<EPI>(), smem, stream>>>(p);
+  if (EPI == EPI_PUSH) kernel<<<grid, gemm_threads<EPI>(), smem, stream>>>(p);
+  else launch_next(kernel, grid, gemm_threads<EPI>(), smem, stream, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
@@ -732,10 +734,12 @@ static int launch_mt(const GemmParams& p, int sms, cudaStream_t stream) {
 template <int A_MN, int B_MN, int EPI, int SCHED>
 static int pairs_resident(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int sms) {
   auto kernel = gemm_tcgen05_kernel<A_MN, B_MN, EPI, SCHED, 1, 1>;
-  attr->id = cudaLaunchAttributeClusterDimension;
-  attr->val.clusterDim.x = 2;
-  attr->val.clusterDim.y = 1;
-  attr->val.clusterDim.z = 1;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg->blockDim = dim3(gemm_threads<EPI>());
   cfg->dynamicSmemBytes = smem_bytes<EPI, 1, 1>();
   cfg->attrs = attr;
@@ -756,11 +760,12 @@ static int pairs_resident(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, in
 template <int A_MN, int B_MN, int EPI, int SCHED>
 static int launch_pair(const GemmParams& p, int sms, cudaStream_t stream) {
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr;
-  const int pairs = pairs_resident<A_MN, B_MN, EPI, SCHED>(&cfg, &attr, sms);
+  cudaLaunchAttribute attr[2];
+  const int pairs = pairs_resident<A_MN, B_MN, EPI, SCHED>(&cfg, attr, sms);
   if (pairs < 1) return -20;
   cfg.gridDim = dim3(2 * pairs);
   cfg.stream = stream;
+  cfg.numAttrs = EPI == EPI_PUSH ? 1 : 2;      // chain.cuh
   if (cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<A_MN, B_MN, EPI, SCHED, 1, 1>, p) != cudaSuccess) {
     cudaGetLastError();
     return -4;
@@ -827,8 +832,8 @@ static TileKind choose_tile(const GemmParams& p, int sms, bool pair_available) {
 template <int A_MN, int B_MN, int EPI, int SCHED>
 static bool pair_available(int sms) {
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr;
-  return pairs_resident<A_MN, B_MN, EPI, SCHED>(&cfg, &attr, sms) >= sms / 2 - 8;   // (nearly) every SM in a pair
+  cudaLaunchAttribute attr[2];
+  return pairs_resident<A_MN, B_MN, EPI, SCHED>(&cfg, attr, sms) >= sms / 2 - 8;   // (nearly) every SM in a pair
 }
 
 template <int A_MN, int B_MN, int EPI, int SCHED>

@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "chain.cuh"
 #include "debug.cuh"
 #include "ptx.cuh"
 
@@ -34,6 +35,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) moe_plan_kernel(const long long*
                                                                 int* __restrict__ offs, int* __restrict__ tile_expert,
                                                                 int* __restrict__ meta, int* __restrict__ counts_out,
                                                                 int capacity_rows) {
+  chain_begin();
   extern __shared__ int plan_smem[];
   constexpr int WARPS = PLAN_THREADS / 32, AHEAD = 8;
   int* const at = plan_smem;                  // [WARPS][E] counts, then the next row of each warp and expert
@@ -157,6 +159,7 @@ __global__ void __launch_bounds__(256) moe_gather_kernel(const __nv_bfloat16* __
                                                          float* __restrict__ dweights,
                                                          __nv_bfloat16* __restrict__ x_perm, int D, int capacity_rows,
                                                          int slots) {
+  chain_begin();
   const int live_rows = min(meta[1], capacity_rows);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int r = blockIdx.x * 8 + warp; r < live_rows; r += gridDim.x * 8) {
@@ -205,6 +208,7 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const __nv_bfloat16* _
                                                           const float* __restrict__ weights,
                                                           const __nv_bfloat16* __restrict__ residual,
                                                           __nv_bfloat16* __restrict__ out, int T, int D, int rows) {
+  chain_begin();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int t = blockIdx.x * 8 + warp; t < T; t += gridDim.x * 8) {
     const int r0 = slot_row[2 * t], r1 = slot_row[2 * t + 1];
@@ -244,6 +248,7 @@ __device__ __forceinline__ float aux_factor(int T, int E) {
 }
 __global__ void __launch_bounds__(1024) moe_aux_kernel(const float* __restrict__ probs, const int* __restrict__ counts,
                                                        float* __restrict__ aux, int T, int E) {
+  chain_begin();
   __shared__ float partial[32];
   float sum = 0.f;
   const long long total = static_cast<long long>(T) * E;
@@ -289,6 +294,7 @@ __global__ void __launch_bounds__(256) moe_dx_kernel(const __nv_bfloat16* __rest
                                                      const float* __restrict__ daux, const int* __restrict__ counts,
                                                      const __nv_bfloat16* __restrict__ w, float* __restrict__ dlogits,
                                                      __nv_bfloat16* __restrict__ dx, int T, int N, int D, int rows) {
+  chain_begin();
   extern __shared__ __nv_bfloat16 dx_ws[];
   __shared__ float grads[8][DX_TOKENS][NN];
   for (int i = threadIdx.x * 8; i < N * D; i += blockDim.x * 8)
@@ -404,17 +410,19 @@ int b2_moe_plan(const long long* idx, int slots, int E, int* slot_row, int* row_
   if (E < 1) return -10;
   if (E > 49) return -11;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = slots >= PLAN_CLUSTER_SLOTS ? 8 : 1;
-  attr.val.clusterDim.y = 1;
-  attr.val.clusterDim.z = 1;
-  cfg.gridDim = dim3(attr.val.clusterDim.x);
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = slots >= PLAN_CLUSTER_SLOTS ? 8 : 1;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(attr[1].val.clusterDim.x);
   cfg.blockDim = dim3(PLAN_THREADS);
   cfg.dynamicSmemBytes = static_cast<size_t>(E) * (PLAN_THREADS / 32) * 4 + (4 * E + 1) * 4;
   cfg.stream = s;
-  cfg.attrs = &attr;
-  cfg.numAttrs = slots >= PLAN_CLUSTER_SLOTS ? 1 : 0;
+  cfg.attrs = attr;
+  cfg.numAttrs = slots >= PLAN_CLUSTER_SLOTS ? 2 : 1;
   if (cudaLaunchKernelEx(&cfg, moe_plan_kernel, idx, slots, E, slot_row, row_slot, offs, tile_expert, meta, counts,
                          capacity_rows) != cudaSuccess) {
     cudaGetLastError();
@@ -426,7 +434,7 @@ int b2_moe_plan(const long long* idx, int slots, int E, int* slot_row, int* row_
 int b2_moe_gather(const void* x, const int* row_slot, const int* meta, const float* scale, const void* y_perm,
                   float* dweights, void* x_perm, int D, int capacity_rows, int slots, cudaStream_t s) {
   if (D % 8) return -10;
-  moe_gather_kernel<<<sm_count_moe() * 8, 256, 0, s>>>((const bf16*)x, row_slot, meta, scale, (const bf16*)y_perm, dweights,
+  launch_next(moe_gather_kernel, sm_count_moe() * 8, 256, 0, s, (const bf16*)x, row_slot, meta, scale, (const bf16*)y_perm, dweights,
                                             (bf16*)x_perm, D, capacity_rows, slots);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
@@ -434,7 +442,7 @@ int b2_moe_gather(const void* x, const int* row_slot, const int* meta, const flo
 int b2_moe_combine(const void* y_perm, const int* slot_row, const float* weights, const void* residual, void* out,
                    int T, int D, int rows, cudaStream_t s) {
   if (D % 8) return -10;
-  moe_combine_kernel<<<min((T + 7) / 8, sm_count_moe() * 8), 256, 0, s>>>((const bf16*)y_perm, slot_row, weights,
+  launch_next(moe_combine_kernel, min((T + 7) / 8, sm_count_moe() * 8), 256, 0, s, (const bf16*)y_perm, slot_row, weights,
                                                                (const bf16*)residual, (bf16*)out, T, D, rows);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
@@ -442,7 +450,7 @@ int b2_moe_combine(const void* y_perm, const int* slot_row, const float* weights
 // probs fp32 [T,E], counts int32 [E] -> aux, one fp32 value.
 int b2_moe_aux(const float* probs, const int* counts, float* aux, int T, int E, cudaStream_t s) {
   if (E < 1 || E > 1024) return -10;
-  moe_aux_kernel<<<1, 1024, 0, s>>>(probs, counts, aux, T, E);
+  launch_next(moe_aux_kernel, 1, 1024, 0, s, probs, counts, aux, T, E);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -460,7 +468,7 @@ int b2_moe_dx(const void* dy, const int* slot_row, const float* dweights, const 
     set = true;
   }
   auto kernel = N <= 8 ? moe_dx_kernel<8> : moe_dx_kernel<16>;
-  kernel<<<min((T + 31) / 32, sm_count_moe() * 2), 256, smem, s>>>((const bf16*)dy, slot_row, dweights, probs, idx, weights,
+  launch_next(kernel, min((T + 31) / 32, sm_count_moe() * 2), 256, smem, s, (const bf16*)dy, slot_row, dweights, probs, idx, weights,
                                                                    daux, counts, (const bf16*)w, dlogits, (bf16*)dx, T, N, D, rows);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

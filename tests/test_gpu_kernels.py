@@ -339,6 +339,53 @@ def test_rmsnorm_row_blocks(native, rows, D):
     native.check_status()
 
 
+@pytest.mark.parametrize("T,D", [(64, 128), (300, 512), (2048, 1024)])
+def test_launches_that_overlap_keep_their_order(native, T, D):
+    """Kernels are placed while the one before them still runs: reads and writes of shared buffers, one after the other,
+    replayed from a graph and on a second stream, give the bits of a run that waits for every kernel."""
+    ids = torch.randint(0, 50, (T,), device="cuda")
+    table, w, w2 = _rand(50, D), _rand(2 * D, D, scale=D ** -0.5), _rand(2 * D, D, scale=(2 * D) ** -0.5)
+    gain = torch.rand(D, device="cuda") + 0.5
+    x, y = _rand(T, D), torch.empty(T, D, device="cuda").bfloat16()
+    acc = torch.zeros(2 * D, D, device="cuda")
+
+    def run(wait):
+        wait()
+        native.zero_many_([acc])
+        wait()
+        cur = native.embedding_fwd(ids, table)
+        for _ in range(6):
+            wait()
+            summed, normed, rstd = native.add_rmsnorm_fwd(cur, x, gain, 1e-5)
+            wait()
+            up = native.gemm_nt(normed, w)
+            wait()
+            native.gemm_nn(up, w2, out=y)
+            wait()
+            native.gemm_tn(up, normed, out=acc, accumulate=True)
+            wait()
+            cur, dgain = native.rmsnorm_bwd(y, summed, gain, rstd)
+        wait()
+        return torch.cat((cur.float().flatten(), acc.flatten(), dgain))
+
+    want = run(torch.cuda.synchronize)
+    none = lambda: None  # noqa: E731
+    assert all(torch.equal(run(none), want) for _ in range(5))
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        other = run(none)
+    torch.cuda.current_stream().wait_stream(side)
+    assert torch.equal(other, want)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = run(none)
+    for _ in range(3):
+        graph.replay()
+        assert torch.equal(captured, want)
+    native.check_status()
+
+
 def test_router_linear_and_top2(native):
     from b200moe import ops
     from b200moe.ops import functional as Fn
