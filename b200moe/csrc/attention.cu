@@ -163,10 +163,10 @@ template <int N> __device__ __forceinline__ void reg_dec() { asm volatile("setma
 struct AttnWork {
   int tile, head;          // 0 = longest; flattened batch * heads + head
 };
-__device__ __forceinline__ AttnWork attn_work(const AttnParams& p, int tiles, int heads) {
+__device__ __forceinline__ AttnWork attn_work(const AttnParams& p, int tiles, int heads, int index) {
   const int per_set = p.set_heads * tiles;
-  const int set = static_cast<int>(blockIdx.x) / per_set;
-  const int rest = static_cast<int>(blockIdx.x) - set * per_set;
+  const int set = index / per_set;
+  const int rest = index - set * per_set;
   const int count = min(p.set_heads, heads - set * p.set_heads);
   return {rest / count, set * p.set_heads + rest % count};
 }
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(FWD_THREADS, 1) attn_fwd_kernel(const __grid_c
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kv_tiles = (p.S + TK - 1) / TK;
   const int pairs = (kv_tiles + 1) / 2;
-  const AttnWork work = attn_work(p, pairs, p.B * p.Hq);
+  const AttnWork work = attn_work(p, pairs, p.B * p.Hq, static_cast<int>(blockIdx.x));
   const int qt0 = 2 * (pairs - 1 - work.tile);
   const int b = work.head / p.Hq, h = work.head - b * p.Hq;
   const int hk = h / (p.Hq / p.Hkv);
@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_fwd_one_tile_kernel(cons
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kv_tiles = (p.S + TK - 1) / TK;
-  const AttnWork work = attn_work(p, kv_tiles, p.B * p.Hq);
+  const AttnWork work = attn_work(p, kv_tiles, p.B * p.Hq, static_cast<int>(blockIdx.x));
   const int qt = kv_tiles - 1 - work.tile;
   const int b = work.head / p.Hq, h = work.head - b * p.Hq;
   const int hk = h / (p.Hq / p.Hkv);
@@ -681,6 +681,21 @@ __global__ void __launch_bounds__(256) attn_stats_kernel(const __nv_bfloat16* __
   }
 }
 
+// 32 columns (chunk c) of a finished gradient row.
+__device__ __forceinline__ void store_grad_chunk(uint32_t (&a)[32], __nv_bfloat16* dst, int pos, float scale,
+                                                 const float* rope_cos, const float* rope_sin, int c) {
+#pragma unroll
+  for (int i = 0; i < 32; ++i) a[i] = __float_as_uint(__uint_as_float(a[i]) * scale);
+  if (rope_cos) unrotate32(a, rope_cos, rope_sin, pos, c * 16);
+  uint4* d4 = reinterpret_cast<uint4*>(dst + c * 32);
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    d4[i] = make_uint4(pack_bf16(__uint_as_float(a[8 * i]), __uint_as_float(a[8 * i + 1])),
+                       pack_bf16(__uint_as_float(a[8 * i + 2]), __uint_as_float(a[8 * i + 3])),
+                       pack_bf16(__uint_as_float(a[8 * i + 4]), __uint_as_float(a[8 * i + 5])),
+                       pack_bf16(__uint_as_float(a[8 * i + 6]), __uint_as_float(a[8 * i + 7])));
+}
+
 // A finished accumulator row of 128 fp32 columns: scaled, rotated back if tables are given, stored as bf16.  The whole
 // warp calls it (tcgen05.ld is a warp instruction); rows behind the sequence are not stored.  CHUNKS of 32 columns from
 // chunk ``first`` on.
@@ -692,18 +707,7 @@ __device__ __forceinline__ void store_grad_row(uint32_t taddr, __nv_bfloat16* ds
     uint32_t a[32];
     tmem_ld_32x32(taddr + c * 32, a);
     tmem_ld_wait();
-    if (pos < S) {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) a[i] = __float_as_uint(__uint_as_float(a[i]) * scale);
-      if (rope_cos) unrotate32(a, rope_cos, rope_sin, pos, c * 16);
-      uint4* d4 = reinterpret_cast<uint4*>(dst + c * 32);
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        d4[i] = make_uint4(pack_bf16(__uint_as_float(a[8 * i]), __uint_as_float(a[8 * i + 1])),
-                           pack_bf16(__uint_as_float(a[8 * i + 2]), __uint_as_float(a[8 * i + 3])),
-                           pack_bf16(__uint_as_float(a[8 * i + 4]), __uint_as_float(a[8 * i + 5])),
-                           pack_bf16(__uint_as_float(a[8 * i + 6]), __uint_as_float(a[8 * i + 7])));
-    }
+    if (pos < S) store_grad_chunk(a, dst, pos, scale, rope_cos, rope_sin, c);
     __syncwarp();
   }
 }
@@ -770,6 +774,56 @@ __device__ __forceinline__ void bwd_exit(BwdSmem& sm, int warp, uint32_t tmem) {
   }
 }
 
+// In grids that leave most SMs idle a cluster of CTAs shares the steps of one tile (launch_bwd): each sums its part in its own
+// tensor memory, each adds up an equal share of the rows, in the order of the parts, and stores it.  The parts meet in the
+// rings' shared memory once every CTA of the cluster has used its tiles.
+__device__ __forceinline__ int cluster_parts() {
+  uint32_t n;
+  asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(n));
+  return static_cast<int>(n);
+}
+// [first, first + count) of ``steps`` for this CTA of its cluster.
+__device__ __forceinline__ void my_steps(int steps, int parts, int& first, int& count) {
+  const int per = (steps + parts - 1) / parts, rank = static_cast<int>(cluster_ctarank());
+  first = min(steps, rank * per);
+  count = min(steps - first, per);
+}
+// 32 columns of a thread's accumulator row (or zeros) to the CTA that adds up this row: ``sums`` is there [parts][rows per
+// CTA][128] floats, 16-byte units swizzled by row.  Stores to the other CTAs' shared memory need no answer; reading the parts
+// from there instead takes a round trip per part.
+__device__ __forceinline__ void put_sums(float* sums, int parts, int row, int chunk, const uint32_t (&v)[32]) {
+  const int rows = 128 / parts, owner = row / rows;
+  const uint32_t dst = mapa_u32(smem_u32(sums + (static_cast<int>(cluster_ctarank()) * rows + row - owner * rows) * 128), owner);
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (((chunk * 8 + i) ^ (row & 7)) << 4)),
+                 "r"(v[4 * i]), "r"(v[4 * i + 1]), "r"(v[4 * i + 2]), "r"(v[4 * i + 3])
+                 : "memory");
+}
+// The sum of the parts for 32 columns of row ``mine`` of this CTA's share (row ``row`` of the tile).
+__device__ __forceinline__ void add_sums(const float* sums, int parts, int mine, int row, int chunk, uint32_t (&v)[32]) {
+  for (int part = 0; part < parts; ++part) {
+    const float4* const src = reinterpret_cast<const float4*>(sums + (part * (128 / parts) + mine) * 128);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float4 x = src[(chunk * 8 + i) ^ (row & 7)];
+      const float y[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[4 * i + k] = __float_as_uint(part == 0 ? y[k] : __uint_as_float(v[4 * i + k]) + y[k]);
+    }
+  }
+}
+// 32 columns of a warp's accumulator rows out of tensor memory, zeros where this CTA had no step.
+__device__ __forceinline__ void take_sums(uint32_t taddr, bool here, uint32_t (&v)[32]) {
+  if (here) {
+    tmem_ld_32x32(taddr, v);
+    tmem_ld_wait();
+  } else {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = 0;
+  }
+}
+
 // Slot and phase of step i in a ring of three.
 __device__ __forceinline__ int slot3(int i) { return i % 3; }
 __device__ __forceinline__ uint32_t phase3(int i) { return (i / 3) & 1; }
@@ -793,27 +847,29 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dkv_kernel(const __g
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q_tiles = (p.S + TQ - 1) / TQ;
-  const AttnWork work = attn_work(p, q_tiles, p.B * p.Hkv);
+  const int parts = cluster_parts();
+  const AttnWork work = attn_work(p, q_tiles, p.B * p.Hkv, static_cast<int>(blockIdx.x) / parts);
   const int kt = work.tile, b = work.head / p.Hkv, hk = work.head - b * p.Hkv;
   const int group = p.Hq / p.Hkv;
   const int q_first = p.causal ? kt : 0;           // causal: query tiles kt .. q_tiles-1
   const int per_head = q_tiles - q_first;
-  const int iters = group * per_head;
+  int it0, iters;                                  // this CTA's steps (query tiles of the group's heads)
+  my_steps(group * per_head, parts, it0, iters);
 
   bwd_init(sm, warp);
   const uint32_t tmem = sm.tmem_slot;
   const uint32_t t_st = tmem, t_dpt = tmem + 128, t_dv = tmem + 256, t_dk = tmem + 384;
 
   if (warp == 8) {
-    if (elect_one()) {
+    if (iters > 0 && elect_one()) {
       mbar_expect_tx(&bars->fixed_full, 2 * TILE_BYTES);
       load_tile(sm.fixed[0], &p.map_k, &bars->fixed_full, hk * HD, kt * TK, b);
       load_tile(sm.fixed[1], &p.map_v, &bars->fixed_full, hk * HD, kt * TK, b);
       int it = 0, a_ahead = 0;
       for (; it < iters && !*abort_flag; ++it) {
         const int s3 = slot3(it), s2 = it & 1;
-        const int hq = hk * group + it / per_head;
-        const int qi = q_first + it % per_head;
+        const int hq = hk * group + (it0 + it) / per_head;
+        const int qi = q_first + (it0 + it) % per_head;
         const float* stat = p.stats + (static_cast<size_t>(b) * p.Hq + hq) * 2 * q_tiles * TQ + qi * TQ;
         if (!mbar_wait(&bars->a_empty[s3], phase3(it) ^ 1)) { ATTN_FAIL(211); break; }
         mbar_expect_tx(&bars->a_full[s3], TILE_BYTES + TQ * 4);
@@ -831,7 +887,7 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dkv_kernel(const __g
       }
     }
   } else if (warp == 9) {
-    if (elect_one()) {
+    if (iters > 0 && elect_one()) {
       constexpr uint32_t idesc_kk = umma_idesc_bf16(128, HALF, 0, 0);  // both operands K-major
       constexpr uint32_t idesc_tn = umma_idesc_bf16(128, 128, 0, 1);   // A from TMEM, B MN-major
       const uint32_t k_addr = smem_u32(sm.fixed[0]), v_addr = smem_u32(sm.fixed[1]);
@@ -916,7 +972,7 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dkv_kernel(const __g
     const uint32_t ts = t_st + lane_base + col0, tp = t_dpt + lane_base + col0;
     const f32x2 scale2 = make_f32x2(p.scale_log2, p.scale_log2);
     for (int it = 0; it < iters && !*abort_flag; ++it) {
-      const int qi = q_first + it % per_head;
+      const int qi = q_first + (it0 + it) % per_head;
       const uint32_t ph = it & 1;
       // statistics of my 64 query columns: four columns per 16-byte broadcast read
       const float4* nlse = reinterpret_cast<const float4*>(sm.b_stat[it & 1] + col0);
@@ -978,14 +1034,43 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dkv_kernel(const __g
       arrive_half(&bars->ds_ready[half], lane);
     }
     // epilogue: group 0 stores dV, group 1 dK
-    if (!*abort_flag) {
-      if (!mbar_wait(&bars->acc_done, 0)) ATTN_FAIL(218);
+    if (!*abort_flag && iters > 0 && !mbar_wait(&bars->acc_done, 0)) ATTN_FAIL(218);
+    if (parts == 1 && !*abort_flag) {
       tc_fence_after();
       const int pos = kt * TK + r;
       const size_t token = static_cast<size_t>(b) * p.S + pos;
       __nv_bfloat16* dst = half ? p.dk + token * p.dk_pitch + hk * HD : p.dv + token * p.dv_pitch + hk * HD;
       store_grad_row(half ? t_dk + lane_base : t_dv + lane_base, dst, pos, p.S, half ? p.scale : 1.f,
                      half ? p.rope_cos : nullptr, p.rope_sin);
+    }
+  }
+  if (parts > 1) {
+    float* const sums = reinterpret_cast<float*>(sm.a);
+    __syncwarp();
+    cluster_sync_all();                            // every CTA of the cluster has used its tiles
+    if (warp < 8) {                                // group 0 hands over dV, group 1 dK
+      const int half = warp >> 2;
+      const bool here = __all_sync(0xffffffffu, iters > 0 && !*abort_flag);
+      tc_fence_after();
+#pragma unroll 1
+      for (int c = 0; c < 4; ++c) {
+        uint32_t v[32];
+        take_sums((half ? t_dk : t_dv) + (static_cast<uint32_t>((warp & 3) * 32) << 16) + c * 32, here, v);
+        put_sums(sums + half * 128 * 128, parts, (warp & 3) * 32 + lane, c, v);
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();
+    const int rows = TK / parts, first = static_cast<int>(cluster_ctarank()) * rows;
+#pragma unroll 1
+    for (int item = threadIdx.x; item < rows * 8; item += ATTN_THREADS) {
+      const int row = first + (item >> 3), which = (item >> 2) & 1, c = item & 3, pos = kt * TK + row;
+      if (pos >= p.S || *abort_flag) continue;
+      uint32_t v[32];
+      add_sums(sums + which * 128 * 128, parts, item >> 3, row, c, v);
+      const size_t token = static_cast<size_t>(b) * p.S + pos;
+      store_grad_chunk(v, which ? p.dk + token * p.dk_pitch + hk * HD : p.dv + token * p.dv_pitch + hk * HD, pos,
+                       which ? p.scale : 1.f, which ? p.rope_cos : nullptr, p.rope_sin, c);
     }
   }
   bwd_exit(sm, warp, tmem);
@@ -1004,18 +1089,20 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dq_kernel(const __gr
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int q_tiles = (p.S + TQ - 1) / TQ;
-  const AttnWork work = attn_work(p, q_tiles, p.B * p.Hq);
+  const int parts = cluster_parts();
+  const AttnWork work = attn_work(p, q_tiles, p.B * p.Hq, static_cast<int>(blockIdx.x) / parts);
   const int qt = q_tiles - 1 - work.tile;
   const int b = work.head / p.Hq, h = work.head - b * p.Hq;
   const int hk = h / (p.Hq / p.Hkv);
-  const int n_kv = p.causal ? qt + 1 : q_tiles;
+  int j0, n_kv;                                    // this CTA's key tiles
+  my_steps(p.causal ? qt + 1 : q_tiles, parts, j0, n_kv);
 
   bwd_init(sm, warp);
   const uint32_t tmem = sm.tmem_slot;
   const uint32_t t_s = tmem, t_dp = tmem + 128, t_dq = tmem + 256, t_q = tmem + 384, t_do = tmem + 448;
 
   if (warp == 8) {
-    if (elect_one()) {
+    if (n_kv > 0 && elect_one()) {
       mbar_expect_tx(&bars->fixed_full, 2 * TILE_BYTES);
       load_tile(sm.fixed[0], &p.map_q, &bars->fixed_full, h * HD, qt * TQ, b);
       load_tile(sm.fixed[1], &p.map_do, &bars->fixed_full, h * HD, qt * TQ, b);
@@ -1024,10 +1111,10 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dq_kernel(const __gr
         const int s3 = slot3(j), s2 = j & 1;
         if (!mbar_wait(&bars->a_empty[s3], phase3(j) ^ 1)) { ATTN_FAIL(221); break; }
         mbar_expect_tx(&bars->a_full[s3], TILE_BYTES);
-        load_tile(sm.a[s3], &p.map_k, &bars->a_full[s3], hk * HD, j * TK, b);
+        load_tile(sm.a[s3], &p.map_k, &bars->a_full[s3], hk * HD, (j0 + j) * TK, b);
         if (!mbar_wait(&bars->b_empty[s2], ((j >> 1) & 1) ^ 1)) { ATTN_FAIL(222); a_ahead = 1; break; }
         mbar_expect_tx(&bars->b_full[s2], TILE_BYTES);
-        load_tile(sm.b[s2], &p.map_v, &bars->b_full[s2], hk * HD, j * TK, b);
+        load_tile(sm.b[s2], &p.map_v, &bars->b_full[s2], hk * HD, (j0 + j) * TK, b);
       }
       if (*abort_flag) {
         mbar_wait(&bars->fixed_full, 0);
@@ -1036,7 +1123,7 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dq_kernel(const __gr
       }
     }
   } else if (warp == 9) {
-    if (elect_one()) {
+    if (n_kv > 0 && elect_one()) {
       constexpr uint32_t idesc_kk = umma_idesc_bf16(128, HALF, 0, 0);
       constexpr uint32_t idesc_tn = umma_idesc_bf16(128, 128, 0, 1);
       auto issue_s = [&](int j, int g) {           // S[q, key half] = Q K^T
@@ -1120,8 +1207,8 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dq_kernel(const __gr
     // dO, a row per thread (16-byte units of the 128-byte-swizzled tile).  From shared memory they were read again for every
     // 64 keys, and the products with N = 64 waited for it (6 KiB per 32 cycles): 32/8 heads of 8192 tokens, causal, backward
     // pass as a whole 1609 -> 1546 us, 128 heads of 640 tokens, every key, 158 -> 153.
-    if (!mbar_wait(&bars->fixed_full, 0)) ATTN_FAIL(224);
-    if (!*abort_flag) {
+    if (n_kv > 0 && !mbar_wait(&bars->fixed_full, 0)) ATTN_FAIL(224);
+    if (n_kv > 0 && !*abort_flag) {
       const uint8_t* row = sm.fixed[half] + r * 128;
 #pragma unroll
       for (int atom = 0; atom < 2; ++atom) {
@@ -1153,9 +1240,9 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dq_kernel(const __gr
         pf[i] = make_f32x2(ex2(e0), ex2(e1));
       }
       // keys that the row does not see: after the query (causal, diagonal tile) or behind the sequence
-      const bool diagonal = p.causal && j == qt;
-      if (diagonal || (j + 1) * TK > p.S) {
-        const int limit = (diagonal ? r + 1 : p.S - j * TK) - col0;
+      const bool diagonal = p.causal && j0 + j == qt;
+      if (diagonal || (j0 + j + 1) * TK > p.S) {
+        const int limit = (diagonal ? r + 1 : p.S - (j0 + j) * TK) - col0;
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
           float e0, e1;
@@ -1179,12 +1266,40 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dq_kernel(const __gr
       tmem_st_wait();
       arrive_half(&bars->ds_ready[half], lane);
     }
-    if (!*abort_flag) {                   // each group stores 64 of the 128 columns
-      if (!mbar_wait(&bars->acc_done, 0)) ATTN_FAIL(227);
+    if (!*abort_flag && n_kv > 0 && !mbar_wait(&bars->acc_done, 0)) ATTN_FAIL(227);
+    if (parts == 1 && !*abort_flag) {     // each group stores 64 of the 128 columns
       tc_fence_after();
       const int pos = qt * TQ + r;
       store_grad_row<2>(t_dq + lane_base, p.dq + (static_cast<size_t>(b) * p.S + pos) * p.dq_pitch + h * HD, pos, p.S,
                         p.scale, p.rope_cos, p.rope_sin, 2 * half);
+    }
+  }
+  if (parts > 1) {
+    float* const sums = reinterpret_cast<float*>(sm.a);
+    __syncwarp();
+    cluster_sync_all();
+    if (warp < 8) {                                // each group hands over 64 columns
+      const int half = warp >> 2;
+      const bool here = __all_sync(0xffffffffu, n_kv > 0 && !*abort_flag);
+      tc_fence_after();
+#pragma unroll 1
+      for (int c = 2 * half; c < 2 * half + 2; ++c) {
+        uint32_t v[32];
+        take_sums(t_dq + (static_cast<uint32_t>((warp & 3) * 32) << 16) + c * 32, here, v);
+        put_sums(sums, parts, (warp & 3) * 32 + lane, c, v);
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();
+    const int rows = TQ / parts, first = static_cast<int>(cluster_ctarank()) * rows;
+#pragma unroll 1
+    for (int item = threadIdx.x; item < rows * 4; item += ATTN_THREADS) {
+      const int row = first + (item >> 2), c = item & 3, pos = qt * TQ + row;
+      if (pos >= p.S || *abort_flag) continue;
+      uint32_t v[32];
+      add_sums(sums, parts, item >> 2, row, c, v);
+      store_grad_chunk(v, p.dq + (static_cast<size_t>(b) * p.S + pos) * p.dq_pitch + h * HD, pos, p.scale, p.rope_cos,
+                       p.rope_sin, c);
     }
   }
   bwd_exit(sm, warp, tmem);
@@ -1231,6 +1346,32 @@ static int sm_count_attn() {
       sms = 0;
   }
   return sms > 0 ? sms : 148;
+}
+
+// A backward kernel over ``tiles`` tiles of at most ``steps`` steps each.  Where the CTAs of several parts per tile still make
+// one wave, two share the steps from five on and four from eight on: below, the two barriers and the exchange cost what a step or
+// two saves; eight parts gain nothing more.  us, whole backward pass, one -> several parts, causal: 2 x 512 tokens, 4/1 heads
+// 45.8 -> 34.0; 1024, 8/2 73.3 -> 41.2; 2048, 8/2 130 -> 68.7; 4 x 1024, 8/2 88.8 -> 70.6; 128, 8/2 (one part) 26.1.
+static int launch_bwd(void (*kernel)(AttnParams), long long tiles, long long steps, const AttnParams& p, cudaStream_t stream) {
+  const int sms = sm_count_attn();
+  int parts = 1;
+  if (steps >= 5 && tiles * 2 <= sms) parts = 2;
+  if (steps >= 8 && tiles * 4 <= sms) parts = 4;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // chain.cuh
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = parts;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.gridDim = dim3(static_cast<unsigned>(tiles * parts));
+  cfg.blockDim = dim3(ATTN_THREADS);
+  cfg.dynamicSmemBytes = BWD_SMEM;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = parts > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, p) == cudaSuccess ? 0 : -4;
 }
 
 template <void (*kernel)(AttnParams), int smem, int threads = ATTN_THREADS>
@@ -1315,9 +1456,9 @@ int b2_attention_bwd_rope(const void* dout, const void* q, const void* k, const 
   launch_next(attn_stats_kernel, static_cast<unsigned>(Sp / 16 * B * Hq), 256, 0, stream, static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(out), lse, stats, S,
       static_cast<int>(Sp), Hq);
   p.set_heads = heads_per_set(B * Hkv, 4LL * S * HD * (Hq / Hkv));
-  launch_next(attn_bwd_dkv_kernel, static_cast<unsigned>(tiles * B * Hkv), ATTN_THREADS, BWD_SMEM, stream, p);
+  if (launch_bwd(attn_bwd_dkv_kernel, tiles * B * Hkv, tiles * (Hq / Hkv), p, stream)) return -4;
   p.set_heads = heads_per_set(B * Hq, 4LL * S * HD * Hkv / Hq);
-  launch_next(attn_bwd_dq_kernel, static_cast<unsigned>(tiles * B * Hq), ATTN_THREADS, BWD_SMEM, stream, p);
+  if (launch_bwd(attn_bwd_dq_kernel, tiles * B * Hq, tiles, p, stream)) return -4;
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 

@@ -998,6 +998,29 @@ def test_flash_attention_in_fp16_keeps_fp16_precision(native, S, causal):
     native.check_status()
 
 
+@pytest.mark.parametrize("B,S,Hq,Hkv,causal", [(1, 640, 4, 4, False), (1, 640, 2, 2, True), (2, 1024, 4, 1, True),
+                                               (1, 1100, 8, 2, True), (1, 1025, 2, 2, False)])
+def test_attention_backward_shared_by_a_cluster(native, B, S, Hq, Hkv, causal):
+    """Tiles whose steps two or four CTAs share: uneven parts, CTAs without a step, a ragged last tile."""
+    q, k, v, dy = (_rand(B, S, h, 128) for h in (Hq, Hkv, Hkv, Hq))
+    out, lse, _, _ = native.attention_fwd(q, k, v, causal=causal)
+    got = native.attention_bwd(dy, q, k, v, out, lse, causal=causal)
+    again = native.attention_bwd(dy, q, k, v, out, lse, causal=causal)
+    leaves = [t.double().requires_grad_(True) for t in (q, k, v)]
+    qh, kh, vh = (t.transpose(1, 2) for t in leaves)
+    kh, vh = (t.repeat_interleave(Hq // Hkv, 1) for t in (kh, vh))
+    scores = qh @ kh.mT * 128 ** -0.5
+    if causal:
+        scores = scores.masked_fill(torch.ones(S, S, dtype=torch.bool, device="cuda").triu(1), -math.inf)
+    want = torch.autograd.grad((scores.softmax(-1) @ vh).transpose(1, 2), leaves, dy.double())
+    for a, b, c in zip(got, again, want):
+        assert torch.equal(a, b) and _rel(a, c) < 1e-2
+        # P and dS are rounded to bf16 (2^-9 each), the row statistic comes from a rounded output
+        rows = (a.double() - c).norm(dim=-1) / (c.norm(dim=-1) + c.norm(dim=-1).mean())
+        assert float(rows.max()) < 3e-2
+    native.check_status()
+
+
 def test_flash_attention_forward_entry(native):
     """``[B, H, S, 128]`` forward-only entry point, fp16 in and out, against an fp32 softmax(QK^T)V."""
     from b200moe.ops.attention import flash_attention_forward
