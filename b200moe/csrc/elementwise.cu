@@ -743,9 +743,17 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dh, const __
 // ------------------------------------------------------------------ cross entropy (in place)
 // logits[t,:] <- (softmax(logits[t,:]) - onehot(target)) * scale ; loss += (lse - logit[target]) * scale
 constexpr int CE_THREADS = 512;
+
+// A CTA's part of the loss, from one thread.  ``wide``: the sum is a double, so that it does not depend on the order of the
+// CTAs as far as fp32 can tell (hundreds of fp32 additions in the order of their arrival are off by 1e-7 from run to run).
+__device__ __forceinline__ void add_loss(void* loss, int wide, double value) {
+  if (wide) atomicAdd(static_cast<double*>(loss), value);
+  else atomicAdd(static_cast<float*>(loss), static_cast<float>(value));
+}
 __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16* __restrict__ logits,
                                                                   const long long* __restrict__ targets,
-                                                                  float* __restrict__ loss, int T, int V, float scale) {
+                                                                  void* __restrict__ loss, int wide, int T, int V,
+                                                                  float scale) {
   chain_begin();
   __shared__ float scratch[CE_THREADS / 32];
   for (int t = blockIdx.x; t < T; t += gridDim.x) {
@@ -770,7 +778,7 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_kernel(__nv_bfloat16
     const int target = static_cast<int>(targets[t]);
     if (threadIdx.x == 0) {
       const float picked = __bfloat162float(row[target]);
-      atomicAdd(loss, (logf(sum) + mx - picked) * scale);
+      add_loss(loss, wide, (logf(sum) + mx - picked) * scale);
     }
     __syncthreads();
     for (int c = threadIdx.x * 8; c < V; c += CE_THREADS * 8) {
@@ -799,10 +807,10 @@ constexpr int CE_REG_CHUNKS = 8;
 template <int CHUNKS>
 __global__ void __launch_bounds__(CE_THREADS, 2)
     cross_entropy_reg_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets,
-                             float* __restrict__ loss, int T, int V, float loss_scale, float grad_scale) {
+                             void* __restrict__ loss, int wide, int T, int V, float loss_scale, float grad_scale) {
   chain_begin();
   __shared__ float scratch[CE_THREADS / 32];
-  float local_loss = 0.f;
+  double local_loss = 0.;
   bf16x8 raw[CHUNKS];
   if (blockIdx.x < T) {
     const __nv_bfloat16* row = logits + static_cast<size_t>(blockIdx.x) * V;
@@ -865,7 +873,7 @@ __global__ void __launch_bounds__(CE_THREADS, 2)
       }
     }
   }
-  if (threadIdx.x == 0 && local_loss != 0.f) atomicAdd(loss, local_loss);   // one atomic per CTA
+  if (threadIdx.x == 0 && local_loss != 0.) add_loss(loss, wide, local_loss);   // one atomic per CTA
 }
 
 // Rows up to 32768 entries: the registers of two CTAs hold the packed rows, not their exponentials in fp32 (formed twice;
@@ -873,8 +881,8 @@ __global__ void __launch_bounds__(CE_THREADS, 2)
 // in shared memory by one bulk copy while the present one is worked on: 165 -> 124 us, 16384 rows 628 -> 467 us.
 __global__ void __launch_bounds__(CE_THREADS, 2)
     cross_entropy_bulk_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets,
-                              float* __restrict__ loss, int* __restrict__ status, int T, int V, float loss_scale,
-                              float grad_scale) {
+                              void* __restrict__ loss, int wide, int* __restrict__ status, int T, int V,
+                              float loss_scale, float grad_scale) {
   chain_begin();
   extern __shared__ __align__(128) uint8_t ce_row[];
   __shared__ float scratch[CE_THREADS / 32];
@@ -889,7 +897,7 @@ __global__ void __launch_bounds__(CE_THREADS, 2)
     }
   }
   __syncthreads();
-  float local_loss = 0.f;
+  double local_loss = 0.;
   uint32_t phase = 0;
   for (int t = blockIdx.x; t < T; t += gridDim.x) {
     __nv_bfloat16* row = logits + static_cast<size_t>(t) * V;
@@ -959,7 +967,7 @@ __global__ void __launch_bounds__(CE_THREADS, 2)
       }
     }
   }
-  if (threadIdx.x == 0 && local_loss != 0.f) atomicAdd(loss, local_loss);   // one atomic per CTA
+  if (threadIdx.x == 0 && local_loss != 0.) add_loss(loss, wide, local_loss);   // one atomic per CTA
 }
 
 __global__ void scale_bf16_kernel(__nv_bfloat16* __restrict__ x, const float* __restrict__ factor, size_t n8) {
@@ -1403,9 +1411,9 @@ int b2_swiglu_bwd(const void* dh, const void* gate, const void* up, void* dgu, v
   return ok();
 }
 
-// ``loss`` (zeroed by the caller) += loss_scale * sum of the rows' losses, logits <- grad_scale * gradient; rows up to
-// 32768 entries are read once and written once.
-int b2_cross_entropy2(void* logits, const long long* targets, float* loss, int T, int V, float loss_scale,
+// ``loss`` (zeroed by the caller; fp32, or a double where ``wide``) += loss_scale * sum of the rows' losses, logits <-
+// grad_scale * gradient; rows up to 32768 entries are read once and written once.
+int b2_cross_entropy2(void* logits, const long long* targets, void* loss, int wide, int T, int V, float loss_scale,
                       float grad_scale, int* status, cudaStream_t s) {
   if (V % 8) return -10;
   if (V > CE_THREADS * 8 * CE_REG_CHUNKS && loss_scale != grad_scale) return -11;   // the streaming kernel has one scale
@@ -1414,7 +1422,7 @@ int b2_cross_entropy2(void* logits, const long long* targets, float* loss, int T
     const int grid = min(T, sm_count_ew() * 2);
     if (V <= CE_THREADS * 32) {
       auto kernel = V <= CE_THREADS * 16 ? cross_entropy_reg_kernel<2> : cross_entropy_reg_kernel<4>;
-      launch_next(kernel, grid, CE_THREADS, 0, s, (bf16*)logits, targets, loss, T, V, loss_scale, grad_scale);
+      launch_next(kernel, grid, CE_THREADS, 0, s, (bf16*)logits, targets, loss, wide, T, V, loss_scale, grad_scale);
       return ok();
     }
     static bool set = false;
@@ -1423,11 +1431,11 @@ int b2_cross_entropy2(void* logits, const long long* targets, float* loss, int T
         return -3;
       set = true;
     }
-    launch_next(cross_entropy_bulk_kernel, grid, CE_THREADS, V * 2, s, (bf16*)logits, targets, loss, status, T, V, loss_scale,
+    launch_next(cross_entropy_bulk_kernel, grid, CE_THREADS, V * 2, s, (bf16*)logits, targets, loss, wide, status, T, V, loss_scale,
                                                               grad_scale);
     return ok();
   }
-  launch_next(cross_entropy_kernel, min(T, sm_count_ew() * 4), CE_THREADS, 0, s, (bf16*)logits, targets, loss, T, V, loss_scale);
+  launch_next(cross_entropy_kernel, min(T, sm_count_ew() * 4), CE_THREADS, 0, s, (bf16*)logits, targets, loss, wide, T, V, loss_scale);
   return ok();
 }
 int b2_scale_bf16(void* x, const float* factor, long long n, cudaStream_t s) {

@@ -41,8 +41,8 @@ int b2_attention_bwd_rope(const void* dout, const void* q, const void* k, const 
                           long long q_pitch, long long k_pitch, long long v_pitch, float* stats, void* dq, void* dk, void* dv,
                           long long dq_pitch, long long dk_pitch, long long dv_pitch, int B, int S, int Hq, int Hkv, float scale,
                           int causal, const float* rope_cos, const float* rope_sin, int* status, cudaStream_t stream);
-int b2_cross_entropy2(void* logits, const long long* targets, float* loss, int T, int V, float loss_scale, float grad_scale,
-                      int* status, cudaStream_t s);
+int b2_cross_entropy2(void* logits, const long long* targets, void* loss, int wide, int T, int V, float loss_scale,
+                      float grad_scale, int* status, cudaStream_t s);
 int b2_router_fwd(const void* x, const void* w, float* weights, long long* idx, float* probs, int T, int N, int K, cudaStream_t s);
 int b2_skinny_tn(const float* dy, const void* x, float* dw, int T, int N, int K, cudaStream_t s);
 int b2_moe_plan(const long long* idx, int slots, int E, int* slot_row, int* row_slot, int* offs, int* tile_expert, int* meta,
@@ -145,13 +145,13 @@ int b2_moe_layer_fwd(const void* x, const void* router, const void* w1, const vo
 // b200moe.ops.native.gemm_nn_swiglu_bwd, which has the figures).
 int b2_swiglu_bwd_in_product(long long M, int F, int K) { return K >= 2048 || M * F <= 1 << 21; }
 
-// One chunk of tokens through the LM head: logits = hidden W^T become their own gradient (and the loss is added to ``loss``),
+// One chunk of tokens through the LM head: logits = hidden W^T become their own gradient (and the loss is added to the double ``loss``),
 // dh = dlogits W, grad (fp32) += dlogits^T hidden.
-int b2_head_chunk(const void* hidden, const void* weight, const long long* targets, void* logits, float* loss, void* dh,
+int b2_head_chunk(const void* hidden, const void* weight, const long long* targets, void* logits, double* loss, void* dh,
                   float* grad, int T, int V, int D, float loss_scale, float grad_scale, int* status, cudaStream_t s) {
   Sequence run;
   run([&] { return b2_gemm_nt(hidden, weight, logits, T, V, D, D, D, V, 1, nullptr, nullptr, 0, 0, status, s); });
-  run([&] { return b2_cross_entropy2(logits, targets, loss, T, V, loss_scale, grad_scale, status, s); });
+  run([&] { return b2_cross_entropy2(logits, targets, loss, 1, T, V, loss_scale, grad_scale, status, s); });
   run([&] { return b2_gemm_nn(logits, weight, nullptr, dh, T, D, V, 0, V, D, D, 1, nullptr, nullptr, 0, nullptr, status, s); });
   run([&] { return b2_gemm_tn(logits, hidden, grad, nullptr, 0, V, D, T, V, D, D, 1, nullptr, nullptr, 1, 1.f, nullptr, status, s); });
   return run.rc;

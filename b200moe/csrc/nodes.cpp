@@ -258,7 +258,7 @@ struct Head : public Function<Head> {
   static Tensor forward(AutogradContext* ctx, const Tensor& hidden, const Tensor& weight, const Tensor& targets, const Tensor& grad,
                         double scale, int64_t chunk, const Tensor& status) {
     const int64_t V = weight.size(0), D = weight.size(1), T = hidden.numel() / D;
-    Tensor loss = at::zeros({}, hidden.options().dtype(at::kFloat)), dh = at::empty_like(hidden);
+    Tensor loss = at::zeros({}, hidden.options().dtype(at::kDouble)), dh = at::empty_like(hidden);
     for (int64_t lo = 0; lo < T; lo += chunk) {
       const int64_t n = std::min(chunk, T - lo);
       Tensor logits = bf16({n, V}, hidden);
@@ -269,7 +269,7 @@ struct Head : public Function<Head> {
     }
     ctx->save_for_backward({dh});
     ctx->saved_data["scale"] = scale;
-    return loss;
+    return loss.to(at::kFloat);
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const Tensor dh = ctx->get_saved_variables()[0];

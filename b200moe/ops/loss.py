@@ -53,7 +53,7 @@ class _LMHeadCE(torch.autograd.Function):
         tokens = h2d.shape[0]
         main_grad = getattr(weight, "main_grad", None)
         eager = wants_grad and grad_scale is not None and main_grad is not None and ctx.needs_input_grad[0]
-        loss = torch.zeros((), dtype=torch.float32, device=hidden.device)
+        loss = torch.zeros((), dtype=torch.float64, device=hidden.device)
         ctx.weight, ctx.shape, ctx.eager, ctx.grad_scale = weight, hidden.shape, eager, grad_scale
         ctx.kept = _kept_tokens(tokens, weight.shape[0]) if wants_grad and not eager else 0
         kept = None
@@ -72,7 +72,7 @@ class _LMHeadCE(torch.autograd.Function):
             ctx.save_for_backward(dh)
         else:
             ctx.save_for_backward(h2d, flat_targets, kept)
-        return loss
+        return loss.float()
 
     @staticmethod
     def backward(ctx, dloss):

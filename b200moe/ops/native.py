@@ -481,11 +481,11 @@ def router_fwd(x, w):
 
 # ------------------------------------------------------------------------------ loss
 def cross_entropy_scaled_(logits, targets, loss, loss_scale: float, grad_scale: float):
-    """Adds ``loss_scale · Σ_rows CE`` to ``loss`` (fp32 scalar tensor) and overwrites ``logits`` (bf16 [T,V]) with
+    """Adds ``loss_scale · Σ_rows CE`` to ``loss`` (fp32 or fp64 scalar tensor) and overwrites ``logits`` (bf16 [T,V]) with
     ``grad_scale · (softmax − onehot)``; rows up to 32768 entries are read once and written once."""
     T, V = logits.shape
-    _call("b2_cross_entropy2", _p(_bf16(logits)), _p(targets.contiguous()), _p(loss), _I(T), _I(V), _F(loss_scale),
-          _F(grad_scale), _p(status_word(logits.device)), _stream())
+    _call("b2_cross_entropy2", _p(_bf16(logits)), _p(targets.contiguous()), _p(loss), _I(int(loss.dtype == torch.float64)), _I(T),
+          _I(V), _F(loss_scale), _F(grad_scale), _p(status_word(logits.device)), _stream())
     return loss
 
 

@@ -497,6 +497,21 @@ def test_cross_entropy_row_sizes(native, T, V):
     native.check_status()
 
 
+@pytest.mark.parametrize("V", [2048, 32000, 33000])
+def test_loss_does_not_depend_on_the_order_of_the_ctas(native, V):
+    T = 1500
+    logits, targets = _rand(T, V), torch.randint(0, V, (T,), device="cuda")
+    want = torch.nn.functional.cross_entropy(logits.double(), targets)
+    got = set()
+    for _ in range(5):
+        loss = torch.zeros((), dtype=torch.float64, device="cuda")
+        native.cross_entropy_scaled_(logits.clone(), targets, loss, 1.0 / T, 1.0 / T)
+        got.add(float(loss.float()))
+    # rows: an fp32 sum of V exponentials, a logarithm and two additions, each good to a few 2^-24 of the row's loss
+    assert len(got) == 1 and abs(got.pop() - float(want)) < 2e-6 * float(want)
+    native.check_status()
+
+
 def test_cross_entropy_and_lm_head(native):
     from b200moe import ops
     T, D, V = 512, 256, 32000
