@@ -37,13 +37,14 @@ def _sources():
     return sorted(f for f in os.listdir(SRC) if f.endswith(".cu"))
 
 
-def _digest(path: str) -> str:
+def _digest(path: str, flags=tuple(NVCC_FLAGS)) -> str:
+    """Of a source, the headers and what it is compiled with."""
     h = hashlib.sha256()
     for name in sorted(os.listdir(SRC)):
         if name.endswith((".cuh", ".h")) or os.path.join(SRC, name) == path:
             with open(os.path.join(SRC, name), "rb") as f:
                 h.update(f.read())
-    h.update(" ".join(NVCC_FLAGS).encode())
+    h.update(" ".join(flags).encode())
     return h.hexdigest()
 
 
@@ -71,7 +72,8 @@ def _compile(name: str, verbose: bool) -> str:
 
 def _build_nodes(verbose: bool) -> None:
     """The C++ autograd nodes (csrc/nodes.cpp), compiled against the installed PyTorch; one file for both libraries, which
-    it binds to at run time.  Skipped where PyTorch is not there (the package's Python nodes do without)."""
+    it binds to at run time.  The package does without (the nodes in Python issue the same launches): skipped where PyTorch
+    is not there; where they cannot be built this says so, leaves none of an earlier build and raises nothing."""
     try:
         import torch
         from torch.utils import cpp_extension
@@ -79,25 +81,31 @@ def _build_nodes(verbose: bool) -> None:
         if verbose:
             print("[b200moe.build] no PyTorch here: C++ autograd nodes not built")
         return
-    import sysconfig
-    source, target = os.path.join(SRC, "nodes.cpp"), os.path.join(HERE, "_C", "b200moe_nodes.so")
-    with open(source, "rb") as f:
-        digest = hashlib.sha256(f.read() + torch.__version__.encode() + sys.version.encode()).hexdigest()
+    target = os.path.join(HERE, "_C", "b200moe_nodes.so")
     stamp = target + ".sha"
-    if os.path.exists(target) and os.path.exists(stamp) and open(stamp).read() == digest:
+    try:
+        source = os.path.join(SRC, "nodes.cpp")
+        digest = _digest(source, [torch.__version__, sys.version])
+        if os.path.exists(target) and os.path.exists(stamp) and open(stamp).read() == digest:
+            return
+        import sysconfig
+        lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+        cuda = os.path.dirname(os.path.dirname(nvcc()))
+        include = [*cpp_extension.include_paths(), os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+        os.makedirs(os.path.dirname(target), exist_ok=True)
+        cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_API_INCLUDE_EXTENSION_H",
+               "-DTORCH_EXTENSION_NAME=b200moe_nodes", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+               *(f"-I{path}" for path in include), source, "-o", target, f"-L{lib}", "-lc10", "-lc10_cuda", "-ltorch",
+               "-ltorch_cpu", "-ltorch_python", "-ldl"]
+        proc = subprocess.run(cmd, capture_output=True, text=True)
+        if proc.returncode:
+            raise RuntimeError(f"g++ failed for nodes.cpp\n{proc.stdout}{proc.stderr}")
+    except Exception as error:
+        for stale in (target, stamp):
+            if os.path.exists(stale):
+                os.unlink(stale)
+        sys.stderr.write(f"[b200moe.build] C++ autograd nodes not built, the nodes in Python stand for them: {error}\n")
         return
-    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
-    cuda = os.path.dirname(os.path.dirname(nvcc()))
-    include = [*cpp_extension.include_paths(), os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
-    os.makedirs(os.path.dirname(target), exist_ok=True)
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_API_INCLUDE_EXTENSION_H",
-           "-DTORCH_EXTENSION_NAME=b200moe_nodes", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-           *(f"-I{path}" for path in include), source, "-o", target, f"-L{lib}", "-lc10", "-lc10_cuda", "-ltorch",
-           "-ltorch_cpu", "-ltorch_python", "-ldl"]
-    proc = subprocess.run(cmd, capture_output=True, text=True)
-    if proc.returncode:
-        sys.stderr.write(proc.stdout + proc.stderr)
-        raise RuntimeError("g++ failed for nodes.cpp")
     with open(stamp, "w") as f:
         f.write(digest)
     if verbose:

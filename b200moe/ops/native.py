@@ -98,27 +98,37 @@ def _stream():
     return ctypes.c_void_p(_raw_stream(_raw_device()))
 
 
-_nodes = None        # the C++ autograd nodes (csrc/nodes.cpp), False where they were not built
+_nodes = None        # the C++ autograd nodes (csrc/nodes.cpp), False where there are none
 
 
-def nodes():
-    """The C++ autograd nodes, bound to this library; ``None`` where the extension was not built (the nodes in Python then
-    issue the same launches) and while launches are timed or marked one by one."""
-    global _nodes
-    if _nodes is None:
-        import importlib.machinery
-        import importlib.util
-        path = os.path.join(_HERE, "_C", "b200moe_nodes.so")
-        _nodes = False
-        if require() is not None and os.path.exists(path):
-            loader = importlib.machinery.ExtensionFileLoader("b200moe_nodes", path)
+def _load_nodes():
+    """The extension, bound to this library; ``False``, with a warning, where it was not built or does not fit the
+    installed PyTorch."""
+    import importlib.machinery
+    import importlib.util
+    import warnings
+    path = os.path.join(_HERE, "_C", "b200moe_nodes.so")
+    reason = "not found"
+    if os.path.exists(path):
+        loader = importlib.machinery.ExtensionFileLoader("b200moe_nodes", path)
+        try:
             module = importlib.util.module_from_spec(importlib.util.spec_from_loader("b200moe_nodes", loader))
             loader.exec_module(module)
             module.bind(_LIB_PATH)
-            _nodes = module
-        else:
-            import warnings
-            warnings.warn(f"{path} not found: small layers run at the speed of Python; run `python -m b200moe.build`")
+            return module
+        except (ImportError, RuntimeError) as error:
+            reason = f"does not load ({error})"
+    warnings.warn(f"{path} {reason}: small layers run at the speed of Python; run `python -m b200moe.build`")
+    return False
+
+
+def nodes():
+    """The C++ autograd nodes; ``None`` where there are none (the nodes in Python then issue the same launches) and while
+    launches are timed or marked one by one."""
+    global _nodes
+    if _nodes is None:
+        require()
+        _nodes = _load_nodes()
     return _nodes if _nodes and _timed is None and not _nvtx else None
 
 

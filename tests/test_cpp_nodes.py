@@ -64,6 +64,43 @@ def test_transformations_that_look_through_nodes_get_the_python_ones():
     assert seen == [None] * 5
 
 
+def test_library_is_built_where_the_nodes_do_not_compile(monkeypatch, tmp_path, capsys):
+    import subprocess
+
+    from b200moe import build
+    run, out = subprocess.run, tmp_path / "_C"
+    out.mkdir()
+    stale = out / "b200moe_nodes.so"
+    for path in (stale, out / "b200moe_nodes.so.sha"):
+        path.write_text("of another build")
+
+    def without_compiler(cmd, **kwargs):
+        return run(["false"], **kwargs) if cmd[0] == "g++" else run(cmd, **kwargs)
+
+    monkeypatch.setattr(build, "HERE", str(tmp_path))
+    monkeypatch.setattr(build, "OUT", str(out))
+    monkeypatch.setattr(build, "LIB", str(out / "lib.so"))
+    monkeypatch.setattr(build, "_sources", lambda: ["pp_link.cu"])
+    monkeypatch.setattr(build.subprocess, "run", without_compiler)
+    build.build_all()
+    assert os.path.getsize(build.LIB) > 0 and not stale.exists() and not (out / "b200moe_nodes.so.sha").exists()
+    assert "C++ autograd nodes not built" in capsys.readouterr().err
+
+
+def test_nodes_that_do_not_load_leave_the_python_ones(monkeypatch, tmp_path):
+    (tmp_path / "_C").mkdir()
+    (tmp_path / "_C" / "b200moe_nodes.so").write_bytes(b"no library")
+    native.require()
+    monkeypatch.setattr(native, "_HERE", str(tmp_path))
+    monkeypatch.setattr(native, "_nodes", None)
+    with pytest.warns(UserWarning, match="does not load"):
+        assert native.nodes() is None
+    import warnings
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")       # said once
+        assert native.nodes() is None
+
+
 # ------------------------------------------------------------------------------ GPU
 def _rel(a, b):
     return float((a.double() - b.double()).norm() / (b.double().norm() + 1e-30))
