@@ -7,6 +7,7 @@
 // caller then goes the general way.  Kernels come from the library that b200moe.ops.native has loaded (``bind``).
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
+#include <torch/csrc/autograd/graph_task.h>
 #include <torch/extension.h>
 
 #include <atomic>
@@ -272,7 +273,8 @@ struct Head : public Function<Head> {
     return loss.to(at::kFloat);
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    const Tensor dh = ctx->get_saved_variables()[0];
+    Tensor dh = ctx->get_saved_variables()[0];
+    if (torch::autograd::get_current_graph_task_keep_graph()) dh = dh.clone();
     const Tensor factor = (grads[0] / ctx->saved_data["scale"].toDouble()).to(dh.device(), at::kFloat);
     check(lib.scale_bf16(mut(dh), ptr(factor), dh.numel(), stream()), "b2_scale_bf16", 1);
     const Tensor none;

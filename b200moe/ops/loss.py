@@ -12,8 +12,9 @@ Where the factor that the caller will back-propagate into the loss is known
 has a ``main_grad`` buffer, all of it happens in the forward pass, a chunk of
 tokens at a time: no full logits tensor exists, and what is kept for the
 backward pass is ``dh`` ``[tokens, d_model]``.  The backward pass multiplies
-``dh`` by ``dloss / grad_scale``, which is one when the caller keeps its word;
-the weight gradient has already been accumulated with ``grad_scale``.
+``dh`` by ``dloss / grad_scale``, which is one when the caller keeps its word
+(in place, unless the graph is retained for another pass); the weight gradient
+has already been accumulated with ``grad_scale``, once whatever follows.
 
 Where it is not known, the forward pass keeps ``d(mean loss)/dlogits`` of as many
 tokens as ``KEEP_BYTES`` hold, and the backward pass is two products over them
@@ -79,6 +80,8 @@ class _LMHeadCE(torch.autograd.Function):
         weight = ctx.weight
         if ctx.eager:
             (dh,) = ctx.saved_tensors
+            if torch._C._autograd._get_current_graph_task_keep_graph():
+                dh = dh.clone()          # a later backward pass through this graph scales what the forward pass left
             native.scale_(dh, dloss / ctx.grad_scale)
             return dh.view(ctx.shape), None, None, None, None
         h2d, flat_targets, kept = ctx.saved_tensors

@@ -209,3 +209,23 @@ def test_head_node_in_chunks(monkeypatch, T, D, V, chunk):
         assert _rel(a, b) < 1e-5
     assert weight.grad is None
     native.check_status()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cpp", [True, False])
+def test_head_with_a_known_factor_twice_through_one_graph(monkeypatch, cpp):
+    from b200moe import ops
+    _nodes()
+    if not cpp:
+        monkeypatch.setattr(native, "nodes", lambda: None)
+    hidden = torch.randn(70, 128, device="cuda").bfloat16().requires_grad_(True)
+    weight = (torch.randn(320, 128, device="cuda") * 0.05).bfloat16().requires_grad_(True)
+    weight.main_grad = torch.zeros(320, 128, device="cuda")
+    targets = torch.randint(0, 320, (70,), device="cuda")
+    loss = ops.lm_head_cross_entropy(hidden, weight, targets, 0.25)
+    summed = weight.main_grad.clone()
+    grads = [torch.autograd.grad(loss, hidden, torch.full_like(loss, f), retain_graph=f < 1)[0].clone() for f in (0.5, 0.25, 0.5, 1.0)]
+    # powers of two: exact; the announced factor is already in dh, and the weight's gradient is added by the forward pass alone
+    assert torch.equal(grads[0], 2 * grads[1]) and torch.equal(grads[0], grads[2]) and torch.equal(grads[3], 4 * grads[1])
+    assert bool(grads[1].any()) and torch.equal(weight.main_grad, summed)
+    native.check_status()
