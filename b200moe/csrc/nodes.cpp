@@ -121,14 +121,44 @@ class Scratch {
   std::vector<void*> at_;
 };
 
-// What a node keeps beside the saved tensors: weights and their gradient buffers, as the Python nodes keep them.
+// Where the gradient of a weight goes in a backward pass: the buffer that the weight carries then (its ``main_grad``; as in the
+// Python nodes, one that took the place of the forward pass's is followed).  A buffer that the kernels do not take, or none,
+// gets the sum afterwards.
+class Gradient {
+ public:
+  Gradient(const Tensor& weight, at::ScalarType kind) : weight_(weight), buffer_(of(weight)) {
+    const bool direct = buffer_.defined() && plain(buffer_, kind, weight) && buffer_.sizes() == weight.sizes();
+    sum_ = direct ? buffer_ : at::zeros(weight.sizes(), weight.options().dtype(kind).requires_grad(false));
+  }
+  void* operator*() const { return sum_.data_ptr(); }
+  // What autograd is told: nothing where there is a buffer.
+  Tensor given() {
+    if (buffer_.is_same(sum_)) return Tensor();
+    if (buffer_.defined()) {
+      buffer_.add_(sum_);
+      return Tensor();
+    }
+    return weight_.requires_grad() ? sum_.to(weight_.scalar_type()) : Tensor();
+  }
+  static Tensor of(const Tensor& weight) {
+    pybind11::gil_scoped_acquire gil;
+    const auto object = pybind11::reinterpret_steal<pybind11::object>(THPVariable_Wrap(weight));
+    const pybind11::object buffer = pybind11::getattr(object, "main_grad", pybind11::none());
+    return THPVariable_Check(buffer.ptr()) ? THPVariable_Unpack(buffer.ptr()) : Tensor();
+  }
+
+ private:
+  Tensor weight_, buffer_, sum_;
+};
+
+// What a node keeps beside the saved tensors: weights, as the Python nodes keep them.
 void keep(AutogradContext* ctx, std::vector<Tensor> tensors) { ctx->saved_data["kept"] = std::move(tensors); }
 std::vector<Tensor> kept(AutogradContext* ctx) { return ctx->saved_data["kept"].toTensorVector(); }
 
 struct Embedding : public Function<Embedding> {
-  static Tensor forward(AutogradContext* ctx, const Tensor& ids, const Tensor& table, const Tensor& grad) {
+  static Tensor forward(AutogradContext* ctx, const Tensor& ids, const Tensor& table) {
     ctx->save_for_backward({ids});
-    keep(ctx, {grad});
+    keep(ctx, {table});
     std::vector<int64_t> sizes = ids.sizes().vec();
     sizes.push_back(table.size(1));
     Tensor out = bf16(sizes, table);
@@ -136,10 +166,11 @@ struct Embedding : public Function<Embedding> {
     return out;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    const Tensor ids = ctx->get_saved_variables()[0], grad = kept(ctx)[0], dy = grads[0].contiguous();
+    const Tensor ids = ctx->get_saved_variables()[0], table = kept(ctx)[0], dy = grads[0].contiguous();
     TORCH_CHECK(dy.scalar_type() == at::kBFloat16, "expected bfloat16, got ", dy.scalar_type());
-    check(lib.embedding_bwd(ptr(ids), ptr(dy), mut(grad), ids.numel(), grad.size(1), stream()), "b2_embedding_bwd", 1);
-    return {Tensor(), Tensor(), Tensor()};
+    Gradient grad(table, at::kFloat);
+    check(lib.embedding_bwd(ptr(ids), ptr(dy), *grad, ids.numel(), table.size(1), stream()), "b2_embedding_bwd", 1);
+    return {Tensor(), grad.given()};
   }
 };
 
@@ -167,9 +198,9 @@ struct RMSNorm : public Function<RMSNorm> {
 };
 
 struct AttnHalf : public Function<AttnHalf> {
-  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& ln1, const Tensor& wqkv, const Tensor& gqkv,
-                               const Tensor& cos, const Tensor& sin, const Tensor& wo, const Tensor& go, const Tensor& ln2,
-                               const Tensor& status, int64_t hq, int64_t hkv, double eps1, double eps2) {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& ln1, const Tensor& wqkv,
+                               const Tensor& cos, const Tensor& sin, const Tensor& wo, const Tensor& ln2, const Tensor& status,
+                               int64_t hq, int64_t hkv, double eps1, double eps2) {
     const int B = x.size(0), S = x.size(1);
     const int64_t T = x.size(0) * x.size(1);
     Tensor n1 = at::empty_like(x), a = at::empty_like(x), proj = at::empty_like(x), sum = at::empty_like(x), n2 = at::empty_like(x);
@@ -178,7 +209,7 @@ struct AttnHalf : public Function<AttnHalf> {
                             mut(proj), mut(sum), mut(n2), mut(stats), B, S, hq, hkv, eps1, eps2, mut(status), stream()),
           "b2_attn_half_fwd", 5);
     ctx->save_for_backward({x, ln1, ln2, cos, sin, n1, qkv, a, sum, stats});
-    keep(ctx, {wqkv, gqkv, wo, go, status});
+    keep(ctx, {wqkv, wo, status});
     ctx->saved_data["heads"] = hq * 4096 + hkv;
     return {sum, n2};
   }
@@ -196,20 +227,20 @@ struct AttnHalf : public Function<AttnHalf> {
     Tensor dx = at::empty_like(x), dln1 = fp32({D}, x), dln2 = fp32({D}, x);
     // dmid, da, dqkv, the norms' partial sums, the attention's row statistics
     const Scratch tmp(x, {2 * T * D, 2 * T * D, 2 * qkv.numel(), int64_t{4} * lib.rmsnorm_bwd_parts(T, D) * D, 8 * T * hq});
-    check(lib.attn_half_bwd(ptr(dsum), ptr(dn2), ptr(x), ptr(ln1), ptr(w[0]), ptr(cos), ptr(sin), ptr(w[2]), ptr(ln2), ptr(n1),
-                            ptr(qkv), ptr(a), ptr(sum), ptr(stats), mut(w[1]), mut(w[3]), mut(dln1), mut(dln2), mut(dx), tmp[0], tmp[1],
-                            tmp[1], tmp[2], static_cast<float*>(tmp[3]), static_cast<float*>(tmp[4]), B, S, hq, hkv, mut(w[4]),
+    Gradient gqkv(w[0], at::kFloat), go(w[1], at::kFloat);
+    check(lib.attn_half_bwd(ptr(dsum), ptr(dn2), ptr(x), ptr(ln1), ptr(w[0]), ptr(cos), ptr(sin), ptr(w[1]), ptr(ln2), ptr(n1),
+                            ptr(qkv), ptr(a), ptr(sum), ptr(stats), *gqkv, *go, mut(dln1), mut(dln2), mut(dx), tmp[0], tmp[1],
+                            tmp[1], tmp[2], static_cast<float*>(tmp[3]), static_cast<float*>(tmp[4]), B, S, hq, hkv, mut(w[2]),
                             stream()),
           "b2_attn_half_bwd", 11);
     const Tensor none;
-    return {dx, dln1, none, none, none, none, none, none, dln2, none, none, none, none, none};
+    return {dx, dln1, gqkv.given(), none, none, go.given(), dln2, none, none, none, none, none};
   }
 };
 
 struct MoELayer : public Function<MoELayer> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& router, const Tensor& w1, const Tensor& w3,
-                               const Tensor& w2, const Optional& residual, const Tensor& grouter, const Tensor& g1,
-                               const Tensor& g3, const Tensor& g2, const Tensor& status, int64_t cap, bool keeps, bool balance) {
+                               const Tensor& w2, const Optional& residual, const Tensor& status, int64_t cap, bool keeps, bool balance) {
     ctx->set_materialize_grads(false);
     const int64_t D = x.size(-1), T = x.numel() / D, E = w1.size(0), F = w1.size(1);
     Tensor weights = fp32({T, 2}, x), probs = fp32({T, E}, x), idx = at::empty({T, 2}, x.options().dtype(at::kLong));
@@ -222,7 +253,7 @@ struct MoELayer : public Function<MoELayer> {
     variable_list saved = {x, weights, idx, probs, tables, x_perm, y_perm};
     if (keeps) saved.insert(saved.end(), {gate, up});
     ctx->save_for_backward(std::move(saved));
-    keep(ctx, {router, w1, w3, w2, grouter, g1, g3, g2, status});
+    keep(ctx, {router, w1, w3, w2, status});
     ctx->saved_data["residual"] = residual.has_value();
     if (!balance) return {out};
     Tensor aux = fp32({}, x);
@@ -244,13 +275,17 @@ struct MoELayer : public Function<MoELayer> {
     // dy_perm, dx_perm, dgu, h, dh, dweights, dlogits, gate and up where they are formed again
     const Scratch tmp(x, {row, row, 2 * wide, wide, own ? wide : 0, 8 * T, 4 * T * E, rebuild ? wide : 0, rebuild ? wide : 0});
     Tensor dx = at::empty_like(x);
+    const Tensor first = Gradient::of(w[1]);
+    const at::ScalarType kind = first.defined() && first.scalar_type() == at::kBFloat16 ? at::kBFloat16 : at::kFloat;
+    Gradient grouter(w[0], at::kFloat), g1(w[1], kind), g3(w[2], kind), g2(w[3], kind);
     check(lib.moe_layer_bwd(ptr(dout), ptr(x), ptr(w[0]), ptr(w[1]), ptr(w[2]), ptr(w[3]), ptr(weights), ptr(idx), ptr(probs),
                             mut(tables), ptr(x_perm), ptr(y_perm), rebuild ? tmp[7] : mut(saved[7]), rebuild ? tmp[8] : mut(saved[8]),
-                            rebuild, ptr(daux), mut(w[5]), mut(w[6]), mut(w[7]), w[5].scalar_type() == at::kFloat ? 1 : 2, mut(w[4]),
-                            tmp[0], tmp[2], tmp[3], tmp[4], tmp[1], tmp[5], tmp[6], mut(dx), T, D, F, E, cap, mut(w[8]), stream()),
+                            rebuild, ptr(daux), *g1, *g3, *g2, kind == at::kFloat ? 1 : 2, *grouter,
+                            tmp[0], tmp[2], tmp[3], tmp[4], tmp[1], tmp[5], tmp[6], mut(dx), T, D, F, E, cap, mut(w[4]), stream()),
           "b2_moe_layer_bwd", 7 + own + rebuild);
     const Tensor none;
-    return {dx, none, none, none, none, ctx->saved_data["residual"].toBool() ? grads[0] : none, none, none, none, none, none, none, none, none};
+    return {dx, grouter.given(), g1.given(), g3.given(), g2.given(), ctx->saved_data["residual"].toBool() ? grads[0] : none,
+            none, none, none, none};
   }
 };
 
@@ -287,7 +322,7 @@ Optional embedding(const Tensor& ids, const Tensor& table, const Tensor& grad) {
   if (!(ids.scalar_type() == at::kLong && ids.is_contiguous() && ids.numel() > 0 && ids.numel() < INT_MAX && table.dim() == 2 &&
         table.size(1) % 8 == 0 && table.is_cuda() && ids.device() == table.device() && trained(table, grad, table)))
     return std::nullopt;
-  return Embedding::apply(ids, table, grad);
+  return Embedding::apply(ids, table);
 }
 
 Optional rmsnorm(const Tensor& x, const Tensor& weight, double eps, const Tensor& status) {
@@ -311,7 +346,7 @@ std::optional<variable_list> attn_half(const Tensor& x, const Tensor& ln1, const
     if (!(gain.dim() == 1 && gain.size(0) == D && plain(gain, at::kFloat, x))) return std::nullopt;
   for (const Tensor& table : {cos, sin})
     if (!(table.dim() == 2 && table.size(1) == 64 && table.size(0) >= S && plain(table, at::kFloat, x))) return std::nullopt;
-  return AttnHalf::apply(x, ln1, wqkv, gqkv, cos, sin, wo, go, ln2, status, hq, hkv, eps1, eps2);
+  return AttnHalf::apply(x, ln1, wqkv, cos, sin, wo, ln2, status, hq, hkv, eps1, eps2);
 }
 
 std::optional<variable_list> moe_layer(const Tensor& x, const Tensor& router, const Tensor& w1, const Tensor& w3, const Tensor& w2,
@@ -332,7 +367,7 @@ std::optional<variable_list> moe_layer(const Tensor& x, const Tensor& router, co
   if (residual && !(plain(*residual, at::kBFloat16, x) && residual->sizes() == x.sizes())) return std::nullopt;
   const bool keeps = !recompute && follows({x, router, w1, w3, w2, residual ? *residual : Tensor()});
   const int64_t cap = (2 * T + E * (align - 1) + align - 1) / align * align;      // moe_fused.capacity_rows
-  return MoELayer::apply(x, router, w1, w3, w2, residual, grouter, g1, g3, g2, status, cap, keeps, balance);
+  return MoELayer::apply(x, router, w1, w3, w2, residual, status, cap, keeps, balance);
 }
 
 Optional head(const Tensor& hidden, const Tensor& weight, const Tensor& targets, const Tensor& grad, double scale, int64_t chunk,

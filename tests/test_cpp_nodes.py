@@ -229,3 +229,42 @@ def test_head_with_a_known_factor_twice_through_one_graph(monkeypatch, cpp):
     assert torch.equal(grads[0], 2 * grads[1]) and torch.equal(grads[0], grads[2]) and torch.equal(grads[3], 4 * grads[1])
     assert bool(grads[1].any()) and torch.equal(weight.main_grad, summed)
     native.check_status()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_gradient_buffers_are_those_of_the_backward_pass(dtype):
+    """A ``main_grad`` replaced between the passes is followed; one that is taken away leaves an ordinary gradient."""
+    _nodes()
+    model = _decoder(blocks=1)
+    inner = model.module.layers[0]
+    weights = [model.module.token_embeddings.compute_weight, inner.attn.qkv_weight, inner.attn.output_proj.compute_weight,
+               inner.ffn.router.compute_weight, inner.ffn.experts.w1, inner.ffn.experts.w3, inner.ffn.experts.w2]
+    ids = torch.randint(0, 320, (2, 129), device="cuda")
+
+    def run(change):
+        model.clear_grad_accumulators()
+        old = [w.main_grad for w in weights]
+        loss = model.loss(ids[:, :-1].contiguous(), ids[:, 1:].contiguous(), grad_scale=1.0)
+        change()
+        loss.backward()
+        got = [w.main_grad if hasattr(w, "main_grad") else w.grad for w in weights]
+        untouched = not any(bool(o.any()) for o in old)
+        for w, o in zip(weights, old):
+            w.main_grad, w.grad = o, None
+        return [g.clone() for g in got], untouched
+
+    def swap():
+        for w in weights:
+            w.main_grad = torch.zeros_like(w.main_grad, dtype=dtype)
+
+    def remove():
+        for w in weights[1:]:                      # (the table of the embedding does not ask for a gradient of its own)
+            del w.main_grad
+
+    kept, _ = run(lambda: None)
+    for change in (swap, remove):
+        got, untouched = run(change)
+        assert untouched or change is remove
+        assert len(got) == 7 and all(_rel(g, k) < (5e-3 if g.dtype == torch.bfloat16 else 1e-4) for g, k in zip(got, kept))
+    native.check_status()
