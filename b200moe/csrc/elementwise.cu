@@ -312,8 +312,8 @@ template <int W, int V>
 __global__ void __launch_bounds__(NORM_THREADS + 32, V == 2 ? 2 : 1)
     rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                        const float* __restrict__ w, const float* __restrict__ rstd,
-                       const __nv_bfloat16* __restrict__ residual, __nv_bfloat16* __restrict__ dx,
-                       float* __restrict__ dw_partial, int* __restrict__ status, int rows, int D, int ring_stages) {
+                       const __nv_bfloat16* residual, __nv_bfloat16* dx, float* __restrict__ dw_partial,
+                       int* __restrict__ status, int rows, int D, int ring_stages) {
   chain_begin();
   constexpr int R = 8 / W;
   extern __shared__ __align__(128) uint8_t norm_ring[];
@@ -1311,7 +1311,8 @@ int b2_rmsnorm_fwd(const void* x, const void* delta, const float* w, void* sum_o
   });
 }
 
-// dw_partial: fp32 [parts, D] scratch with parts = b2_rmsnorm_bwd_parts(rows, D); dw: fp32 [D] (overwritten).
+// dw_partial: fp32 [parts, D] scratch with parts = b2_rmsnorm_bwd_parts(rows, D); dw: fp32 [D] (overwritten).  dx may be residual:
+// one CTA holds a row of all tensors before it stores that row.
 // two CTAs are resident per SM (registers): one wave, and as few partial rows as possible for the column sum
 int b2_rmsnorm_bwd_parts(int rows, int D) {
   const int R = norm_rows_at_once(D);

@@ -101,7 +101,7 @@ int b2_attn_half_fwd(const void* x, const float* ln1, const void* wqkv, const fl
 
 // Its backward pass: dx for the gradients dsum and dn2; the weights' gradients are added to gqkv and go (fp32), the gains' are
 // stored to dln1 and dln2 (fp32 [D]).  Scratch: dmid, da, dn1 [T, D], dqkv [T, N], partial fp32 (rmsnorm_bwd's),
-// row_stats fp32 [B Hq, 2, S].
+// row_stats fp32 [B Hq, 2, S].  dn1 may be da, and dmid may be dx (see b2_rmsnorm_bwd).
 int b2_attn_half_bwd(const void* dsum, const void* dn2, const void* x, const float* ln1, const void* wqkv, const float* cos_t,
                      const float* sin_t, const void* wo, const float* ln2, const void* n1, const void* qkv, const void* a,
                      const void* sum, const float* stats, float* gqkv, float* go, float* dln1, float* dln2, void* dx, void* dmid, void* da,
@@ -157,15 +157,15 @@ int b2_head_chunk(const void* hidden, const void* weight, const long long* targe
   return run.rc;
 }
 
-// Backward pass of the routed layer.  The gradients of w1, w3, w2 are added to g1, g3, g2 (expert_kind 1: fp32, 2: bf16), the router's to
-// grouter (fp32).  rebuild: gate and up are scratch and are formed again.  dh: scratch [cap, F] where the SwiGLU backward is a
-// kernel of its own, null where it rides in the product.  Scratch besides: dy_perm, dx_perm [cap, D], dgu [cap, 2F], h [cap, F],
-// dweights [T, 2], dlogits [T, E].
-int b2_moe_layer_bwd(const void* dout, const void* x, const void* router, const void* w1, const void* w3, const void* w2,
-                     const float* weights, const long long* idx, const float* probs, int* tables, const void* x_perm,
-                     const void* y_perm, void* gate, void* up, int rebuild, const float* daux, void* g1, void* g3, void* g2,
-                     int expert_kind, float* grouter, void* dy_perm, void* dgu, void* h, void* dh, void* dx_perm, float* dweights,
-                     float* dlogits, void* dx, int T, int D, int F, int E, int cap, int* status, cudaStream_t s) {
+// Backward pass of the routed layer, the experts: dx_perm and dweights [T, 2] for the output's gradient; those of w1, w3, w2 are
+// added to g1, g3, g2 (expert_kind 1: fp32, 2: bf16).  rebuild: gate and up are scratch and are formed again.  dh: scratch
+// [cap, F] where the SwiGLU backward is a kernel of its own, null where it rides in the product.  Scratch besides: dy_perm
+// [cap, D], dgu [cap, 2F], h [cap, F].  dx_perm [cap, D] may overlap dh, and gate and up where they are scratch: it is stored
+// behind the kernels that read them.
+int b2_moe_experts_bwd(const void* dout, const void* w1, const void* w3, const void* w2, const float* weights, int* tables,
+                       const void* x_perm, const void* y_perm, void* gate, void* up, int rebuild, void* g1, void* g3, void* g2,
+                       int expert_kind, void* dy_perm, void* dgu, void* h, void* dh, void* dx_perm, float* dweights, int T, int D,
+                       int F, int E, int cap, int* status, cudaStream_t s) {
   const Tables t(tables, 2 * T, cap, E);
   Sequence run;
   if (rebuild)
@@ -182,6 +182,16 @@ int b2_moe_layer_bwd(const void* dout, const void* x, const void* router, const 
   run([&] {
     return b2_gemm_tn(dgu, x_perm, g1, g3, F, 2 * F, D, cap, 2 * F, D, D, E, t.offs, t.counts, expert_kind, 1.f, nullptr, status, s);
   });
+  return run.rc;
+}
+
+// Its router, behind the experts (whose scratch the caller may have given back): dx [T, D]; the gradient of the router's weights is
+// added to grouter (fp32).  Scratch: dlogits [T, E].
+int b2_moe_router_bwd(const void* x, const void* router, const float* weights, const long long* idx, const float* probs, int* tables,
+                      const float* daux, float* grouter, const void* dx_perm, const float* dweights, float* dlogits, void* dx, int T,
+                      int D, int E, int cap, cudaStream_t s) {
+  const Tables t(tables, 2 * T, cap, E);
+  Sequence run;
   run([&] { return b2_moe_dx(dx_perm, t.slot_row, dweights, probs, idx, weights, daux, t.counts, router, dlogits, dx, T, E, D, cap, s); });
   run([&] { return b2_skinny_tn(dlogits, x, grouter, T, E, D, s); });
   return run.rc;

@@ -30,9 +30,11 @@ struct Library {
                        void*, void*, void*, void*, void*, void*, void*, int, int, int, int, void*, void*);
   int (*moe_layer_fwd)(const void*, const void*, const void*, const void*, const void*, const void*, void*, void*, void*, void*,
                        void*, void*, void*, void*, void*, void*, int, int, int, int, int, void*, void*);
-  int (*moe_layer_bwd)(const void*, const void*, const void*, const void*, const void*, const void*, const void*, const void*,
-                       const void*, void*, const void*, const void*, void*, void*, int, const void*, void*, void*, void*, int,
-                       void*, void*, void*, void*, void*, void*, void*, void*, void*, int, int, int, int, int, void*, void*);
+  int (*moe_experts_bwd)(const void*, const void*, const void*, const void*, const void*, void*, const void*, const void*, void*,
+                         void*, int, void*, void*, void*, int, void*, void*, void*, void*, void*, void*, int, int, int, int, int,
+                         void*, void*);
+  int (*moe_router_bwd)(const void*, const void*, const void*, const void*, const void*, void*, const void*, void*, const void*,
+                        const void*, void*, void*, int, int, int, int, void*);
   int (*moe_aux)(const void*, const void*, void*, int, int, void*);
   int (*rmsnorm_fwd)(const void*, const void*, const void*, void*, void*, void*, int, int, float, void*, void*);
   int (*rmsnorm_bwd)(const void*, const void*, const void*, const void*, const void*, void*, void*, void*, int, int, void*, void*);
@@ -55,7 +57,8 @@ void bind(const std::string& path) {
   resolve(lib.attn_half_fwd, "b2_attn_half_fwd");
   resolve(lib.attn_half_bwd, "b2_attn_half_bwd");
   resolve(lib.moe_layer_fwd, "b2_moe_layer_fwd");
-  resolve(lib.moe_layer_bwd, "b2_moe_layer_bwd");
+  resolve(lib.moe_experts_bwd, "b2_moe_experts_bwd");
+  resolve(lib.moe_router_bwd, "b2_moe_router_bwd");
   resolve(lib.moe_aux, "b2_moe_aux");
   resolve(lib.rmsnorm_fwd, "b2_rmsnorm_fwd");
   resolve(lib.rmsnorm_bwd, "b2_rmsnorm_bwd");
@@ -223,15 +226,15 @@ struct AttnHalf : public Function<AttnHalf> {
     const int64_t T = x.size(0) * x.size(1);
     const Tensor dsum = grads[0].contiguous(), dn2 = grads[1].contiguous();
     TORCH_CHECK(dsum.scalar_type() == at::kBFloat16 && dn2.scalar_type() == at::kBFloat16, "expected bfloat16 gradients");
-    // the gradient of the first norm's output takes the place of the attention output's, which is used up by then
+    // The gradient of the first norm's output takes the place of the attention output's, which is used up by then, and dx that
+    // of the sum's, which the first norm's kernel adds row by row before it stores the row: as much as the separate nodes hold.
     Tensor dx = at::empty_like(x), dln1 = fp32({D}, x), dln2 = fp32({D}, x);
-    // dmid, da, dqkv, the norms' partial sums, the attention's row statistics
-    const Scratch tmp(x, {2 * T * D, 2 * T * D, 2 * qkv.numel(), int64_t{4} * lib.rmsnorm_bwd_parts(T, D) * D, 8 * T * hq});
+    // da, dqkv, the norms' partial sums, the attention's row statistics
+    const Scratch tmp(x, {2 * T * D, 2 * qkv.numel(), int64_t{4} * lib.rmsnorm_bwd_parts(T, D) * D, 8 * T * hq});
     Gradient gqkv(w[0], at::kFloat), go(w[1], at::kFloat);
     check(lib.attn_half_bwd(ptr(dsum), ptr(dn2), ptr(x), ptr(ln1), ptr(w[0]), ptr(cos), ptr(sin), ptr(w[1]), ptr(ln2), ptr(n1),
-                            ptr(qkv), ptr(a), ptr(sum), ptr(stats), *gqkv, *go, mut(dln1), mut(dln2), mut(dx), tmp[0], tmp[1],
-                            tmp[1], tmp[2], static_cast<float*>(tmp[3]), static_cast<float*>(tmp[4]), B, S, hq, hkv, mut(w[2]),
-                            stream()),
+                            ptr(qkv), ptr(a), ptr(sum), ptr(stats), *gqkv, *go, mut(dln1), mut(dln2), mut(dx), mut(dx), tmp[0],
+                            tmp[0], tmp[1], tmp[2], tmp[3], B, S, hq, hkv, mut(w[2]), stream()),
           "b2_attn_half_bwd", 11);
     const Tensor none;
     return {dx, dln1, gqkv.given(), none, none, go.given(), dln2, none, none, none, none, none};
@@ -272,17 +275,23 @@ struct MoELayer : public Function<MoELayer> {
     Tensor daux = grads.size() > 1 && grads[1].defined() ? grads[1].to(x.device(), at::kFloat) : Tensor();
     const int64_t row = 2 * cap * D, wide = 2 * cap * F;
     const bool own = !lib.swiglu_bwd_in_product(cap, F, D);      // the SwiGLU backward is a kernel of its own
-    // dy_perm, dx_perm, dgu, h, dh, dweights, dlogits, gate and up where they are formed again
-    const Scratch tmp(x, {row, row, 2 * wide, wide, own ? wide : 0, 8 * T, 4 * T * E, rebuild ? wide : 0, rebuild ? wide : 0});
-    Tensor dx = at::empty_like(x);
     const Tensor first = Gradient::of(w[1]);
     const at::ScalarType kind = first.defined() && first.scalar_type() == at::kBFloat16 ? at::kBFloat16 : at::kFloat;
     Gradient grouter(w[0], at::kFloat), g1(w[1], kind), g3(w[2], kind), g2(w[3], kind);
-    check(lib.moe_layer_bwd(ptr(dout), ptr(x), ptr(w[0]), ptr(w[1]), ptr(w[2]), ptr(w[3]), ptr(weights), ptr(idx), ptr(probs),
-                            mut(tables), ptr(x_perm), ptr(y_perm), rebuild ? tmp[7] : mut(saved[7]), rebuild ? tmp[8] : mut(saved[8]),
-                            rebuild, ptr(daux), *g1, *g3, *g2, kind == at::kFloat ? 1 : 2, *grouter,
-                            tmp[0], tmp[2], tmp[3], tmp[4], tmp[1], tmp[5], tmp[6], mut(dx), T, D, F, E, cap, mut(w[4]), stream()),
-          "b2_moe_layer_bwd", 7 + own + rebuild);
+    // dx_perm takes the place of what is used up by then: dh, and gate and up where they are formed again.  dweights, dlogits.
+    const Scratch tmp(x, {std::max(row, (own + 2 * rebuild) * wide), 8 * T, 4 * T * E});
+    char* const used = static_cast<char*>(tmp[0]);
+    char* const formed = used + own * wide;
+    {
+      const Scratch inner(x, {row, 2 * wide, wide});              // dy_perm, dgu, h
+      check(lib.moe_experts_bwd(ptr(dout), ptr(w[1]), ptr(w[2]), ptr(w[3]), ptr(weights), mut(tables), ptr(x_perm), ptr(y_perm),
+                                rebuild ? formed : mut(saved[7]), rebuild ? formed + wide : mut(saved[8]), rebuild, *g1, *g3, *g2,
+                                kind == at::kFloat ? 1 : 2, inner[0], inner[1], inner[2], own ? used : nullptr, used, tmp[1], T, D,
+                                F, E, cap, mut(w[4]), stream()), "b2_moe_experts_bwd", 5 + own + rebuild);
+    }
+    Tensor dx = at::empty_like(x);
+    check(lib.moe_router_bwd(ptr(x), ptr(w[0]), ptr(weights), ptr(idx), ptr(probs), mut(tables), ptr(daux), *grouter, used, tmp[1],
+                             tmp[2], mut(dx), T, D, E, cap, stream()), "b2_moe_router_bwd", 2);
     const Tensor none;
     return {dx, grouter.given(), g1.given(), g3.given(), g2.given(), ctx->saved_data["residual"].toBool() ? grads[0] : none,
             none, none, none, none};

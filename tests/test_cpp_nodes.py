@@ -268,3 +268,36 @@ def test_gradient_buffers_are_those_of_the_backward_pass(dtype):
         assert untouched or change is remove
         assert len(got) == 7 and all(_rel(g, k) < (5e-3 if g.dtype == torch.bfloat16 else 1e-4) for g, k in zip(got, kept))
     native.check_status()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("part,recompute", [("attention", False), ("experts", False), ("experts", True)])
+def test_backward_passes_hold_no_more_memory_than_the_python_nodes(monkeypatch, part, recompute):
+    from b200moe import ops
+    _nodes()
+    layer = _decoder(D=1024, heads=8, ffn=3584, blocks=1, expert_grad=torch.bfloat16).module.layers[0]
+    layer.ffn.recompute = recompute
+    x = torch.randn(16, 256, 1024, device="cuda").bfloat16().requires_grad_(True)
+
+    def outputs():
+        if part == "experts":
+            return (layer.ffn(x),)
+        half = layer._attention_half(x)
+        return half if half is not None else ops.add_rmsnorm(x, layer.attn(layer.ln1(x)), layer.ln2.weight, layer.ln2.eps)
+
+    peaks, grads = [], []
+    for _ in range(2):
+        out = outputs()
+        douts = [torch.full_like(o, 0.01) for o in out]
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()                        # (blocks left by others may be larger than what is asked for)
+        before = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        grads.append(torch.autograd.grad(out, x, douts)[0])
+        torch.cuda.synchronize()
+        peaks.append(torch.cuda.max_memory_allocated() - before)
+        del out, douts
+        monkeypatch.setattr(native, "nodes", lambda: None)
+    assert peaks[0] <= peaks[1] + (2 << 20), peaks      # the allocator's granularity
+    assert _rel(*grads) < 1e-2
+    native.check_status()
