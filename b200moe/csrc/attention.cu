@@ -19,6 +19,7 @@
 // A sequence may have any length: its last tile reads zeros behind it and is masked.
 // Every barrier wait is bounded; a wait that runs out sets the status word.
 #include "chain.cuh"
+#include "entries.h"
 #include "ptx.cuh"
 #include "tensormap.cuh"
 

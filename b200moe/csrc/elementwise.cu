@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include "chain.cuh"
+#include "entries.h"
 #include "ptx.cuh"
 
 namespace b2 {

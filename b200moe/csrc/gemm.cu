@@ -18,6 +18,7 @@
 // ring of {A 128x64, B 256x64} bf16 tiles in the 128-byte-swizzled layout that
 // both TMA and the MMA descriptors understand.
 #include "chain.cuh"
+#include "entries.h"
 #include "peer.cuh"
 #include "ptx.cuh"
 #include "tensormap.cuh"

@@ -16,6 +16,7 @@
 
 #include "chain.cuh"
 #include "debug.cuh"
+#include "entries.h"
 #include "ptx.cuh"
 
 namespace b2 {

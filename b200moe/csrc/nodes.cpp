@@ -12,6 +12,8 @@
 
 #include <atomic>
 
+#include "entries.h"
+
 using torch::autograd::AutogradContext;
 using torch::autograd::Function;
 using torch::autograd::variable_list;
@@ -23,27 +25,20 @@ namespace {
 std::atomic<long long> launches{0};
 
 struct Library {
-  int (*attn_half_fwd)(const void*, const void*, const void*, const void*, const void*, const void*, const void*, void*, void*,
-                       void*, void*, void*, void*, void*, int, int, int, int, float, float, void*, void*);
-  int (*attn_half_bwd)(const void*, const void*, const void*, const void*, const void*, const void*, const void*, const void*,
-                       const void*, const void*, const void*, const void*, const void*, const void*, void*, void*, void*, void*,
-                       void*, void*, void*, void*, void*, void*, void*, int, int, int, int, void*, void*);
-  int (*moe_layer_fwd)(const void*, const void*, const void*, const void*, const void*, const void*, void*, void*, void*, void*,
-                       void*, void*, void*, void*, void*, void*, int, int, int, int, int, void*, void*);
-  int (*moe_experts_bwd)(const void*, const void*, const void*, const void*, const void*, void*, const void*, const void*, void*,
-                         void*, int, void*, void*, void*, int, void*, void*, void*, void*, void*, void*, int, int, int, int, int,
-                         void*, void*);
-  int (*moe_router_bwd)(const void*, const void*, const void*, const void*, const void*, void*, const void*, void*, const void*,
-                        const void*, void*, void*, int, int, int, int, void*);
-  int (*moe_aux)(const void*, const void*, void*, int, int, void*);
-  int (*rmsnorm_fwd)(const void*, const void*, const void*, void*, void*, void*, int, int, float, void*, void*);
-  int (*rmsnorm_bwd)(const void*, const void*, const void*, const void*, const void*, void*, void*, void*, int, int, void*, void*);
-  int (*rmsnorm_bwd_parts)(int, int);
-  int (*swiglu_bwd_in_product)(long long, int, int);
-  int (*head_chunk)(const void*, const void*, const void*, void*, void*, void*, void*, int, int, int, float, float, void*, void*);
-  int (*scale_bf16)(void*, const void*, long long, void*);
-  int (*embedding_fwd)(const void*, const void*, void*, int, int, void*);
-  int (*embedding_bwd)(const void*, const void*, void*, int, int, void*);
+  decltype(&b2_attn_half_fwd) attn_half_fwd;
+  decltype(&b2_attn_half_bwd) attn_half_bwd;
+  decltype(&b2_moe_layer_fwd) moe_layer_fwd;
+  decltype(&b2_moe_experts_bwd) moe_experts_bwd;
+  decltype(&b2_moe_router_bwd) moe_router_bwd;
+  decltype(&b2_moe_aux) moe_aux;
+  decltype(&b2_rmsnorm_fwd) rmsnorm_fwd;
+  decltype(&b2_rmsnorm_bwd) rmsnorm_bwd;
+  decltype(&b2_rmsnorm_bwd_parts) rmsnorm_bwd_parts;
+  decltype(&b2_swiglu_bwd_in_product) swiglu_bwd_in_product;
+  decltype(&b2_head_chunk) head_chunk;
+  decltype(&b2_scale_bf16) scale_bf16;
+  decltype(&b2_embedding_fwd) embedding_fwd;
+  decltype(&b2_embedding_bwd) embedding_bwd;
 } lib;
 
 void bind(const std::string& path) {
@@ -70,13 +65,22 @@ void bind(const std::string& path) {
   resolve(lib.embedding_bwd, "b2_embedding_bwd");
 }
 
-void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+cudaStream_t stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 void check(int code, const char* name, int count) {
   TORCH_CHECK(code == 0, name, " failed with code ", code);
   launches += count;
 }
-const void* ptr(const Tensor& t) { return t.defined() ? t.const_data_ptr() : nullptr; }
-void* mut(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+// Addresses as the entry points type them; the tensors' types have been looked at by then.
+struct Const {
+  const void* at;
+  template <typename T> operator const T*() const { return static_cast<const T*>(at); }
+};
+struct Mutable {
+  void* at;
+  template <typename T> operator T*() const { return static_cast<T*>(at); }
+};
+Const ptr(const Tensor& t) { return {t.defined() ? t.const_data_ptr() : nullptr}; }
+Mutable mut(const Tensor& t) { return {t.defined() ? t.data_ptr() : nullptr}; }
 Tensor fp32(at::IntArrayRef sizes, const Tensor& like) { return at::empty(sizes, like.options().dtype(at::kFloat)); }
 Tensor bf16(at::IntArrayRef sizes, const Tensor& like) { return at::empty(sizes, like.options().dtype(at::kBFloat16)); }
 Tensor int32(at::IntArrayRef sizes, const Tensor& like) { return at::empty(sizes, like.options().dtype(at::kInt)); }
@@ -112,14 +116,13 @@ class Scratch {
         next += (b + 255) / 256 * 256;
       } else {
         held_.push_back(b ? at::empty({b}, options) : Tensor());
-        at_.push_back(mut(held_.back()));
+        at_.push_back(mut(held_.back()).at);
       }
     }
   }
-  void* operator[](size_t i) const { return at_[i]; }
+  Mutable operator[](size_t i) const { return {at_[i]}; }
 
  private:
-  static void* mut(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
   std::vector<Tensor> held_;
   std::vector<void*> at_;
 };
@@ -133,7 +136,7 @@ class Gradient {
     const bool direct = buffer_.defined() && plain(buffer_, kind, weight) && buffer_.sizes() == weight.sizes();
     sum_ = direct ? buffer_ : at::zeros(weight.sizes(), weight.options().dtype(kind).requires_grad(false));
   }
-  void* operator*() const { return sum_.data_ptr(); }
+  Mutable operator*() const { return {sum_.data_ptr()}; }
   // What autograd is told: nothing where there is a buffer.
   Tensor given() {
     if (buffer_.is_same(sum_)) return Tensor();
@@ -250,7 +253,7 @@ struct MoELayer : public Function<MoELayer> {
     Tensor tables = int32({2 * T + cap + 2 * E + cap / 128 + 4}, x);
     Tensor x_perm = bf16({cap, D}, x), y_perm = bf16({cap, D}, x), h = bf16({cap, F}, x), out = at::empty_like(x), gate, up;
     if (keeps) gate = at::empty_like(h), up = at::empty_like(h);
-    check(lib.moe_layer_fwd(ptr(x), ptr(router), ptr(w1), ptr(w3), ptr(w2), residual ? ptr(*residual) : nullptr, mut(weights),
+    check(lib.moe_layer_fwd(ptr(x), ptr(router), ptr(w1), ptr(w3), ptr(w2), ptr(residual ? *residual : Tensor()), mut(weights),
                             mut(idx), mut(probs), mut(tables), mut(x_perm), mut(h), mut(gate), mut(up), mut(y_perm), mut(out), T, D,
                             F, E, cap, mut(status), stream()), "b2_moe_layer_fwd", 6);
     variable_list saved = {x, weights, idx, probs, tables, x_perm, y_perm};
@@ -280,12 +283,12 @@ struct MoELayer : public Function<MoELayer> {
     Gradient grouter(w[0], at::kFloat), g1(w[1], kind), g3(w[2], kind), g2(w[3], kind);
     // dx_perm takes the place of what is used up by then: dh, and gate and up where they are formed again.  dweights, dlogits.
     const Scratch tmp(x, {std::max(row, (own + 2 * rebuild) * wide), 8 * T, 4 * T * E});
-    char* const used = static_cast<char*>(tmp[0]);
+    char* const used = tmp[0];
     char* const formed = used + own * wide;
     {
       const Scratch inner(x, {row, 2 * wide, wide});              // dy_perm, dgu, h
       check(lib.moe_experts_bwd(ptr(dout), ptr(w[1]), ptr(w[2]), ptr(w[3]), ptr(weights), mut(tables), ptr(x_perm), ptr(y_perm),
-                                rebuild ? formed : mut(saved[7]), rebuild ? formed + wide : mut(saved[8]), rebuild, *g1, *g3, *g2,
+                                rebuild ? formed : mut(saved[7]).at, rebuild ? formed + wide : mut(saved[8]).at, rebuild, *g1, *g3, *g2,
                                 kind == at::kFloat ? 1 : 2, inner[0], inner[1], inner[2], own ? used : nullptr, used, tmp[1], T, D,
                                 F, E, cap, mut(w[4]), stream()), "b2_moe_experts_bwd", 5 + own + rebuild);
     }
@@ -307,9 +310,9 @@ struct Head : public Function<Head> {
     for (int64_t lo = 0; lo < T; lo += chunk) {
       const int64_t n = std::min(chunk, T - lo);
       Tensor logits = bf16({n, V}, hidden);
-      check(lib.head_chunk(static_cast<const char*>(ptr(hidden)) + 2 * lo * D, ptr(weight),
-                           static_cast<const char*>(ptr(targets)) + 8 * lo, mut(logits), mut(loss),
-                           static_cast<char*>(mut(dh)) + 2 * lo * D, mut(grad), n, V, D, 1.0 / T, scale / T, mut(status), stream()),
+      check(lib.head_chunk(static_cast<const char*>(ptr(hidden).at) + 2 * lo * D, ptr(weight),
+                           static_cast<const long long*>(ptr(targets)) + lo, mut(logits), mut(loss),
+                           static_cast<char*>(mut(dh).at) + 2 * lo * D, mut(grad), n, V, D, 1.0 / T, scale / T, mut(status), stream()),
             "b2_head_chunk", 4);
     }
     ctx->save_for_backward({dh});
