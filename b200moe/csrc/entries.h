@@ -54,6 +54,7 @@ int b2_embedding_fwd(const long long* ids, const void* table, void* out, int T, 
 int b2_embedding_bwd(const long long* ids, const void* dy, float* dtable, int T, int D, cudaStream_t s);
 int b2_moe_aux(const float* probs, const int* counts, float* aux, int T, int E, cudaStream_t s);
 // layers.cu
+const char* b2_layers_refused();
 int b2_attn_half_fwd(const void* x, const float* ln1, const void* wqkv, const float* cos_t, const float* sin_t, const void* wo,
                      const float* ln2, void* n1, void* qkv, void* a, void* proj, void* sum, void* n2, float* stats, int B, int S,
                      int Hq, int Hkv, float eps1, float eps2, int* status, cudaStream_t s);

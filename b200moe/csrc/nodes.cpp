@@ -25,6 +25,7 @@ namespace {
 std::atomic<long long> launches{0};
 
 struct Library {
+  decltype(&b2_layers_refused) layers_refused;
   decltype(&b2_attn_half_fwd) attn_half_fwd;
   decltype(&b2_attn_half_bwd) attn_half_bwd;
   decltype(&b2_moe_layer_fwd) moe_layer_fwd;
@@ -49,6 +50,7 @@ void bind(const std::string& path) {
     TORCH_CHECK(symbol, path, " has no ", name);
     entry = reinterpret_cast<std::remove_reference_t<decltype(entry)>>(symbol);
   };
+  resolve(lib.layers_refused, "b2_layers_refused");
   resolve(lib.attn_half_fwd, "b2_attn_half_fwd");
   resolve(lib.attn_half_bwd, "b2_attn_half_bwd");
   resolve(lib.moe_layer_fwd, "b2_moe_layer_fwd");
@@ -66,8 +68,18 @@ void bind(const std::string& path) {
 }
 
 cudaStream_t stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+// Raises what b200moe.ops.native raises for a refused launch; ``name``: its entry point, null for a sequence of layers.cu.
 void check(int code, const char* name, int count) {
-  TORCH_CHECK(code == 0, name, " failed with code ", code);
+  if (code != 0) {
+    if (!name) name = lib.layers_refused();
+    std::string detail;
+    try {
+      pybind11::gil_scoped_acquire gil;
+      detail = pybind11::module_::import("b200moe.ops.native").attr("_failure_detail")(name, code).cast<std::string>();
+    } catch (pybind11::error_already_set&) {      // the code alone, then
+    }
+    TORCH_CHECK(false, name, " failed with code ", code, detail);
+  }
   launches += count;
 }
 // Addresses as the entry points type them; the tensors' types have been looked at by then.
@@ -213,7 +225,7 @@ struct AttnHalf : public Function<AttnHalf> {
     Tensor qkv = bf16({T, 128 * (hq + 2 * hkv)}, x), stats = fp32({T * (2 + hq)}, x);
     check(lib.attn_half_fwd(ptr(x), ptr(ln1), ptr(wqkv), ptr(cos), ptr(sin), ptr(wo), ptr(ln2), mut(n1), mut(qkv), mut(a),
                             mut(proj), mut(sum), mut(n2), mut(stats), B, S, hq, hkv, eps1, eps2, mut(status), stream()),
-          "b2_attn_half_fwd", 5);
+          nullptr, 5);
     ctx->save_for_backward({x, ln1, ln2, cos, sin, n1, qkv, a, sum, stats});
     keep(ctx, {wqkv, wo, status});
     ctx->saved_data["heads"] = hq * 4096 + hkv;
@@ -238,7 +250,7 @@ struct AttnHalf : public Function<AttnHalf> {
     check(lib.attn_half_bwd(ptr(dsum), ptr(dn2), ptr(x), ptr(ln1), ptr(w[0]), ptr(cos), ptr(sin), ptr(w[1]), ptr(ln2), ptr(n1),
                             ptr(qkv), ptr(a), ptr(sum), ptr(stats), *gqkv, *go, mut(dln1), mut(dln2), mut(dx), mut(dx), tmp[0],
                             tmp[0], tmp[1], tmp[2], tmp[3], B, S, hq, hkv, mut(w[2]), stream()),
-          "b2_attn_half_bwd", 11);
+          nullptr, 11);
     const Tensor none;
     return {dx, dln1, gqkv.given(), none, none, go.given(), dln2, none, none, none, none, none};
   }
@@ -255,7 +267,7 @@ struct MoELayer : public Function<MoELayer> {
     if (keeps) gate = at::empty_like(h), up = at::empty_like(h);
     check(lib.moe_layer_fwd(ptr(x), ptr(router), ptr(w1), ptr(w3), ptr(w2), ptr(residual ? *residual : Tensor()), mut(weights),
                             mut(idx), mut(probs), mut(tables), mut(x_perm), mut(h), mut(gate), mut(up), mut(y_perm), mut(out), T, D,
-                            F, E, cap, mut(status), stream()), "b2_moe_layer_fwd", 6);
+                            F, E, cap, mut(status), stream()), nullptr, 6);
     variable_list saved = {x, weights, idx, probs, tables, x_perm, y_perm};
     if (keeps) saved.insert(saved.end(), {gate, up});
     ctx->save_for_backward(std::move(saved));
@@ -290,11 +302,11 @@ struct MoELayer : public Function<MoELayer> {
       check(lib.moe_experts_bwd(ptr(dout), ptr(w[1]), ptr(w[2]), ptr(w[3]), ptr(weights), mut(tables), ptr(x_perm), ptr(y_perm),
                                 rebuild ? formed : mut(saved[7]).at, rebuild ? formed + wide : mut(saved[8]).at, rebuild, *g1, *g3, *g2,
                                 kind == at::kFloat ? 1 : 2, inner[0], inner[1], inner[2], own ? used : nullptr, used, tmp[1], T, D,
-                                F, E, cap, mut(w[4]), stream()), "b2_moe_experts_bwd", 5 + own + rebuild);
+                                F, E, cap, mut(w[4]), stream()), nullptr, 5 + own + rebuild);
     }
     Tensor dx = at::empty_like(x);
     check(lib.moe_router_bwd(ptr(x), ptr(w[0]), ptr(weights), ptr(idx), ptr(probs), mut(tables), ptr(daux), *grouter, used, tmp[1],
-                             tmp[2], mut(dx), T, D, E, cap, stream()), "b2_moe_router_bwd", 2);
+                             tmp[2], mut(dx), T, D, E, cap, stream()), nullptr, 2);
     const Tensor none;
     return {dx, grouter.given(), g1.given(), g3.given(), g2.given(), ctx->saved_data["residual"].toBool() ? grads[0] : none,
             none, none, none, none};
@@ -313,7 +325,7 @@ struct Head : public Function<Head> {
       check(lib.head_chunk(static_cast<const char*>(ptr(hidden).at) + 2 * lo * D, ptr(weight),
                            static_cast<const long long*>(ptr(targets)) + lo, mut(logits), mut(loss),
                            static_cast<char*>(mut(dh).at) + 2 * lo * D, mut(grad), n, V, D, 1.0 / T, scale / T, mut(status), stream()),
-            "b2_head_chunk", 4);
+            nullptr, 4);
     }
     ctx->save_for_backward({dh});
     ctx->saved_data["scale"] = scale;
@@ -398,6 +410,7 @@ Optional head(const Tensor& hidden, const Tensor& weight, const Tensor& targets,
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   using Release = pybind11::call_guard<pybind11::gil_scoped_release>;
   m.def("bind", &bind);
+  m.def("check", &check, Release());
   m.def("launches", [] { return launches.load(); });
   m.def("embedding", &embedding, Release());
   m.def("rmsnorm", &rmsnorm, Release());

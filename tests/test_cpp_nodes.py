@@ -101,6 +101,20 @@ def test_nodes_that_do_not_load_leave_the_python_ones(monkeypatch, tmp_path):
         assert native.nodes() is None
 
 
+def test_refused_launch_is_named_as_the_python_bindings_name_it():
+    import ctypes
+    nodes, lib = _nodes(), native.require()
+    nodes.check(0, None, 0)
+    with pytest.raises(RuntimeError, match=r"^b2_attention_fwd_ex failed with code -12 \(tensor map k: driver result 0\)"):
+        nodes.check(-12, "b2_attention_fwd_ex", 1)
+    # rows of 65 * 128 columns: the first launch of the sequence is refused before anything touches a device
+    null, pointers = ctypes.c_void_p(0), 14
+    code = lib.b2_attn_half_fwd(*[null] * pointers, *[ctypes.c_int(v) for v in (1, 128, 65, 65)], ctypes.c_float(1e-5),
+                                ctypes.c_float(1e-5), null, null)
+    with pytest.raises(RuntimeError, match="^b2_rmsnorm_fwd failed with code -10"):
+        nodes.check(code, None, 1)
+
+
 # ------------------------------------------------------------------------------ GPU
 def _rel(a, b):
     return float((a.double() - b.double()).norm() / (b.double().norm() + 1e-30))
