@@ -122,10 +122,10 @@ class AdamW(torch.optim.Optimizer):
             group["t"] = t + 1
 
     def zero_grad(self, set_to_none: bool = True):
-        """As the base class, without its profiler range where gradients are dropped (a fifth of a small step's host time
-        outside the layers)."""
-        if not set_to_none:
-            return super().zero_grad(set_to_none=False)
+        """As the base class, whose profiler range (a fifth of a small step's host time outside the layers) is opened where
+        there is a profiler to see it."""
+        if not set_to_none or torch.autograd._profiler_enabled():
+            return super().zero_grad(set_to_none=set_to_none)
         for group in self.param_groups:
             for p in group["params"]:
                 p.grad = None

@@ -350,3 +350,17 @@ def test_differentiable_attention_refuses_fp16_before_it_runs(monkeypatch):
         ops.rope_attention(q, q, q, None, None)
     q = torch.zeros(1, 128, 1, 128, dtype=torch.bfloat16, requires_grad=True)
     assert ops.rope_attention(q, q, q, None, None).requires_grad
+
+
+def test_adamw_zero_grad_is_seen_by_a_profiler():
+    p = torch.nn.Parameter(torch.ones(3))
+    optimizer = AdamW([p])
+    for profiled in (True, False):
+        p.grad = torch.ones(3)
+        if profiled:
+            with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU]) as seen:
+                optimizer.zero_grad()
+            assert "Optimizer.zero_grad#AdamW.zero_grad" in [event.key for event in seen.key_averages()]
+        else:
+            optimizer.zero_grad()
+        assert p.grad is None
