@@ -23,6 +23,8 @@
 #include "ptx.cuh"
 #include "tensormap.cuh"
 
+#include <atomic>
+
 namespace b2 {
 
 constexpr int HD = 128;
@@ -1349,15 +1351,53 @@ static int sm_count_attn() {
   return sms > 0 ? sms : 148;
 }
 
-// A backward kernel over ``tiles`` tiles of at most ``steps`` steps each.  Where the CTAs of several parts per tile still make
-// one wave, two share the steps from five on and four from eight on: below, the two barriers and the exchange cost what a step or
-// two saves; eight parts gain nothing more.  us, whole backward pass, one -> several parts, causal: 2 x 512 tokens, 4/1 heads
-// 45.8 -> 34.0; 1024, 8/2 73.3 -> 41.2; 2048, 8/2 130 -> 68.7; 4 x 1024, 8/2 88.8 -> 70.6; 128, 8/2 (one part) 26.1.
-static int launch_bwd(void (*kernel)(AttnParams), long long tiles, long long steps, const AttnParams& p, cudaStream_t stream) {
+// Clusters of ``parts`` (2 or 4) backward CTAs that the device holds at once; a cluster lies in one GPC, so that 148 SMs hold 74 of
+// two and 33 of four.  Asked once per device.
+template <void (*kernel)(AttnParams)>
+static int bwd_clusters_resident(int parts) {
+  constexpr int DEVICES = 64;
+  static std::atomic<int> known[DEVICES][2];                            // 0: not asked yet, else the number + 1
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= DEVICES) return 0;
+  std::atomic<int>& slot = known[dev][parts == 4];
+  if (slot.load() == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = parts;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(parts);
+    cfg.blockDim = dim3(ATTN_THREADS);
+    cfg.dynamicSmemBytes = BWD_SMEM;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int count = 0;
+    if (cudaOccupancyMaxActiveClusters(&count, kernel, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      count = 0;
+    }
+    slot.store(count + 1);
+  }
+  return slot.load() - 1;
+}
+
+// A backward kernel over ``tiles`` tiles of at most ``steps`` steps each.  Where the clusters of several parts per tile make one
+// wave, two share the steps from seven on and four from eight on: below, the two barriers and the exchange cost what the steps
+// save (two parts against one: five steps 29.0, 25.0; six 29.5, 27.5); eight parts gain nothing more.  One wave is what the
+// device holds in clusters, 33 of four CTAs, not 148 / 4: 36 tiles of nine steps in four parts are 61 us, in two 35, in one 39.  Causal
+// tiles of many steps may make a second wave, which the shortest of them fill: 36 tiles of up to 36 steps in four parts 53,
+// in two 59.  us, whole backward pass, one -> several parts, causal: 2 x 512 tokens, 4/1 heads 45.8 -> 34.0; 1024, 8/2 73.3 ->
+// 41.2; 2048, 8/2 130 -> 68.7; 4 x 1024, 8/2 88.8 -> 70.6; 128, 8/2 (one part) 26.1.
+template <void (*kernel)(AttnParams)>
+static int launch_bwd(long long tiles, long long steps, const AttnParams& p, cudaStream_t stream) {
   const int sms = sm_count_attn();
   int parts = 1;
-  if (steps >= 5 && tiles * 2 <= sms) parts = 2;
-  if (steps >= 8 && tiles * 4 <= sms) parts = 4;
+  if (steps >= 7 && tiles * 2 <= sms && tiles <= bwd_clusters_resident<kernel>(2)) parts = 2;
+  if (steps >= 8 && tiles * 4 <= sms) {
+    const int held = bwd_clusters_resident<kernel>(4);
+    if (tiles <= held || (held > 0 && p.causal && steps >= 24)) parts = 4;
+  }
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // chain.cuh
@@ -1372,7 +1412,9 @@ static int launch_bwd(void (*kernel)(AttnParams), long long tiles, long long ste
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = parts > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, kernel, p) == cudaSuccess ? 0 : -4;
+  if (cudaLaunchKernelEx(&cfg, kernel, p) == cudaSuccess) return 0;
+  cudaGetLastError();                                                   // not the next launch's
+  return -4;
 }
 
 template <void (*kernel)(AttnParams), int smem, int threads = ATTN_THREADS>
@@ -1454,12 +1496,12 @@ int b2_attention_bwd_rope(const void* dout, const void* q, const void* k, const 
   }
   const long long tiles = (S + TQ - 1) / TQ, Sp = tiles * TQ;
   if (Sp / 16 * B * Hq > 0x7fffffffLL) return -10;
-  launch_next(attn_stats_kernel, static_cast<unsigned>(Sp / 16 * B * Hq), 256, 0, stream, static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(out), lse, stats, S,
-      static_cast<int>(Sp), Hq);
+  launch_next(attn_stats_kernel, static_cast<unsigned>(Sp / 16 * B * Hq), 256, 0, stream, static_cast<const __nv_bfloat16*>(dout),
+              static_cast<const __nv_bfloat16*>(out), lse, stats, S, static_cast<int>(Sp), Hq);
   p.set_heads = heads_per_set(B * Hkv, 4LL * S * HD * (Hq / Hkv));
-  if (launch_bwd(attn_bwd_dkv_kernel, tiles * B * Hkv, tiles * (Hq / Hkv), p, stream)) return -4;
+  if (launch_bwd<attn_bwd_dkv_kernel>(tiles * B * Hkv, tiles * (Hq / Hkv), p, stream)) return -4;
   p.set_heads = heads_per_set(B * Hq, 4LL * S * HD * Hkv / Hq);
-  if (launch_bwd(attn_bwd_dq_kernel, tiles * B * Hq, tiles, p, stream)) return -4;
+  if (launch_bwd<attn_bwd_dq_kernel>(tiles * B * Hq, tiles, p, stream)) return -4;
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 

@@ -1014,7 +1014,8 @@ def test_flash_attention_in_fp16_keeps_fp16_precision(native, S, causal):
 
 
 @pytest.mark.parametrize("B,S,Hq,Hkv,causal", [(1, 640, 4, 4, False), (1, 640, 2, 2, True), (2, 1024, 4, 1, True),
-                                               (1, 1100, 8, 2, True), (1, 1025, 2, 2, False)])
+                                               (1, 1100, 8, 2, True), (1, 1025, 2, 2, False), (1, 896, 2, 2, True),
+                                               (1, 4224, 1, 1, True), (1, 1152, 4, 4, False), (1, 1152, 16, 4, True)])
 def test_attention_backward_shared_by_a_cluster(native, B, S, Hq, Hkv, causal):
     """Tiles whose steps two or four CTAs share: uneven parts, CTAs without a step, a ragged last tile."""
     q, k, v, dy = (_rand(B, S, h, 128) for h in (Hq, Hkv, Hkv, Hq))
