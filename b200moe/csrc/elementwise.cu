@@ -308,8 +308,9 @@ __global__ void __launch_bounds__(NORM_THREADS) rmsnorm_fwd_row_kernel(const __n
   }
 }
 
-// dx = rstd * (dy*w - xhat * mean(dy*w*xhat)) [+ residual]; dw partial per CTA.
-template <int W, int V>
+// dx = rstd * (dy*w - xhat * mean(dy*w*xhat)) [+ residual]; dw partial per CTA.  RING 0: no CTA has more than one block of rows,
+// which its warps read straight from global memory (us with the column sum: 1 x 512 4.0 -> 3.7, 300 x 2048 7.5 -> 6.7).
+template <int W, int V, int RING>
 __global__ void __launch_bounds__(NORM_THREADS + 32, V == 2 ? 2 : 1)
     rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                        const float* __restrict__ w, const float* __restrict__ rstd,
@@ -320,7 +321,7 @@ __global__ void __launch_bounds__(NORM_THREADS + 32, V == 2 ? 2 : 1)
   extern __shared__ __align__(128) uint8_t norm_ring[];
   __shared__ NormBars bars;
   __shared__ float scratch[2][R][8];
-  norm_init(bars);
+  if (RING) norm_init(bars);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool worker = warp < NORM_THREADS / 32;
   const int slot = warp / W, in_row = warp % W;
@@ -345,25 +346,26 @@ __global__ void __launch_bounds__(NORM_THREADS + 32, V == 2 ? 2 : 1)
     bool here = true;
     float next_r = static_cast<int>(blockIdx.x) * R + slot < rows ? rstd[blockIdx.x * R + slot] : 0.f;
     for (int block = blockIdx.x; block < blocks; block += gridDim.x, ++count) {
-      const int s = count % ring_stages;
+      const int s = RING ? count % ring_stages : 0;
       const int row = block * R + slot, after = row + static_cast<int>(gridDim.x) * R;
       const bool live = row < rows;
       const float r = next_r;
       if (after < rows) next_r = rstd[after];
       const __nv_bfloat16* in = reinterpret_cast<const __nv_bfloat16*>(norm_ring) + (static_cast<size_t>(s) * 3 * R + slot) * D;
-      here = norm_arrived(here, bars.full[s], (count / ring_stages) & 1, status);
+      const size_t base = static_cast<size_t>(row) * D;
+      if (RING) here = norm_arrived(here, bars.full[s], (count / ring_stages) & 1, status);
       bf16x8 a[V], b[V], res[V];
 #pragma unroll
       for (int c = 0; c < V; ++c) {
         const int col = ((c * W + in_row) * 32 + lane) * 8;
         if (live && col < D) {
-          a[c] = *reinterpret_cast<const bf16x8*>(in + col);
-          b[c] = *reinterpret_cast<const bf16x8*>(in + static_cast<size_t>(R) * D + col);
-          if (residual) res[c] = *reinterpret_cast<const bf16x8*>(in + static_cast<size_t>(2 * R) * D + col);
+          a[c] = *reinterpret_cast<const bf16x8*>(RING ? in + col : dy + base + col);
+          b[c] = *reinterpret_cast<const bf16x8*>(RING ? in + static_cast<size_t>(R) * D + col : x + base + col);
+          if (residual) res[c] = *reinterpret_cast<const bf16x8*>(RING ? in + static_cast<size_t>(2 * R) * D + col : residual + base + col);
         }
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bars.empty[s]);
+      if (RING && lane == 0) mbar_arrive(&bars.empty[s]);
       float part[V];
 #pragma unroll
       for (int c = 0; c < V; ++c) part[c] = 0.f;
@@ -399,7 +401,7 @@ __global__ void __launch_bounds__(NORM_THREADS + 32, V == 2 ? 2 : 1)
 #pragma unroll
             for (int i = 0; i < 8; ++i) o[i] += add[i];
           }
-          *reinterpret_cast<bf16x8*>(dx + static_cast<size_t>(row) * D + col) = pack8(o);
+          *reinterpret_cast<bf16x8*>(dx + base + col) = pack8(o);
         }
       }
     }
@@ -420,7 +422,7 @@ __global__ void __launch_bounds__(NORM_THREADS + 32, V == 2 ? 2 : 1)
       }
     }
     __syncthreads();
-    for (int col = threadIdx.x; col < D; col += NORM_THREADS + 32) {
+    for (int col = threadIdx.x; col < D; col += blockDim.x) {
       float total = 0.f;
 #pragma unroll
       for (int k = 0; k < R; ++k) total += sums[static_cast<size_t>(k) * D + col];
@@ -441,22 +443,26 @@ __global__ void __launch_bounds__(NORM_THREADS + 32, V == 2 ? 2 : 1)
 
 // out[col] = sum over parts of partial[part][col].  One CTA per 32 columns: lane = column (coalesced 128-byte reads), the
 // 32 warps take every 32nd part (eight warps in four chains each were 7.6 us at 296 parts of 512 columns, this 2.5),
-// shared memory adds the 32 partial sums.
-__global__ void __launch_bounds__(1024) column_sum_kernel(const float* __restrict__ partial, float* __restrict__ out,
+// shared memory adds the 32 partial sums.  Eight warps for up to eight parts: the same sums without the warps that add zeros.
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) column_sum_kernel(const float* __restrict__ partial, float* __restrict__ out,
                                                          int parts, int D) {
   chain_begin();
-  __shared__ float acc[32][33];
+  __shared__ float acc[WARPS][33];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int col = blockIdx.x * 32 + lane;
   float s = 0.f;
   if (col < D) {
 #pragma unroll 10
-    for (int p = warp; p < parts; p += 32) s += partial[static_cast<size_t>(p) * D + col];
+    for (int p = warp; p < parts; p += WARPS) s += partial[static_cast<size_t>(p) * D + col];
   }
   acc[warp][lane] = s;
   __syncthreads();
-  s = warp_sum(acc[lane][warp]);             // transposed: warp = column, lane = part
-  if (lane == 0 && blockIdx.x * 32 + warp < D) out[blockIdx.x * 32 + warp] = s;
+#pragma unroll
+  for (int c = warp; c < 32; c += WARPS) {    // transposed: warp = column, lane = part
+    s = warp_sum(lane < WARPS ? acc[lane][c] : 0.f);
+    if (lane == 0 && blockIdx.x * 32 + c < D) out[blockIdx.x * 32 + c] = s;
+  }
 }
 
 // ------------------------------------------------------------------ router softmax / top-2
@@ -1266,7 +1272,7 @@ template <typename F>
 static int launch_norm(int D, int tensors, F launch) {
   const int slot = norm_rows_at_once(D) * D * 2 * tensors;
   const int stages = min(NORM_RING, NORM_SMEM / slot);
-  // (backward: the sums of the rows at once, four bytes a column, fit into two stages)
+  // (backward: the sums of the rows at once, four bytes a column, fit into one stage of three tensors)
   const int smem = max(stages, 1) * slot;
   if (D <= 512) return launch(Int<1>{}, Int<NORM_VECS>{}, smem, stages);
   if (D <= 1024) return launch(Int<2>{}, Int<NORM_VECS>{}, smem, stages);
@@ -1314,25 +1320,33 @@ int b2_rmsnorm_fwd(const void* x, const void* delta, const float* w, void* sum_o
 
 // dw_partial: fp32 [parts, D] scratch with parts = b2_rmsnorm_bwd_parts(rows, D); dw: fp32 [D] (overwritten).  dx may be residual:
 // one CTA holds a row of all tensors before it stores that row.
-// two CTAs are resident per SM (registers): one wave, and as few partial rows as possible for the column sum
+// One wave, and as few partial rows as possible for the column sum: two CTAs are resident per SM, beyond 4096 columns one
+// (registers; with twice as many 1024 x 8192 took 24.3 us instead of 19.7, 16384 x 8192 218 instead of 209).
 int b2_rmsnorm_bwd_parts(int rows, int D) {
   const int R = norm_rows_at_once(D);
-  return min((rows + R - 1) / R, sm_count_ew() * 2);
+  return min((rows + R - 1) / R, sm_count_ew() * (D <= 4096 ? 2 : 1));
 }
 int b2_rmsnorm_bwd(const void* dy, const void* x, const float* w, const float* rstd, const void* residual, void* dx,
                    float* dw_partial, float* dw, int rows, int D, int* status, cudaStream_t s) {
   if (D % 8 || D > NORM_MAX_D) return -10;
   if ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(residual)) % 16) return -12;
-  const int parts = b2_rmsnorm_bwd_parts(rows, D);
+  const int parts = b2_rmsnorm_bwd_parts(rows, D), at_once = norm_rows_at_once(D);
   const int rc = launch_norm(D, 3, [&](auto W, auto V, int smem, int stages) {
-    auto kernel = rmsnorm_bwd_kernel<decltype(W)::value, decltype(V)::value>;
-    if (const int rc = norm_smem<decltype(W)::value, decltype(V)::value, 1>(kernel)) return rc;
+    constexpr int w_ = decltype(W)::value, v_ = decltype(V)::value;
+    if ((rows + at_once - 1) / at_once <= parts) {
+      launch_next(rmsnorm_bwd_kernel<w_, v_, 0>, parts, NORM_THREADS, at_once * D * 4, s, (const bf16*)dy, (const bf16*)x, w, rstd,
+                  (const bf16*)residual, (bf16*)dx, dw_partial, status, rows, D, stages);
+      return ok();
+    }
+    auto kernel = rmsnorm_bwd_kernel<w_, v_, 1>;
+    if (const int rc = norm_smem<w_, v_, 1>(kernel)) return rc;
     launch_next(kernel, parts, NORM_THREADS + 32, smem, s, (const bf16*)dy, (const bf16*)x, w, rstd, (const bf16*)residual, (bf16*)dx,
-                                                  dw_partial, status, rows, D, stages);
+                dw_partial, status, rows, D, stages);
     return ok();
   });
   if (rc) return rc;
-  launch_next(column_sum_kernel, (D + 31) / 32, 1024, 0, s, dw_partial, dw, parts, D);
+  if (parts <= 8) launch_next(column_sum_kernel<8>, (D + 31) / 32, 256, 0, s, dw_partial, dw, parts, D);
+  else launch_next(column_sum_kernel<32>, (D + 31) / 32, 1024, 0, s, dw_partial, dw, parts, D);
   return ok();
 }
 

@@ -315,9 +315,11 @@ def test_rmsnorm_forward_backward(native):
         assert _rel(w.grad, wr2.grad) < 8e-3
 
 
-@pytest.mark.parametrize("rows,D", [(1, 8), (3563, 512), (1800, 520), (1777, 1024), (893, 2048), (451, 2056), (450, 8192)])
+@pytest.mark.parametrize("rows,D", [(1, 8), (3563, 512), (1800, 520), (1777, 1024), (893, 2048), (451, 2056), (450, 8192),
+                                    (65, 512), (2368, 512), (2369, 512), (592, 2048), (148, 8192), (149, 4104)])
 def test_rmsnorm_row_blocks(native, rows, D):
-    """Blocks of eight to one rows through the ring, the last one cut short; the one-CTA-per-row form of few rows."""
+    """Blocks of eight to one rows through the ring, the last one cut short; the one-CTA-per-row form of few rows; backward
+    without the ring where no CTA has a second block."""
     x, delta, dy, res = (_rand(rows, D) for _ in range(4))
     w = torch.rand(D, device="cuda") + 0.5
     summed, y, rstd = native.add_rmsnorm_fwd(x, delta, w, 1e-5)
@@ -336,6 +338,8 @@ def test_rmsnorm_row_blocks(native, rows, D):
         assert _rel(dx, want) < 4e-3
         bound = (rows + 8) * 2.0 ** -23 * (dy64 * xhat).abs().sum(0)
         assert bool(((dw.double() - (dy64 * xhat).sum(0)).abs() <= bound + 1e-30).all())
+        if rows > 1:                              # rows do not depend on how many there are, ring or not
+            assert torch.equal(native.rmsnorm_bwd(dy[-1:], summed[-1:], w, rstd[-1:], None if residual is None else res[-1:])[0], dx[-1:])
     native.check_status()
 
 
