@@ -814,7 +814,13 @@ static TileKind choose_tile(const GemmParams& p, int sms, bool pair_available) {
     const long long groups = SCHED == SCHED_WGRAD ? p.num_experts : 1;
     const auto waves = [&](int width) { return ((rows + 127) / 128 * ((p.N + width - 1) / width) * groups + sms - 1) / sms; };
     const long long w256 = waves(256), w128 = waves(128);
-    if (waves(64) == 1) return TILE_N64;
+    if (waves(64) == 1) {
+      // Loads of an A operand below 128 KiB are slow, whatever its shape (4096 columns, 64 CTAs: K 4096 21.4 us at 15 rows and 12.9
+      // at 16, K 8192 37.8 at 6 and 22.4 at 8), and the slower the more CTAs read it: 128 columns where 64 make more than 32 CTAs
+      // (6144 columns, one row, K 4096: 64 columns 28, 128 21.9, 256 22; 4096 columns 21.4, 16.4, 21.9).
+      const bool small_a = SCHED == SCHED_FLAT && static_cast<long long>(p.M) * p.K * 2 < 128 * 1024;
+      return small_a && (p.N + 63) / 64 > 32 ? TILE_N128 : TILE_N64;
+    }
     if (w128 == 1 || (w256 == 2 && w128 == 3)) return TILE_N128;
   }
   if (!legal || g_tile_mode == 1) return TILE_128;

@@ -62,6 +62,39 @@ def test_gemm_tn_accumulates(native, tile_mode, R, M, N, dtype):
     native.check_status()
 
 
+def test_fp32_additions_keep_subnormals_and_round_the_scaled_product(native, tile_mode):
+    """What the memory system adds is what the SM would add: exact with subnormal terms and sums; with a factor the product is
+    rounded, then added."""
+    for old, left, right in ((1e-39, 0.0, 0.0), (0.0, 2.0 ** -70, 2.0 ** -63), (2.0 ** -126, 2.0 ** -70, 2.0 ** -63),
+                             (-2.0 ** -126, 2.0 ** -65, 2.0 ** -62)):
+        dy, x = (torch.zeros(64, n, device="cuda").bfloat16() for n in (136, 96))
+        dy[5], x[5] = left, right
+        got = torch.full((136, 96), old, device="cuda")
+        want = float(got[0, 0].double()) + left * right             # a sum that fp32 holds
+        native.gemm_tn(dy, x, out=got, accumulate=True)
+        assert bool((got.double() == want).all())
+    dy, x, factor, old = _rand(100, 136), _rand(100, 96), torch.tensor(0.3, device="cuda"), torch.randn(136, 96, device="cuda")
+    want = native.gemm_tn(dy, x) * factor + old
+    native.gemm_tn(dy, x, out=old, accumulate=True, alpha=factor)
+    assert torch.equal(old, want)
+    native.check_status()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 2112, 64), (15, 4096, 4096), (16, 4096, 4096), (7, 9472, 512)])
+def test_products_of_few_rows(native, M, N, K):
+    """An A operand below 128 KiB, where 64 columns per tile would make many CTAs, and the first one that is not."""
+    x, w = _rand(M, K), _rand(N, K, scale=K ** -0.5)
+    got = native.gemm_nt(x, w)
+    want = x.double() @ w.double().t()
+    # bf16 result: half an ulp, beside K additions of 2^-24
+    assert bool(((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + K * 2.0 ** -23 * (x.double().abs() @ w.double().abs().t())).all())
+    native.set_gemm_tile_mode(1)
+    assert torch.equal(native.gemm_nt(x, w), got) and torch.equal(native.gemm_nn(x, w.t().contiguous()), got)
+    native.set_gemm_tile_mode(0)
+    assert torch.equal(native.gemm_nn(x, w.t().contiguous()), got)
+    native.check_status()
+
+
 @pytest.mark.parametrize("mode", [6, 7], ids=["128x128", "128x64"])
 @pytest.mark.parametrize("M,N,K", [(1, 32, 64), (129, 96, 128), (200, 320, 576), (300, 2080, 64), (2100, 1312, 192)])
 def test_narrow_tiles_give_the_bits_of_wide_ones(native, mode, M, N, K):
