@@ -554,12 +554,12 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
         }
         if (F32) {
           // fp32 results leave as 32 x 32 boxes that the memory system writes or adds: a warp stages its rows of 32 columns
-          // (16-byte units, XOR-swizzled by row as the tensor map has it) and one lane sends them off.  Each value is added once per launch, so
-          // results do not depend on the order of the tiles (an fp32 subnormal counts as zero in that addition).  Before, the
-          // warp read the old values, added and stored: twice the traffic through the SM, beside the operands of the next
-          // tile.  us, before -> now: 8 experts of 3584 x 1024, 1024 rows each 82.7 -> 72.7, both halves in one launch 140.6 ->
-          // 130.6 (470 MB of results alone are 73), 768 x 512 K 1024 15.1 -> 12.6, 6144 x 4096 K 16384 575 -> 558.  Reading
-          // the old values a chunk ahead instead, or 16 contiguous bytes per lane, gave nothing.
+          // (16-byte units, XOR-swizzled by row as the tensor map has it) and one lane sends them off.  Each value is added once
+          // per launch, so results do not depend on the order of the tiles; the addition is the SM's, subnormals included.
+          // Before, the warp read the old values, added and stored (the same bits): twice the traffic through the SM, beside
+          // the operands of the next tile.  us, before -> now: 8 experts of 3584 x 1024, 1024 rows each 82.7 -> 72.7, both
+          // halves in one launch 140.6 -> 130.6 (470 MB of results alone are 73), 768 x 512 K 1024 15.1 -> 12.6, 6144 x 4096 K
+          // 16384 575 -> 558.  Reading the old values a chunk ahead instead, or 16 contiguous bytes per lane, gave nothing.
 #pragma unroll 1
           for (int c = half * (NT / 2); c < (half + 1) * (NT / 2); c += 32) {
             if (col_base + c >= p.N || row0 >= p.M || (add && empty_k)) break;

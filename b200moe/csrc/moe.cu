@@ -409,6 +409,8 @@ extern "C" {
 int b2_moe_plan(const long long* idx, int slots, int E, int* slot_row, int* row_slot, int* offs, int* tile_expert,
                 int* meta, int* counts, int capacity_rows, cudaStream_t s) {
   if (E < 1) return -10;
+  // 49 experts is what an earlier form of the kernel held in shared memory; this one needs 144 bytes an expert.  The limit stays: no
+  // caller has more (the router takes 64 at most, the routed layer 16 on one rank), and nothing beyond has been tested.
   if (E > 49) return -11;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];

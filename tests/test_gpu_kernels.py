@@ -423,6 +423,60 @@ def test_launches_that_overlap_keep_their_order(native, T, D):
     native.check_status()
 
 
+@pytest.mark.parametrize("T,S", [(256, 128), (2048, 1024)])
+def test_overlapping_launches_of_routing_attention_loss_and_optimizer(native, T, S):
+    """The same for the kernels of a block around the products (from 1280 tokens on the plan is a cluster's, 1024 tokens a sequence
+    share backward steps between CTAs), with PyTorch operations in between."""
+    D, F_, E, V = 512, 256, 4, 320
+    cap = (2 * T + E * 255 + 255) // 256 * 256
+    x0, router = _rand(T, D), _rand(E, D, scale=D ** -0.5)
+    w1, w3, w2 = _rand(E, F_, D, scale=D ** -0.5), _rand(E, F_, D, scale=D ** -0.5), _rand(E, D, F_, scale=F_ ** -0.5)
+    head, targets = _rand(V, D, scale=D ** -0.5), torch.randint(0, V, (T,), device="cuda")
+    m, v = torch.zeros(V, D, device="cuda"), torch.zeros(V, D, device="cuda")
+    acc, master = torch.zeros(V, D, device="cuda"), torch.zeros(V, D, device="cuda")
+
+    def run(wait):
+        def after(value):
+            wait()
+            return value
+
+        native.zero_many_([acc, m, v, master])
+        x = after(x0 * 1)
+        for _ in range(3):
+            weights, idx, probs = after(native.router_fwd(x, router))
+            slot_row, row_slot, offs, tiles, meta, counts = after(native.moe_plan(idx, E, cap))
+            rows = after(native.moe_gather(x, row_slot, meta, cap))
+            h, gate, up = after(native.gemm_swiglu(rows, w1, w3, tiles, meta[:1], align256=True))
+            y = after(native.gemm_nt(h, w2, tile_expert=tiles, num_m_tiles=meta[:1], num_experts=E, align256=True))
+            x = after(native.moe_combine(y, slot_row, weights, T, residual=x))
+            aux = after(native.moe_aux(probs, counts))
+            dweights = torch.empty(T, 2, device="cuda")
+            dy = after(native.moe_gather(x, row_slot, meta, cap, scale=weights.view(-1), y_perm=y, dweights=dweights.view(-1)))
+            dx, dlogits = after(native.moe_dx(dy, slot_row, dweights, probs, idx, weights, router, aux, counts))
+            q = after((x + dx).view(T // S, S, 4, 128).clamp(-4, 4))
+            out, lse, _, _ = after(native.attention_fwd(q, q, q))
+            grads = after(native.attention_bwd(q, q, q, q, out, lse))
+            x = after(sum(grads).clamp(-4, 4).reshape(T, D))
+            logits = after(native.gemm_nt(x, head))
+            loss = after(native.cross_entropy_scaled_(logits, targets, torch.zeros((), dtype=torch.float64, device="cuda"), 1 / T, 1.0))
+            after(native.gemm_tn(logits, x, out=acc, accumulate=True))
+            after(native.adamw_(master, acc, m, v, 1e-3, 0.9, 0.999, 1e-8, 0.0, 1e-3))
+        wait()
+        return torch.cat([t.float().flatten() for t in (x, dlogits, loss, acc, master, m, v)])
+
+    want = run(torch.cuda.synchronize)
+    assert bool(torch.isfinite(want).all())
+    none = lambda: None  # noqa: E731
+    assert all(torch.equal(run(none), want) for _ in range(3))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = run(none)
+    for _ in range(3):
+        graph.replay()
+        assert torch.equal(captured, want)
+    native.check_status()
+
+
 def test_router_linear_and_top2(native):
     from b200moe import ops
     from b200moe.ops import functional as Fn
