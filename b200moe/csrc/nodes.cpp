@@ -115,10 +115,11 @@ bool follows(std::initializer_list<Tensor> inputs) {
 // buffer, as blocks that the allocator has use for elsewhere.
 class Scratch {
  public:
+  static constexpr int64_t TOGETHER = 16 << 20;
   Scratch(const Tensor& like, std::initializer_list<int64_t> bytes) {
     int64_t total = 0;
     for (int64_t b : bytes) total += (b + 255) / 256 * 256;
-    const bool together = total <= 16 << 20;
+    const bool together = total <= TOGETHER;
     const auto options = like.options().dtype(at::kByte);
     if (together) held_.push_back(at::empty({total}, options));
     char* next = together ? static_cast<char*>(held_[0].data_ptr()) : nullptr;
@@ -144,7 +145,7 @@ class Scratch {
 // gets the sum afterwards.
 class Gradient {
  public:
-  Gradient(const Tensor& weight, at::ScalarType kind) : weight_(weight), buffer_(of(weight)) {
+  Gradient(const Tensor& weight, const Tensor& buffer, at::ScalarType kind) : weight_(weight), buffer_(buffer) {
     const bool direct = buffer_.defined() && plain(buffer_, kind, weight) && buffer_.sizes() == weight.sizes();
     sum_ = direct ? buffer_ : at::zeros(weight.sizes(), weight.options().dtype(kind).requires_grad(false));
   }
@@ -158,11 +159,18 @@ class Gradient {
     }
     return weight_.requires_grad() ? sum_.to(weight_.scalar_type()) : Tensor();
   }
-  static Tensor of(const Tensor& weight) {
+  // The buffers that ``count`` weights carry.
+  static std::vector<Tensor> of(const std::vector<Tensor>& weights, size_t count) {
+    std::vector<Tensor> buffers(count);
     pybind11::gil_scoped_acquire gil;
-    const auto object = pybind11::reinterpret_steal<pybind11::object>(THPVariable_Wrap(weight));
-    const pybind11::object buffer = pybind11::getattr(object, "main_grad", pybind11::none());
-    return THPVariable_Check(buffer.ptr()) ? THPVariable_Unpack(buffer.ptr()) : Tensor();
+    static PyObject* const name = PyUnicode_InternFromString("main_grad");
+    for (size_t i = 0; i < count; ++i) {
+      const auto object = pybind11::reinterpret_steal<pybind11::object>(THPVariable_Wrap(weights[i]));
+      const auto buffer = pybind11::reinterpret_steal<pybind11::object>(PyObject_GetAttr(object.ptr(), name));
+      if (!buffer) PyErr_Clear();
+      else if (THPVariable_Check(buffer.ptr())) buffers[i] = THPVariable_Unpack(buffer.ptr());
+    }
+    return buffers;
   }
 
  private:
@@ -184,10 +192,11 @@ struct Embedding : public Function<Embedding> {
     return out;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    const Tensor ids = ctx->get_saved_variables()[0], table = kept(ctx)[0], dy = grads[0].contiguous();
+    const Tensor ids = ctx->get_saved_variables()[0], dy = grads[0].contiguous();
+    const std::vector<Tensor> w = kept(ctx);
     TORCH_CHECK(dy.scalar_type() == at::kBFloat16, "expected bfloat16, got ", dy.scalar_type());
-    Gradient grad(table, at::kFloat);
-    check(lib.embedding_bwd(ptr(ids), ptr(dy), *grad, ids.numel(), table.size(1), stream()), "b2_embedding_bwd", 1);
+    Gradient grad(w[0], Gradient::of(w, 1)[0], at::kFloat);
+    check(lib.embedding_bwd(ptr(ids), ptr(dy), *grad, ids.numel(), w[0].size(1), stream()), "b2_embedding_bwd", 1);
     return {Tensor(), grad.given()};
   }
 };
@@ -246,7 +255,8 @@ struct AttnHalf : public Function<AttnHalf> {
     Tensor dx = at::empty_like(x), dln1 = fp32({D}, x), dln2 = fp32({D}, x);
     // da, dqkv, the norms' partial sums, the attention's row statistics
     const Scratch tmp(x, {2 * T * D, 2 * qkv.numel(), int64_t{4} * lib.rmsnorm_bwd_parts(T, D) * D, 8 * T * hq});
-    Gradient gqkv(w[0], at::kFloat), go(w[1], at::kFloat);
+    const std::vector<Tensor> buffers = Gradient::of(w, 2);
+    Gradient gqkv(w[0], buffers[0], at::kFloat), go(w[1], buffers[1], at::kFloat);
     check(lib.attn_half_bwd(ptr(dsum), ptr(dn2), ptr(x), ptr(ln1), ptr(w[0]), ptr(cos), ptr(sin), ptr(w[1]), ptr(ln2), ptr(n1),
                             ptr(qkv), ptr(a), ptr(sum), ptr(stats), *gqkv, *go, mut(dln1), mut(dln2), mut(dx), mut(dx), tmp[0],
                             tmp[0], tmp[1], tmp[2], tmp[3], B, S, hq, hkv, mut(w[2]), stream()),
@@ -290,19 +300,23 @@ struct MoELayer : public Function<MoELayer> {
     Tensor daux = grads.size() > 1 && grads[1].defined() ? grads[1].to(x.device(), at::kFloat) : Tensor();
     const int64_t row = 2 * cap * D, wide = 2 * cap * F;
     const bool own = !lib.swiglu_bwd_in_product(cap, F, D);      // the SwiGLU backward is a kernel of its own
-    const Tensor first = Gradient::of(w[1]);
-    const at::ScalarType kind = first.defined() && first.scalar_type() == at::kBFloat16 ? at::kBFloat16 : at::kFloat;
-    Gradient grouter(w[0], at::kFloat), g1(w[1], kind), g3(w[2], kind), g2(w[3], kind);
+    const std::vector<Tensor> buffers = Gradient::of(w, 4);
+    const at::ScalarType kind = buffers[1].defined() && buffers[1].scalar_type() == at::kBFloat16 ? at::kBFloat16 : at::kFloat;
+    Gradient grouter(w[0], buffers[0], at::kFloat), g1(w[1], buffers[1], kind), g3(w[2], buffers[2], kind), g2(w[3], buffers[3], kind);
     // dx_perm takes the place of what is used up by then: dh, and gate and up where they are formed again.  dweights, dlogits.
-    const Scratch tmp(x, {std::max(row, (own + 2 * rebuild) * wide), 8 * T, 4 * T * E});
+    // Behind them dy_perm, dgu and h, which large calls hold no longer than the experts need them.
+    const int64_t used_bytes = std::max(row, (own + 2 * rebuild) * wide), few = used_bytes + row + 3 * wide <= Scratch::TOGETHER;
+    const Scratch tmp(x, {used_bytes, 8 * T, 4 * T * E, few * row, few * 2 * wide, few * wide});
     char* const used = tmp[0];
     char* const formed = used + own * wide;
     {
-      const Scratch inner(x, {row, 2 * wide, wide});              // dy_perm, dgu, h
+      std::optional<Scratch> large;
+      if (!few) large.emplace(x, std::initializer_list<int64_t>{row, 2 * wide, wide});
+      const auto inner = [&](size_t i) { return few ? tmp[3 + i] : (*large)[i]; };
       check(lib.moe_experts_bwd(ptr(dout), ptr(w[1]), ptr(w[2]), ptr(w[3]), ptr(weights), mut(tables), ptr(x_perm), ptr(y_perm),
-                                rebuild ? formed : mut(saved[7]).at, rebuild ? formed + wide : mut(saved[8]).at, rebuild, *g1, *g3, *g2,
-                                kind == at::kFloat ? 1 : 2, inner[0], inner[1], inner[2], own ? used : nullptr, used, tmp[1], T, D,
-                                F, E, cap, mut(w[4]), stream()), nullptr, 5 + own + rebuild);
+                                rebuild ? formed : mut(saved[7]).at, rebuild ? formed + wide : mut(saved[8]).at, rebuild, *g1, *g3,
+                                *g2, kind == at::kFloat ? 1 : 2, inner(0), inner(1), inner(2), own ? used : nullptr, used, tmp[1],
+                                T, D, F, E, cap, mut(w[4]), stream()), nullptr, 5 + own + rebuild);
     }
     Tensor dx = at::empty_like(x);
     check(lib.moe_router_bwd(ptr(x), ptr(w[0]), ptr(weights), ptr(idx), ptr(probs), mut(tables), ptr(daux), *grouter, used, tmp[1],
