@@ -1080,8 +1080,9 @@ __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dkv_kernel(const __g
 }
 
 // ================================================================= backward: dQ
-// TMEM: S [0,128), dP / dS [128,256), dQ [256,384), Q and dO as A operands [384,448) and [448,512).  Thread layout as above with query rows: group g handles key columns
-// [64 g, 64 g + 64).  The ring of three holds K tiles, the ring of two V tiles.  P stays in registers, so the next
+// TMEM: S [0,128), dP / dS [128,256), dQ [256,384), Q and dO as A operands [384,448) and [448,512).  Thread layout as above with
+// query rows: group g handles key columns [64 g, 64 g + 64).  The ring of three holds K tiles, the ring of two V tiles.  P stays in
+// registers, so the next
 // scores of a half are issued as soon as its warps have read the present ones (p_ready counts that).  MMA order:
 //   S0(j+1) | dQ1(j-1) dP1(j) | S1(j+1) | dQ0(j) dP0(j+1)
 __global__ void __launch_bounds__(ATTN_THREADS, 1) attn_bwd_dq_kernel(const __grid_constant__ AttnParams p) {
@@ -1385,9 +1386,9 @@ static int bwd_clusters_resident(int parts) {
 // A backward kernel over ``tiles`` tiles of at most ``steps`` steps each.  Where the clusters of several parts per tile make one
 // wave, two share the steps from seven on and four from eight on: below, the two barriers and the exchange cost what the steps
 // save (two parts against one: five steps 29.0, 25.0; six 29.5, 27.5); eight parts gain nothing more.  One wave is what the
-// device holds in clusters, 33 of four CTAs, not 148 / 4: 36 tiles of nine steps in four parts are 61 us, in two 35, in one 39.  Causal
-// tiles of many steps may make a second wave, which the shortest of them fill: 36 tiles of up to 36 steps in four parts 53,
-// in two 59.  us, whole backward pass, one -> several parts, causal: 2 x 512 tokens, 4/1 heads 45.8 -> 34.0; 1024, 8/2 73.3 ->
+// device holds in clusters, 33 of four CTAs, not 148 / 4: 36 tiles of nine steps in four parts are 61 us, in two 35, in one 39.
+// Causal tiles of many steps may make a second wave, which the shortest of them fill: 36 tiles of up to 36 steps in four parts
+// 53, in two 59.  us, whole backward pass, one -> several parts, causal: 2 x 512 tokens, 4/1 heads 45.8 -> 34.0; 1024, 8/2 73.3 ->
 // 41.2; 2048, 8/2 130 -> 68.7; 4 x 1024, 8/2 88.8 -> 70.6; 128, 8/2 (one part) 26.1.
 template <void (*kernel)(AttnParams)>
 static int launch_bwd(long long tiles, long long steps, const AttnParams& p, cudaStream_t stream) {

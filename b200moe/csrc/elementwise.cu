@@ -102,7 +102,8 @@ __device__ __forceinline__ void norm_producer(const __nv_bfloat16* const (&src)[
 #pragma unroll
     for (int i = 0; i < TENSORS; ++i)
       if (src[i])
-        bulk_load(ring + (static_cast<size_t>(s) * TENSORS + i) * slot, src[i] + static_cast<size_t>(block) * R * D, &bars.full[s], bytes);
+        bulk_load(ring + (static_cast<size_t>(s) * TENSORS + i) * slot, src[i] + static_cast<size_t>(block) * R * D, &bars.full[s],
+                  bytes);
   }
   // copies of a CTA whose other warps gave up land before it exits
   for (int i = max(0, count - ring_stages); i < count; ++i) mbar_wait(&bars.full[i % ring_stages], (i / ring_stages) & 1);
@@ -361,7 +362,8 @@ __global__ void __launch_bounds__(NORM_THREADS + 32, V == 2 ? 2 : 1)
         if (live && col < D) {
           a[c] = *reinterpret_cast<const bf16x8*>(RING ? in + col : dy + base + col);
           b[c] = *reinterpret_cast<const bf16x8*>(RING ? in + static_cast<size_t>(R) * D + col : x + base + col);
-          if (residual) res[c] = *reinterpret_cast<const bf16x8*>(RING ? in + static_cast<size_t>(2 * R) * D + col : residual + base + col);
+          if (residual)
+            res[c] = *reinterpret_cast<const bf16x8*>(RING ? in + static_cast<size_t>(2 * R) * D + col : residual + base + col);
         }
       }
       __syncwarp();
@@ -1305,15 +1307,15 @@ int b2_rmsnorm_fwd(const void* x, const void* delta, const float* w, void* sum_o
   const int at_once = norm_rows_at_once(D);
   if ((rows + at_once - 1) / at_once <= sm_count_ew() * NORM_FWD_CTAS) {
     auto kernel = D <= 2048 ? rmsnorm_fwd_row_kernel<1> : D <= 4096 ? rmsnorm_fwd_row_kernel<2> : rmsnorm_fwd_row_kernel<4>;
-    launch_next(kernel, min(rows, sm_count_ew() * 8), NORM_THREADS, 0, s, (const bf16*)x, (const bf16*)delta, w, (bf16*)sum_out, (bf16*)y,
-                                                                 rstd, rows, D, eps);
+    launch_next(kernel, min(rows, sm_count_ew() * 8), NORM_THREADS, 0, s, (const bf16*)x, (const bf16*)delta, w, (bf16*)sum_out,
+                (bf16*)y, rstd, rows, D, eps);
     return ok();
   }
   return launch_norm(D, 2, [&](auto W, auto V, int smem, int stages) {
     auto kernel = rmsnorm_fwd_kernel<decltype(W)::value, decltype(V)::value>;
     if (const int rc = norm_smem<decltype(W)::value, decltype(V)::value, 0>(kernel)) return rc;
-    launch_next(kernel, sm_count_ew() * NORM_FWD_CTAS, NORM_THREADS + 32, smem, s, (const bf16*)x, (const bf16*)delta, w, (bf16*)sum_out, (bf16*)y, rstd, status,
-                                                 rows, D, eps, stages);
+    launch_next(kernel, sm_count_ew() * NORM_FWD_CTAS, NORM_THREADS + 32, smem, s, (const bf16*)x, (const bf16*)delta, w,
+                (bf16*)sum_out, (bf16*)y, rstd, status, rows, D, eps, stages);
     return ok();
   });
 }
@@ -1340,8 +1342,8 @@ int b2_rmsnorm_bwd(const void* dy, const void* x, const float* w, const float* r
     }
     auto kernel = rmsnorm_bwd_kernel<w_, v_, 1>;
     if (const int rc = norm_smem<w_, v_, 1>(kernel)) return rc;
-    launch_next(kernel, parts, NORM_THREADS + 32, smem, s, (const bf16*)dy, (const bf16*)x, w, rstd, (const bf16*)residual, (bf16*)dx,
-                dw_partial, status, rows, D, stages);
+    launch_next(kernel, parts, NORM_THREADS + 32, smem, s, (const bf16*)dy, (const bf16*)x, w, rstd, (const bf16*)residual,
+                (bf16*)dx, dw_partial, status, rows, D, stages);
     return ok();
   });
   if (rc) return rc;
@@ -1423,7 +1425,8 @@ int b2_router_top2_bwd(const float* dweights, const float* probs, const long lon
 int b2_swiglu_bwd(const void* dh, const void* gate, const void* up, void* dgu, void* h, const int* live_rows, int rows,
                   int F, cudaStream_t s) {
   if (F % 8) return -10;
-  launch_next(swiglu_bwd_kernel, grid_for(static_cast<size_t>(rows) * F / 8, 256), 256, 0, s, (const bf16*)dh, (const bf16*)gate, (const bf16*)up, (bf16*)dgu, (bf16*)h, live_rows, rows, F);
+  launch_next(swiglu_bwd_kernel, grid_for(static_cast<size_t>(rows) * F / 8, 256), 256, 0, s, (const bf16*)dh, (const bf16*)gate,
+              (const bf16*)up, (bf16*)dgu, (bf16*)h, live_rows, rows, F);
   return ok();
 }
 
@@ -1451,7 +1454,8 @@ int b2_cross_entropy2(void* logits, const long long* targets, void* loss, int wi
                                                               grad_scale);
     return ok();
   }
-  launch_next(cross_entropy_kernel, min(T, sm_count_ew() * 4), CE_THREADS, 0, s, (bf16*)logits, targets, loss, wide, T, V, loss_scale);
+  launch_next(cross_entropy_kernel, min(T, sm_count_ew() * 4), CE_THREADS, 0, s, (bf16*)logits, targets, loss, wide, T, V,
+              loss_scale);
   return ok();
 }
 int b2_scale_bf16(void* x, const float* factor, long long n, cudaStream_t s) {
@@ -1549,7 +1553,8 @@ int b2_rope(void* x, const float* cos_t, const float* sin_t, int tokens, int S, 
 int b2_rope_copy(const void* q, const void* k, void* q_out, void* k_out, const float* cos_t, const float* sin_t,
                  int tokens, int S, int Hq, int Hkv, long long q_pitch, long long k_pitch, cudaStream_t s) {
   if (q_pitch % 8 || k_pitch % 8 || S < 1) return -10;
-  launch_next(rope_copy_kernel, grid_for(static_cast<size_t>(tokens) * (Hq + Hkv) * 16, 256), 256, 0, s, (const bf16*)q, (const bf16*)k, (bf16*)q_out, (bf16*)k_out, cos_t, sin_t, tokens, S, Hq, Hkv, q_pitch, k_pitch);
+  launch_next(rope_copy_kernel, grid_for(static_cast<size_t>(tokens) * (Hq + Hkv) * 16, 256), 256, 0, s, (const bf16*)q,
+              (const bf16*)k, (bf16*)q_out, (bf16*)k_out, cos_t, sin_t, tokens, S, Hq, Hkv, q_pitch, k_pitch);
   return ok();
 }
 

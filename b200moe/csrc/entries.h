@@ -60,8 +60,8 @@ int b2_attn_half_fwd(const void* x, const float* ln1, const void* wqkv, const fl
                      int Hq, int Hkv, float eps1, float eps2, int* status, cudaStream_t s);
 int b2_attn_half_bwd(const void* dsum, const void* dn2, const void* x, const float* ln1, const void* wqkv, const float* cos_t,
                      const float* sin_t, const void* wo, const float* ln2, const void* n1, const void* qkv, const void* a,
-                     const void* sum, const float* stats, float* gqkv, float* go, float* dln1, float* dln2, void* dx, void* dmid, void* da,
-                     void* dn1, void* dqkv, float* partial, float* row_stats, int B, int S, int Hq, int Hkv, int* status,
+                     const void* sum, const float* stats, float* gqkv, float* go, float* dln1, float* dln2, void* dx, void* dmid,
+                     void* da, void* dn1, void* dqkv, float* partial, float* row_stats, int B, int S, int Hq, int Hkv, int* status,
                      cudaStream_t s);
 int b2_moe_layer_fwd(const void* x, const void* router, const void* w1, const void* w3, const void* w2, const void* residual,
                      float* weights, long long* idx, float* probs, int* tables, void* x_perm, void* h, void* gate, void* up,
@@ -73,7 +73,7 @@ int b2_moe_experts_bwd(const void* dout, const void* w1, const void* w3, const v
                        const void* x_perm, const void* y_perm, void* gate, void* up, int rebuild, void* g1, void* g3, void* g2,
                        int expert_kind, void* dy_perm, void* dgu, void* h, void* dh, void* dx_perm, float* dweights, int T, int D,
                        int F, int E, int cap, int* status, cudaStream_t s);
-int b2_moe_router_bwd(const void* x, const void* router, const float* weights, const long long* idx, const float* probs, int* tables,
-                      const float* daux, float* grouter, const void* dx_perm, const float* dweights, float* dlogits, void* dx, int T,
-                      int D, int E, int cap, cudaStream_t s);
+int b2_moe_router_bwd(const void* x, const void* router, const float* weights, const long long* idx, const float* probs,
+                      int* tables, const float* daux, float* grouter, const void* dx_perm, const float* dweights, float* dlogits,
+                      void* dx, int T, int D, int E, int cap, cudaStream_t s);
 }

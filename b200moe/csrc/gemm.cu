@@ -602,7 +602,8 @@ __global__ void __launch_bounds__(gemm_threads<EPI>(), 1) gemm_tcgen05_kernel(co
           }
         }
 #pragma unroll 1
-        for (int c = half * (NT / 2); !F32 && (NT < 128 || (EPI != EPI_STORE_BF16 && (EPI != EPI_ACC_BF16 || add))) && c < (half + 1) * (NT / 2); c += 32) {
+        for (int c = half * (NT / 2);
+             !F32 && (NT < 128 || (EPI != EPI_STORE_BF16 && (EPI != EPI_ACC_BF16 || add))) && c < (half + 1) * (NT / 2); c += 32) {
           const long long col = col_base + c + q * 8;     // N is a multiple of 32 (checked on the host)
           if (col_base + c >= p.N) break;
           if (OLD && !EARLY) fetch_old(t, sub, c);

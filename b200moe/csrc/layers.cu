@@ -3,8 +3,8 @@
 // host: an operation takes some 25 us from Python (arguments, allocations, autograd) beside 2-3 us for the launch itself, so a
 // training step of two blocks of width 512 spent 4.7 ms on 1.5 ms of kernels.
 //
-// Every entry point returns 0, or the code of the first launch that was refused (b2_layers_refused: its entry point).  Buffers are the
-// caller's.
+// Every entry point returns 0, or the code of the first launch that was refused (b2_layers_refused: its entry point).  Buffers
+// are the caller's.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -65,8 +65,8 @@ int b2_attn_half_fwd(const void* x, const float* ln1, const void* wqkv, const fl
 // row_stats fp32 [B Hq, 2, S].  dn1 may be da, and dmid may be dx (see b2_rmsnorm_bwd).
 int b2_attn_half_bwd(const void* dsum, const void* dn2, const void* x, const float* ln1, const void* wqkv, const float* cos_t,
                      const float* sin_t, const void* wo, const float* ln2, const void* n1, const void* qkv, const void* a,
-                     const void* sum, const float* stats, float* gqkv, float* go, float* dln1, float* dln2, void* dx, void* dmid, void* da,
-                     void* dn1, void* dqkv, float* partial, float* row_stats, int B, int S, int Hq, int Hkv, int* status,
+                     const void* sum, const float* stats, float* gqkv, float* go, float* dln1, float* dln2, void* dx, void* dmid,
+                     void* da, void* dn1, void* dqkv, float* partial, float* row_stats, int B, int S, int Hq, int Hkv, int* status,
                      cudaStream_t s) {
   const int T = B * S, D = Hq * 128, N = (Hq + 2 * Hkv) * 128;
   const bf16* const q = static_cast<const bf16*>(qkv);
@@ -118,8 +118,8 @@ int b2_moe_layer_fwd(const void* x, const void* router, const void* w1, const vo
 // b200moe.ops.native.gemm_nn_swiglu_bwd, which has the figures).
 int b2_swiglu_bwd_in_product(long long M, int F, int K) { return K >= 2048 || M * F <= 1 << 21; }
 
-// One chunk of tokens through the LM head: logits = hidden W^T become their own gradient (and the loss is added to the double ``loss``),
-// dh = dlogits W, grad (fp32) += dlogits^T hidden.
+// One chunk of tokens through the LM head: logits = hidden W^T become their own gradient (and the loss is added to the double
+// ``loss``), dh = dlogits W, grad (fp32) += dlogits^T hidden.
 int b2_head_chunk(const void* hidden, const void* weight, const long long* targets, void* logits, double* loss, void* dh,
                   float* grad, int T, int V, int D, float loss_scale, float grad_scale, int* status, cudaStream_t s) {
   Sequence run;
@@ -174,11 +174,11 @@ int b2_moe_experts_bwd(const void* dout, const void* w1, const void* w3, const v
   return run.rc;
 }
 
-// Its router, behind the experts (whose scratch the caller may have given back): dx [T, D]; the gradient of the router's weights is
-// added to grouter (fp32).  Scratch: dlogits [T, E].
-int b2_moe_router_bwd(const void* x, const void* router, const float* weights, const long long* idx, const float* probs, int* tables,
-                      const float* daux, float* grouter, const void* dx_perm, const float* dweights, float* dlogits, void* dx, int T,
-                      int D, int E, int cap, cudaStream_t s) {
+// Its router, behind the experts (whose scratch the caller may have given back): dx [T, D]; the gradient of the router's weights
+// is added to grouter (fp32).  Scratch: dlogits [T, E].
+int b2_moe_router_bwd(const void* x, const void* router, const float* weights, const long long* idx, const float* probs,
+                      int* tables, const float* daux, float* grouter, const void* dx_perm, const float* dweights, float* dlogits,
+                      void* dx, int T, int D, int E, int cap, cudaStream_t s) {
   const Tables t(tables, 2 * T, cap, E);
   Sequence run;
   run("b2_moe_dx", [&] {

@@ -409,8 +409,8 @@ extern "C" {
 int b2_moe_plan(const long long* idx, int slots, int E, int* slot_row, int* row_slot, int* offs, int* tile_expert,
                 int* meta, int* counts, int capacity_rows, cudaStream_t s) {
   if (E < 1) return -10;
-  // 49 experts is what an earlier form of the kernel held in shared memory; this one needs 144 bytes an expert.  The limit stays: no
-  // caller has more (the router takes 64 at most, the routed layer 16 on one rank), and nothing beyond has been tested.
+  // 49 experts are what an earlier form of the kernel held in shared memory; this one needs 144 bytes an expert.  The limit
+  // stays what callers and tests know.
   if (E > 49) return -11;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
@@ -437,8 +437,8 @@ int b2_moe_plan(const long long* idx, int slots, int E, int* slot_row, int* row_
 int b2_moe_gather(const void* x, const int* row_slot, const int* meta, const float* scale, const void* y_perm,
                   float* dweights, void* x_perm, int D, int capacity_rows, int slots, cudaStream_t s) {
   if (D % 8) return -10;
-  launch_next(moe_gather_kernel, sm_count_moe() * 8, 256, 0, s, (const bf16*)x, row_slot, meta, scale, (const bf16*)y_perm, dweights,
-                                            (bf16*)x_perm, D, capacity_rows, slots);
+  launch_next(moe_gather_kernel, sm_count_moe() * 8, 256, 0, s, (const bf16*)x, row_slot, meta, scale, (const bf16*)y_perm,
+              dweights, (bf16*)x_perm, D, capacity_rows, slots);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -446,7 +446,7 @@ int b2_moe_combine(const void* y_perm, const int* slot_row, const float* weights
                    int T, int D, int rows, cudaStream_t s) {
   if (D % 8) return -10;
   launch_next(moe_combine_kernel, min((T + 7) / 8, sm_count_moe() * 8), 256, 0, s, (const bf16*)y_perm, slot_row, weights,
-                                                               (const bf16*)residual, (bf16*)out, T, D, rows);
+              (const bf16*)residual, (bf16*)out, T, D, rows);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -471,8 +471,8 @@ int b2_moe_dx(const void* dy, const int* slot_row, const float* dweights, const 
     set = true;
   }
   auto kernel = N <= 8 ? moe_dx_kernel<8> : moe_dx_kernel<16>;
-  launch_next(kernel, min((T + 31) / 32, sm_count_moe() * 2), 256, smem, s, (const bf16*)dy, slot_row, dweights, probs, idx, weights,
-                                                                   daux, counts, (const bf16*)w, dlogits, (bf16*)dx, T, N, D, rows);
+  launch_next(kernel, min((T + 31) / 32, sm_count_moe() * 2), 256, smem, s, (const bf16*)dy, slot_row, dweights, probs, idx,
+              weights, daux, counts, (const bf16*)w, dlogits, (bf16*)dx, T, N, D, rows);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

@@ -268,7 +268,8 @@ struct AttnHalf : public Function<AttnHalf> {
 
 struct MoELayer : public Function<MoELayer> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& router, const Tensor& w1, const Tensor& w3,
-                               const Tensor& w2, const Optional& residual, const Tensor& status, int64_t cap, bool keeps, bool balance) {
+                               const Tensor& w2, const Optional& residual, const Tensor& status, int64_t cap, bool keeps,
+                               bool balance) {
     ctx->set_materialize_grads(false);
     const int64_t D = x.size(-1), T = x.numel() / D, E = w1.size(0), F = w1.size(1);
     Tensor weights = fp32({T, 2}, x), probs = fp32({T, E}, x), idx = at::empty({T, 2}, x.options().dtype(at::kLong));
@@ -305,7 +306,8 @@ struct MoELayer : public Function<MoELayer> {
     Gradient grouter(w[0], buffers[0], at::kFloat), g1(w[1], buffers[1], kind), g3(w[2], buffers[2], kind), g2(w[3], buffers[3], kind);
     // dx_perm takes the place of what is used up by then: dh, and gate and up where they are formed again.  dweights, dlogits.
     // Behind them dy_perm, dgu and h, which large calls hold no longer than the experts need them.
-    const int64_t used_bytes = std::max(row, (own + 2 * rebuild) * wide), few = used_bytes + row + 3 * wide <= Scratch::TOGETHER;
+    const int64_t used_bytes = std::max(row, (own + 2 * rebuild) * wide);
+    const int64_t few = used_bytes + row + 3 * wide <= Scratch::TOGETHER;
     const Scratch tmp(x, {used_bytes, 8 * T, 4 * T * E, few * row, few * 2 * wide, few * wide});
     char* const used = tmp[0];
     char* const formed = used + own * wide;
@@ -338,7 +340,8 @@ struct Head : public Function<Head> {
       Tensor logits = bf16({n, V}, hidden);
       check(lib.head_chunk(static_cast<const char*>(ptr(hidden).at) + 2 * lo * D, ptr(weight),
                            static_cast<const long long*>(ptr(targets)) + lo, mut(logits), mut(loss),
-                           static_cast<char*>(mut(dh).at) + 2 * lo * D, mut(grad), n, V, D, 1.0 / T, scale / T, mut(status), stream()),
+                           static_cast<char*>(mut(dh).at) + 2 * lo * D, mut(grad), n, V, D, 1.0 / T, scale / T, mut(status),
+                           stream()),
             nullptr, 4);
     }
     ctx->save_for_backward({dh});
